@@ -121,4 +121,36 @@ __device__ __forceinline__ double div_rn_rcp(double a, double b, double y) {
   return ieee_div(a, b);
 }
 
+// RN(a/b) without a certificate, for |a| < 2|b|: returns true with the
+// quotient in *q, or false (*q unspecified) when the caller has to divide
+// with the operator.  Markstein's method with two residual steps:
+//   y0 ~ 1/b with |1 - b*y0| < 2^-19; two Newton-Raphson steps give y within
+//   (1/2 + 2^-23) ulp of 1/b;
+//   q0 = a*y;  q1 = q0 + (a - b*q0)*y  is within (1/2 + 2^-50) ulp of a/b;
+//   r = a - b*q1 is exact, and q = RN(q1 + r*y).
+// Scaled to 1 <= b < 2, the last sum misses a/b by |a/b - q1|*|b*y - 1| <=
+// (1/2 + 2^-50)(1/2 + 2^-23) b 2^-53 ulp(q), while a/b keeps at least 2^-53/b
+// ulp(q) from every midpoint m of two doubles (a - b*m is a nonzero multiple
+// of 2^-53 ulp(q)): q = RN(a/b) whenever b < 2(1 - 2^-22).  Divisors whose
+// leading 20 mantissa bits are all ones are refused; the estimate's error is
+// at most 2^-19.9 over all leading 20-bit mantissas (the bits it depends on),
+// measured on B200.  |a| >= 2^-700 and 2^-200 <= |b| < 2^201 keep every
+// intermediate normal and the residual exact (see above); a zero dividend is
+// refused.
+__device__ __forceinline__ bool quot_rn(double a, double b, double *q) {
+  const unsigned ha = (unsigned)__double2hiint(a) & 0x7fffffffu, hb = (unsigned)__double2hiint(b) & 0x7fffffffu;
+  constexpr unsigned ALO = (1023u - 700u) << 20, BLO = (1023u - 200u) << 20, BHI = (1023u + 201u) << 20;
+  double y = rcp_approx(b);
+  double e = fma(-b, y, 1.0);
+  y = fma(y, e, y);
+  e = fma(-b, y, 1.0);
+  y = fma(y, e, y);
+  double v = a * y;
+  double r = fma(-b, v, a);
+  v = fma(r, y, v);
+  r = fma(-b, v, a);
+  *q = fma(r, y, v);
+  return ha >= ALO && (hb - BLO) < (BHI - BLO) && (hb & 0xfffffu) != 0xfffffu;
+}
+
 }  // namespace a3g

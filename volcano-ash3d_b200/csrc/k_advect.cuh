@@ -1225,28 +1225,143 @@ static void launch_col(a3g_ctx *ctx) {
 }
 
 // ---------------------------------------------------------------------------
-// Column march fed by TMA chunks (y and z sweeps).  The march of k_advect_col
-// -- one warp per 32 lines of 32 consecutive i at one (other index, grain),
-// each interface formed once, the same step() arithmetic and so the same bits
-// -- but the interior steps read the concentration and the wind of cell c+2
-// from shared memory: chunks of ACH cells of both arrive by two tensor loads
-// into one of two buffers per warp, the next chunk in flight while the lanes
-// march through the current one, and the geometry of the chunk's cells
-// (sigma, dt/kappa: the same for the warp's lines) is staged beside them.
-// The prologue and the few checked steps at the line ends keep the global
-// loads of k_advect_col.  Warps are ordered grain-fastest, so the grains of a
-// tile run side by side and share its wind rows through L2.  Taken when the
-// geometry is constant along i and the fall speed is one value per grain.
+// The marching step that the TMA-fed sweeps share.
+// ---------------------------------------------------------------------------
+// max(0, x) and min(0, x) by the sign bit: two logic operations per half
+// instead of a compare and two selects.  A NaN stays a NaN in one of them.
+__device__ __forceinline__ double pos_part(double x) {
+  const int h = __double2hiint(x), m = ~(h >> 31);
+  return __hiloint2double(h & m, __double2loint(x) & m);
+}
+__device__ __forceinline__ double neg_part(double x) {
+  const int h = __double2hiint(x), m = h >> 31;
+  return __hiloint2double(h & m, __double2loint(x) & m);
+}
+
+// Second-order flux of one interface, cf*ldq (0 where the reference cycles),
+// the same value as fss_select's.  Superbee's factor is 0 for ratios dqu/dq
+// <= 0, 2 from 2 up, 1 on [1/2, 1], and 2*theta or theta in between, and
+// rounding to nearest cannot move a quotient across those bounds, so the
+// class comes from comparisons of dqu with dq and 2*dq, the quotient is
+// needed in two classes only, and it is divided by the operator only where
+// one of those lanes holds operands out of quot_rn's range.  `up` may be
+// either for usig = 0, where cf = 0.
+static __device__ __noinline__ double ieee_theta(double dqu, double dq, bool twice) {
+  const double th = dqu / dq;
+  return twice ? th + th : th;
+}
+
+template <int LIM>
+__device__ __forceinline__ double fss_step(double dqm, double dq, double dqp, bool up, double cf, double eps,
+                                           bool nocycle) {
+  if (LIM == A3G_LIM_NONE) return 0.0;
+  if (LIM != A3G_LIM_SUPERBEE) return fss_select<LIM>(dqm, dq, dqp, up, cf, true, eps, nocycle);
+  const double dqu = up ? dqm : dqp;
+  const double a = fabs(dqu), b = fabs(dq);
+  const bool lt = a + a < b, gt = a > b;
+  bool ge2 = a >= b + b, none = b <= eps;
+  if (nocycle) {  // the clamp of :201 without the cycle of :183
+    ge2 = ge2 || b < eps;
+    none = false;
+  }
+  none = none || (__double2hiint(dqu) ^ __double2hiint(dq)) < 0;
+  const bool need = !none && !ge2 && (lt || gt);
+  double th;
+  const bool ok = quot_rn(dqu, dq, &th);
+  int hi = __double2hiint(th) + (lt ? 1 << 20 : 0), lo = __double2loint(th);  // 2*theta of a normal theta
+  if (need && !ok) {
+    th = ieee_theta(dqu, dq, lt);
+    hi = __double2hiint(th);
+    lo = __double2loint(th);
+  }
+  const int flat = none ? 0 : (ge2 ? 0x40000000 : 0x3ff00000);  // 0, 2 or 1
+  const double phi = __hiloint2double(need ? hi : flat, need ? lo : 0);
+  return cf * (dq * phi);
+}
+
+// The values a march carries from cell c to cell c+1.
+struct March {
+  double q0, q1, d0, d1;   // q(c), q(c+1), q(c)-q(c-1), q(c+1)-q(c)
+  double us, vB;           // usig(c+1), vel(c+1)
+  double upA, upB, unB;    // max(0,usig(c)), max(0,usig(c+1)), min(0,usig(c+1))
+  double fss0, fsr0, dtv0; // fss(c), fs_r(c), dt/kappa(c)
+};
+
+// One interior step (no range checks): interface c+1 from q2 = q(c+2), d2 =
+// q2 - q(c+1), vn = vel(c+2), hs = sigma(c+2)/2 and dtv1 = dt/kappa(c+1).
+// Returns the sum whose product with dt/kappa(c) is taken off q(c) (:264-281).
+// usig = 0.5*(v+v')*sigma is (v+v')*(sigma/2): halving is exact.  QUIET: the
+// caller knows that |dq| <= EPS_THRESH at this interface.
+template <int LIM, bool QUIET>
+__device__ __forceinline__ double march_step(March &m, double q2, double d2, double vn, double hs, double dtv1,
+                                             double eps, bool nocycle) {
+  const double usC = (m.vB + vn) * hs;
+  const double upC = pos_part(usC), unC = neg_part(usC);
+  double fss1 = 0.0;
+  if (!QUIET && LIM != A3G_LIM_NONE) {
+    const double aus = fabs(m.us);
+    const double cf = 0.5 * aus * (1.0 - dtv1 * aus);
+    fss1 = fss_step<LIM>(m.d0, m.d1, d2, __double2hiint(m.us) >= 0, cf, eps, nocycle);
+  }
+  double fsr1 = m.upB * m.d1;
+  double fsl1 = m.unB * m.d1;
+  fsr1 = fsr1 + m.q1 * (unC - m.unB);
+  fsl1 = fsl1 + m.q0 * (m.upB - m.upA);
+  const double sum = fsl1 + m.fsr0 + fss1 - m.fss0;
+  m.us = usC;
+  m.vB = vn;
+  m.upA = m.upB;
+  m.upB = upC;
+  m.unB = unC;
+  m.fss0 = fss1;
+  m.fsr0 = fsr1;
+  m.q0 = m.q1;
+  m.q1 = q2;
+  m.d0 = m.d1;
+  m.d1 = d2;
+  return sum;
+}
+
+// ---------------------------------------------------------------------------
+// Column march fed by TMA chunks (y and z sweeps).  One warp per 32 lines of
+// 32 consecutive i at one (other index, grain), lanes along i, marching the
+// line with each interface formed once and the values of block_body (the same
+// bits).  The concentration and the wind of cell c+2 come from shared memory:
+// chunks of ACH cells of both arrive by two tensor loads into one of two
+// buffers per warp, the next chunk in flight while the lanes march through
+// the current one, and the geometry of the chunk's cells (sigma/2, dt/kappa:
+// the same for the warp's lines) is staged beside them.  Every cell of the
+// line takes the same unchecked step: concentrations beyond the line arrive
+// as the zeros of Set_BC(1), the wind beyond its last cell is written into
+// the last chunk, and the flux areas beyond the box are zero because their
+// sigma is staged as zero.  The interface the line starts from and the two
+// outflow cells are formed outside the loop.  Warps are ordered
+// grain-fastest, so the grains of a tile run side by side and share its wind
+// rows through L2.  Taken when the geometry is constant along i and the fall
+// speed is one value per grain.
+//
+// Bound by instruction issue (67 % of cycles on the C2 slab) and the FP64 pipe
+// (45 %).  march_step() forms an interface in about 100 instructions where
+// block_body's expressions and the checked steps at the line ends took 190,
+// and a chunk whose differences are all within EPS_THRESH on every lane -- the
+// air around a cloud -- takes steps without the limiter: 720x360x60, 10
+// grains, y 1.12 -> 0.58 ms and z 1.27 -> 0.66 ms a sweep.
+// Lines are cut into segments of `seg` cells where whole lines would leave
+// the chip short of warps (launch_colt); a segment repeats one interface.
 // ---------------------------------------------------------------------------
 constexpr int ACT_WARPS = 2;
+constexpr int ACT_MINB = 8;  // 128 registers, none spilled: 9 and 10 blocks spill and run 5 % slower
+constexpr int ACT_U = 4;     // steps unrolled: 4 measured faster than 8 (instruction cache) and than 2
 // doubles per warp: two buffers of (q, v) chunks and two of staged geometry
 constexpr int ACT_WARP_D = 2 * 2 * ACH * 32 + 2 * 2 * ACH;
 static_assert((ACT_WARP_D * 8) % 128 == 0, "warp regions stay 128-byte aligned");
+struct TrueT { static constexpr bool value = true; };
+struct FalseT { static constexpr bool value = false; };
 
 template <int DIR, int LIM>
-__global__ void __launch_bounds__(32 * ACT_WARPS) k_advect_colt(
+__global__ void __launch_bounds__(32 * ACT_WARPS, ACT_MINB) k_advect_colt(
     const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tv, Layout L, Box box,
-    int nocycle, double eps, const double *__restrict__ cin, double *__restrict__ cout,
+    int nocycle, double eps, int nseg, int seg, const double *__restrict__ cin, double *__restrict__ cout,
     const double *__restrict__ vel, const double *__restrict__ vghost, Geo4 vf, Geo3 sig, Geo3 dtvt,
     const int32_t *__restrict__ aloft, DevScalars *sc, double *__restrict__ out1, double *__restrict__ out2) {
   static_assert(DIR == 1 || DIR == 2, "lanes along i: y and z sweeps only");
@@ -1255,178 +1370,195 @@ __global__ void __launch_bounds__(32 * ACT_WARPS) k_advect_colt(
   uint64_t *bar = reinterpret_cast<uint64_t *>(act_smem) + 2 * wid;
   double *wsm = reinterpret_cast<double *>(act_smem + 128) + (long)wid * ACT_WARP_D;
   // buffer b: q chunk at wsm + b*2*ACH*32, v chunk after it; geometry of
-  // buffer b at wsm + 4*ACH*32 + b*2*ACH (sigma(c+2), then dt/kappa(c+1))
+  // buffer b at wsm + 4*ACH*32 + b*2*ACH: pairs (sigma(c+2)/2, dt/kappa(c+1))
   const int nother = (DIR == 1) ? L.nz : L.ny;
   const int nti = (L.nx + 31) >> 5;
   const long t = (long)blockIdx.x * ACT_WARPS + wid;
-  if (t >= (long)nti * nother * L.ns) return;  // whole warps only; no block barrier below
+  if (t >= (long)nti * nother * L.ns * nseg) return;  // whole warps only; no block barrier below
   const int g = (int)(t % L.ns);
-  const long rr = t / L.ns;
+  long rr = t / L.ns;
   const int it = (int)(rr % nti);
-  const int o = (int)(rr / nti) + 1;  // k (y sweep) or j (z sweep)
+  rr /= nti;
+  const int o = (int)(rr % nother) + 1;  // k (y sweep) or j (z sweep)
+  const int s0 = (int)(rr / nother) * seg + 1;
   const int a = (it << 5) + lane + 1;  // i
   const bool valid = a <= L.nx;
   const int n = (DIR == 1) ? L.ny : L.nz;
+  const int s1 = min(n, s0 + seg - 1);
   const int rmin = (DIR == 1) ? box.jmin : box.kmin;
   const int rmax = (DIR == 1) ? box.jmax : box.kmax;
-  const int ncells = rmax - rmin + 1;
   const int st = (DIR == 1) ? (int)L.P : (int)L.PY;
   const int ac = valid ? a : 1;
-  const long base = (DIR == 1) ? L.cell(ac, 1, o) : L.cell(ac, o, 1);
   const bool lane_active = (DIR == 1) ? (a >= box.imin && a <= box.imax && o >= box.kmin && o <= box.kmax)
                                       : (a >= box.imin && a <= box.imax && o >= box.jmin && o <= box.jmax);
   const bool al = valid && lane_active && aloft[g] != 0;
-  double *po = cout + (long)g * L.PG + base;
-  if (!__any_sync(0xffffffffu, al)) {  // the reference leaves zeros
-    if (valid)
-      for (int c = 1; c <= n; c++) po[(c - 1) * st] = 0.0;
-    return;
+  double *po = cout + (long)g * L.PG + ((DIR == 1) ? L.cell(ac, 1, o) : L.cell(ac, o, 1));
+  const int c0 = max(s0, rmin), c1 = min(s1, rmax);  // the cells marched
+  // the reference leaves zeros outside the box and for grains not aloft
+  if (valid) {
+    const int z0 = (al && c0 <= c1) ? c0 : s1 + 1;
+    for (int c = s0; c < z0; c++) po[(c - 1) * st] = 0.0;
+    for (int c = max(c1 + 1, z0); c <= s1; c++) po[(c - 1) * st] = 0.0;
   }
-  if (valid && !al)
-    for (int c = 1; c <= n; c++) po[(c - 1) * st] = 0.0;
+  if (c0 > c1 || !__any_sync(0xffffffffu, al)) return;
+  const bool out_hi = rmax == n;
+  // update_cc(ncells+1) for z (:309-311): cell n+1 of a box on the ground
+  const int ctop = (DIR == 2) ? rmax - rmin + 2 : rmax + 1;
+  if (DIR == 2 && out_hi && ctop < rmin - 1 && lane == 0) raise_error(sc, A3G_ERR_UNSUPPORTED, 311);
+  const int nchunk = (c1 - c0) / ACH + 1;
+  // chunk k holds cells C0(k) .. C0(k)+ACH-1, C0(k) = c0+2+k*ACH: the cell
+  // c+2 of the steps c = c0+k*ACH ..
+  auto issue = [&](int k) {
+    double *qb = wsm + (k & 1) * 2 * ACH * 32;
+    const int C0 = c0 + 2 + k * ACH;
+    if (lane == 0) {
+      uint64_t *b = &bar[k & 1];
+      mbar_arrive_expect_tx(b, 2u * ACH * 32u * 8u);
+      if (DIR == 1) {
+        tma_load_4d(qb, &tq, b, it << 5, C0 - 1, o - 1, g);
+        tma_load_4d(qb + ACH * 32, &tv, b, it << 5, C0 - 1, o - 1, 0);
+      } else {
+        tma_load_4d(qb, &tq, b, it << 5, o - 1, C0 - 1, g);
+        tma_load_4d(qb + ACH * 32, &tv, b, it << 5, o - 1, C0 - 1, 0);
+      }
+    }
+    const LineGeo gsig = line_of<DIR>(sig, 1, o), gdtv = line_of<DIR>(dtvt, 1, o);  // constant along i
+    double2 *gb = reinterpret_cast<double2 *>(wsm + 4 * ACH * 32 + (k & 1) * 2 * ACH);
+    const int I = C0 + lane;
+    if (lane < ACH && I <= n + 2) gb[lane] = make_double2(I <= rmax + 1 ? 0.5 * gsig.at(I) : 0.0, gdtv.at(I - 1));
+  };
   if (lane == 0) {
     mbar_init(&bar[0], 1);
     mbar_init(&bar[1], 1);
     mbar_init_fence();
   }
   __syncwarp();
-  const double *pq = cin + (long)g * L.PG + base;
-  const double *pv = vel + base;
-  const double *pvg = vghost + base;
-  const LineGeo gsig = line_of<DIR>(sig, ac, o);   // constant along i: the same line for every lane
-  const LineGeo gdtv = line_of<DIR>(dtvt, ac, o);
+  issue(0);
   const double vf0 = (DIR == 2) ? vf.p[(long)g * vf.sg] : 0.0;  // one fall speed per grain
-  const bool out_lo = rmin == 1;
-  const bool out_hi = rmax == n;
-  const int ctop = (DIR == 2) ? ncells + 1 : rmax + 1;  // update_cc(ncells+1) for z (:309-311)
-  if (DIR == 2 && out_hi && ctop < rmin - 1 && lane == 0) raise_error(sc, A3G_ERR_UNSUPPORTED, 311);
-  const long na = L.nx;
-  const long oo = (long)g * na * nother + (long)(o - 1) * na + (ac - 1);
-  auto fs_ok = [&](int I) { return I >= rmin - 1 && I <= rmax + 1; };
-  auto fss_ok = [&](int I) { return I >= rmin && I <= rmax + 1; };
-  auto qload = [&](int c) -> double {
-    return (c >= rmin - 2 && c <= rmax + 2 && c >= 1 && c <= n) ? pq[(c - 1) * st] : 0.0;
-  };
-  auto vload = [&](int c) -> double {
-    const int cl = c < 1 ? 1 : (c > n ? n : c);
-    double v = ((DIR == 2 && (c < 1 || c > n)) ? pvg : pv)[(cl - 1) * st];
-    if (DIR == 2) v = v + vf0;
-    return v;
-  };
-  const int cs = out_lo ? 0 : 1;
-  const int ce = out_hi ? n + 1 : n;
-  // ---- interface cs and the window at cs (k_advect_col's prologue) ----------
-  double q0 = qload(cs), q1 = qload(cs + 1);
-  double d0 = q0 - qload(cs - 1), d1 = q1 - q0;
-  double usA, usB, vB, dtv0 = gdtv.at(cs), fss0, fsr0;
+  const long oo = (long)g * L.nx * nother + (long)(o - 1) * L.nx + (ac - 1);
+  // ---- interface c0 and the window at c0; vedge: the wind beyond the line ----
+  March m;
+  double vedge;
   {
-    const double vm2 = vload(cs - 2), vm1 = vload(cs - 1), v0 = vload(cs);
-    vB = vload(cs + 1);
-    const double usm1 = fs_ok(cs - 1) ? 0.5 * (vm2 + vm1) * gsig.at(cs - 1) : 0.0;
-    usA = fs_ok(cs) ? 0.5 * (vm1 + v0) * gsig.at(cs) : 0.0;
-    usB = fs_ok(cs + 1) ? 0.5 * (v0 + vB) * gsig.at(cs + 1) : 0.0;
-    const double qm1 = qload(cs - 1);
-    const double dm = qm1 - qload(cs - 2);
-    const Iface f = make_iface(usm1, usA, usB, dtv0, fss_ok(cs), fs_ok(cs));
-    fss0 = fss_select<LIM>(dm, d0, d1, f.up, f.cf, f.fss_ok, eps, nocycle);
-    fsr0 = f.fs_ok ? (f.usp * d0) + q0 * f.divm : 0.0;
+    const long base = (DIR == 1) ? L.cell(ac, 1, o) : L.cell(ac, o, 1);
+    const double *pq = cin + (long)g * L.PG + base;
+    const double *pv = vel + base, *pvg = vghost + base;
+    const LineGeo gsig = line_of<DIR>(sig, 1, o), gdtv = line_of<DIR>(dtvt, 1, o);
+    auto qload = [&](int c) -> double {
+      return (c >= rmin - 2 && c <= rmax + 2 && c >= 1 && c <= n) ? pq[(c - 1) * st] : 0.0;
+    };
+    auto vload = [&](int c) -> double {  // edge winds; the z ghost levels read the plain vertical wind
+      const int cl = c < 1 ? 1 : (c > n ? n : c);
+      const double v = ((DIR == 2 && (c < 1 || c > n)) ? pvg : pv)[(cl - 1) * st];
+      return (DIR == 2) ? v + vf0 : v;
+    };
+    vedge = ((DIR == 2) ? pvg : pv)[(n - 1) * st];
+    m.q0 = qload(c0);
+    m.q1 = qload(c0 + 1);
+    const double qm1 = qload(c0 - 1), qm2 = qload(c0 - 2);
+    m.d0 = m.q0 - qm1;
+    m.d1 = m.q1 - m.q0;
+    m.dtv0 = gdtv.at(c0);
+    const double vm2 = vload(c0 - 2), vm1 = vload(c0 - 1), v0 = vload(c0);
+    m.vB = vload(c0 + 1);
+    const double usm1 = 0.5 * (vm2 + vm1) * gsig.at(c0 - 1);
+    const double usA = 0.5 * (vm1 + v0) * gsig.at(c0);
+    m.us = 0.5 * (v0 + m.vB) * gsig.at(c0 + 1);
+    const double dm = qm1 - qm2;
+    const Iface f = make_iface(usm1, usA, m.us, m.dtv0, true, true);
+    m.fss0 = fss_select<LIM>(dm, m.d0, m.d1, f.up, f.cf, true, eps, nocycle);
+    m.fsr0 = f.usp * m.d0;
+    m.fsr0 = m.fsr0 + m.q0 * f.divm;
+    // cell rmin-1: the low outflow of a box at the edge (or the z quirk's cell)
+    if (c0 == rmin && (rmin == 1 || (DIR == 2 && out_hi && ctop == rmin - 1))) {
+      double fsl = f.usm * m.d0;
+      fsl = fsl + qm1 * f.divp;
+      double fsr = pos_part(usm1) * dm;
+      fsr = fsr + qm1 * (neg_part(usA) - neg_part(usm1));
+      const double upd = cell_update(gdtv.at(c0 - 1), fsl, fsr, m.fss0, 0.0);
+      if (al) (rmin == 1 ? out1 : out2)[oo] += upd;
+    }
+    m.upA = pos_part(usA);
+    m.upB = pos_part(m.us);
+    m.unB = neg_part(m.us);
   }
-  // ---- one step: interface c+1 and the update of cell c (k_advect_col's) ----
-  auto step = [&](int c, auto checked, double q2, double vn, double s2, double dtv1) {
-    constexpr bool CK = decltype(checked)::value;
-    const int I = c + 1;
-    const bool fsok2 = !CK || fs_ok(c + 2);
-    const double usC = fsok2 ? 0.5 * (vB + vn) * s2 : 0.0;
-    vB = vn;
-    const Iface f = make_iface(usA, usB, usC, dtv1, !CK || fss_ok(I), !CK || fs_ok(I));
-    usA = usB;
-    usB = usC;
-    const double d2 = q2 - q1;
-    const double fss1 = fss_select<LIM>(d0, d1, d2, f.up, f.cf, f.fss_ok, eps, nocycle);
-    double fsr1 = 0.0, fsl1 = 0.0;
-    if (f.fs_ok) {
-      fsr1 = f.usp * d1;
-      fsl1 = f.usm * d1;
-      fsr1 = fsr1 + q1 * f.divm;
-      fsl1 = fsl1 + q0 * f.divp;
+  const bool nocyc = nocycle != 0;
+  const int eps_hi = nocyc ? 0 : __double2hiint(eps);  // |d| < eps for certain, by its high word alone
+  po += (long)(c0 - 1) * st;                           // cell c's place from here on
+  // the step c from the values of cell c+2 at slot e of the chunk
+  auto step = [&](auto quiet, const double *qv, const double2 *gb, int e) {
+    const double2 sd = gb[e];
+    const double q0 = m.q0, q2 = qv[e * 32];
+    const double vn = (DIR == 2) ? qv[(ACH + e) * 32] + vf0 : qv[(ACH + e) * 32];
+    const double sum = march_step<LIM, decltype(quiet)::value>(m, q2, q2 - m.q1, vn, sd.x, sd.y, eps, nocyc);
+    const double upd = m.dtv0 * sum;
+    if (al) *po = q0 - upd;
+    po += st;
+    m.dtv0 = sd.y;
+    return upd;
+  };
+  uint32_t ph = 0u;
+  for (int k = 0, c = c0; k < nchunk; k++) {
+    const int bi = k & 1;
+    if (k + 1 < nchunk) issue(k + 1);
+    if (!mbar_wait(&bar[bi], (ph >> bi) & 1u)) {
+      if (lane == 0) raise_error(sc, A3G_ERR_TIMEOUT, 3);
+      return;
     }
-    const double upd = cell_update(dtv0, fsl1, fsr0, fss1, fss0);
-    if (al) {
-      if (!CK || (c >= 1 && c <= n)) {
-        const bool inbox = !CK || (c >= rmin && c <= rmax);
-        po[(c - 1) * st] = inbox ? q0 + upd : 0.0;
+    ph ^= 1u << bi;
+    double *qv = wsm + bi * 2 * ACH * 32 + lane;
+    // cells of the chunk's steps; the wind of cell n+1 (only the last chunk holds it)
+    const int cnt = min(ACH, c1 - c + 1);
+    if (c + 2 <= n + 1 && n + 1 <= c + 1 + cnt) qv[(ACH + n - 1 - c) * 32] = vedge;
+    __syncwarp();
+    const double2 *gb = reinterpret_cast<const double2 *>(wsm + 4 * ACH * 32 + bi * 2 * ACH);
+    int e = 0;
+    // a chunk that holds the z sweep's ctop (a box off the ground) runs the loop
+    if (!(DIR == 2 && out_hi && ctop <= rmax)) {
+      // the differences the chunk's interfaces limit: d1 and the first cnt-1 new ones
+      int top = __double2hiint(m.d1) & 0x7fffffff;
+      double prev = m.q1;
+#pragma unroll
+      for (int u = 0; u < ACH - 1; u++) {
+        const double x = qv[u * 32];
+        top = max(top, __double2hiint(x - prev) & 0x7fffffff);
+        prev = x;
       }
-      if (CK && out_lo && c == 0) out1[oo] += upd;
-      if (out_hi && c == ctop) out2[oo] += upd;
-    }
-    fss0 = fss1;
-    fsr0 = fsr1;
-    q0 = q1;
-    q1 = q2;
-    d0 = d1;
-    d1 = d2;
-    dtv0 = dtv1;
-  };
-  auto checked_step = [&](int c) {
-    step(c, CkT{}, qload(c + 2), vload(c + 2), fs_ok(c + 2) ? gsig.at(c + 2) : 0.0, gdtv.at(c + 1));
-  };
-  // steps without range checks: c >= rmin, c+2 <= min(n, rmax+1)
-  int fa = max(cs, rmin), fb = min(n - 2, rmax - 1);
-  if (fb < fa) { fa = ce + 1; fb = ce; }
-  int c = cs;
-  for (; c < fa; c++) checked_step(c);
-  if (fa <= fb) {
-    // chunk m holds cells C0(m) .. C0(m)+ACH-1, C0(m) = fa+2+m*ACH: the cell
-    // c+2 of the steps c = fa+m*ACH .. (clipped to fb)
-    const int nchunk = (fb - fa) / ACH + 1;
-    constexpr uint32_t bytes = 2u * ACH * 32u * 8u;
-    auto issue = [&](int m) {
-      const int bi = m & 1;
-      double *qb = wsm + bi * 2 * ACH * 32;
-      const int C0 = fa + 2 + m * ACH;
-      if (lane == 0) {
-        mbar_arrive_expect_tx(&bar[bi], bytes);
-        if (DIR == 1) {
-          tma_load_4d(qb, &tq, &bar[bi], it << 5, C0 - 1, o - 1, g);
-          tma_load_4d(qb + ACH * 32, &tv, &bar[bi], it << 5, C0 - 1, o - 1, 0);
-        } else {
-          tma_load_4d(qb, &tq, &bar[bi], it << 5, o - 1, C0 - 1, g);
-          tma_load_4d(qb + ACH * 32, &tv, &bar[bi], it << 5, o - 1, C0 - 1, 0);
+      if (LIM == A3G_LIM_NONE || __all_sync(0xffffffffu, top < eps_hi || !al)) {
+        for (; e + 2 <= cnt; e += 2) {
+          step(TrueT{}, qv, gb, e);
+          step(TrueT{}, qv, gb, e + 1);
+        }
+      } else {
+        for (; e + ACT_U <= cnt; e += ACT_U) {
+#pragma unroll
+          for (int u = 0; u < ACT_U; u++) step(FalseT{}, qv, gb, e + u);
         }
       }
-      double *gb = wsm + 4 * ACH * 32 + bi * 2 * ACH;
-      if (lane < ACH && C0 + lane <= fb + 2) {
-        gb[lane] = gsig.at(C0 + lane);            // sigma(c+2)
-        gb[ACH + lane] = gdtv.at(C0 + lane - 1);  // dt/kappa(c+1)
-      }
-    };
-    uint32_t ph = 0u;
-    issue(0);
-    for (int m = 0; m < nchunk; m++) {
-      const int bi = m & 1;
-      if (m + 1 < nchunk) issue(m + 1);
-      if (!mbar_wait(&bar[bi], (ph >> bi) & 1u)) {
-        if (lane == 0) raise_error(sc, A3G_ERR_TIMEOUT, 3);
-        return;
-      }
-      ph ^= 1u << bi;
-      __syncwarp();
-      const double *qb = wsm + bi * 2 * ACH * 32 + lane;
-      const double *vb = qb + ACH * 32;
-      const double *gb = wsm + 4 * ACH * 32 + bi * 2 * ACH;
-      const int cend = min(fb, fa + m * ACH + ACH - 1);
-      if (cend - c + 1 == ACH) {  // a whole chunk: straight-line steps
-#pragma unroll
-        for (int e = 0; e < ACH; e++, c++)
-          step(c, FastT{}, qb[e * 32], (DIR == 2) ? vb[e * 32] + vf0 : vb[e * 32], gb[e], gb[ACH + e]);
-      } else {
-        for (int e = 0; c <= cend; c++, e++)
-          step(c, FastT{}, qb[e * 32], (DIR == 2) ? vb[e * 32] + vf0 : vb[e * 32], gb[e], gb[ACH + e]);
-      }
-      __syncwarp();
     }
+    for (; e < cnt; e++) {
+      const double upd = step(FalseT{}, qv, gb, e);
+      if (DIR == 2 && al && out_hi && c + e == ctop) out2[oo] -= upd;
+    }
+    c += cnt;
+    __syncwarp();
   }
-  for (; c <= ce; c++) checked_step(c);
+  // cell n+1: interface n+2 lies outside the box and carries nothing
+  if (al && s1 == n && out_hi && ctop == n + 1) out2[oo] += cell_update(m.dtv0, 0.0, m.fsr0, 0.0, m.fss0);
+}
+
+// Segments a marched line of n cells is cut into, given the warps that whole
+// lines would make: enough to give every SM about 20 warps (its registers hold
+// 16 at once), in segments of at least MARCH_SEG_MIN cells, below which the
+// repeated interface costs more than the added warps give (93x131x37, 2
+// grains: y 56 -> 16 us, z 27 -> 14 us a sweep; whole lines would take 45, 22).
+constexpr int MARCH_SEG_MIN = 10;
+static inline int march_segments(int n, long warps) {
+  const long want = 148L * 20;
+  if (warps >= want) return 1;
+  const long most = n / MARCH_SEG_MIN > 1 ? n / MARCH_SEG_MIN : 1;
+  const long s = (want + warps - 1) / warps;
+  return (int)(s < most ? s : most);
 }
 
 // Launches the TMA-fed column march; false when its conditions do not hold
@@ -1444,11 +1576,15 @@ static bool launch_colt(a3g_ctx *ctx) {
     return false;
   const size_t smem = 128 + (size_t)ACT_WARPS * ACT_WARP_D * sizeof(double);
   static_assert(128 + ACT_WARPS * ACT_WARP_D * 8 <= 48 * 1024, "fits the default dynamic limit");
+  const int n = (DIR == 1) ? L.ny : L.nz;
   const int nother = (DIR == 1) ? L.nz : L.ny;
-  const long nw = (long)((L.nx + 31) / 32) * nother * L.ns;
+  const long nlw = (long)((L.nx + 31) / 32) * nother * L.ns;  // warps of whole lines
+  const int nseg = march_segments(n, nlw);
+  const int seg = (n + nseg - 1) / nseg;
+  const long nw = nlw * ((n + seg - 1) / seg);
   k_advect_colt<DIR, LIM><<<(unsigned)((nw + ACT_WARPS - 1) / ACT_WARPS), 32 * ACT_WARPS, smem, ctx->stream>>>(
-      tq, tv, L, ctx->box, ctx->prm.nocycle, ctx->prm.eps_thresh, ctx->c0, ctx->c1, vel, dir_vghost(ctx, DIR),
-      ctx->vf, sg, ctx->dtv, ctx->aloft, ctx->sc, (DIR == 1) ? ctx->out_xz1 : ctx->out_xy1,
+      tq, tv, L, ctx->box, ctx->prm.nocycle, ctx->prm.eps_thresh, (n + seg - 1) / seg, seg, ctx->c0, ctx->c1, vel,
+      dir_vghost(ctx, DIR), ctx->vf, sg, ctx->dtv, ctx->aloft, ctx->sc, (DIR == 1) ? ctx->out_xz1 : ctx->out_xy1,
       (DIR == 1) ? ctx->out_xz2 : ctx->out_xy2);
   return true;
 }
