@@ -384,8 +384,9 @@ int a3g_kernel_times(a3g_ctx *ctx, double *ms, uint64_t *count);
  * variant 0 marching threads, 1 blocks of 4 cells, 2 blocks of 8 cells, and
  * for x only 3, warps marching 32 rows through shared-memory tiles, 4,
  * one warp per row walking it in 32-cell chunks with the lanes along i, and
- * 5, the same with the interior chunks staged one ahead by TMA tensor copies
- * (defaults: x 5, y 6, z 6).
+ * 5, warps marching 32 rows, a row per lane, through chunks that TMA tensor
+ * copies bring and take away (where the geometry varies along i, variant 4
+ * with its interior chunks staged by TMA) (defaults: x 5, y 6, z 6).
  * dir 3: the Crank-Nicolson x solve, variant 0 warp-tiled, 1 one thread per
  * line, 2 warp-tiled with each tile loaded one chunk ahead by a TMA tensor
  * copy (default).  dir 4: the Crank-Nicolson y and z solves, variant 0 one

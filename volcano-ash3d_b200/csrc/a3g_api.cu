@@ -192,11 +192,11 @@ int a3g_create(const a3g_grid_desc *grid, const a3g_params *params, int device, 
   ctx->h_aloft.assign(grid->ns, 1);
   ctx->n_gs_aloft = grid->ns;
   ctx->last_bc = 0;
-  // fastest measured advection variants on B200 (x: warp-row chunks with
-  // the interior chunks fed by TMA, C2 1.27 ms against 1.38 without and 2.16
-  // for marching rows; y, z: the column march fed by TMA chunks, C2 y 1.43 ->
-  // 1.24 ms and z 1.64 -> 1.28 ms against 4-cell blocks, which remain where
-  // the march's conditions do not hold); a3g_set_variant overrides them
+  // fastest measured advection variants on B200: marches fed by TMA chunks,
+  // along rows (x) and columns (y, z) -- 720x360x60, 10 grains: x 0.67 ms
+  // against 1.08 for the warp rows, y 0.58 and z 0.66 against 1.43 and 1.64
+  // for 4-cell blocks.  Where their conditions do not hold the warp rows and
+  // the blocks run; a3g_set_variant overrides them
   ctx->tune_advect[0] = 5;
   ctx->tune_advect[1] = 6;
   ctx->tune_advect[2] = 6;

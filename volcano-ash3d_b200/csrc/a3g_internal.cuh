@@ -79,6 +79,8 @@ struct Box {
 //   TM_ADV_VX      wind array, 32 i (an x chunk)
 //   TM_XROWS       level as a 2-D array of rows (i, row = (grain, k, j)),
 //                  36 i x 32 rows (a CN x tile with its neighbour cells)
+//   TM_QROWS/VROWS level / wind array as rows, 8 i x 32 rows in the 64-byte
+//                  swizzle (an x march chunk)
 enum TmapKind {
   TM_COLUMN = 0,
   TM_YCHUNK_IN = 1,
@@ -90,7 +92,9 @@ enum TmapKind {
   TM_ADV_QX1 = 7,
   TM_ADV_QX2 = 8,
   TM_ADV_VX = 9,
-  TM_XROWS = 10
+  TM_XROWS = 10,
+  TM_QROWS = 11,
+  TM_VROWS = 12
 };
 constexpr int YT_CH = 16;            // cells per CN y chunk
 constexpr int YT_ROWS = YT_CH + 2;   // with the cell before and the cell after

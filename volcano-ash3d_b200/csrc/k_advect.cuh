@@ -838,8 +838,8 @@ static void launch_advect_xt(a3g_ctx *ctx) {
 // the march's expressions (make_iface, iface_grain, cell_update), so the
 // results are the same bits.  Nothing is carried in registers between
 // chunks, which keeps the register count and the L1 traffic low.
-// With TMA, the loads of the interior chunks (the ones without range checks)
-// arrive by tensor copies instead: the warp's GC grains and the wind of the
+// With TMA (rows whose geometry varies along i), the loads of the interior
+// chunks (the ones without range checks) arrive by tensor copies instead: the warp's GC grains and the wind of the
 // chunk, one chunk ahead, into one of two staging buffers, so that the
 // lanes no longer wait on global loads there.  Same arithmetic, same bits.
 // ---------------------------------------------------------------------------
@@ -1030,17 +1030,15 @@ static void launch_advect_xw(a3g_ctx *ctx, bool tma) {
   if (tma && !(tensor_map(ctx, ctx->c0, gc == 2 ? TM_ADV_QX2 : TM_ADV_QX1, &tq) &&
                tensor_map(ctx, ctx->vx, TM_ADV_VX, &tv)))
     tma = false;
-#define A3G_XW(GC_, PER_, LC_)                                                                              \
-  if (tma)                                                                                                   \
-    k_advect_xw<LIM, GC_, PER_, LC_, true><<<blocks, 32 * XW_WARPS, 0, ctx->stream>>>(                      \
-        tq, tv, L, ctx->box, ctx->prm.nocycle, ctx->prm.eps_thresh, ngroups, ctx->c0, ctx->c1, ctx->vx,      \
-        ctx->snx, ctx->dtv, ctx->aloft, ctx->sc, ctx->out_yz1, ctx->out_yz2);                                \
-  else                                                                                                       \
-    k_advect_xw<LIM, GC_, PER_, LC_, false><<<blocks, 32 * XW_WARPS, 0, ctx->stream>>>(                     \
-        tq, tv, L, ctx->box, ctx->prm.nocycle, ctx->prm.eps_thresh, ngroups, ctx->c0, ctx->c1, ctx->vx,      \
-        ctx->snx, ctx->dtv, ctx->aloft, ctx->sc, ctx->out_yz1, ctx->out_yz2)
-#define A3G_XW_LC(GC_, PER_) \
-  if (lc) { A3G_XW(GC_, PER_, true); } else { A3G_XW(GC_, PER_, false); }
+#define A3G_XW(GC_, PER_, LC_, TMA_)                                                                        \
+  k_advect_xw<LIM, GC_, PER_, LC_, TMA_><<<blocks, 32 * XW_WARPS, 0, ctx->stream>>>(                        \
+      tq, tv, L, ctx->box, ctx->prm.nocycle, ctx->prm.eps_thresh, ngroups, ctx->c0, ctx->c1, ctx->vx,        \
+      ctx->snx, ctx->dtv, ctx->aloft, ctx->sc, ctx->out_yz1, ctx->out_yz2)
+  // rows of constant geometry come here only without tensor maps (k_advect_xm)
+#define A3G_XW_LC(GC_, PER_)                      \
+  if (lc) { A3G_XW(GC_, PER_, true, false); }     \
+  else if (tma) { A3G_XW(GC_, PER_, false, true); } \
+  else { A3G_XW(GC_, PER_, false, false); }
   if (gc == 2) {
     if (ctx->grid.periodic) { A3G_XW_LC(2, true); } else { A3G_XW_LC(2, false); }
   } else {
@@ -1590,6 +1588,256 @@ static bool launch_colt(a3g_ctx *ctx) {
 }
 
 // ---------------------------------------------------------------------------
+// Row march fed by TMA chunks (x sweep).  A warp owns 32 rows of one grain
+// (row r = (k-1)*ny + j-1 of the plane) with one row per lane, and marches
+// them with march_step() as the column march does: no exchange between lanes
+// and no ring in shared memory.  Chunks of 8 cells x 32 rows of the
+// concentration and the wind arrive by tensor loads in the 64-byte swizzle,
+// under which the lanes' 16-byte reads of their own rows meet no bank twice;
+// the new cells replace the chunk's old ones in place, two cells behind, and
+// leave by a tensor store.  Chunk t holds the cells s0+2+8t .. of a segment
+// that starts at s0 = 1 (mod 8), so that loads start on an even cell and
+// stores on a multiple of 8 (the 16-byte rule).  Three concentration buffers
+// turn: one being marched, one loading, one being stored.  A tile whose 32
+// rows are not all this plane's (the last of a grain) is stored by the lanes.
+// Taken when sigma and dt/kappa do not vary along the row.
+//
+// Bound, like the column march, by issue (58 % of cycles on the C2 slab, 16
+// warps per SM by registers) and the FP64 pipe (40 %).  720x360x60, 10 grains:
+// 1.08 -> 0.67 ms a sweep against the warp-row kernel, whose lanes pass each
+// value on through shared-memory rings (188 instructions a cell against 95).
+// ---------------------------------------------------------------------------
+constexpr int AXM_WARPS = 2;
+constexpr int AXM_BUF = 32 * 8 * 8;                    // bytes of a chunk
+constexpr int AXM_WARP_B = 5 * AXM_BUF;                // 3 concentration and 2 wind buffers
+constexpr int AXM_SMEM = 512 + 512 + AXM_WARPS * AXM_WARP_B;  // barriers, room to align, buffers
+
+template <int LIM, bool PER>
+__global__ void __launch_bounds__(32 * AXM_WARPS, ACT_MINB) k_advect_xm(
+    const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tv,
+    const __grid_constant__ CUtensorMap to, Layout L, Box box, int nocycle, double eps, int nseg, int seg,
+    const double *__restrict__ cin, double *__restrict__ cout, const double *__restrict__ vel, Geo3 sig, Geo3 dtvt,
+    const int32_t *__restrict__ aloft, DevScalars *sc, double *__restrict__ out1, double *__restrict__ out2) {
+  extern __shared__ unsigned char axm_smem[];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  unsigned char *const sm = axm_smem + ((512u - (smem_u32(axm_smem) & 511u)) & 511u);  // the swizzle's period
+  uint64_t *bar = reinterpret_cast<uint64_t *>(sm) + 2 * wid;
+  unsigned char *const qbuf = sm + 512 + wid * AXM_WARP_B, *const vbuf = qbuf + 3 * AXM_BUF;
+  const int nrows = L.ny * L.nz;
+  const int ntile = (nrows + 31) >> 5;
+  const long t = (long)blockIdx.x * AXM_WARPS + wid;
+  if (t >= (long)ntile * L.ns * nseg) return;  // whole warps only; no block barrier below
+  const int g = (int)(t % L.ns);
+  const long rr = t / L.ns;
+  const int r0 = (int)(rr % ntile) * 32;
+  const int s0 = (int)(rr / ntile) * seg + 1;
+  const int n = L.nx, s1 = min(n, s0 + seg - 1);
+  const int r = min(r0 + lane, nrows - 1);
+  const int j = r % L.ny + 1, k = r / L.ny + 1;
+  const int rmin = box.imin, rmax = box.imax;
+  const bool al = r0 + lane < nrows && j >= box.jmin && j <= box.jmax && k >= box.kmin && k <= box.kmax &&
+                  aloft[g] != 0;
+  const long grow = (long)g * nrows;  // this grain's first row in the level
+  double *const po = cout + (grow + r0) * L.P;
+  auto zero = [&](int ca, int cb) {   // cells ca..cb of the tile's rows: the reference leaves zeros
+    for (int row = 0; row < min(32, nrows - r0); row++)
+      for (int c = ca + lane; c <= cb; c += 32) po[(long)row * L.P + (c - 1)] = 0.0;
+  };
+  const int c0 = max(s0, rmin), c1 = min(s1, rmax);  // the cells marched
+  if (c0 > c1 || !__any_sync(0xffffffffu, al)) {
+    zero(s0, s1);
+    return;
+  }
+  const int t0 = (c0 - s0) >> 3, t1 = (c1 - s0) >> 3;
+  zero(s0, s0 + 8 * t0 - 1);
+  zero(s0 + 8 * t1 + 8, s1);
+  auto issue = [&](int c) {  // chunk c; its concentration buffer was stored from two chunks ago
+    if (lane == 0) {
+      uint64_t *b = &bar[c & 1];
+      bulk_wait_read1();
+      mbar_arrive_expect_tx(b, 2u * AXM_BUF);
+      tma_load_2d(qbuf + (c % 3) * AXM_BUF, &tq, b, s0 + 1 + 8 * c, (int)(grow + r0));
+      tma_load_2d(vbuf + (c & 1) * AXM_BUF, &tv, b, s0 + 1 + 8 * c, r0);
+    }
+  };
+  if (lane == 0) {
+    mbar_init(&bar[0], 1);
+    mbar_init(&bar[1], 1);
+    mbar_init_fence();
+  }
+  __syncwarp();
+  issue(t0);
+  const double *const pv = vel + (long)r * L.P;
+  const double *const pq = cin + (grow + r) * L.P;
+  // ghost-aware loads (Set_BC(1): zero or wrapped concentration, edge or wrapped winds)
+  auto qload = [&](int c) -> double {
+    if (c < rmin - 2 || c > rmax + 2) return 0.0;
+    if (c >= 1 && c <= n) return pq[c - 1];
+    return PER ? pq[(c < 1 ? c + n : c - n) - 1] : 0.0;
+  };
+  auto vload = [&](int c) -> double {
+    if (PER) return pv[(c < 1 ? c + n : c > n ? c - n : c) - 1];
+    return pv[(c < 1 ? 1 : c > n ? n : c) - 1];
+  };
+  // sigma and dt/kappa of the row
+  const double sg = sig.p[(long)(j + 1) * sig.sj + (long)(k + 1) * sig.sk], hs = 0.5 * sg;
+  const double dtv = dtvt.p[(long)(j + 1) * dtvt.sj + (long)(k + 1) * dtvt.sk];
+  // ---- interface c0 and the window at c0 -------------------------------------
+  March m;
+  {
+    m.q0 = qload(c0);
+    m.q1 = qload(c0 + 1);
+    const double qm1 = qload(c0 - 1), qm2 = qload(c0 - 2);
+    m.d0 = m.q0 - qm1;
+    m.d1 = m.q1 - m.q0;
+    const double vm2 = vload(c0 - 2), vm1 = vload(c0 - 1), v0 = vload(c0);
+    m.vB = vload(c0 + 1);
+    const double usm1 = 0.5 * (vm2 + vm1) * sg;
+    const double usA = 0.5 * (vm1 + v0) * sg;
+    m.us = 0.5 * (v0 + m.vB) * sg;
+    const double dm = qm1 - qm2;
+    const Iface f = make_iface(usm1, usA, m.us, dtv, true, true);
+    m.fss0 = fss_select<LIM>(dm, m.d0, m.d1, f.up, f.cf, true, eps, nocycle);
+    m.fsr0 = f.usp * m.d0;
+    m.fsr0 = m.fsr0 + m.q0 * f.divm;
+    if (!PER && c0 == 1 && al) {  // the low outflow, cell 0
+      double fsl = f.usm * m.d0;
+      fsl = fsl + qm1 * f.divp;
+      double fsr = pos_part(usm1) * dm;
+      fsr = fsr + qm1 * (neg_part(usA) - neg_part(usm1));
+      out1[grow + r] += cell_update(dtv, fsl, fsr, m.fss0, 0.0);
+    }
+    m.upA = pos_part(usA);
+    m.upB = pos_part(m.us);
+    m.unB = neg_part(m.us);
+  }
+  const bool nocyc = nocycle != 0;
+  const int eps_hi = nocyc ? 0 : __double2hiint(eps);  // |d| < eps for certain, by its high word alone
+  // this lane's row of a buffer: cells 2p, 2p+1 at pair(p), cell e at cell(e)
+  const int row_b = lane << 6, row_s = ((lane >> 1) & 3) << 4;
+  auto pair = [&](unsigned char *b, int p) { return reinterpret_cast<double2 *>(b + row_b + ((p << 4) ^ row_s)); };
+  auto cell = [&](unsigned char *b, int e) { return reinterpret_cast<double *>(pair(b, e >> 1)) + (e & 1); };
+  auto step = [&](auto quiet, double q2, double vn) {
+    const double q0 = m.q0;
+    const double sum = march_step<LIM, decltype(quiet)::value>(m, q2, q2 - m.q1, vn, hs, dtv, eps, nocyc);
+    const double upd = dtv * sum;
+    return q0 - upd;
+  };
+  auto two = [&](auto quiet, unsigned char *qb, unsigned char *vb, int p) {  // cells 2p, 2p+1 of the chunk
+    double2 *q = pair(qb, p);
+    const double2 x = *q, v = *pair(vb, p);
+    double2 y;
+    y.x = step(quiet, x.x, v.x);
+    y.y = step(quiet, x.y, v.y);
+    *q = y;
+  };
+  const bool whole = r0 + 32 <= nrows, all_al = __all_sync(0xffffffffu, al);
+  uint32_t ph = 0u;
+  for (int c = t0; c <= t1; c++) {
+    if (c < t1) issue(c + 1);
+    if (!mbar_wait(&bar[c & 1], (ph >> (c & 1)) & 1u)) {
+      if (lane == 0) {
+        raise_error(sc, A3G_ERR_TIMEOUT, 4);
+        bulk_wait0();
+      }
+      return;
+    }
+    ph ^= 1u << (c & 1);
+    unsigned char *const qb = qbuf + (c % 3) * AXM_BUF, *const vb = vbuf + (c & 1) * AXM_BUF;
+    const int cb = s0 + 8 * c;                       // slot e: the step of cell cb+e, holding cell cb+e+2
+    const int e0 = max(c0 - cb, 0), e1 = min(c1 - cb, 7);
+    if (cb + 9 > n) {                                // the ghosts beyond the row's end
+#pragma unroll
+      for (int x = n + 1; x <= n + 2; x++) {
+        const int e = x - cb - 2;
+        if (e >= 0 && e < 8) {
+          if (PER) *cell(qb, e) = qload(x);
+          *cell(vb, e) = vload(x);
+        }
+      }
+    }
+    // the differences the chunk's interfaces limit: d1 and the first 7 new ones
+    int top = __double2hiint(m.d1) & 0x7fffffff;
+    {
+      double prev = m.q1;
+#pragma unroll
+      for (int p = 0; p < 4; p++) {
+        const double2 x = *pair(qb, p);
+        top = max(top, __double2hiint(x.x - prev) & 0x7fffffff);
+        if (p < 3) top = max(top, __double2hiint(x.y - x.x) & 0x7fffffff);
+        prev = x.y;
+      }
+    }
+    const bool quiet = LIM == A3G_LIM_NONE || __all_sync(0xffffffffu, top < eps_hi || !al);
+    if (e0 == 0 && e1 == 7) {
+      if (quiet) {
+        for (int p = 0; p < 4; p++) two(TrueT{}, qb, vb, p);
+      } else {
+        for (int p = 0; p < 4; p += ACT_U / 2) {
+#pragma unroll
+          for (int u = 0; u < ACT_U / 2; u++) two(FalseT{}, qb, vb, p + u);
+        }
+      }
+    } else {
+      for (int e = 0; e < 8; e++) {
+        double *q = cell(qb, e);
+        double y = 0.0;  // outside the box
+        if (e >= e0 && e <= e1) y = step(FalseT{}, *q, *cell(vb, e));
+        *q = y;
+      }
+    }
+    if (!all_al && !al) {
+#pragma unroll
+      for (int p = 0; p < 4; p++) *pair(qb, p) = make_double2(0.0, 0.0);
+    }
+    fence_proxy_async_smem();
+    __syncwarp();
+    if (whole) {
+      if (lane == 0) {
+        tma_store_2d(&to, qb, cb - 1, (int)(grow + r0));
+        bulk_commit();
+      }
+    } else {
+      const int e = lane & 7, x = cb + e;
+#pragma unroll
+      for (int h = 0; h < 8; h++) {
+        const int row = 4 * h + (lane >> 3);
+        if (r0 + row < nrows && x <= n)
+          po[(long)row * L.P + (x - 1)] = *reinterpret_cast<const double *>(
+              qb + (row << 6) + ((((e >> 1) ^ ((row >> 1) & 3)) << 4) | ((e & 1) << 3)));
+      }
+      __syncwarp();
+    }
+  }
+  // cell n+1: interface n+2 lies outside the box and carries nothing
+  if (!PER && al && s1 == n && rmax == n) out2[grow + r] += cell_update(dtv, 0.0, m.fsr0, 0.0, m.fss0);
+  if (lane == 0) bulk_wait0();
+}
+
+// Launches the TMA-fed row march; false when its conditions do not hold.
+template <int LIM>
+static bool launch_advect_xm(a3g_ctx *ctx) {
+  const Layout &L = ctx->L;
+  if (along<0>(ctx->snx) != 0 || along<0>(ctx->dtv) != 0) return false;
+  CUtensorMap tq, tv, to;
+  if (!tensor_map(ctx, ctx->c0, TM_QROWS, &tq) || !tensor_map(ctx, ctx->vx, TM_VROWS, &tv) ||
+      !tensor_map(ctx, ctx->c1, TM_QROWS, &to))
+    return false;
+  const long nlw = (long)(((long)L.ny * L.nz + 31) / 32) * L.ns;
+  const int want = march_segments(L.nx, nlw);
+  const int seg = (L.nx + want - 1) / want + 7 & ~7;  // whole chunks
+  const int nseg = (L.nx + seg - 1) / seg;
+  const unsigned blocks = (unsigned)((nlw * nseg + AXM_WARPS - 1) / AXM_WARPS);
+#define A3G_XM(PER_)                                                                                           \
+  k_advect_xm<LIM, PER_><<<blocks, 32 * AXM_WARPS, AXM_SMEM, ctx->stream>>>(                                    \
+      tq, tv, to, L, ctx->box, ctx->prm.nocycle, ctx->prm.eps_thresh, nseg, seg, ctx->c0, ctx->c1, ctx->vx,     \
+      ctx->snx, ctx->dtv, ctx->aloft, ctx->sc, ctx->out_yz1, ctx->out_yz2)
+  if (ctx->grid.periodic) A3G_XM(true); else A3G_XM(false);
+#undef A3G_XM
+  return true;
+}
+
+// ---------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------
 template <int DIR, int LIM, int GC, bool PER, bool TOPO = false>
@@ -1658,6 +1906,7 @@ static void launch_dir_lim(a3g_ctx *ctx) {
       launch_advect_xt<LIM>(ctx);
       return;
     }
+    if (variant == 5 && launch_advect_xm<LIM>(ctx)) return;
     if (variant == 4 || variant == 5) {
       launch_advect_xw<LIM>(ctx, variant == 5);
       return;

@@ -1293,11 +1293,17 @@ bool tensor_map(a3g_ctx *ctx, const double *p, int kind, CUtensorMap *out) {
   cuuint32_t box[4] = {32, 1, 1, 1};
   cuuint32_t rank = 4;
   // the rows of a level form a 2-D array: row r = (g*nz + k-1)*ny + j-1 at r*P
-  const cuuint64_t rdims[2] = {(cuuint64_t)L.nx, (cuuint64_t)L.ny * L.nz * L.ns};
+  const cuuint64_t rdims[2] = {(cuuint64_t)L.nx, (cuuint64_t)L.ny * L.nz * (kind == TM_VROWS ? 1 : L.ns)};
+  CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_NONE;
   if (kind == TM_XROWS) {
     rank = 2;
     box[0] = XT2_COLS;
     box[1] = 32;
+  } else if (kind == TM_QROWS || kind == TM_VROWS) {
+    rank = 2;
+    box[0] = 8;
+    box[1] = 32;
+    swizzle = CU_TENSOR_MAP_SWIZZLE_64B;
   } else if (kind == TM_COLUMN) {
     if (L.nz > 256) return false;
     box[2] = (cuuint32_t)L.nz;
@@ -1323,7 +1329,7 @@ bool tensor_map(a3g_ctx *ctx, const double *p, int kind, CUtensorMap *out) {
   e.kind = kind;
   if (enc(&e.map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, rank, const_cast<double *>(p), rank == 2 ? rdims : dims,
           strides, box, estr,
-          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+          CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
     return false;
   // a step uses about 17 (two levels alternating under each tile shape, and
