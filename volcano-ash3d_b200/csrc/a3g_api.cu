@@ -200,15 +200,15 @@ int a3g_create(const a3g_grid_desc *grid, const a3g_params *params, int device, 
   ctx->tune_advect[0] = 5;
   ctx->tune_advect[1] = 6;
   ctx->tune_advect[2] = 6;
-  // CN x solve: warp tiles loaded one chunk ahead by TMA (C2 1.35 -> 1.16 ms
-  // against the synchronous tile loads of variant 0)
+  // CN x solve: row tiles through TMA (C2 0.82 ms against 1.35 for the
+  // synchronous tile loads of variant 0)
   ctx->tune_cn_x = 2;
   ctx->ov_cloudcon = 1.0e-3;   // CLOUDCON_THRESH, src/Output_Vars.f90:119
   ctx->ov_cloudload = 2.0e-1;  // CLOUDLOAD_THRESH, :114
   ctx->ov_depo = 1.0e-2;       // DEPO_THRESH, :113
   ctx->ov_density = 1000.0;    // DepositDensity, src/Tephra.f90:55
-  // CN y and z solves through TMA tiles (C2 on B200: y 1.55 -> 1.25 ms, z
-  // 1.23 -> 0.66 ms against two grains per thread)
+  // CN y and z solves through TMA tiles (C2 on B200: y 0.91, z 0.71 ms against
+  // 1.55 and 1.23 for two grains per thread)
   ctx->tune_cn_yz = 3;
   auto dmalloc = [&](void **p, size_t n) -> cudaError_t {
     cudaError_t e = cudaMalloc(p, n);

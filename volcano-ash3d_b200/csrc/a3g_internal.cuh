@@ -71,20 +71,18 @@ struct Box {
 // A TMA tensor map over one concentration level or one wind array (cached
 // per device pointer and tile shape; see tensor_map()).  Tile kinds:
 //   TM_COLUMN      level, 32 i x 1 j x nz k (the CN z solve's column tile)
-//   TM_YCHUNK_IN   level, 32 i x (YT_CH + 2) j (a CN y chunk and its neighbours)
-//   TM_YCHUNK_OUT  level, 32 i x YT_CH j (the CN y chunk it stores)
+//   TM_YCHUNK      level, 32 i x YT_CH j (a CN y chunk)
 //   TM_ADV_QY/QZ   level, 32 i x ACH j / ACH k (an advection chunk)
 //   TM_ADV_VY/VZ   wind array, the same chunks
 //   TM_ADV_QX1/QX2 level, 32 i x 1 j x 1 k x 1 / 2 grains (an x chunk)
 //   TM_ADV_VX      wind array, 32 i (an x chunk)
 //   TM_XROWS       level as a 2-D array of rows (i, row = (grain, k, j)),
-//                  36 i x 32 rows (a CN x tile with its neighbour cells)
+//                  CX_CH i x 32 rows in the 128-byte swizzle (a CN x chunk)
 //   TM_QROWS/VROWS level / wind array as rows, 8 i x 32 rows in the 64-byte
 //                  swizzle (an x march chunk)
 enum TmapKind {
   TM_COLUMN = 0,
-  TM_YCHUNK_IN = 1,
-  TM_YCHUNK_OUT = 2,
+  TM_YCHUNK = 1,
   TM_ADV_QY = 3,
   TM_ADV_QZ = 4,
   TM_ADV_VY = 5,
@@ -97,9 +95,8 @@ enum TmapKind {
   TM_VROWS = 12
 };
 constexpr int YT_CH = 16;            // cells per CN y chunk
-constexpr int YT_ROWS = YT_CH + 2;   // with the cell before and the cell after
 constexpr int ACH = 8;               // cells per advection chunk
-constexpr int XT2_COLS = 36;         // cells per CN x tile row as loaded (even start, 16-byte rule)
+constexpr int CX_CH = 16;            // cells per CN x chunk
 struct TmapEntry {
   const void *p;
   int kind;
@@ -171,13 +168,17 @@ struct a3g_ctx {
   double *h_tot;            // pinned totals staging
   // CN factor tables, one region per direction (cn_tab[d] inside cn_buf),
   // reused while dt, the box, the geometry and the diffusivity stay the same:
-  // cn_state = {dt of each table (3), skip flags (3)} on the device
+  // cn_state holds two slots of the dt a table was built for per direction on
+  // the device, cn_slot the one the next build reads; cn_stamp is the
+  // dt_stamp a table was last brought up to date for
   double *cn_buf;
   size_t cn_len;
   double *cn_tab[3];
   bool cn_valid[3];
   a3g::Box cn_box[3];
   double *cn_state;
+  int cn_slot[3];
+  uint64_t cn_stamp[3];
 
   a3g::Box box;
   int last_bc;
@@ -243,8 +244,7 @@ struct a3g_ctx {
   a3g_inv *inv;
   // TMA tensor maps over the levels and winds the tiled kernels read and
   // write, and per tiled CN kernel its set-up state: 0 until its first
-  // launch, then the persistent grid size (z: [0], y: [1]) or 1 once its
-  // shared-memory attributes are set (x: [2])
+  // launch, then the persistent grid size (z: [0], y: [1], x: [2])
   std::vector<a3g::TmapEntry> tmaps;
   int tma_grid[4];
   // optional per-kernel timing (a3g_kernel_timing)

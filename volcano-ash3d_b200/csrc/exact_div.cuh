@@ -153,4 +153,30 @@ __device__ __forceinline__ bool quot_rn(double a, double b, double *q) {
   return ha >= ALO && (hb - BLO) < (BHI - BLO) && (hb & 0xfffffu) != 0xfffffu;
 }
 
+// RN(a/b) from 1/b = zh + zl + zll (zh = RN(1/b), zl = RN(1/b - zh), zll =
+// RN(1/b - zh - zl)) in three dependent operations and no test of the result:
+// q = RN(a*zh + RN(a*zl + RN(a*zll))).  The idea of multiplying by a reciprocal
+// in more than one word is N. Brisebarre, J.-M. Muller and S. K. Raina,
+// "Accelerating correctly rounded floating-point division when the divisor is
+// known in advance" (IEEE Trans. Computers 53, 2004); the third word removes
+// their exceptional divisors.  Scaled to 1 <= a, b < 2: |zl| <= 2^-54, so the
+// correction is below 2^-53 and its rounding error at most 2^-107 (+ 2^-158 for
+// the rest), while a/b keeps 2^-106/b > 2^-107 from every midpoint of two
+// doubles (2^-105/b when a >= b): the last rounding gives RN(a/b).  Divisors
+// within 2^-20 of twice a power of two, where the margin closes, and those
+// outside [2^-50, 2^51) are not covered (div_rn_3_covers).  The dividend has
+// to be in [2^-900, 2^901) or zero (div_rn_3_takes); a zero quotient's sign is
+// not kept.
+__device__ __forceinline__ double div_rn_3(double a, double zh, double zl, double zll) {
+  return fma(a, zh, fma(a, zl, a * zll));
+}
+__device__ __forceinline__ bool div_rn_3_covers(double b) {
+  return exp_in<-50, 50, false>(b) && ((unsigned)__double2hiint(b) & 0xfffffu) != 0xfffffu;
+}
+__device__ __forceinline__ bool div_rn_3_takes(double a) {
+  const unsigned h = (unsigned)__double2hiint(a) & 0x7fffffffu;
+  constexpr unsigned LO = (1023u - 900u) << 20, HI = (1023u + 901u) << 20;
+  return h - LO < HI - LO || (h | (unsigned)__double_as_longlong(a)) == 0u;
+}
+
 }  // namespace a3g

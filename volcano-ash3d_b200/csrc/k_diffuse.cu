@@ -86,11 +86,33 @@ __global__ void __launch_bounds__(256) k_diff(Layout L, Box box, int periodic,
 // ---------------------------------------------------------------------------
 // Crank-Nicolson line tables
 // ---------------------------------------------------------------------------
-// Table fields, stored [field][position][line] so that neighbouring lines
-// (neighbouring threads) read neighbouring words.
-// CN_RDP holds RN(1/D'), so that the back substitution's quotients can be
-// formed by exact_div.cuh's certified path.
-enum { CN_FACT = 0, CN_DP = 1, CN_DU = 2, CN_CL = 3, CN_CC = 4, CN_CR = 5, CN_RDP = 6, CN_NF = 7 };
+// Per row of a distinct line: dgtsv's multiplier, the right-hand side's
+// weights, the upper diagonal, the pivot D', and 1/D' as a sum of up to three
+// doubles (exact_div.cuh, div_rn_3).  Two layouts:
+//   by field, [field][row][line] (neighbouring lines in neighbouring words):
+//     the x tables, whose solve runs a line per lane, and y or z tables whose
+//     lines differ along i; without CN_ZL and CN_ZLL;
+//   by row, [line][row][8] with D' behind it as [line][row]: the y and z
+//     tables that a warp's 32 lines share, so that a chunk's rows are one
+//     contiguous copy.
+enum {
+  CN_FACT = 0, CN_CL = 1, CN_CC = 2, CN_CR = 3, CN_DU = 4, CN_ZH = 5, CN_DP = 6, CN_NFX = 7,  // by field
+  CN_ROW = 8, CN_ZL = 6, CN_ZLL = 7, CN_NF = 9                                               // by row
+};
+
+struct CnTab {
+  const double *p;
+  long F, U;  // rows x lines, lines
+  int n;      // rows of a line
+  bool byrow;
+  __device__ __forceinline__ double at(int f, int l, long u) const {  // f: CN_FACT .. CN_ZH or CN_DP
+    if (!byrow) return p[f * F + (long)l * U + u];
+    const long r = u * n + l;
+    return f == CN_DP ? p[CN_ROW * F + r] : p[CN_ROW * r + f];
+  }
+  // per line: the run [lo, hi] (below) and whether a pivot is one div_rn_3 does not cover
+  __host__ __device__ __forceinline__ const double *runs() const { return p + (byrow ? CN_NF : CN_NFX) * F; }
+};
 
 // Constant runs.  Along a line whose geometry and diffusivity do not change
 // (every x line of a lon/lat grid, every line of a projected grid with
@@ -98,31 +120,31 @@ enum { CN_FACT = 0, CN_DP = 1, CN_DU = 2, CN_CL = 3, CN_CC = 4, CN_CR = 5, CN_RD
 // elimination factors of dgtsv settle to a fixed point after a few rows, so
 // the table rows become bit-identical.  Per distinct line the table keeps the
 // run [lo, hi] of identical rows that ends at the last interior row
-// (hi = ncells-2): row lo is stored, rows lo+1..hi are not, and readers take
-// them from registers.  The values are the same bits either way.  The run
-// bounds follow the CN_NF fields: [2][U] doubles holding lo and hi.
+// (hi = ncells-2): row lo is stored, rows lo+1..hi of the x tables are not,
+// and readers take them from registers.  The values are the same bits either
+// way.
 struct CnRun {
   int lo, hi;
-  double v[CN_NF];
+  double v[CN_NFX];
 };
 
-__device__ __forceinline__ void cn_load_run(const double *__restrict__ t, long F, long U,
-                                            const double *__restrict__ runs, long u, CnRun &R) {
+__device__ __forceinline__ void cn_load_run(const CnTab &t, long u, CnRun &R) {
+  const double *runs = t.runs();
   R.lo = (int)runs[u];
-  R.hi = (int)runs[U + u];
+  R.hi = (int)runs[t.U + u];
 #pragma unroll
-  for (int f = 0; f < CN_NF; f++) R.v[f] = t[f * F + (long)R.lo * U];
+  for (int f = 0; f < CN_NFX; f++) R.v[f] = t.p[f * t.F + (long)R.lo * t.U + u];
 }
 
-// Field f of row l: from the run registers inside (lo, hi], else from the table.
-__device__ __forceinline__ double cn_coef(const double *__restrict__ t, long F, long U, const CnRun &R,
-                                          int f, int l) {
-  return (l > R.lo && l <= R.hi) ? R.v[f] : t[f * F + (long)l * U];
+// Field f of row l of an x line: from the run registers inside (lo, hi], else from the table.
+__device__ __forceinline__ double cn_coef(const CnTab &t, long u, const CnRun &R, int f, int l) {
+  return (l > R.lo && l <= R.hi) ? R.v[f] : t.p[f * t.F + (long)l * t.U + u];
 }
 
 struct LineMap {  // distinct-line indexing for one sweep direction
   int na, nb;     // extents of the two fixed indices (a fastest)
   int da, db;     // 1 if the coefficients vary with a / b
+  int ds;         // 1 if they vary along the sweep
   int U;          // number of distinct lines
   __host__ __device__ __forceinline__ int u(int a, int b) const {
     return (da ? a - 1 : 0) + (da ? na : 1) * (db ? b - 1 : 0);
@@ -133,129 +155,177 @@ __device__ __forceinline__ bool same_bits(double a, double b) {
   return __double_as_longlong(a) == __double_as_longlong(b);
 }
 
-// Only the x tables (read by the warp-tiled x solve) leave their final run
-// unstored; the y and z tables are written in full, because their solves
-// read every row.
-template <int DIR>
-__global__ void k_cn_table(Layout L, Box box, double imp, LineMap map, Geo3 sig, Geo3 kap, Geo3 kk,
-                           DevScalars *sc, const double *__restrict__ cstate, double *__restrict__ tab) {
+// The tables of LPB lines per block (256 threads), in tiles of CN_TR rows:
+//   the rows' coefficients (four IEEE divisions each) by all threads, then
+//   the elimination -- fact = DL/D'(l-1), D' = D - fact*DU(l-1), the only
+//   serial part -- by one lane per line, then the pivots' reciprocals by all.
+// One thread per line doing all of it took 55 us a table on 317x211x53 (53
+// lines) and 150 us on 201x151x41 over terrain; the chain of one division,
+// product and difference per row is what is left.  A lane that reaches the
+// fixed point of a line whose remaining interior rows have the same inputs
+// stops; LPB = 1 (few lines, more rows per tile) or 32.
+//
+// The tables are kept between steps: st_old holds the dt this table was built
+// for, and while that is the step's dt (and the host allows it, `may`: same
+// box, geometry and diffusivity) the blocks return at once.  st_new is the
+// slot the next launch reads, so that no block can see this launch's write.
+template <int DIR, int LPB>
+__global__ void __launch_bounds__(256) k_cn_table(Layout L, Box box, double imp, LineMap map, Geo3 sig, Geo3 kap,
+                                                  Geo3 kk, DevScalars *sc, const double *__restrict__ st_old,
+                                                  double *__restrict__ st_new, int may, int byrow,
+                                                  double *__restrict__ tab) {
   constexpr bool COMPRESS = (DIR == 0);
-  const int u = blockIdx.x * blockDim.x + threadIdx.x;
-  if (u >= map.U) return;
-  if (cstate[3 + DIR] != 0.0) return;  // the table already holds this dt's factors
-  // representative fixed indices of this distinct line
+  constexpr int TR = LPB == 1 ? 256 : 32;  // rows per tile
+  __shared__ double sD[TR * LPB], sDL[TR * LPB], sDU[TR * LPB], sF[TR * LPB], sP[TR * LPB];
+  __shared__ double cF[LPB], cP[LPB];      // fact and D' of the row before the tile
+  __shared__ int sRun[LPB], sBad[LPB], sBrk;
+  const double dt = sc->dt;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *st_new = dt;
+  if (may && *st_old == dt) return;
+  const int u0 = blockIdx.x * LPB;
+  const int tid = threadIdx.x;
+  // representative fixed indices of a distinct line
   const int amin = (DIR == 0) ? box.jmin : box.imin;
   const int bmin = (DIR == 2) ? box.jmin : box.kmin;
   const int na1 = map.da ? map.na : 1;
-  const int a = map.da ? (u % na1) + 1 : amin;
-  const int b = map.db ? (u / na1) + 1 : bmin;
   const int rmin = (DIR == 0) ? box.imin : (DIR == 1) ? box.jmin : box.kmin;
   const int rmax = (DIR == 0) ? box.imax : (DIR == 1) ? box.jmax : box.kmax;
-  const int ncells = rmax - rmin + 1;
-  auto G = [&](const Geo3 &g3, int m) {
+  const int n = rmax - rmin + 1;
+  const long U = map.U, F = (long)n * U;
+  auto G = [&](const Geo3 &g3, int u, int m) {
+    const int a = map.da ? (u % na1) + 1 : amin, b = map.db ? (u / na1) + 1 : bmin;
     return (DIR == 0) ? g3.at(m, a, b) : (DIR == 1) ? g3.at(a, m, b) : g3.at(a, b, m);
   };
-  const double dt = sc->dt;
-  const long U = map.U;
-  const long F = (long)ncells * U;
-  auto put = [&](int l, const double *v) {
-#pragma unroll
-    for (int f = 0; f < CN_NF; f++) tab[f * F + (long)l * U + u] = v[f];
+  auto put = [&](int u, int l, int f, double v) {
+    if (!byrow) tab[f * F + (long)l * U + u] = v;
+    else tab[CN_ROW * ((long)u * n + l) + f] = v;
   };
-  double dp_prev = 0.0, du_prev = 0.0;
-  double rv[CN_NF];   // first row of the current run
-  int s = 0;          // index of that row
-  bool cont = false;  // row l-1 repeated row l-2
-  double pin[8];      // inputs of row l-1
-  for (int l = 0; l < ncells - 1; l++) {
-    const int c = rmin + l;
-    const double in[8] = {G(kap, c - 1), G(kap, c), G(kap, c + 1), G(kk, c - 1),
-                          G(kk, c),      G(kk, c + 1), G(sig, c),   G(sig, c + 1)};
-    bool same_in = l >= 2;
-#pragma unroll
-    for (int e = 0; e < 8; e++) {
-      if (l >= 2) same_in = same_in && same_bits(in[e], pin[e]);
-      pin[e] = in[e];
-    }
-    // an interior row with the inputs and the carried (D', DU) of its
-    // predecessor repeats it: nothing to compute or store
-    if (cont && same_in) {
-      if (!COMPRESS) put(l, rv);
-      continue;
-    }
-    // :794-801 and :809-811
-    const double vavgL = 0.5 * (in[0] + in[1]);
-    const double kavgL = 0.5 * (in[3] + in[4]);
-    const double dsL = in[6] / vavgL;
-    const double kdsL = kavgL * dsL;
-    const double vavgR = 0.5 * (in[1] + in[2]);
-    const double kavgR = 0.5 * (in[4] + in[5]);
-    const double dsR = in[7] / vavgR;
-    const double kdsR = kavgR * dsR;
-    const double Lf = dt * kdsL * in[6] / in[1];
-    const double Rf = dt * kdsR * in[7] / in[1];
-    const double Cf = Lf + Rf;
-    double D, DU = 0.0;
-    if (l == 0) {
-      D = 1.0 + imp * Cf - imp * Lf;
-      DU = -(imp * Rf);
-    } else {
-      D = 1.0 + imp * Cf;
-      DU = -(imp * Rf);
-    }
-    double fact = 0.0, Dp = D;
-    if (l > 0) {
-      const double DL = -(imp * Lf);  // DL_d(l-1)
-      if (!(fabs(dp_prev) >= fabs(DL)) || dp_prev == 0.0) raise_error(sc, A3G_ERR_PIVOT, l + 1);
-      fact = DL / dp_prev;
-      Dp = D - fact * du_prev;
-    }
-    const double v[CN_NF] = {fact, Dp, DU, (1.0 - imp) * Lf, 1.0 - (1.0 - imp) * Cf, (1.0 - imp) * Rf,
-                             1.0 / Dp};
-    bool same = l >= 1;
-#pragma unroll
-    for (int f = 0; f < CN_NF; f++) same = same && same_bits(v[f], rv[f]);
-    cont = same;
-    dp_prev = Dp;
-    du_prev = DU;
-    if (same) {
-      if (!COMPRESS) put(l, rv);
-      continue;
-    }
-    if (COMPRESS)
-      for (int m = s + 1; m < l; m++) put(m, rv);  // materialise the finished run
-    put(l, v);
-#pragma unroll
-    for (int f = 0; f < CN_NF; f++) rv[f] = v[f];
-    s = l;
+  if (tid == 0) sBrk = map.ds ? 0 : 1;
+  if (tid < LPB) {
+    sRun[tid] = n;  // first row of the final run, once known
+    sBad[tid] = 0;
   }
-  // last row (always distinct: DU = 0); the run ending at ncells-2 stays unstored
-  {
-    const int l = ncells - 1;
-    const int c = rmin + l;
-    const double vavgL = 0.5 * (G(kap, c - 1) + G(kap, c));
-    const double kavgL = 0.5 * (G(kk, c - 1) + G(kk, c));
-    const double dsL = G(sig, c) / vavgL;
-    const double kdsL = kavgL * dsL;
-    const double vavgR = 0.5 * (G(kap, c) + G(kap, c + 1));
-    const double kavgR = 0.5 * (G(kk, c) + G(kk, c + 1));
-    const double dsR = G(sig, c + 1) / vavgR;
-    const double kdsR = kavgR * dsR;
-    const double Lf = dt * kdsL * G(sig, c) / G(kap, c);
-    const double Rf = dt * kdsR * G(sig, c + 1) / G(kap, c);
-    const double Cf = Lf + Rf;
-    const double D = 1.0 + imp * Cf - imp * Rf;
-    const double DL = -(imp * Lf);
-    if (!(fabs(dp_prev) >= fabs(DL)) || dp_prev == 0.0) raise_error(sc, A3G_ERR_PIVOT, l + 1);
-    const double fact = DL / dp_prev;
-    const double Dp = D - fact * du_prev;
-    if (Dp == 0.0) raise_error(sc, A3G_ERR_PIVOT, ncells);
-    const double v[CN_NF] = {fact, Dp, 0.0, (1.0 - imp) * Lf, 1.0 - (1.0 - imp) * Cf, (1.0 - imp) * Rf,
-                             1.0 / Dp};
-    put(l, v);
-    double *runs = tab + CN_NF * F;
-    runs[u] = (double)s;
-    runs[U + u] = (double)(ncells - 2);
+  __syncthreads();
+  if (map.ds) {  // the last interior row whose inputs differ from its predecessor's, over the block's lines
+    int last = 1;
+    if (LPB > 1) {
+      last = n;
+    } else {
+      for (int l = n - 2 - tid; l >= 2 && last == 1; l -= 256) {
+        const int c = rmin + l;
+        bool same = true;
+        for (int d = -1; d <= 1; d++)
+          same = same && same_bits(G(kap, u0, c + d), G(kap, u0, c + d - 1)) &&
+                 same_bits(G(kk, u0, c + d), G(kk, u0, c + d - 1)) &&
+                 (d < 0 || same_bits(G(sig, u0, c + d), G(sig, u0, c + d - 1)));
+        if (!same) last = l;
+      }
+    }
+    atomicMax(&sBrk, last);
+    __syncthreads();
+  }
+  const int brk = sBrk;
+  double dp = 0.0, du = 0.0, fa = 0.0;  // of the row before (the serial lanes)
+  for (int b0 = 0; b0 < n; b0 += TR) {
+    const int cnt = min(TR, n - b0);
+    // ---- coefficients (:794-811) ----
+    for (int e = tid; e < cnt * LPB; e += 256) {
+      const int ln = e % LPB, l = b0 + e / LPB, u = u0 + ln;
+      if (u >= U || (l > sRun[ln] && l < n - 1 && COMPRESS)) continue;
+      const int c = rmin + l;
+      const double k0 = G(kap, u, c - 1), k1 = G(kap, u, c), k2 = G(kap, u, c + 1);
+      const double sl = G(sig, u, c), sr = G(sig, u, c + 1);
+      const double vavgL = 0.5 * (k0 + k1);
+      const double kavgL = 0.5 * (G(kk, u, c - 1) + G(kk, u, c));
+      const double dsL = sl / vavgL;
+      const double kdsL = kavgL * dsL;
+      const double vavgR = 0.5 * (k1 + k2);
+      const double kavgR = 0.5 * (G(kk, u, c) + G(kk, u, c + 1));
+      const double dsR = sr / vavgR;
+      const double kdsR = kavgR * dsR;
+      const double Lf = dt * kdsL * sl / k1;
+      const double Rf = dt * kdsR * sr / k1;
+      const double Cf = Lf + Rf;
+      double D = 1.0 + imp * Cf;
+      if (l == n - 1) D = D - imp * Rf;
+      else if (l == 0) D = D - imp * Lf;
+      const double DU = l == n - 1 ? 0.0 : -(imp * Rf);
+      sD[e] = D;
+      sDL[e] = -(imp * Lf);  // DL_d(l-1)
+      sDU[e] = DU;
+      put(u, l, CN_CL, (1.0 - imp) * Lf);
+      put(u, l, CN_CC, 1.0 - (1.0 - imp) * Cf);
+      put(u, l, CN_CR, (1.0 - imp) * Rf);
+      put(u, l, CN_DU, DU);
+    }
+    __syncthreads();
+    // ---- elimination ----
+    if (tid < LPB) {
+      cF[tid] = fa;
+      cP[tid] = dp;
+      if (u0 + tid < U) {
+        int l = b0;
+        if (sRun[tid] < n) l = max(l, n - 1);  // in the final run: only the last row is left
+        for (; l < b0 + cnt; l++) {
+          const int e = (l - b0) * LPB + tid;
+          double f = 0.0, p = sD[e];
+          if (l > 0) {
+            f = div_rn(sDL[e], dp);
+            p = p - f * du;
+          }
+          sF[e] = f;
+          sP[e] = p;
+          // (fact, D') repeat and so do all later inputs: the run that ends at row n-2
+          if (l > brk && l < n - 2 && same_bits(p, dp) && same_bits(f, fa) && same_bits(sDU[e], du)) {
+            sRun[tid] = l - 1;
+            l = n - 2;  // the loop's next row is the last one, in this tile or a later one
+          }
+          dp = p;
+          fa = f;
+          if (l < n - 1) du = sDU[e];
+        }
+      }
+    }
+    __syncthreads();
+    // ---- pivots and their reciprocals ----
+    for (int e = tid; e < cnt * LPB; e += 256) {
+      const int ln = e % LPB, l = b0 + e / LPB, u = u0 + ln;
+      if (u >= U) continue;
+      const int s = sRun[ln];
+      const bool in_run = l > s && l < n - 1;
+      if (in_run && COMPRESS) continue;
+      // the values of row s stand for the run's; its row is in this tile or was the carry
+      const int es = (s - b0) * LPB + ln;
+      const double f = !in_run ? sF[e] : s >= b0 ? sF[es] : cF[ln];
+      const double p = !in_run ? sP[e] : s >= b0 ? sP[es] : cP[ln];
+      const double pm = l == 0 ? 1.0 : (l - 1 > s && l - 1 < n - 1) || l == b0
+                                           ? (l - 1 > s && s >= b0 ? sP[es] : cP[ln])
+                                           : sP[e - LPB];
+      if (l > 0 && (!(fabs(pm) >= fabs(sDL[e])) || pm == 0.0)) raise_error(sc, A3G_ERR_PIVOT, l + 1);
+      if (l == n - 1 && p == 0.0) raise_error(sc, A3G_ERR_PIVOT, n);
+      const double zh = 1.0 / p;
+      put(u, l, CN_FACT, f);
+      put(u, l, CN_ZH, zh);
+      if (byrow) {
+        const double r = fma(-p, zh, 1.0);
+        const double zl = r / p;
+        put(u, l, CN_ZL, zl);
+        put(u, l, CN_ZLL, fma(-p, zl, r) / p);
+        tab[CN_ROW * F + (long)u * n + l] = p;
+      } else {
+        put(u, l, CN_DP, p);
+      }
+      if (!div_rn_3_covers(p)) sBad[ln] = 1;
+    }
+    if (__syncthreads_and(tid >= LPB || u0 + tid >= U || sRun[tid] < n) && COMPRESS && b0 + TR < n - 1)
+      b0 = (n - 1) / TR * TR - TR;  // every line is in its final run: on to the last row's tile
+  }
+  if (tid < LPB && u0 + tid < U) {
+    double *runs = tab + (byrow ? CN_NF : CN_NFX) * F;
+    const int u = u0 + tid;
+    runs[u] = (double)min(sRun[tid], n - 2);
+    runs[U + u] = (double)(n - 2);
+    runs[2 * U + u] = (double)sBad[tid];
   }
 }
 // Solve of one line (a, b) of grain g from the table.  The eliminated
@@ -265,7 +335,7 @@ __global__ void k_cn_table(Layout L, Box box, double imp, LineMap map, Geo3 sig,
 template <int DIR>
 __device__ __forceinline__ void cn_line(const Layout &L, const Box &box, const LineMap &map,
                                         const double *__restrict__ cin, double *__restrict__ cout,
-                                        const double *__restrict__ tab,
+                                        const CnTab &tab,
                                         const int32_t *__restrict__ aloft, int a, int b, int g) {
   constexpr int PF = 4;
   const int n = (DIR == 0) ? L.nx : (DIR == 1) ? L.ny : L.nz;
@@ -293,14 +363,11 @@ __device__ __forceinline__ void cn_line(const Layout &L, const Box &box, const L
   }
   for (int c = 1; c < rmin; c++) x[(long)(c - 1) * st] = 0.0;
   for (int c = rmax + 1; c <= n; c++) x[(long)(c - 1) * st] = 0.0;
-  const long U = map.U;
-  const long F = (long)ncells * U;
   const long u = map.u(a, b);
-  const double *t = tab + u;
   CnRun R;
-  if (DIR == 0) cn_load_run(t, F, U, tab + CN_NF * F, u, R);
+  if (DIR == 0) cn_load_run(tab, u, R);
   auto co = [&](int f, int l) {  // the y and z tables are stored in full
-    return (DIR == 0) ? cn_coef(t, F, U, R, f, l) : t[f * F + (long)l * U];
+    return (DIR == 0) ? cn_coef(tab, u, R, f, l) : tab.at(f, l, u);
   };
   const double *qq = q + (long)(rmin - 1) * st;  // cell rmin
   double *xx = x + (long)(rmin - 1) * st;
@@ -332,7 +399,7 @@ __device__ __forceinline__ void cn_line(const Layout &L, const Box &box, const L
         const int lp = l - PF;  // refill this slot for the next round
         ring[p] = (lp >= 0) ? xx[(long)lp * st] : 0.0;
         const double num = (l == ncells - 1) ? b2 : b2 - co(CN_DU, l) * xn;
-        const double v = div_rn_rcp(num, co(CN_DP, l), co(CN_RDP, l));
+        const double v = div_rn_rcp(num, co(CN_DP, l), co(CN_ZH, l));
         xx[(long)l * st] = v;
         xn = v;
       }
@@ -347,7 +414,7 @@ __device__ __forceinline__ void cn_line(const Layout &L, const Box &box, const L
 template <int DIR, int GC>
 __device__ __forceinline__ void cn_line_gc(const Layout &L, const Box &box, const LineMap &map,
                                            const double *__restrict__ cin, double *__restrict__ cout,
-                                           const double *__restrict__ tab,
+                                           const CnTab &tab,
                                            const int32_t *__restrict__ aloft, int a, int b, int g0) {
   constexpr int PF = 4;
   const int n = (DIR == 1) ? L.ny : L.nz;
@@ -381,10 +448,8 @@ __device__ __forceinline__ void cn_line_gc(const Layout &L, const Box &box, cons
     }
   }
   if (!any) return;
-  const long U = map.U;
-  const long F = (long)ncells * U;
-  const double *t = tab + map.u(a, b);
-  auto co = [&](int f, int l) { return t[f * F + (long)l * U]; };
+  const long line = map.u(a, b);
+  auto co = [&](int f, int l) { return tab.at(f, l, line); };
   const long off = (long)(rmin - 1) * st;
   // forward elimination with the right-hand side built on the fly, :813-851
   double qm[GC], qc[GC], bp[GC];
@@ -423,7 +488,7 @@ __device__ __forceinline__ void cn_line_gc(const Layout &L, const Box &box, cons
       const int l = l0 - p;
       if (l >= 0) {
         const int lp = l - PF;
-        const double du = co(CN_DU, l), dp = co(CN_DP, l), rd = co(CN_RDP, l);
+        const double du = co(CN_DU, l), dp = co(CN_DP, l), rd = co(CN_ZH, l);
 #pragma unroll
         for (int u = 0; u < GC; u++) {
           const double b2 = ring[u][p];
@@ -442,7 +507,7 @@ template <int DIR, int GC>
 __device__ __forceinline__ void cn_solve_gc_thread(const Layout &L, const Box &box, const LineMap &map,
                                                    const double *__restrict__ cin,
                                                    double *__restrict__ cout,
-                                                   const double *__restrict__ tab,
+                                                   const CnTab &tab,
                                                    const int32_t *__restrict__ aloft) {
   const int na = L.nx;
   const int nb = (DIR == 2) ? L.ny : L.nz;
@@ -463,7 +528,7 @@ template <int DIR, int GC>
 __global__ void __launch_bounds__(128) k_cn_solve_gc(Layout L, Box box, LineMap map,
                                                      const double *__restrict__ cin,
                                                      double *__restrict__ cout,
-                                                     const double *__restrict__ tab,
+                                                     CnTab tab,
                                                      const int32_t *__restrict__ aloft) {
   cn_solve_gc_thread<DIR, GC>(L, box, map, cin, cout, tab, aloft);
 }
@@ -474,13 +539,13 @@ template <int GC>
 __global__ void __launch_bounds__(128, 12) k_cn_solve_gc_y(Layout L, Box box, LineMap map,
                                                            const double *__restrict__ cin,
                                                            double *__restrict__ cout,
-                                                           const double *__restrict__ tab,
+                                                           CnTab tab,
                                                            const int32_t *__restrict__ aloft) {
   cn_solve_gc_thread<1, GC>(L, box, map, cin, cout, tab, aloft);
 }
 
 template <int DIR, int GC>
-static void launch_cn_solve_gc(a3g_ctx *ctx, const LineMap &map, const double *tab) {
+static void launch_cn_solve_gc(a3g_ctx *ctx, const LineMap &map, const CnTab &tab) {
   const Layout &L = ctx->L;
   const long n = (long)map.na * map.nb * ((L.ns + GC - 1) / GC);
   const unsigned grid = (unsigned)((n + 127) / 128);
@@ -497,7 +562,7 @@ template <int DIR>
 __global__ void __launch_bounds__(128) k_cn_solve(Layout L, Box box, LineMap map,
                                                   const double *__restrict__ cin,
                                                   double *__restrict__ cout,
-                                                  const double *__restrict__ tab,
+                                                  CnTab tab,
                                                   const int32_t *__restrict__ aloft) {
   const int na = (DIR == 0) ? L.ny : L.nx;
   const int nb = (DIR == 2) ? L.ny : L.nz;
@@ -530,7 +595,7 @@ constexpr int XT_S = 35;  // tile row stride in doubles: 34 columns, odd stride
 __global__ void __launch_bounds__(128, 5) k_cn_solve_xt(Layout L, Box box, LineMap map,
                                                      const double *__restrict__ cin,
                                                      double *__restrict__ cout,
-                                                     const double *__restrict__ tab,
+                                                     CnTab tab,
                                                      const int32_t *__restrict__ aloft) {
   __shared__ double sh[XT_WARPS][32 * XT_S];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -561,12 +626,9 @@ __global__ void __launch_bounds__(128, 5) k_cn_solve_xt(Layout L, Box box, LineM
   double *x0 = cout + r0 * P + (rmin - 1);
   const double *qown = q0 + (long)lane * P;
   double *xown = x0 + (long)lane * P;
-  const long U = map.U;
-  const long F = (long)ncells * U;
   const long u = map.u(j, k);
-  const double *t = tab + u;
   CnRun R;
-  cn_load_run(t, F, U, tab + CN_NF * F, u, R);
+  cn_load_run(tab, u, R);
   double *tr = tile + lane * XT_S;  // this lane's row of the tile
   const int nch = (ncells + 31) >> 5;
 
@@ -596,7 +658,7 @@ __global__ void __launch_bounds__(128, 5) k_cn_solve_xt(Layout L, Box box, LineM
   for (int o = 16; o > 0; o >>= 1) lo_w = max(lo_w, __shfl_xor_sync(0xffffffffu, lo_w, o));
   auto fast_chunk = [&](int l0, int cnt) { return cnt == 32 && l0 > lo_w && l0 + 31 <= ncells - 2; };
   const double fCL = R.v[CN_CL], fCC = R.v[CN_CC], fCR = R.v[CN_CR], fFA = R.v[CN_FACT];
-  const double fDU = R.v[CN_DU], fDP = R.v[CN_DP], fRD = R.v[CN_RDP];
+  const double fDU = R.v[CN_DU], fDP = R.v[CN_DP], fRD = R.v[CN_ZH];
 
   // pass 1: forward elimination, checkpoints only (:813-851 and dgtsv)
   double qm = 0.0, qc = 0.0, bp = 0.0;
@@ -624,9 +686,9 @@ __global__ void __launch_bounds__(128, 5) k_cn_solve_xt(Layout L, Box box, LineM
     for (int c = 0; c < cnt; c++) {
       const int l = l0 + c;
       const double qp = (l + 1 < ncells) ? tr[c + 2] : qc;  // BC_right_t0 = q(rmax)
-      const double B = cn_coef(t, F, U, R, CN_CL, l) * qm + cn_coef(t, F, U, R, CN_CC, l) * qc +
-                       cn_coef(t, F, U, R, CN_CR, l) * qp;
-      bp = (l == 0) ? B : B - cn_coef(t, F, U, R, CN_FACT, l) * bp;
+      const double B = cn_coef(tab, u, R, CN_CL, l) * qm + cn_coef(tab, u, R, CN_CC, l) * qc +
+                       cn_coef(tab, u, R, CN_CR, l) * qp;
+      bp = (l == 0) ? B : B - cn_coef(tab, u, R, CN_FACT, l) * bp;
       qm = qc;
       qc = qp;
     }
@@ -664,9 +726,9 @@ __global__ void __launch_bounds__(128, 5) k_cn_solve_xt(Layout L, Box box, LineM
     for (int c = 0; c < cnt; c++) {
       const int l = l0 + c;
       const double qp = (l + 1 < ncells) ? tr[c + 2] : qc2;
-      const double B = cn_coef(t, F, U, R, CN_CL, l) * qm2 + cn_coef(t, F, U, R, CN_CC, l) * qc2 +
-                       cn_coef(t, F, U, R, CN_CR, l) * qp;
-      bq = (l == 0) ? B : B - cn_coef(t, F, U, R, CN_FACT, l) * bq;
+      const double B = cn_coef(tab, u, R, CN_CL, l) * qm2 + cn_coef(tab, u, R, CN_CC, l) * qc2 +
+                       cn_coef(tab, u, R, CN_CR, l) * qp;
+      bq = (l == 0) ? B : B - cn_coef(tab, u, R, CN_FACT, l) * bq;
       tr[c + 1] = bq;
       qm2 = qc2;
       qc2 = qp;
@@ -674,8 +736,8 @@ __global__ void __launch_bounds__(128, 5) k_cn_solve_xt(Layout L, Box box, LineM
     for (int c = cnt - 1; c >= 0; c--) {
       const int l = l0 + c;
       const double b2 = tr[c + 1];
-      const double num = (l == ncells - 1) ? b2 : b2 - cn_coef(t, F, U, R, CN_DU, l) * xn;
-      const double v = div_rn_rcp(num, cn_coef(t, F, U, R, CN_DP, l), cn_coef(t, F, U, R, CN_RDP, l));
+      const double num = (l == ncells - 1) ? b2 : b2 - cn_coef(tab, u, R, CN_DU, l) * xn;
+      const double v = div_rn_rcp(num, cn_coef(tab, u, R, CN_DP, l), cn_coef(tab, u, R, CN_ZH, l));
       tr[c + 1] = v;
       xn = v;
     }
@@ -691,45 +753,58 @@ __global__ void __launch_bounds__(128, 5) k_cn_solve_xt(Layout L, Box box, LineM
 }
 
 // ---------------------------------------------------------------------------
-// x lines, warp-tiled, with TMA tiles.  The walk of k_cn_solve_xt (a warp
-// owns 32 consecutive x rows, chunks of 32 cells, checkpoints of B' in pass
-// 1, recompute and back substitution in pass 2; the same operations and the
-// same bits), but each chunk's tile arrives by one tensor load of 36 cells x
-// 32 rows (the rows of a level are a 2-D array of pitch P) into a dense
-// staging buffer, one chunk ahead: the lanes copy it into the odd-stride
-// tile (conflict-free per-lane rows), and the next chunk's load then runs
-// while they work through the current one.  The load starts on the even
-// cell at or before the chunk's left neighbour (the 16-byte rule for the
-// innermost coordinate); cells outside the level read as zero.
-// Chunks are loaded in the order the two passes use them (0 .. nch-1, then
-// nch-2 .. 0): the last chunk of pass 1 is still in the tile for pass 2.
+// The tiled solves through TMA (x, y and z).  Each lane runs one line:
+//   forward  B' = (CL*q(l-1) + CC*q(l) + CR*q(l+1)) - FACT*B'(l-1)
+//   backward x(l) = (B' - DU*x(l+1)) / D'
+// in cn_line's operations (row 0 has FACT = 0 and the last row DU = 0, so that
+// the end rows need no tests).  The division is the three dependent
+// operations of div_rn_3: a batch of rows runs without a branch, and the rare
+// batch with a dividend outside its range (a diffused tail below 2^-900) or a
+// pivot it does not cover is done again with the division operator.
 // ---------------------------------------------------------------------------
 constexpr int ZT_BAR_BYTES = 128;  // barriers ahead of the tiles (keeps tiles 128-byte aligned)
-constexpr int XT2_WARPS = 2;
-constexpr int XT2_DENSE = 32 * XT2_COLS;             // doubles of the staging buffer
-constexpr int XT2_WARP_D = XT2_DENSE + 32 * XT_S;    // staging buffer + tile
-static_assert((XT2_DENSE * 8) % 128 == 0 && (XT2_WARP_D * 8) % 128 == 0, "128-byte aligned buffers");
 
-__global__ void __launch_bounds__(32 * XT2_WARPS) k_cn_solve_xt2(const __grid_constant__ CUtensorMap trow,
-                                                                Layout L, Box box, LineMap map,
-                                                                const double *__restrict__ cin,
-                                                                double *__restrict__ cout,
-                                                                const double *__restrict__ tab,
-                                                                const int32_t *__restrict__ aloft,
-                                                                DevScalars *sc) {
-  extern __shared__ __align__(128) unsigned char x2_smem[];
+// x lines.  A warp owns 32 consecutive rows (row r = (g*nz + k-1)*ny + j-1 at
+// r*P), a row per lane, and walks them in chunks of CX_CH cells that arrive
+// and leave by tensor copies in the 128-byte swizzle (the lanes' 16-byte
+// accesses of their own rows meet no bank twice), three buffers turning.
+// Positions count cells from the even cell at or before the box's first one
+// (the 16-byte rule).
+//   pass 1 (forward): the elimination over the row, keeping only B' of every
+//     chunk's first cell, parked in the output where the chunk will go (the
+//     32 lanes' values side by side in its first two rows; the last chunk's
+//     stays in a register);
+//   pass 2 (backward, last chunk first): the chunk's other B' again from the
+//     parked one, read a chunk ahead (same operations, same bits), back
+//     substitution in place, and the chunk's store.
+// Chunks are loaded 0 .. nch-1, then nch-2 .. 0: the last one of pass 1 is
+// still in its buffer for pass 2.  Chunks inside every lane's constant run
+// take their coefficients from registers.
+//
+// Bound by the latency of the two recurrences at 16 warps per SM (registers),
+// with 24 B per cell of traffic at 4.5 TB/s.  720x360x60, 10 grains: 1.27 ->
+// 0.82 ms, 317x211x53, 7 grains: 275 -> 180 us, against dense tiles that the
+// lanes copied into an odd-stride one and certified quotients (96 warp
+// instructions a cell against 55).  Issuing loads two chunks ahead instead of
+// one changed nothing; parking the values a sector each per row cost 1.33 ms.
+constexpr int CXT_WARPS = 2;
+constexpr int CXT_BUF = 32 * CX_CH * 8;
+constexpr int CXT_SMEM = 1024 + 1024 + CXT_WARPS * 3 * CXT_BUF;  // room to align, barriers, buffers
+
+__global__ void __launch_bounds__(32 * CXT_WARPS, 8) k_cn_solve_xt2(const __grid_constant__ CUtensorMap tin,
+                                                                   const __grid_constant__ CUtensorMap tout,
+                                                                   Layout L, Box box, LineMap map,
+                                                                   double *__restrict__ cout, CnTab tab,
+                                                                   const int32_t *__restrict__ aloft,
+                                                                   DevScalars *sc) {
+  extern __shared__ unsigned char x2_smem[];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  uint64_t *bar = reinterpret_cast<uint64_t *>(x2_smem) + w;
-  double *dense = reinterpret_cast<double *>(x2_smem + ZT_BAR_BYTES) + (long)w * XT2_WARP_D;
-  double *tile = dense + XT2_DENSE;
+  unsigned char *const sm = x2_smem + ((1024u - (smem_u32(x2_smem) & 1023u)) & 1023u);  // the swizzle's period
+  uint64_t *bar = reinterpret_cast<uint64_t *>(sm) + 3 * w;
+  unsigned char *const bufs = sm + 1024 + w * 3 * CXT_BUF;
   const long nrows = (long)L.ny * L.nz * L.ns;
-  const long r0 = ((long)blockIdx.x * XT2_WARPS + w) * 32;
+  const long r0 = ((long)blockIdx.x * CXT_WARPS + w) * 32;
   if (r0 >= nrows) return;  // uniform over the warp
-  if (lane == 0) {
-    mbar_init(bar, 1);
-    mbar_init_fence();
-  }
-  __syncwarp();
   const long r = r0 + lane;
   const bool valid = r < nrows;
   const long rc = valid ? r : nrows - 1;
@@ -739,181 +814,238 @@ __global__ void __launch_bounds__(32 * XT2_WARPS) k_cn_solve_xt2(const __grid_co
   const int g = (int)(t1 / L.nz);
   const bool active =
       valid && j >= box.jmin && j <= box.jmax && k >= box.kmin && k <= box.kmax && aloft[g] != 0;
-  const unsigned amask = __ballot_sync(0xffffffffu, active);
-  const int nvalid = (int)((nrows - r0) < 32 ? (nrows - r0) : 32);
   const int rmin = box.imin, rmax = box.imax;
   const int ncells = rmax - rmin + 1;
   const long P = L.P;
-  if (valid) {  // cells outside [rmin, rmax] (FAST_SUBGRID box)
-    double *xr = cout + r * P;
-    for (int c = 1; c < rmin; c++) xr[c - 1] = 0.0;
-    for (int c = rmax + 1; c <= L.nx; c++) xr[c - 1] = 0.0;
+  const int xa = (rmin - 1) & ~1, off = (rmin - 1) - xa;  // 0-based cell of position 0; positions before the box
+  const int np = off + ncells, nch = (np + CX_CH - 1) / CX_CH;
+  const bool any = __any_sync(0xffffffffu, active);
+  {  // cells that no chunk store covers (outside the FAST_SUBGRID box): zeros
+    const int nr = (int)(nrows - r0 < 32 ? nrows - r0 : 32);
+    const int za = any ? xa : L.nx, zb = any ? xa + nch * CX_CH : L.nx;
+    if (za > 0 || zb < L.nx)
+      for (int row = 0; row < nr; row++) {
+        double *xr = cout + (r0 + row) * P;
+        for (int c = lane; c < za; c += 32) xr[c] = 0.0;
+        for (int c = zb + lane; c < L.nx; c += 32) xr[c] = 0.0;
+      }
   }
-  double *x0 = cout + r0 * P + (rmin - 1);
-  double *xown = x0 + (long)lane * P;
-  const long U = map.U;
-  const long F = (long)ncells * U;
+  if (!any) return;
+  if (lane == 0) {
+    mbar_init(&bar[0], 1);
+    mbar_init(&bar[1], 1);
+    mbar_init(&bar[2], 1);
+    mbar_init_fence();
+  }
+  __syncwarp();
+  const int nload = 2 * nch - 1;
+  auto issue = [&](int p) {  // load p, once its buffer's last store has been read
+    if (lane == 0 && p < nload) {
+      const int ch = p < nch ? p : 2 * nch - 2 - p;
+      bulk_wait_read0();
+      mbar_arrive_expect_tx(&bar[p % 3], CXT_BUF);
+      tma_load_2d(bufs + (p % 3) * CXT_BUF, &tin, &bar[p % 3], xa + ch * CX_CH, (int)r0);
+    }
+  };
+  issue(0);
+  issue(1);
+  // this lane's parking place of chunk ch: park[ch*CX_CH]
+  double *const park = cout + (r0 + (lane >> 4)) * P + xa + (lane & 15);
   const long u = map.u(j, k);
-  const double *t = tab + u;
   CnRun R;
-  cn_load_run(t, F, U, tab + CN_NF * F, u, R);
-  double *tr = tile + lane * XT_S;  // this lane's row of the tile
-  const int nch = (ncells + 31) >> 5;
-  const int nload = 2 * nch - 1;  // chunks 0 .. nch-1, then nch-2 .. 0
-  auto chunk_of = [&](int p) { return p < nch ? p : 2 * nch - 2 - p; };
-  // tile columns: 0 = cell l0-1, 1..32 = cells l0..l0+31, 33 = cell l0+32;
-  // cell l0-1 is line position l0-1, 0-based x = rmin + l0 - 2
-  auto issue = [&](int p) {
-    if (lane == 0) {
-      const int xa = rmin + (chunk_of(p) << 5) - 2;
-      mbar_arrive_expect_tx(bar, XT2_DENSE * 8);
-      tma_load_2d(dense, &trow, bar, xa & ~1, (int)r0);
-    }
-  };
-  uint32_t phase = 0u;
-  bool ok = true;
-  // waits for load p, copies it into the tile, then starts load p+1
-  auto next_tile = [&](int p) {
-    if (!mbar_wait(bar, phase)) {
-      ok = false;
-      return;
-    }
-    phase ^= 1u;
-    const int off = (rmin + (chunk_of(p) << 5) - 2) & 1;
-#pragma unroll 8
-    for (int row = 0; row < 32; row++) tile[row * XT_S + lane] = dense[row * XT2_COLS + off + lane];
-    tr[32] = dense[lane * XT2_COLS + off + 32];
-    tr[33] = dense[lane * XT2_COLS + off + 33];
-    __syncwarp();
-    if (p + 1 < nload) issue(p + 1);
-  };
-
+  cn_load_run(tab, u, R);
   int lo_w = R.lo;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) lo_w = max(lo_w, __shfl_xor_sync(0xffffffffu, lo_w, o));
-  auto fast_chunk = [&](int l0, int cnt) { return cnt == 32 && l0 > lo_w && l0 + 31 <= ncells - 2; };
   const double fCL = R.v[CN_CL], fCC = R.v[CN_CC], fCR = R.v[CN_CR], fFA = R.v[CN_FACT];
-  const double fDU = R.v[CN_DU], fDP = R.v[CN_DP], fRD = R.v[CN_RDP];
+  const double fDU = R.v[CN_DU], fDP = R.v[CN_DP], fZH = R.v[CN_ZH];
+  const double rz = fma(-fDP, fZH, 1.0), fZL = rz / fDP, fZLL = fma(-fDP, fZL, rz) / fDP;
+  const bool hard = !div_rn_3_covers(fDP);
+  auto co = [&](int f, int l) { return cn_coef(tab, u, R, f, l); };
+  // this lane's row of a buffer: positions 2e, 2e+1 at pair(e), position e at cell(e)
+  const int row_b = lane << 7, row_s = (lane & 7) << 4;
+  auto pair = [&](unsigned char *b, int e) { return reinterpret_cast<double2 *>(b + row_b + ((e << 4) ^ row_s)); };
+  auto cell = [&](unsigned char *b, int e) { return reinterpret_cast<double *>(pair(b, e >> 1)) + (e & 1); };
 
-  // pass 1: forward elimination, checkpoints only (:813-851 and dgtsv)
+  // pass 1
+  bool ok = true;
   double qm = 0.0, qc = 0.0, bp = 0.0;
-  issue(0);
   for (int ch = 0; ch < nch; ch++) {
-    const int l0 = ch << 5;
-    const int cnt = (ncells - l0) < 32 ? (ncells - l0) : 32;
-    next_tile(ch);
-    if (!ok) break;
-    if (ch == 0) {
-      qm = tr[1];  // BC_left_t0 = q(rmin)
-      qc = qm;
-    }
-    if (fast_chunk(l0, cnt)) {  // rows l0..l0+31 < ncells-1: qp always from the tile
-#pragma unroll 8
-      for (int c = 0; c < 32; c++) {
-        const double qp = tr[c + 2];
-        const double B = fCL * qm + fCC * qc + fCR * qp;
+    issue(ch + 2);
+    ok = mbar_wait(&bar[ch % 3], (ch / 3) & 1);
+    if (!ok || nch == 1) break;
+    unsigned char *const b = bufs + (ch % 3) * CXT_BUF;
+    const int l0 = ch * CX_CH - off;  // line row of position e: l0 + e; reading it finishes row l0 + e - 1
+    if (l0 - 1 > lo_w && l0 + CX_CH - 2 <= ncells - 2 && ch + 1 < nch) {
+      double q[CX_CH];
+#pragma unroll
+      for (int e = 0; e < CX_CH / 2; e++) {
+        const double2 x = *pair(b, e);
+        q[2 * e] = x.x;
+        q[2 * e + 1] = x.y;
+      }
+#pragma unroll
+      for (int e = 0; e < CX_CH; e++) {
+        const double B = fCL * qm + fCC * qc + fCR * q[e];
         bp = B - fFA * bp;
+        if (e == 1 && valid) park[ch * CX_CH] = bp;
         qm = qc;
-        qc = qp;
+        qc = q[e];
       }
     } else {
-      for (int c = 0; c < cnt; c++) {
-        const int l = l0 + c;
-        const double qp = (l + 1 < ncells) ? tr[c + 2] : qc;  // BC_right_t0 = q(rmax)
-        const double B = cn_coef(t, F, U, R, CN_CL, l) * qm + cn_coef(t, F, U, R, CN_CC, l) * qc +
-                         cn_coef(t, F, U, R, CN_CR, l) * qp;
-        bp = (l == 0) ? B : B - cn_coef(t, F, U, R, CN_FACT, l) * bp;
-        qm = qc;
-        qc = qp;
+      const int cnt = min(np - ch * CX_CH, ch + 1 < nch ? CX_CH : 2);  // of the last chunk: its first row
+#pragma unroll 2
+      for (int e = 0; e < cnt; e++) {
+        const int l = l0 + e;
+        if (l < 0) continue;
+        const double qv = *cell(b, e);
+        if (l == 0) {
+          qm = qv;  // BC_left_t0 = q(rmin)
+        } else {
+          const double B = co(CN_CL, l - 1) * qm + co(CN_CC, l - 1) * qc + co(CN_CR, l - 1) * qv;
+          bp = B - co(CN_FACT, l - 1) * bp;
+          if (e == 1 && valid && ch + 1 < nch) park[ch * CX_CH] = bp;
+          qm = qc;
+        }
+        qc = qv;
+      }
+      if (ch + 1 == nch && cnt == 1) {  // the last row is a chunk's first; BC_right_t0 = q(rmax)
+        const int l = ncells - 1;
+        const double B = co(CN_CL, l) * qm + co(CN_CC, l) * qc + co(CN_CR, l) * qc;
+        bp = B - co(CN_FACT, l) * bp;
       }
     }
-    if (valid && ch + 1 < nch) xown[l0 + 31] = bp;  // checkpoint B'(l0+31)
-    if (ch + 1 < nch) __syncwarp();  // the last chunk stays in the tile for pass 2
+    __syncwarp();
   }
+  fence_proxy_async_all();  // the parked values land before any store of this row's chunks
 
-  // pass 2: per chunk, last first: recompute B', back-substitute, store
-  double xn = 0.0;
+  // pass 2
+  double xn = 0.0, qn = 0.0;  // x and q of the row after the chunk
+  double ahead = bp;          // B' of the next chunk's first cell
   for (int ch = nch - 1; ch >= 0 && ok; ch--) {
-    const int l0 = ch << 5;
-    const int cnt = (ncells - l0) < 32 ? (ncells - l0) : 32;
+    const int p = 2 * nch - 2 - ch;
+    double bq = ahead;
+    ahead = (valid && ch > 1) ? park[(ch - 1) * CX_CH] : 0.0;
     if (ch != nch - 1) {
-      next_tile(2 * nch - 2 - ch);
+      ok = mbar_wait(&bar[p % 3], (p / 3) & 1);
       if (!ok) break;
     }
-    double bq = (valid && ch > 0) ? xown[l0 - 1] : 0.0;
-    double qm2 = (ch == 0) ? tr[1] : tr[0];
-    double qc2 = tr[1];
-    if (fast_chunk(l0, cnt)) {
-#pragma unroll 8
-      for (int c = 0; c < 32; c++) {
-        const double qp = tr[c + 2];
-        const double B = fCL * qm2 + fCC * qc2 + fCR * qp;
-        bq = B - fFA * bq;
-        tr[c + 1] = bq;
-        qm2 = qc2;
-        qc2 = qp;
+    unsigned char *const b = bufs + (p % 3) * CXT_BUF;
+    const int l0 = ch * CX_CH - off;
+    if (ch == 0) bq = 0.0;
+    if (ch > 0 && l0 > lo_w && l0 + CX_CH - 1 <= ncells - 2) {
+      double q[CX_CH + 1], y[CX_CH];
+#pragma unroll
+      for (int e = 0; e < CX_CH / 2; e++) {
+        const double2 x = *pair(b, e);
+        q[2 * e] = x.x;
+        q[2 * e + 1] = x.y;
       }
-#pragma unroll 8
-      for (int c = 31; c >= 0; c--) {
-        const double num = tr[c + 1] - fDU * xn;
-        const double v = div_rn_rcp(num, fDP, fRD);
-        tr[c + 1] = v;
-        xn = v;
+      q[CX_CH] = qn;
+      qn = q[0];
+      y[0] = bq;
+#pragma unroll
+      for (int e = 1; e < CX_CH; e++) {
+        const double B = fCL * q[e - 1] + fCC * q[e] + fCR * q[e + 1];
+        y[e] = B - fFA * y[e - 1];
+      }
+      if (ch != nch - 1) issue(p + 2);  // the store of the chunk before has had the time to be read
+      const double xs = xn;
+      bool bad = hard;
+#pragma unroll
+      for (int e = CX_CH - 1; e >= 0; e--) {
+        const double num = y[e] - fDU * xn;
+        bad = bad || !div_rn_3_takes(num);
+        xn = div_rn_3(num, fZH, fZL, fZLL);
+        q[e] = xn;
+      }
+      if (bad) {
+#pragma unroll
+        for (int e = 0; e < CX_CH; e++) *cell(b, e) = y[e];
+        xn = xs;
+        for (int e = CX_CH - 1; e >= 0; e--) {
+          double *T = cell(b, e);
+          xn = ieee_div(*T - fDU * xn, fDP);
+          *T = xn;
+        }
+      } else {
+#pragma unroll
+        for (int e = 0; e < CX_CH / 2; e++) *pair(b, e) = make_double2(q[2 * e], q[2 * e + 1]);
       }
     } else {
-      for (int c = 0; c < cnt; c++) {
-        const int l = l0 + c;
-        const double qp = (l + 1 < ncells) ? tr[c + 2] : qc2;
-        const double B = cn_coef(t, F, U, R, CN_CL, l) * qm2 + cn_coef(t, F, U, R, CN_CC, l) * qc2 +
-                         cn_coef(t, F, U, R, CN_CR, l) * qp;
-        bq = (l == 0) ? B : B - cn_coef(t, F, U, R, CN_FACT, l) * bq;
-        tr[c + 1] = bq;
-        qm2 = qc2;
-        qc2 = qp;
+      const int cnt = min(np - ch * CX_CH, CX_CH);
+      double pm = 0.0, first = 0.0;
+      for (int e = 0; e < CX_CH; e++) {
+        const int l = l0 + e;
+        double *T = cell(b, e);
+        if (l < 0 || e >= cnt) {  // outside the box
+          *T = 0.0;
+          continue;
+        }
+        const double qv = *T;
+        const double qp = l + 1 < ncells ? (e + 1 < CX_CH ? *cell(b, e + 1) : qn) : qv;  // BC_right_t0 = q(rmax)
+        if (e == 0) first = qv;
+        if (l == 0) pm = qv;  // BC_left_t0 = q(rmin)
+        if (e > 0 || ch == 0) {
+          const double B = co(CN_CL, l) * pm + co(CN_CC, l) * qv + co(CN_CR, l) * qp;
+          bq = B - co(CN_FACT, l) * bq;
+        }
+        *T = bq;
+        pm = qv;
       }
-      for (int c = cnt - 1; c >= 0; c--) {
-        const int l = l0 + c;
-        const double b2 = tr[c + 1];
-        const double num = (l == ncells - 1) ? b2 : b2 - cn_coef(t, F, U, R, CN_DU, l) * xn;
-        const double v = div_rn_rcp(num, cn_coef(t, F, U, R, CN_DP, l), cn_coef(t, F, U, R, CN_RDP, l));
-        tr[c + 1] = v;
-        xn = v;
+      qn = first;
+      if (ch != nch - 1) issue(p + 2);
+#pragma unroll 2
+      for (int e = cnt - 1; e >= 0; e--) {
+        const int l = l0 + e;
+        if (l < 0) break;
+        double *T = cell(b, e);
+        xn = div_rn_rcp(*T - co(CN_DU, l) * xn, co(CN_DP, l), co(CN_ZH, l));
+        *T = xn;
       }
     }
-    __syncwarp();
-#pragma unroll 8
-    for (int row = 0; row < 32; row++) {
-      if (row < nvalid && lane < cnt)
-        x0[(long)row * P + l0 + lane] = ((amask >> row) & 1u) ? tile[row * XT_S + 1 + lane] : 0.0;
+    if (!active) {  // the reference leaves zeros
+#pragma unroll
+      for (int e = 0; e < CX_CH / 2; e++) *pair(b, e) = make_double2(0.0, 0.0);
     }
+    fence_proxy_async_smem();
     __syncwarp();
+    if (lane == 0) {  // rows past the last one lie outside the tensor
+      tma_store_2d(&tout, b, xa + ch * CX_CH, (int)r0);
+      bulk_commit();
+    }
   }
-  if (!ok && lane == 0) raise_error(sc, A3G_ERR_TIMEOUT, 5);
+  if (lane == 0) {
+    if (!ok) raise_error(sc, A3G_ERR_TIMEOUT, 5);
+    bulk_wait0();
+  }
 }
 
-// ---------------------------------------------------------------------------
-// z lines through TMA column tiles.  A warp owns the 32 z lines of 32
-// consecutive i at one (j, grain): one tensor load brings the whole tile
-// (32 i x nz levels, tile[k][lane]) into shared memory, each lane runs its
-// line's elimination and back substitution in place (the same operations as
-// cn_line, so the same bits), and one tensor store writes the tile back.  The
-// level is read once and written once, with no B' round trip through global
-// memory, and the copies run asynchronously to the other warps' arithmetic.
-// The factor-table rows of the tile's line (the same for its 32 lines: the
-// coefficients do not vary along i) are staged in shared memory by the warp,
-// so the recurrences read only shared memory.  Warps are persistent and take
-// contiguous runs of tiles (neighbouring i, then j), which share table rows.
-// ---------------------------------------------------------------------------
+// z lines.  A warp owns the 32 z lines of 32 consecutive i at one (j, grain):
+// one tensor load brings the whole tile (32 i x nz levels, tile[k][lane]) into
+// shared memory, each lane runs its line's elimination and back substitution
+// in place, and one tensor store writes the tile back: the level is read once
+// and written once.  The table rows of the tile's line (the same for its 32
+// lines: the coefficients do not vary along i) come with the first tile that
+// needs them by one bulk copy.  Warps are persistent and take contiguous runs
+// of tiles (neighbouring i, then j), which share table rows.  Rows go in
+// batches of four whose operands are read before the batch's first store, so
+// that the reads do not wait on it.
+// Bound by the recurrences' latency at the 11 lines per lane that 227 KB of
+// shared memory hold for 60 levels.  480x401x50, 6 grains in a box: 148 -> 125
+// us; 317x211x53, 7 grains: 133 -> 104 us a solve (44 warp instructions a cell
+// against 60).
+constexpr int ZT_U = 4;
 
 // doubles of shared memory per warp: the tile and the staged table rows,
 // rounded up to 128 bytes so that every warp's tile stays aligned
 __host__ __device__ __forceinline__ long zt_warp_doubles(int nz) {
-  return (32L * nz + CN_NF * (long)nz + 15) / 16 * 16;
+  return (32L * nz + CN_ROW * (long)nz + 15) / 16 * 16;
 }
 
 __global__ void __launch_bounds__(64, 8) k_cn_solve_zt(const __grid_constant__ CUtensorMap tin,
                                                     const __grid_constant__ CUtensorMap tout, Layout L,
-                                                    Box box, LineMap map, const double *__restrict__ tab,
+                                                    Box box, LineMap map, CnTab tab,
                                                     const int32_t *__restrict__ aloft, DevScalars *sc,
                                                     int wpb) {
   extern __shared__ __align__(128) unsigned char zt_smem[];
@@ -921,7 +1053,7 @@ __global__ void __launch_bounds__(64, 8) k_cn_solve_zt(const __grid_constant__ C
   const int nz = L.nz;
   uint64_t *bar = reinterpret_cast<uint64_t *>(zt_smem) + wid;
   double *tile = reinterpret_cast<double *>(zt_smem + ZT_BAR_BYTES) + (long)wid * zt_warp_doubles(nz);
-  double *stab = tile + 32L * nz;  // staged table: field f, row l at stab[f*nz + l]
+  double *stab = tile + 32L * nz;  // staged rows, CN_ROW doubles each
   if (lane == 0) {
     mbar_init(bar, 1);
     mbar_init_fence();
@@ -937,12 +1069,11 @@ __global__ void __launch_bounds__(64, 8) k_cn_solve_zt(const __grid_constant__ C
   const long t1 = t0 + per < ntiles ? t0 + per : ntiles;
   const int rmin = box.kmin, rmax = box.kmax;
   const int ncells = rmax - rmin + 1;
-  const long U = map.U;
-  const long F = (long)ncells * U;
-  const uint32_t tile_bytes = 32u * (uint32_t)nz * 8u;
+  const uint32_t tile_bytes = 32u * (uint32_t)nz * 8u, tab_bytes = (uint32_t)ncells * CN_ROW * 8u;
   uint32_t phase = 0;
   int staged = -1;            // the line index u whose rows stab holds
-  double *col = tile + lane;  // this lane's line: level k (1-based) at col[(k-1)*32]
+  double *xx = tile + lane + (long)(rmin - 1) * 32;  // row l of this lane's line at xx[l*32]
+  const double2 *const row2 = reinterpret_cast<const double2 *>(stab);  // FACT,CL  CC,CR  DU,ZH  ZL,ZLL
   for (long t = t0; t < t1; t++) {
     const int it = (int)(t % nti);
     const long r = t / nti;
@@ -952,22 +1083,17 @@ __global__ void __launch_bounds__(64, 8) k_cn_solve_zt(const __grid_constant__ C
     const bool act = i <= L.nx && i >= box.imin && i <= box.imax && j >= box.jmin && j <= box.jmax &&
                      aloft[g] != 0;
     const bool any = __any_sync(0xffffffffu, act);
+    const int u = map.u(1, j);  // the coefficients do not vary along i (map.da == 0)
     // the previous tile's store must have read the buffer before it is refilled
     if (lane == 0) bulk_wait_read0();
     __syncwarp();
     if (any) {
       if (lane == 0) {
-        mbar_arrive_expect_tx(bar, tile_bytes);
+        mbar_arrive_expect_tx(bar, tile_bytes + (u != staged ? tab_bytes : 0u));
         tma_load_4d(tile, &tin, bar, it << 5, j - 1, 0, g);
+        if (u != staged) bulk_load(stab, tab.p + (long)CN_ROW * u * ncells, tab_bytes, bar);
       }
-      const int u = map.u(1, j);  // the coefficients do not vary along i (map.da == 0)
-      if (u != staged) {          // stage the rows while the tile is in flight
-        const double *tl = tab + u;
-        for (int l = lane; l < ncells; l += 32)
-#pragma unroll
-          for (int f = 0; f < CN_NF; f++) stab[f * nz + l] = tl[f * F + (long)l * U];
-        staged = u;
-      }
+      staged = u;
       if (!mbar_wait(bar, phase)) {
         if (lane == 0) {
           raise_error(sc, A3G_ERR_TIMEOUT, 2);
@@ -979,52 +1105,80 @@ __global__ void __launch_bounds__(64, 8) k_cn_solve_zt(const __grid_constant__ C
       __syncwarp();
     }
     if (act) {
-      auto co = [&](int f, int l) { return stab[f * nz + l]; };
-      double *xx = col + (long)(rmin - 1) * 32;  // row l at xx[l*32]
-      // forward elimination with the right-hand side built on the fly, :813-851
-      // (ncells >= 2: a single-row line is skipped before the launch; the
-      // first and last rows are taken out of the loops, which then need no
-      // per-row boundary tests)
-      double qm = xx[0];  // BC_left_t0 = q(rmin)
-      double qc = qm;
-      double bp;
-      {
-        const double qp = xx[32];
-        bp = co(CN_CL, 0) * qm + co(CN_CC, 0) * qc + co(CN_CR, 0) * qp;
-        xx[0] = bp;
-        qm = qc;
-        qc = qp;
+      double qm = xx[0], qc = qm, bp = 0.0;  // BC_left_t0 = q(rmin)
+      int l = 0;
+      for (; l + ZT_U < ncells; l += ZT_U) {
+        double q[ZT_U];
+        double2 a[ZT_U], b[ZT_U];
+#pragma unroll
+        for (int e = 0; e < ZT_U; e++) {
+          q[e] = xx[(l + 1 + e) * 32];
+          a[e] = row2[(l + e) * 4];
+          b[e] = row2[(l + e) * 4 + 1];
+        }
+#pragma unroll
+        for (int e = 0; e < ZT_U; e++) {
+          const double B = a[e].y * qm + b[e].x * qc + b[e].y * q[e];
+          bp = B - a[e].x * bp;
+          xx[(l + e) * 32] = bp;
+          qm = qc;
+          qc = q[e];
+        }
       }
-#pragma unroll 4
-      for (int l = 1; l < ncells - 1; l++) {
-        const double qp = xx[(l + 1) * 32];
-        const double B = co(CN_CL, l) * qm + co(CN_CC, l) * qc + co(CN_CR, l) * qp;
-        bp = B - co(CN_FACT, l) * bp;
+      for (; l < ncells; l++) {
+        const double qp = l + 1 < ncells ? xx[(l + 1) * 32] : qc;  // BC_right_t0 = q(rmax)
+        const double2 a = row2[l * 4], b = row2[l * 4 + 1];
+        const double B = a.y * qm + b.x * qc + b.y * qp;
+        bp = B - a.x * bp;
         xx[l * 32] = bp;
         qm = qc;
         qc = qp;
-      }
-      {
-        const int l = ncells - 1;
-        const double qp = qc;  // BC_right_t0 = q(rmax)
-        const double B = co(CN_CL, l) * qm + co(CN_CC, l) * qc + co(CN_CR, l) * qp;
-        bp = B - co(CN_FACT, l) * bp;
-        xx[l * 32] = bp;
       }
       // back substitution
-      double xn = div_rn_rcp(xx[(ncells - 1) * 32], co(CN_DP, ncells - 1), co(CN_RDP, ncells - 1));
-      xx[(ncells - 1) * 32] = xn;
-#pragma unroll 4
-      for (int l = ncells - 2; l >= 0; l--) {
-        const double num = xx[l * 32] - co(CN_DU, l) * xn;
-        const double v = div_rn_rcp(num, co(CN_DP, l), co(CN_RDP, l));
-        xx[l * 32] = v;
-        xn = v;
+      const bool hard = tab.runs()[2 * tab.U + u] != 0.0;
+      double xn = 0.0;
+      int top = ncells;  // rows below are to do
+      for (; top >= ZT_U; top -= ZT_U) {
+        double y[ZT_U], x[ZT_U];
+        double2 a[ZT_U], b[ZT_U];
+#pragma unroll
+        for (int e = 0; e < ZT_U; e++) {
+          y[e] = xx[(top - 1 - e) * 32];
+          a[e] = row2[(top - 1 - e) * 4 + 2];
+          b[e] = row2[(top - 1 - e) * 4 + 3];
+        }
+        const double xs = xn;
+        bool bad = hard;
+#pragma unroll
+        for (int e = 0; e < ZT_U; e++) {
+          const double num = y[e] - a[e].x * xn;
+          bad = bad || !div_rn_3_takes(num);
+          xn = div_rn_3(num, a[e].y, b[e].x, b[e].y);
+          x[e] = xn;
+        }
+        if (bad) {
+          xn = xs;
+          for (int e = 0; e < ZT_U; e++) {
+            const int m = top - 1 - e;
+            xn = ieee_div(xx[m * 32] - row2[m * 4 + 2].x * xn, tab.at(CN_DP, m, u));
+            xx[m * 32] = xn;
+          }
+        } else {
+#pragma unroll
+          for (int e = 0; e < ZT_U; e++) xx[(top - 1 - e) * 32] = x[e];
+        }
       }
-      for (int k = 1; k < rmin; k++) col[(k - 1) * 32] = 0.0;  // outside the box
-      for (int k = rmax + 1; k <= nz; k++) col[(k - 1) * 32] = 0.0;
+      for (int m = top - 1; m >= 0; m--) {
+        const double2 a = row2[m * 4 + 2], b = row2[m * 4 + 3];
+        const double num = xx[m * 32] - a.x * xn;
+        xn = div_rn_3(num, a.y, b.x, b.y);
+        if (hard || !div_rn_3_takes(num)) xn = ieee_div(num, tab.at(CN_DP, m, u));
+        xx[m * 32] = xn;
+      }
+      for (int k = 1; k < rmin; k++) tile[(k - 1) * 32 + lane] = 0.0;  // outside the box
+      for (int k = rmax + 1; k <= nz; k++) tile[(k - 1) * 32 + lane] = 0.0;
     } else {
-      for (int k = 1; k <= nz; k++) col[(k - 1) * 32] = 0.0;  // the reference leaves zeros
+      for (int k = 1; k <= nz; k++) tile[(k - 1) * 32 + lane] = 0.0;  // the reference leaves zeros
     }
     fence_proxy_async_smem();
     __syncwarp();
@@ -1036,42 +1190,31 @@ __global__ void __launch_bounds__(64, 8) k_cn_solve_zt(const __grid_constant__ C
   if (lane == 0) bulk_wait0();
 }
 
-// ---------------------------------------------------------------------------
-// y lines through TMA chunk tiles.  A warp owns the 32 y lines of 32
-// consecutive i at one (k, grain) and walks them in chunks of YT_CH cells;
-// each chunk arrives by one tensor load as a tile of YT_CH + 2 rows (the
-// cell before the chunk and the cell after it included; row r holds line
-// position l0 - 1 + r), tile[r][lane].  Two buffers per warp: the next
-// chunk's load is in flight while the lanes work on the current one.
-//   pass 1 (forward): the elimination of B' over the whole line, keeping only
-//     B' at the last cell of every chunk (a checkpoint, parked in the output
-//     line at that cell, which the chunk's own store overwrites later);
-//   pass 2 (backward, last chunk first, which pass 1 left in its buffer):
-//     recompute the chunk's B' from the previous chunk's checkpoint (same
-//     operations, same bits), back-substitute in place, and store the chunk
-//     with one tensor store.
-// The arithmetic is cn_line's, operation for operation.  Each chunk's
-// factor-table rows (the same for the warp's 32 lines) are staged in shared
-// memory while its tile is in flight.  Warps take contiguous runs of line
-// groups (neighbouring i, then k), which share table rows.
-// ---------------------------------------------------------------------------
+// y lines.  A warp owns the 32 y lines of 32 consecutive i at one (k, grain)
+// and walks them as the x solve walks its rows: chunks of YT_CH cells,
+// tile[row][lane], with the chunk's table rows beside them (one bulk copy; the
+// same for the warp's 32 lines), three buffers turning; pass 1 parks B' of
+// every chunk's first row in the output line, pass 2 solves and stores chunk
+// by chunk from the last (the last chunk's B' stays in a register, the others
+// are read a chunk ahead).  Warps are persistent and take contiguous runs of
+// line groups (neighbouring i, then k), which share table rows.
+// Bound as the x solve; 720x360x60, 10 grains: 1.04 -> 0.91 ms, 93x131x37, 2
+// grains: 45 -> 29 us a solve.
+constexpr int YT_BUF_D = YT_CH * 32 + YT_CH * CN_ROW;  // doubles of a buffer: the tile, the table rows
 
-__global__ void __launch_bounds__(64, 10) k_cn_solve_yt(const __grid_constant__ CUtensorMap tin,
+__global__ void __launch_bounds__(64, 8) k_cn_solve_yt(const __grid_constant__ CUtensorMap tin,
                                                     const __grid_constant__ CUtensorMap tout, Layout L,
-                                                    Box box, LineMap map, double *__restrict__ cout,
-                                                    const double *__restrict__ tab,
+                                                    Box box, LineMap map, double *__restrict__ cout, CnTab tab,
                                                     const int32_t *__restrict__ aloft, DevScalars *sc,
                                                     int wpb) {
   extern __shared__ __align__(128) unsigned char yt_smem[];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  constexpr int BUF = 32 * YT_ROWS;  // doubles per buffer (a multiple of 16: 128-byte aligned buffers)
-  uint64_t *bar = reinterpret_cast<uint64_t *>(yt_smem) + 2 * wid;
-  double *wbase = reinterpret_cast<double *>(yt_smem + ZT_BAR_BYTES) + (long)wid * (2 * BUF + CN_NF * 32);
-  auto buf = [&](int bi) { return wbase + (bi ? BUF : 0); };
-  double *stab = wbase + 2 * BUF;  // staged table of the chunk: field f, row c at stab[f*32 + c]
+  uint64_t *bar = reinterpret_cast<uint64_t *>(yt_smem) + 3 * wid;
+  double *const bufs = reinterpret_cast<double *>(yt_smem + ZT_BAR_BYTES) + (long)wid * 3 * YT_BUF_D;
   if (lane == 0) {
     mbar_init(&bar[0], 1);
     mbar_init(&bar[1], 1);
+    mbar_init(&bar[2], 1);
     mbar_init_fence();
     prefetch_tensormap(&tin);
     prefetch_tensormap(&tout);
@@ -1085,11 +1228,9 @@ __global__ void __launch_bounds__(64, 10) k_cn_solve_yt(const __grid_constant__ 
   const long t1 = t0 + per < ngroups ? t0 + per : ngroups;
   const int rmin = box.jmin, rmax = box.jmax;
   const int ncells = rmax - rmin + 1;
-  const int nch = (ncells + YT_CH - 1) / YT_CH;
-  const long U = map.U;
-  const long F = (long)ncells * U;
-  const uint32_t tile_bytes = 32u * YT_ROWS * 8u;
-  uint32_t ph = 0u;  // bit b: the parity of buffer b's barrier
+  const int nch = (ncells + YT_CH - 1) / YT_CH, nload = 2 * nch - 1;
+  const int cnt_last = ncells - (nch - 1) * YT_CH;
+  uint32_t s0 = 0;  // loads of the groups before: load p of this one is the warp's load s0 + p
   for (long t = t0; t < t1; t++) {
     const int it = (int)(t % nti);
     const long r = t / nti;
@@ -1109,132 +1250,147 @@ __global__ void __launch_bounds__(64, 10) k_cn_solve_yt(const __grid_constant__ 
       for (int j = 1; j < rmin; j++) xg[(long)(j - 1) * L.P] = 0.0;
       for (int j = rmin + nch * YT_CH; j <= L.ny; j++) xg[(long)(j - 1) * L.P] = 0.0;
     }
-    auto issue = [&](int bi, int ch) {  // tensor load of chunk ch into buffer bi
-      if (lane == 0) {
-        bulk_wait_read0();  // a store from this buffer must have read it first
-        mbar_arrive_expect_tx(&bar[bi], tile_bytes);
-        tma_load_4d(buf(bi), &tin, &bar[bi], it << 5, rmin - 2 + ch * YT_CH, k - 1, g);
+    xg += (long)(rmin - 1) * L.P;  // row 0
+    const long u = map.u(1, k);    // the coefficients do not vary along i (map.da == 0)
+    auto buf = [&](int p) { return bufs + ((s0 + (uint32_t)p) % 3u) * YT_BUF_D; };
+    auto issue = [&](int p) {  // load p, once its buffer's last store has been read
+      if (lane == 0 && p < nload) {
+        const int ch = p < nch ? p : 2 * nch - 2 - p;
+        const uint32_t tb = (uint32_t)(ch + 1 < nch ? YT_CH : cnt_last) * CN_ROW * 8u;
+        uint64_t *b = &bar[(s0 + (uint32_t)p) % 3u];
+        bulk_wait_read0();
+        mbar_arrive_expect_tx(b, YT_CH * 32u * 8u + tb);
+        tma_load_4d(buf(p), &tin, b, it << 5, rmin - 1 + ch * YT_CH, k - 1, g);
+        bulk_load(buf(p) + YT_CH * 32, tab.p + CN_ROW * (u * ncells + (long)ch * YT_CH), tb, b);
       }
     };
+    auto wait = [&](int p) {
+      const uint32_t s = s0 + (uint32_t)p;
+      return mbar_wait(&bar[s % 3u], (s / 3u) & 1u);
+    };
+    issue(0);
+    issue(1);
+    // pass 1: forward elimination, B' of the chunks' first rows only
     bool ok = true;
-    auto wait = [&](int bi) {
-      ok = mbar_wait(&bar[bi], (ph >> bi) & 1u);
-      ph ^= 1u << bi;
-    };
-    const double *tl = tab + map.u(1, k);  // the coefficients do not vary along i (map.da == 0)
-    auto stage = [&](int l0, int nf) {      // fields 0..nf-1 of the chunk's rows into stab
-      const int l = l0 + lane;
-      if (lane < YT_CH && l < ncells)
-        for (int f = 0; f < nf; f++) stab[f * 32 + lane] = tl[f * F + (long)l * U];
-    };
-    auto co = [&](int f, int c) { return stab[f * 32 + c]; };
-    // pass 1: forward elimination, checkpoints only (:813-851 and dgtsv)
     double qm = 0.0, qc = 0.0, bp = 0.0;
-    issue(0, 0);
-    for (int ch = 0; ch < nch && ok; ch++) {
-      const int bi = ch & 1;
-      if (ch + 1 < nch) issue(bi ^ 1, ch + 1);
-      const int l0 = ch * YT_CH;
-      stage(l0, CN_CR + 1);  // FACT, DP, DU, CL, CC, CR
-      wait(bi);
-      if (!ok) break;
-      __syncwarp();
-      const double *T = buf(bi) + lane;
-      const int cnt = (ncells - l0) < YT_CH ? (ncells - l0) : YT_CH;
-      if (act) {
-        if (ch == 0) {
-          qm = T[32];  // BC_left_t0 = q(rmin)
-          qc = qm;
-        }
-        if (ch > 0 && l0 + YT_CH <= ncells - 1) {  // interior chunk: rows 1 .. ncells-2 only
+    double2 ca = make_double2(0.0, 0.0), cb = ca;  // FACT,CL and CC,CR of the chunk before's last row
+    for (int ch = 0; ch < nch; ch++) {
+      issue(ch + 2);
+      ok = wait(ch);
+      if (!ok || nch == 1) break;
+      const double *T = buf(ch) + lane;
+      const double2 *row2 = reinterpret_cast<const double2 *>(buf(ch) + YT_CH * 32);
+      auto row = [&](double2 a, double2 b, double qp) {  // the next row of the elimination
+        const double B = a.y * qm + b.x * qc + b.y * qp;
+        bp = B - a.x * bp;
+        qm = qc;
+        qc = qp;
+      };
+      if (ch == 0) {
+        qm = T[0];  // BC_left_t0 = q(rmin)
+        qc = qm;
+      } else {
+        row(ca, cb, T[0]);
+      }
+      if (ch + 1 < nch) {
+        double q[YT_CH];
 #pragma unroll
-          for (int c = 0; c < YT_CH; c++) {
-            const double qp = T[(c + 2) * 32];
-            const double B = co(CN_CL, c) * qm + co(CN_CC, c) * qc + co(CN_CR, c) * qp;
-            bp = B - co(CN_FACT, c) * bp;
-            qm = qc;
-            qc = qp;
-          }
-        } else {
-#pragma unroll 4
-          for (int c = 0; c < cnt; c++) {
-            const int l = l0 + c;
-            const double qp = (l + 1 < ncells) ? T[(c + 2) * 32] : qc;  // BC_right_t0 = q(rmax)
-            const double B = co(CN_CL, c) * qm + co(CN_CC, c) * qc + co(CN_CR, c) * qp;
-            bp = (l == 0) ? B : B - co(CN_FACT, c) * bp;
-            qm = qc;
-            qc = qp;
-          }
+        for (int e = 1; e < YT_CH; e++) q[e] = T[e * 32];
+#pragma unroll
+        for (int e = 1; e < YT_CH; e++) {
+          row(row2[(e - 1) * 4], row2[(e - 1) * 4 + 1], q[e]);
+          if (e == 1 && act) xg[(long)(ch * YT_CH) * L.P] = bp;
         }
-        if (ch + 1 < nch) xg[(long)(rmin + l0 + YT_CH - 2) * L.P] = bp;  // checkpoint B'(l0+YT_CH-1)
+        ca = row2[(YT_CH - 1) * 4];
+        cb = row2[(YT_CH - 1) * 4 + 1];
+      } else {  // of the last chunk: its first row; BC_right_t0 = q(rmax)
+        row(row2[0], row2[1], cnt_last > 1 ? T[32] : qc);
       }
       __syncwarp();
     }
-    fence_proxy_async_all();  // the checkpoints land before any store of this line's chunks
-    // pass 2: per chunk, last first: recompute B', back-substitute, store
-    double xn = 0.0;
+    fence_proxy_async_all();  // the parked values land before any store of this line's chunks
+    // pass 2
+    const bool hard = tab.runs()[2 * tab.U + u] != 0.0;
+    double xn = 0.0, qn = 0.0;  // x and q of the row after the chunk
+    double ahead = bp;          // B' of the next chunk's first row
     for (int ch = nch - 1; ch >= 0 && ok; ch--) {
-      const int bi = ch & 1;
-      if (ch - 1 >= 0) issue(bi ^ 1, ch - 1);
-      const int l0 = ch * YT_CH;
-      stage(l0, CN_NF);
+      const int p = 2 * nch - 2 - ch;
+      double b0 = ahead;
+      ahead = (act && ch > 1) ? xg[(long)((ch - 1) * YT_CH) * L.P] : 0.0;
       if (ch != nch - 1) {
-        wait(bi);
+        ok = wait(p);
         if (!ok) break;
       }
-      __syncwarp();
-      double *T = buf(bi) + lane;
-      const int cnt = (ncells - l0) < YT_CH ? (ncells - l0) : YT_CH;
-      if (act) {
-        double bq = ch > 0 ? xg[(long)(rmin + l0 - 2) * L.P] : 0.0;
-        double qm2 = (ch == 0) ? T[32] : T[0];
-        double qc2 = T[32];
-        if (ch > 0 && l0 + YT_CH <= ncells - 1) {  // interior chunk: rows 1 .. ncells-2 only
+      double *T = buf(p) + lane;
+      const double2 *row2 = reinterpret_cast<const double2 *>(buf(p) + YT_CH * 32);
+      const int cnt = ch + 1 < nch ? YT_CH : cnt_last;
+      const double q0 = T[0];
+      if (ch == 0) {
+        const double q1 = ncells > 1 ? T[32] : q0;
+        b0 = row2[0].y * q0 + row2[1].x * q0 + row2[1].y * q1;  // FACT = 0
+      }
+      if (cnt == YT_CH) {  // lanes outside the box run along: their tile is cleared below
+        double q[YT_CH + 1], y[YT_CH];
 #pragma unroll
-          for (int c = 0; c < YT_CH; c++) {
-            const double qp = T[(c + 2) * 32];
-            const double B = co(CN_CL, c) * qm2 + co(CN_CC, c) * qc2 + co(CN_CR, c) * qp;
-            bq = B - co(CN_FACT, c) * bq;
-            T[(c + 1) * 32] = bq;
-            qm2 = qc2;
-            qc2 = qp;
-          }
+        for (int e = 0; e < YT_CH; e++) q[e] = T[e * 32];
+        q[YT_CH] = ch + 1 < nch ? qn : q[YT_CH - 1];  // BC_right_t0 = q(rmax)
+        y[0] = b0;
 #pragma unroll
-          for (int c = YT_CH - 1; c >= 0; c--) {
-            const double num = T[(c + 1) * 32] - co(CN_DU, c) * xn;
-            const double v = div_rn_rcp(num, co(CN_DP, c), co(CN_RDP, c));
-            T[(c + 1) * 32] = v;
-            xn = v;
-          }
-        } else {
-#pragma unroll 4
-          for (int c = 0; c < cnt; c++) {
-            const int l = l0 + c;
-            const double qp = (l + 1 < ncells) ? T[(c + 2) * 32] : qc2;
-            const double B = co(CN_CL, c) * qm2 + co(CN_CC, c) * qc2 + co(CN_CR, c) * qp;
-            bq = (l == 0) ? B : B - co(CN_FACT, c) * bq;
-            T[(c + 1) * 32] = bq;
-            qm2 = qc2;
-            qc2 = qp;
-          }
-#pragma unroll 4
-          for (int c = cnt - 1; c >= 0; c--) {
-            const int l = l0 + c;
-            const double b2 = T[(c + 1) * 32];
-            const double num = (l == ncells - 1) ? b2 : b2 - co(CN_DU, c) * xn;
-            const double v = div_rn_rcp(num, co(CN_DP, c), co(CN_RDP, c));
-            T[(c + 1) * 32] = v;
-            xn = v;
+        for (int e = 1; e < YT_CH; e++) {
+          const double2 a = row2[e * 4], b = row2[e * 4 + 1];
+          const double B = a.y * q[e - 1] + b.x * q[e] + b.y * q[e + 1];
+          y[e] = B - a.x * y[e - 1];
+        }
+        if (ch != nch - 1) issue(p + 2);  // the store of the chunk before has had the time to be read
+        const double xs = xn;
+        bool bad = hard;
+#pragma unroll
+        for (int e = YT_CH - 1; e >= 0; e--) {
+          const double2 a = row2[e * 4 + 2], b = row2[e * 4 + 3];
+          const double num = y[e] - a.x * xn;
+          bad = bad || !div_rn_3_takes(num);
+          xn = div_rn_3(num, a.y, b.x, b.y);
+          T[e * 32] = xn;
+        }
+        if (bad && act) {
+#pragma unroll
+          for (int e = 0; e < YT_CH; e++) T[e * 32] = y[e];
+          xn = xs;
+          for (int e = YT_CH - 1; e >= 0; e--) {
+            xn = ieee_div(T[e * 32] - row2[e * 4 + 2].x * xn, tab.at(CN_DP, ch * YT_CH + e, u));
+            T[e * 32] = xn;
           }
         }
-        for (int c = cnt; c < YT_CH; c++) T[(c + 1) * 32] = 0.0;  // beyond rmax
-      } else {
-        for (int c = 0; c < YT_CH; c++) T[(c + 1) * 32] = 0.0;  // the reference leaves zeros
+      } else if (act) {
+        double pm = q0, bq = b0;
+        T[0] = b0;
+#pragma unroll 2
+        for (int e = 1; e < cnt; e++) {
+          const double qv = T[e * 32], qp = e + 1 < cnt ? T[(e + 1) * 32] : qv;  // BC_right_t0 = q(rmax)
+          const double2 a = row2[e * 4], b = row2[e * 4 + 1];
+          const double B = a.y * pm + b.x * qv + b.y * qp;
+          bq = B - a.x * bq;
+          T[e * 32] = bq;
+          pm = qv;
+        }
+#pragma unroll 2
+        for (int e = cnt - 1; e >= 0; e--) {
+          const double2 a = row2[e * 4 + 2], b = row2[e * 4 + 3];
+          const double num = T[e * 32] - a.x * xn;
+          xn = div_rn_3(num, a.y, b.x, b.y);
+          if (hard || !div_rn_3_takes(num)) xn = ieee_div(num, tab.at(CN_DP, ch * YT_CH + e, u));
+          T[e * 32] = xn;
+        }
+        for (int e = cnt; e < YT_CH; e++) T[e * 32] = 0.0;  // beyond rmax
+      }
+      qn = q0;
+      if (!act) {
+        for (int e = 0; e < YT_CH; e++) T[e * 32] = 0.0;  // the reference leaves zeros
       }
       fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) {
-        tma_store_4d(&tout, buf(bi) + 32, it << 5, rmin - 1 + l0, k - 1, g);
+        tma_store_4d(&tout, buf(p), it << 5, rmin - 1 + ch * YT_CH, k - 1, g);
         bulk_commit();
       }
     }
@@ -1245,6 +1401,7 @@ __global__ void __launch_bounds__(64, 10) k_cn_solve_yt(const __grid_constant__ 
       }
       return;
     }
+    s0 += (uint32_t)nload;
   }
   if (lane == 0) bulk_wait0();
 }
@@ -1297,8 +1454,9 @@ bool tensor_map(a3g_ctx *ctx, const double *p, int kind, CUtensorMap *out) {
   CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_NONE;
   if (kind == TM_XROWS) {
     rank = 2;
-    box[0] = XT2_COLS;
+    box[0] = CX_CH;
     box[1] = 32;
+    swizzle = CU_TENSOR_MAP_SWIZZLE_128B;
   } else if (kind == TM_QROWS || kind == TM_VROWS) {
     rank = 2;
     box[0] = 8;
@@ -1307,9 +1465,7 @@ bool tensor_map(a3g_ctx *ctx, const double *p, int kind, CUtensorMap *out) {
   } else if (kind == TM_COLUMN) {
     if (L.nz > 256) return false;
     box[2] = (cuuint32_t)L.nz;
-  } else if (kind == TM_YCHUNK_IN) {
-    box[1] = YT_ROWS;
-  } else if (kind == TM_YCHUNK_OUT) {
+  } else if (kind == TM_YCHUNK) {
     box[1] = YT_CH;
   } else if (kind == TM_ADV_QY || kind == TM_ADV_VY) {
     box[1] = ACH;
@@ -1340,9 +1496,24 @@ bool tensor_map(a3g_ctx *ctx, const double *p, int kind, CUtensorMap *out) {
   return true;
 }
 
+// Opts a tiled kernel in to the largest dynamic shared memory; `per_sm`: its
+// resident blocks per SM.
+template <typename K>
+static bool tile_kernel_setup(a3g_ctx *ctx, K kernel, int threads, size_t smem, int *per_sm, int *nsm) {
+  int optin = 0;
+  // the opt-in maximum, so that contexts of any extent can share the attribute
+  return cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device) == cudaSuccess &&
+         (size_t)optin >= smem &&
+         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, optin) == cudaSuccess &&
+         cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                              cudaSharedmemCarveoutMaxShared) == cudaSuccess &&
+         cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, kernel, threads, smem) == cudaSuccess &&
+         cudaDeviceGetAttribute(nsm, cudaDevAttrMultiProcessorCount, ctx->device) == cudaSuccess && *per_sm >= 1;
+}
+
 // Launches the z solve through column tiles; false when the shape is outside
 // what the tiles cover (the caller takes the per-thread kernel).
-static bool launch_cn_solve_zt(a3g_ctx *ctx, const LineMap &map, const double *tab) {
+static bool launch_cn_solve_zt(a3g_ctx *ctx, const LineMap &map, const CnTab &tab) {
   const Layout &L = ctx->L;
   if (L.nz > 256 || map.da) return false;
   CUtensorMap tin, tout;
@@ -1350,18 +1521,8 @@ static bool launch_cn_solve_zt(a3g_ctx *ctx, const LineMap &map, const double *t
   const int wpb = L.nz <= 128 ? 2 : 1;
   const size_t smem = ZT_BAR_BYTES + (size_t)wpb * zt_warp_doubles(L.nz) * sizeof(double);
   if (ctx->tma_grid[0] == 0) {
-    // the opt-in maximum, so that contexts of any nz can share the attribute
-    int optin = 0;
-    if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device) != cudaSuccess ||
-        (size_t)optin < smem ||
-        cudaFuncSetAttribute(k_cn_solve_zt, cudaFuncAttributeMaxDynamicSharedMemorySize, optin) != cudaSuccess ||
-        cudaFuncSetAttribute(k_cn_solve_zt, cudaFuncAttributePreferredSharedMemoryCarveout,
-                             cudaSharedmemCarveoutMaxShared) != cudaSuccess)
-      return false;
     int per_sm = 0, nsm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cn_solve_zt, 32 * wpb, smem) != cudaSuccess ||
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx->device) != cudaSuccess || per_sm < 1)
-      return false;
+    if (!tile_kernel_setup(ctx, k_cn_solve_zt, 32 * wpb, smem, &per_sm, &nsm)) return false;
     ctx->tma_grid[0] = per_sm * nsm;
   }
   const long ntiles = (long)((L.nx + 31) / 32) * L.ny * L.ns;
@@ -1374,26 +1535,16 @@ static bool launch_cn_solve_zt(a3g_ctx *ctx, const LineMap &map, const double *t
 
 // Launches the y solve through chunk tiles; false when the maps cannot be
 // made (the caller takes the per-thread kernel).
-static bool launch_cn_solve_yt(a3g_ctx *ctx, const LineMap &map, const double *tab) {
+static bool launch_cn_solve_yt(a3g_ctx *ctx, const LineMap &map, const CnTab &tab) {
   const Layout &L = ctx->L;
   if (map.da) return false;
   CUtensorMap tin, tout;
-  if (!tensor_map(ctx, ctx->c0, TM_YCHUNK_IN, &tin) || !tensor_map(ctx, ctx->c1, TM_YCHUNK_OUT, &tout))
-    return false;
+  if (!tensor_map(ctx, ctx->c0, TM_YCHUNK, &tin) || !tensor_map(ctx, ctx->c1, TM_YCHUNK, &tout)) return false;
   const int wpb = 2;
-  const size_t smem = ZT_BAR_BYTES + (size_t)wpb * (2 * 32 * YT_ROWS + CN_NF * 32) * sizeof(double);
+  const size_t smem = ZT_BAR_BYTES + (size_t)wpb * 3 * YT_BUF_D * sizeof(double);
   if (ctx->tma_grid[1] == 0) {
-    int optin = 0;
-    if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device) != cudaSuccess ||
-        (size_t)optin < smem ||
-        cudaFuncSetAttribute(k_cn_solve_yt, cudaFuncAttributeMaxDynamicSharedMemorySize, optin) != cudaSuccess ||
-        cudaFuncSetAttribute(k_cn_solve_yt, cudaFuncAttributePreferredSharedMemoryCarveout,
-                             cudaSharedmemCarveoutMaxShared) != cudaSuccess)
-      return false;
     int per_sm = 0, nsm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cn_solve_yt, 32 * wpb, smem) != cudaSuccess ||
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx->device) != cudaSuccess || per_sm < 1)
-      return false;
+    if (!tile_kernel_setup(ctx, k_cn_solve_yt, 32 * wpb, smem, &per_sm, &nsm)) return false;
     ctx->tma_grid[1] = per_sm * nsm;
   }
   const long ngroups = (long)((L.nx + 31) / 32) * L.nz * L.ns;
@@ -1404,23 +1555,19 @@ static bool launch_cn_solve_yt(a3g_ctx *ctx, const LineMap &map, const double *t
   return true;
 }
 
-// Launches the x solve through TMA tiles; false when the map cannot be made.
-static bool launch_cn_solve_xt2(a3g_ctx *ctx, const LineMap &map, const double *tab) {
+// Launches the x solve through TMA tiles; false when the maps cannot be made.
+static bool launch_cn_solve_xt2(a3g_ctx *ctx, const LineMap &map, const CnTab &tab) {
   const Layout &L = ctx->L;
-  CUtensorMap trow;
-  if (!tensor_map(ctx, ctx->c0, TM_XROWS, &trow)) return false;
-  const size_t smem = ZT_BAR_BYTES + (size_t)XT2_WARPS * XT2_WARP_D * sizeof(double);
+  CUtensorMap tin, tout;
+  if (!tensor_map(ctx, ctx->c0, TM_XROWS, &tin) || !tensor_map(ctx, ctx->c1, TM_XROWS, &tout)) return false;
   if (ctx->tma_grid[2] == 0) {
-    int optin = 0;
-    if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device) != cudaSuccess ||
-        (size_t)optin < smem ||
-        cudaFuncSetAttribute(k_cn_solve_xt2, cudaFuncAttributeMaxDynamicSharedMemorySize, optin) != cudaSuccess)
-      return false;
-    ctx->tma_grid[2] = 1;
+    int per_sm = 0, nsm = 0;
+    if (!tile_kernel_setup(ctx, k_cn_solve_xt2, 32 * CXT_WARPS, CXT_SMEM, &per_sm, &nsm)) return false;
+    ctx->tma_grid[2] = per_sm * nsm;
   }
   const long nwarps = ((long)L.ny * L.nz * L.ns + 31) / 32;
-  k_cn_solve_xt2<<<(unsigned)((nwarps + XT2_WARPS - 1) / XT2_WARPS), 32 * XT2_WARPS, smem, ctx->stream>>>(
-      trow, L, ctx->box, map, ctx->c0, ctx->c1, tab, ctx->aloft, ctx->sc);
+  k_cn_solve_xt2<<<(unsigned)((nwarps + CXT_WARPS - 1) / CXT_WARPS), 32 * CXT_WARPS, CXT_SMEM, ctx->stream>>>(
+      tin, tout, L, ctx->box, map, ctx->c1, tab, ctx->aloft, ctx->sc);
   return true;
 }
 
@@ -1451,27 +1598,30 @@ static inline bool varies(const Geo3 &g, int idx) {  // idx 0:i 1:j 2:k
   return (idx == 0 ? g.si : idx == 1 ? g.sj : g.sk) != 0;
 }
 
-size_t cn_table_doubles(const a3g_ctx *ctx, int dir) {
+template <int DIR>
+static LineMap line_map(const a3g_ctx *ctx) {
   const Layout &L = ctx->L;
-  const Geo3 &sig = (dir == 0) ? ctx->snx : (dir == 1) ? ctx->sny : ctx->snz;
-  const Geo3 &kk = (dir == 0) ? ctx->kx : (dir == 1) ? ctx->ky : ctx->kz;
-  const int ia = (dir == 0) ? 1 : 0, ib = (dir == 2) ? 1 : 2;
-  const int na = (dir == 0) ? L.ny : L.nx, nb = (dir == 2) ? L.ny : L.nz;
-  const bool da = varies(ctx->kappa, ia) || varies(sig, ia) || varies(kk, ia);
-  const bool db = varies(ctx->kappa, ib) || varies(sig, ib) || varies(kk, ib);
-  const size_t n = (dir == 0) ? L.nx : (dir == 1) ? L.ny : L.nz;
-  const size_t U = (size_t)(da ? na : 1) * (size_t)(db ? nb : 1);
-  return (size_t)CN_NF * n * U + 2 * U;
+  const Geo3 &sig = (DIR == 0) ? ctx->snx : (DIR == 1) ? ctx->sny : ctx->snz;
+  const Geo3 &kk = (DIR == 0) ? ctx->kx : (DIR == 1) ? ctx->ky : ctx->kz;
+  const int ia = (DIR == 0) ? 1 : 0, ib = (DIR == 2) ? 1 : 2;
+  auto any = [&](int i) { return varies(ctx->kappa, i) || varies(sig, i) || varies(kk, i); };
+  LineMap map;
+  map.na = (DIR == 0) ? L.ny : L.nx;
+  map.nb = (DIR == 2) ? L.ny : L.nz;
+  map.da = any(ia);
+  map.db = any(ib);
+  map.ds = any(DIR);
+  map.U = (map.da ? map.na : 1) * (map.db ? map.nb : 1);
+  return map;
 }
 
-// Decides on the device whether direction dir's table can be kept: the host
-// allows it (same box, geometry and diffusivity as when it was built) and
-// the step's dt equals the table's.
-__global__ void k_cn_check(const DevScalars *__restrict__ sc, double *__restrict__ st, int dir, int may) {
-  const double dt = sc->dt;
-  const bool keep = may && st[dir] == dt;
-  st[3 + dir] = keep ? 1.0 : 0.0;
-  st[dir] = dt;
+// the y and z tables are stored by row unless their lines differ along i
+static bool cn_byrow(int dir, const LineMap &map) { return dir != 0 && !map.da; }
+
+size_t cn_table_doubles(const a3g_ctx *ctx, int dir) {
+  const LineMap map = dir == 0 ? line_map<0>(ctx) : dir == 1 ? line_map<1>(ctx) : line_map<2>(ctx);
+  const size_t n = (dir == 0) ? ctx->L.nx : (dir == 1) ? ctx->L.ny : ctx->L.nz;
+  return ((cn_byrow(dir, map) ? CN_NF : CN_NFX) * n + 3) * (size_t)map.U;
 }
 
 static inline bool same_box(const Box &a, const Box &b) {
@@ -1481,17 +1631,28 @@ static inline bool same_box(const Box &a, const Box &b) {
 
 // The factor table of direction DIR for the step's dt: built by k_cn_table,
 // or kept from the previous build when nothing it depends on has changed.
+// No launch at all while the host knows that dt has not been set since.
 template <int DIR>
-static int cn_table(a3g_ctx *ctx, const LineMap &map, const Geo3 &sig, const Geo3 &kk) {
-  const bool may = ctx->cn_valid[DIR] && same_box(ctx->cn_box[DIR], ctx->box);
-  k_cn_check<<<1, 1, 0, ctx->stream>>>(ctx->sc, ctx->cn_state, DIR, may ? 1 : 0);
+static int cn_table(a3g_ctx *ctx, const LineMap &map, const Geo3 &sig, const Geo3 &kk, CnTab *out) {
+  const Box &box = ctx->box;
+  const int n = (DIR == 0) ? box.imax - box.imin + 1 : (DIR == 1) ? box.jmax - box.jmin + 1 : box.kmax - box.kmin + 1;
+  const bool may = ctx->cn_valid[DIR] && same_box(ctx->cn_box[DIR], box);
+  *out = CnTab{ctx->cn_tab[DIR], (long)n * map.U, map.U, n, cn_byrow(DIR, map)};
+  if (may && ctx->cn_stamp[DIR] == ctx->dt_stamp) return A3G_OK;
+  double *const st = ctx->cn_state + 2 * DIR;
+  const int slot = ctx->cn_slot[DIR];
+#define A3G_TABLE(LPB_)                                                                                       \
+  k_cn_table<DIR, LPB_><<<(map.U + LPB_ - 1) / LPB_, 256, 0, ctx->stream>>>(                                   \
+      ctx->L, box, ctx->prm.imp_fac, map, sig, ctx->kappa, kk, ctx->sc, st + slot, st + (slot ^ 1), may ? 1 : 0, \
+      out->byrow ? 1 : 0, ctx->cn_tab[DIR])
+  // many lines: 32 share a block's serial warp; few: a block each, more of its rows at once
+  if (map.U >= 1024) A3G_TABLE(32); else A3G_TABLE(1);
+#undef A3G_TABLE
   A3G_LAUNCH_CHECK(ctx);
-  k_cn_table<DIR><<<(map.U + 127) / 128, 128, 0, ctx->stream>>>(ctx->L, ctx->box, ctx->prm.imp_fac, map, sig,
-                                                                ctx->kappa, kk, ctx->sc, ctx->cn_state,
-                                                                ctx->cn_tab[DIR]);
-  A3G_LAUNCH_CHECK(ctx);
+  ctx->cn_slot[DIR] ^= 1;
+  ctx->cn_stamp[DIR] = ctx->dt_stamp;
   ctx->cn_valid[DIR] = true;
-  ctx->cn_box[DIR] = ctx->box;
+  ctx->cn_box[DIR] = box;
   return A3G_OK;
 }
 
@@ -1508,18 +1669,12 @@ static int launch_cn_dir(a3g_ctx *ctx) {
   }
   const Geo3 &sig = (DIR == 0) ? ctx->snx : (DIR == 1) ? ctx->sny : ctx->snz;
   const Geo3 &kk = (DIR == 0) ? ctx->kx : (DIR == 1) ? ctx->ky : ctx->kz;
-  const int ia = (DIR == 0) ? 1 : 0, ib = (DIR == 2) ? 1 : 2;
-  LineMap map;
-  map.na = (DIR == 0) ? L.ny : L.nx;
-  map.nb = (DIR == 2) ? L.ny : L.nz;
-  map.da = varies(ctx->kappa, ia) || varies(sig, ia) || varies(kk, ia);
-  map.db = varies(ctx->kappa, ib) || varies(sig, ib) || varies(kk, ib);
-  map.U = (map.da ? map.na : 1) * (map.db ? map.nb : 1);
+  const LineMap map = line_map<DIR>(ctx);
+  CnTab tab;
   tbegin(ctx, A3G_K_CN_TABLE);
-  int rc = cn_table<DIR>(ctx, map, sig, kk);
+  int rc = cn_table<DIR>(ctx, map, sig, kk, &tab);
   tend(ctx);
   if (rc) return rc;
-  const double *tab = ctx->cn_tab[DIR];
   const long nlines = (long)map.na * map.nb * L.ns;
   tbegin(ctx, A3G_K_CN_SOLVE_X + DIR);
   if (DIR == 0 && ctx->tune_cn_x == 2 && launch_cn_solve_xt2(ctx, map, tab)) {
@@ -1615,7 +1770,7 @@ __global__ void __launch_bounds__(256) k_adj_diff(Layout L, int periodic, const 
 // columns of N).  One thread per line; z is parked in the output line.
 template <int DIR>
 __global__ void __launch_bounds__(128) k_adj_cn(Layout L, LineMap map, const double *__restrict__ lin,
-                                                double *__restrict__ lout, const double *__restrict__ tab,
+                                                double *__restrict__ lout, CnTab tab,
                                                 const int32_t *__restrict__ aloft) {
   const int na = (DIR == 0) ? L.ny : L.nx;
   const int nb = (DIR == 2) ? L.ny : L.nz;
@@ -1638,13 +1793,10 @@ __global__ void __launch_bounds__(128) k_adj_cn(Layout L, LineMap map, const dou
     for (int r = 0; r < n; r++) lo[(long)r * st] = 0.0;
     return;
   }
-  const long U = map.U;
-  const long F = (long)n * U;
   const long u = map.u(a, b);
-  const double *t = tab + u;
   CnRun R;
-  if (DIR == 0) cn_load_run(t, F, U, tab + CN_NF * F, u, R);
-  auto co = [&](int f, int l) { return (DIR == 0) ? cn_coef(t, F, U, R, f, l) : t[f * F + (long)l * U]; };
+  if (DIR == 0) cn_load_run(tab, u, R);
+  auto co = [&](int f, int l) { return (DIR == 0) ? cn_coef(tab, u, R, f, l) : tab.at(f, l, u); };
   // U^T z = lam
   double zp = 0.0;
   for (int r = 0; r < n; r++) {
@@ -1695,18 +1847,13 @@ static int launch_adj_cn_dir(a3g_ctx *ctx, const double *lin, double *lout) {
   }
   const Geo3 &sig = (DIR == 0) ? ctx->snx : (DIR == 1) ? ctx->sny : ctx->snz;
   const Geo3 &kk = (DIR == 0) ? ctx->kx : (DIR == 1) ? ctx->ky : ctx->kz;
-  const int ia = (DIR == 0) ? 1 : 0, ib = (DIR == 2) ? 1 : 2;
-  LineMap map;
-  map.na = (DIR == 0) ? L.ny : L.nx;
-  map.nb = (DIR == 2) ? L.ny : L.nz;
-  map.da = varies(ctx->kappa, ia) || varies(sig, ia) || varies(kk, ia);
-  map.db = varies(ctx->kappa, ib) || varies(sig, ib) || varies(kk, ib);
-  map.U = (map.da ? map.na : 1) * (map.db ? map.nb : 1);
+  const LineMap map = line_map<DIR>(ctx);
+  CnTab tab;
   tbegin(ctx, A3G_K_ADJOINT);
-  int rc = cn_table<DIR>(ctx, map, sig, kk);
+  int rc = cn_table<DIR>(ctx, map, sig, kk, &tab);
   if (rc) return rc;
   const long nlines = (long)map.na * map.nb * L.ns;
-  k_adj_cn<DIR><<<(unsigned)((nlines + 127) / 128), 128, 0, ctx->stream>>>(L, map, lin, lout, ctx->cn_tab[DIR],
+  k_adj_cn<DIR><<<(unsigned)((nlines + 127) / 128), 128, 0, ctx->stream>>>(L, map, lin, lout, tab,
                                                                            ctx->aloft);
   tend(ctx);
   A3G_LAUNCH_CHECK(ctx);

@@ -85,6 +85,15 @@ __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, u
       : "memory");
 }
 
+// Untiled load of `bytes` contiguous bytes (a multiple of 16, both addresses
+// 16-byte aligned) into shared memory; completes on bar as the tiled loads do.
+__device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes, uint64_t *bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                   smem_u32(dst)),
+               "l"(reinterpret_cast<uint64_t>(src)), "r"(bytes), "r"(smem_u32(bar))
+               : "memory");
+}
+
 // Tiled 4-D tensor store of one box from shared memory; elements outside the
 // tensor are not written.  Tracked by the issuing thread's bulk groups.
 __device__ __forceinline__ void tma_store_4d(const CUtensorMap *map, const void *src, int x, int y, int z,
