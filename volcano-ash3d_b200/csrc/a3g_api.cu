@@ -234,6 +234,8 @@ int a3g_create(const a3g_grid_desc *grid, const a3g_params *params, int device, 
   if (e == cudaSuccess) e = dmalloc((void **)&ctx->sc, sizeof(DevScalars));
   ctx->red_len = (size_t)2 * 296 * 7 * ns + 7 * ns;
   if (e == cudaSuccess) e = dmalloc((void **)&ctx->red_buf, sizeof(double) * ctx->red_len);
+  if (e == cudaSuccess) e = dmalloc((void **)&ctx->cfl_part, sizeof(double) * 3 * CFL_BLOCKS);
+  if (e == cudaSuccess) e = dmalloc((void **)&ctx->block_count, sizeof(unsigned) * 2);
   if (e == cudaSuccess) e = dmalloc((void **)&ctx->plane_flags, sizeof(int32_t) * (L.nx + L.ny + L.nz + 3));
   if (e == cudaSuccess) e = dmalloc((void **)&ctx->src_buf, sizeof(double) * (L.nz + 1) * ns);
   if (e == cudaSuccess) e = cudaMallocHost((void **)&ctx->h_sc, sizeof(DevScalars));
@@ -281,6 +283,8 @@ int a3g_destroy(a3g_ctx *ctx) {
   if (ctx->met) cudaFree(ctx->met);
   if (ctx->aloft) cudaFree(ctx->aloft);
   if (ctx->sc) cudaFree(ctx->sc);
+  if (ctx->cfl_part) cudaFree(ctx->cfl_part);
+  if (ctx->block_count) cudaFree(ctx->block_count);
   if (ctx->plane_flags) cudaFree(ctx->plane_flags);
   if (ctx->h_sc) cudaFreeHost(ctx->h_sc);
   if (ctx->h_plane_flags) cudaFreeHost(ctx->h_plane_flags);
@@ -1276,9 +1280,11 @@ int a3g_timestep_totals(a3g_ctx *ctx, double *out4, double *mass_aloft) {
   CTX_CHECK(ctx);
   if (!out4) return fail(A3G_ERR_ARG, "null out4");
   if (!ctx->have_geometry) return fail(A3G_ERR_STATE, "geometry not set");
-  int rc = launch_totals(ctx, out4, mass_aloft);
+  int rc = launch_totals_partials(ctx, ctx->h_tot);
   if (rc) return rc;
-  if ((rc = sync_scalars(ctx))) return rc;
+  rc = sync_scalars(ctx);  // waits for the totals too; a device error leaves them written
+  totals_volumes(ctx, ctx->h_tot, out4, mass_aloft);
+  if (rc) return rc;
   // The reference carries a NaN on silently (its mass-conservation stop
   // test compares false); the totals are still written, but the caller is told.
   for (int q = 0; q < 4; q++)

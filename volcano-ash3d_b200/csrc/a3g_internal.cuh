@@ -97,6 +97,7 @@ enum TmapKind {
 constexpr int YT_CH = 16;            // cells per CN y chunk
 constexpr int ACH = 8;               // cells per advection chunk
 constexpr int CX_CH = 16;            // cells per CN x chunk
+constexpr int CFL_BLOCKS = 148 * 4;  // blocks of the CFL reduction
 struct TmapEntry {
   const void *p;
   int kind;
@@ -160,6 +161,8 @@ struct a3g_ctx {
   a3g::DevScalars *h_sc;    // pinned host mirror
   double *red_buf;          // reduction partials
   size_t red_len;
+  double *cfl_part;         // per-block CFL maxima (3*CFL_BLOCKS)
+  unsigned *block_count;    // blocks done: [0] totals, [1] CFL (zero between launches)
   int32_t *plane_flags;     // subgrid plane occupancy (nx+ny+nz+3)
   int32_t *h_plane_flags;   // pinned
   double *src_buf;          // device source column (nz+1)*ns
@@ -291,9 +294,10 @@ int launch_cfl_maxima_meso(a3g_ctx *ctx, int slot);
 int launch_cfl_maxima_meso_ptr(a3g_ctx *ctx, const float *met_step);
 void inv_free(a3g_ctx *ctx);
 int launch_fast_dt(a3g_ctx *ctx, double frac, double time, double next_write_time, double simtime);
-int launch_totals(a3g_ctx *ctx, double *out4, double *mass_aloft);
+double *claim_dtv(a3g_ctx *ctx);
 int launch_plane_flags(a3g_ctx *ctx);
 int launch_interp_winds(a3g_ctx *ctx, double frac);
+int launch_interp_pair(a3g_ctx *ctx, const float *last, const float *next, double frac);
 int launch_vmod_topo(a3g_ctx *ctx);
 int launch_totals_partials(a3g_ctx *ctx, double *h_dst);
 void totals_volumes(a3g_ctx *ctx, const double *h_src, double *out4, double *mass_aloft);

@@ -111,7 +111,14 @@ __global__ void k_inv_grad(Layout L, int ivent, int jvent, const double *__restr
   grad[o] = grad[o] + dts[n] * lam[(long)g * L.PG + L.cell(ivent, jvent, k)] / kv;
 }
 
-__global__ void k_set_dt(DevScalars *sc, const double *__restrict__ dts, int n) { sc->dt = dts[n]; }
+// the step's dt and (dtv not null) dt/kappa with it
+__global__ void k_set_dt(DevScalars *sc, const double *__restrict__ dts, int n, const double *__restrict__ kap,
+                         double *__restrict__ dtv, int dtv_len) {
+  const double dt = dts[n];
+  if (threadIdx.x == 0) sc->dt = dt;
+  if (dtv)
+    for (int t = threadIdx.x; t < dtv_len; t += blockDim.x) dtv[t] = dt / kap[t];
+}
 
 // DepositThickness(i,j) = sum_g dep(i,j,g) * dz_vec(1) / KM2_2_M2 / DepositDensity * M_2_MM
 // (src/Output_Vars.f90:880-884), unmasked; dep in the device's [g][j][i] order
@@ -139,23 +146,6 @@ __global__ void k_adj_dep(int nx, int ny, int ns, const double *__restrict__ w, 
 __global__ void k_resid(long n, const double *__restrict__ a, const double *__restrict__ b, double *__restrict__ r) {
   const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (t < n) r[t] = a[t] - b[t];
-}
-
-__global__ void k_interp_from(Layout L, const float *__restrict__ last, const float *__restrict__ next, long n,
-                              double frac, double *__restrict__ vx, double *__restrict__ vy, double *__restrict__ vz) {
-  for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < n; t += (long)gridDim.x * blockDim.x) {
-    const int i = (int)(t % L.nx) + 1;
-    const long r = t / L.nx;
-    const int j = (int)(r % L.ny) + 1;
-    const int k = (int)(r / L.ny) + 1;
-    const long c = L.cell(i, j, k);
-    const float dx = next[t] - last[t];
-    const float dy = next[n + t] - last[n + t];
-    const float dz = next[2 * n + t] - last[2 * n + t];
-    vx[c] = ((double)last[t] + (double)dx * frac) * 3.6;
-    vy[c] = ((double)last[n + t] + (double)dy * frac) * 3.6;
-    vz[c] = ((double)last[2 * n + t] + (double)dz * frac) * 3.6;
-  }
 }
 
 }  // namespace a3g
@@ -320,20 +310,13 @@ int winds(a3g_ctx *ctx, a3g_inv *v, int hour, double frac) {
   const float *last, *next;
   int rc = load_pair(ctx, v, hour, &last, &next);
   if (rc) return rc;
-  const Layout &L = ctx->L;
-  const long n = (long)L.nx * L.ny * L.nz;
-  int blocks = (int)((n + 255) / 256);
-  if (blocks > 148 * 16) blocks = 148 * 16;
-  tbegin(ctx, A3G_K_WINDS);
-  k_interp_from<<<blocks, 256, 0, ctx->stream>>>(L, last, next, n, frac, ctx->vx, ctx->vy, ctx->vz);
-  tend(ctx);
-  A3G_LAUNCH_CHECK(ctx);
+  if ((rc = launch_interp_pair(ctx, last, next, frac))) return rc;
   ctx->have_winds = true;
   return A3G_OK;
 }
 
 int set_step_dt(a3g_ctx *ctx, a3g_inv *v, int n) {
-  k_set_dt<<<1, 1, 0, ctx->stream>>>(ctx->sc, v->dts, n);
+  k_set_dt<<<1, 256, 0, ctx->stream>>>(ctx->sc, v->dts, n, ctx->kappa.p, claim_dtv(ctx), (int)ctx->kappa_len);
   A3G_LAUNCH_CHECK(ctx);
   ctx->host_dt = v->steps[n].dt;
   ctx->dt_stamp++;

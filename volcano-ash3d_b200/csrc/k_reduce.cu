@@ -2,9 +2,9 @@
 //
 //  * CFL maxima and the dt arithmetic of Adjust_DT (src/Adjust_dt.f90:136-332):
 //    maxima are exact and order independent, so the result is bit-identical
-//    to the CPU loop; they are combined with atomicMax on the IEEE bit
-//    patterns (valid for non-negative doubles; NaNs are skipped as the
-//    reference's `if (tmp.gt.max)` skips them).
+//    to the CPU loop (NaNs are skipped as the reference's `if (tmp.gt.max)`
+//    skips them; a met step's are combined with atomicMax on the IEEE bit
+//    patterns of non-negative doubles).
 //  * mass totals (src/Output_Vars.f90:1255-1459): per-grain sums of c*kappa
 //    accumulated in double-double (TwoSum) and combined in a fixed order, so
 //    the result is deterministic and within a few ulp of the exact sum.
@@ -36,18 +36,88 @@ __device__ __forceinline__ double warp_min(double v) {
   return v;
 }
 
-// One thread per interior cell (grid-stride).  vmax[0]: |vx| (projected) or
-// max |vx|*minsig/kappa (lon/lat); vmax[1] the same for y; vmax[2] the
-// vertical (|vz| + max_g |vf|)/dz_k.  src/Adjust_dt.f90:136-173.
+// What Adjust_DT's last block does with the maxima (k_dt_finalize's arguments).
+struct DtArgs {
+  int latlon, use_diffusion, use_cn, n_gs_aloft;
+  double dx, dy, cfl, dt_min, dt_max, imp_dt_fac, eps_small, time, next_write_time, simtime;
+  int diff_fresh, meso;
+};
+
+// dt arithmetic, src/Adjust_dt.f90:176-179 and :288-332.
+// meso (FAST_DT, Adjust_DT(mesostep=.true.)): bit 1 first copies
+// dt_meso_next to dt_meso_last (the toggle of src/MesoInterpolater.f90:187),
+// bit 0 stores the dt formed here as dt_meso_next (src/Adjust_dt.f90:335-337).
+__device__ void dt_finalize(const DtArgs &a, DevScalars *sc) {
+  if (a.meso & 2) sc->dt_meso_last = sc->dt_meso_next;
+  double vx_dx = sc->vmax[0], vy_dy = sc->vmax[1], vz_dz = sc->vmax[2];
+  if (!a.latlon) {
+    vx_dx = vx_dx / a.dx;
+    vy_dy = vy_dy / a.dy;
+  }
+  if (a.n_gs_aloft == 0) vz_dz = 0.0;
+  const double time_advect = 1.0 / fmx(fmx(vx_dx, vy_dy), vz_dz);
+  double td;
+  if (a.use_diffusion) {
+    if (a.diff_fresh) {
+      td = sc->time_diffuse;  // min(DT_MAX, min_cells tmp4)
+      td = a.use_cn ? td * a.imp_dt_fac : td * 0.5;
+      sc->time_diffuse = td;
+      sc->have_diffuse = 1;
+    } else {
+      td = sc->time_diffuse;
+    }
+  } else {
+    td = a.dt_max;
+  }
+  const double dt_tmp = fmn(time_advect, td);
+  double dt;
+  if (dt_tmp < a.dt_min) dt = a.dt_min;
+  else if (dt_tmp > a.dt_max) dt = a.dt_max;
+  else dt = fmn(1.0, a.cfl) * dt_tmp;
+  const long long fac = (long long)(dt / a.dt_min);
+  dt = a.dt_min * (double)fac;
+  if ((a.next_write_time - a.time) > a.eps_small && (a.next_write_time - a.time) < dt) dt = a.next_write_time - a.time;
+  if (a.time + dt > a.simtime) dt = a.simtime - a.time;
+  sc->dt = dt;
+  if (a.meso & 1) sc->dt_meso_next = dt;
+}
+
+// The last block of a grid to come here (true in every thread of that block):
+// what the others wrote before is visible to it.  The counter is left at zero.
+__device__ bool last_block(unsigned *counter, unsigned nblocks) {
+  __shared__ bool last;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(counter, 1u) == nblocks - 1;
+    if (last) {
+      *counter = 0u;
+      __threadfence();
+    }
+  }
+  __syncthreads();
+  return last;
+}
+
+// CFL maxima: vmax[0] |vx| (projected) or max |vx|*minsig/kappa (lon/lat);
+// vmax[1] the same for y; vmax[2] the vertical (|vz| + max_g |vf|)/dz_k
+// (src/Adjust_dt.f90:136-173); then, with `finish`, the step's dt and (dtv not
+// null, a small kappa table) dt/kappa, by the last block.  A warp takes a row:
+// where the row's geometry and settling speeds are constant along i, the
+// products and quotients are formed once, from the row's largest winds --
+// rounding is monotone, so the maximum is the same.  Bound by the winds' 24 B a
+// cell; with per-warp atomics on three words, a memset before and the dt in a
+// kernel of its own this took 26 us on 93x131x37 where the loads take under 2.
 __global__ void __launch_bounds__(256) k_cfl(Layout L, int latlon, const double *__restrict__ vx,
                                              const double *__restrict__ vy,
                                              const double *__restrict__ vz, Geo4 vf, Geo3 snx,
                                              Geo3 sny, Geo3 kap, const double *__restrict__ dz_vec,
-                                             DevScalars *sc) {
-  // block-strided rows (j,k), threads along i (a maximum does not depend on
-  // the visiting order)
-  const int nrow = L.ny * L.nz;
+                                             double *__restrict__ part, unsigned *__restrict__ counter, int finish,
+                                             DtArgs args, double *__restrict__ dtv, int dtv_len, DevScalars *sc) {
+  __shared__ double sh[3][8];
+  const int nrow = L.ny * L.nz, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const bool vf_const = vf.si == 0 && vf.sj == 0 && vf.sk == 0;  // per-grain settling speeds
+  const bool row_const = vf_const && (!latlon || (snx.si == 0 && sny.si == 0 && kap.si == 0));
   double vf0 = 0.0;
   if (vf_const)
     for (int g = 0; g < L.ns; g++) {
@@ -55,43 +125,85 @@ __global__ void __launch_bounds__(256) k_cfl(Layout L, int latlon, const double 
       if (g == 0 || a > vf0) vf0 = a;
     }
   double m0 = 0.0, m1 = 0.0, m2 = 0.0;
-  for (int r = blockIdx.x; r < nrow; r += gridDim.x) {
-    const int j = r % L.ny + 1, k = r / L.ny + 1;
-    const double rdz = dz_vec[k + 1];
-    const long rb = L.cell(1, j, k);
-    for (int i = threadIdx.x + 1; i <= L.nx; i += blockDim.x) {
-      const long c = rb + (i - 1);
-      const double ax = fabs(vx[c]), ay = fabs(vy[c]);
-      double t1, t2;
-      if (latlon) {
-        const double kp = kap.at(i, j, k);
-        t1 = ax * fmn(snx.at(i, j, k), snx.at(i + 1, j, k)) / kp;
-        t2 = ay * fmn(sny.at(i, j, k), sny.at(i, j + 1, k)) / kp;
-      } else {
-        t1 = ax;
-        t2 = ay;
-      }
-      double vfm = vf0;
-      if (!vf_const) {
-        vfm = 0.0;
-        for (int g = 0; g < L.ns; g++) {
-          const double a = fabs(vf.at(i, j, k, g));
-          if (g == 0 || a > vfm) vfm = a;
-        }
-      }
-      const double t3 = (fabs(vz[c]) + vfm) / rdz;
-      if (t1 > m0) m0 = t1;
-      if (t2 > m1) m1 = t2;
-      if (t3 > m2) m2 = t3;
+  auto cell = [&](int i, int j, int k, double ax, double ay, double az, double vfm) {
+    double t1 = ax, t2 = ay;
+    if (latlon) {
+      const double kp = kap.at(i, j, k);
+      t1 = ax * fmn(snx.at(i, j, k), snx.at(i + 1, j, k)) / kp;
+      t2 = ay * fmn(sny.at(i, j, k), sny.at(i, j + 1, k)) / kp;
     }
+    const double t3 = (az + vfm) / dz_vec[k + 1];
+    if (t1 > m0) m0 = t1;
+    if (t2 > m1) m1 = t2;
+    if (t3 > m2) m2 = t3;
+  };
+  for (int r = blockIdx.x * 8 + w; r < nrow; r += gridDim.x * 8) {
+    const int j = r % L.ny + 1, k = r / L.ny + 1;
+    const long rb = (long)r * L.P;
+    double ax = 0.0, ay = 0.0, az = 0.0;
+#pragma unroll 4
+    for (int i = lane; i < L.nx; i += 32) {
+      const double x = fabs(vx[rb + i]), y = fabs(vy[rb + i]), z = fabs(vz[rb + i]);
+      if (row_const) {
+        if (x > ax) ax = x;
+        if (y > ay) ay = y;
+        if (z > az) az = z;
+      } else {
+        double vfm = vf0;
+        if (!vf_const) {
+          vfm = 0.0;
+          for (int g = 0; g < L.ns; g++) {
+            const double a = fabs(vf.at(i + 1, j, k, g));
+            if (g == 0 || a > vfm) vfm = a;
+          }
+        }
+        cell(i + 1, j, k, x, y, z, vfm);
+      }
+    }
+    if (row_const) cell(1, j, k, ax, ay, az, vf0);
   }
-  m0 = warp_max(m0);
-  m1 = warp_max(m1);
-  m2 = warp_max(m2);
-  if ((threadIdx.x & 31) == 0) {
-    atomic_max_pos(&sc->vmax[0], m0);
-    atomic_max_pos(&sc->vmax[1], m1);
-    atomic_max_pos(&sc->vmax[2], m2);
+  auto block_max = [&]() {  // the block's maxima, in thread 0
+    m0 = warp_max(m0);
+    m1 = warp_max(m1);
+    m2 = warp_max(m2);
+    if (lane == 0) {
+      sh[0][w] = m0;
+      sh[1][w] = m1;
+      sh[2][w] = m2;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0)
+      for (int q = 1; q < 8; q++) {
+        m0 = fmx(m0, sh[0][q]);
+        m1 = fmx(m1, sh[1][q]);
+        m2 = fmx(m2, sh[2][q]);
+      }
+  };
+  block_max();
+  if (threadIdx.x == 0) {
+    part[3 * blockIdx.x] = m0;
+    part[3 * blockIdx.x + 1] = m1;
+    part[3 * blockIdx.x + 2] = m2;
+  }
+  if (!last_block(counter, gridDim.x)) return;
+  m0 = m1 = m2 = 0.0;
+  for (int q = threadIdx.x; q < (int)gridDim.x; q += 256) {
+    m0 = fmx(m0, __ldcg(part + 3 * q));
+    m1 = fmx(m1, __ldcg(part + 3 * q + 1));
+    m2 = fmx(m2, __ldcg(part + 3 * q + 2));
+  }
+  block_max();
+  if (threadIdx.x == 0) {
+    sc->vmax[0] = m0;
+    sc->vmax[1] = m1;
+    sc->vmax[2] = m2;
+    sc->vmax[3] = 0.0;
+    if (finish) dt_finalize(args, sc);
+  }
+  if (finish && dtv) {
+    __syncthreads();
+    const double dt = sc->dt;
+    for (int t = threadIdx.x; t < dtv_len; t += 256) dtv[t] = dt / kap.p[t];
   }
 }
 
@@ -121,47 +233,7 @@ __global__ void __launch_bounds__(256) k_diff_limit(Layout L, Geo3 snx, Geo3 sny
   if ((threadIdx.x & 31) == 0) atomic_min_pos(&sc->time_diffuse, m);
 }
 
-// dt arithmetic, src/Adjust_dt.f90:176-179 and :288-332.
-// meso (FAST_DT, Adjust_DT(mesostep=.true.)): bit 1 first copies
-// dt_meso_next to dt_meso_last (the toggle of src/MesoInterpolater.f90:187),
-// bit 0 stores the dt formed here as dt_meso_next (src/Adjust_dt.f90:335-337).
-__global__ void k_dt_finalize(int latlon, int use_diffusion, int use_cn, int n_gs_aloft, double dx,
-                              double dy, double cfl, double dt_min, double dt_max, double imp_dt_fac,
-                              double eps_small, double time, double next_write_time,
-                              double simtime, int diff_fresh, int meso, DevScalars *sc) {
-  if (meso & 2) sc->dt_meso_last = sc->dt_meso_next;
-  double vx_dx = sc->vmax[0], vy_dy = sc->vmax[1], vz_dz = sc->vmax[2];
-  if (!latlon) {
-    vx_dx = vx_dx / dx;
-    vy_dy = vy_dy / dy;
-  }
-  if (n_gs_aloft == 0) vz_dz = 0.0;
-  const double time_advect = 1.0 / fmx(fmx(vx_dx, vy_dy), vz_dz);
-  double td;
-  if (use_diffusion) {
-    if (diff_fresh) {
-      td = sc->time_diffuse;  // min(DT_MAX, min_cells tmp4)
-      td = use_cn ? td * imp_dt_fac : td * 0.5;
-      sc->time_diffuse = td;
-      sc->have_diffuse = 1;
-    } else {
-      td = sc->time_diffuse;
-    }
-  } else {
-    td = dt_max;
-  }
-  const double dt_tmp = fmn(time_advect, td);
-  double dt;
-  if (dt_tmp < dt_min) dt = dt_min;
-  else if (dt_tmp > dt_max) dt = dt_max;
-  else dt = fmn(1.0, cfl) * dt_tmp;
-  const long long fac = (long long)(dt / dt_min);
-  dt = dt_min * (double)fac;
-  if ((next_write_time - time) > eps_small && (next_write_time - time) < dt) dt = next_write_time - time;
-  if (time + dt > simtime) dt = simtime - time;
-  sc->dt = dt;
-  if (meso & 1) sc->dt_meso_next = dt;
-}
+__global__ void k_dt_finalize(DtArgs args, DevScalars *sc) { dt_finalize(args, sc); }
 
 // Adjust_DT(mesostep=.true.), the FAST_DT branch of src/Adjust_dt.f90:96-135:
 // the maxima over the FP32 met step `vx,vy,vz` (m/s, [k][j][i] without
@@ -214,13 +286,27 @@ __global__ void __launch_bounds__(256) k_cfl_meso(Layout L, int latlon, const fl
 // The FAST_DT step dt of src/MesoInterpolater.f90:250-258: interpolated
 // between the met steps' dt (no DT_MIN rounding), then clipped to the next
 // write time and the end of the simulation.
+// Every thread forms it, thread 0 stores it, and (dtv not null) all write dt/kappa.
 __global__ void k_fast_dt(double frac, double eps_small, double time, double next_write_time, double simtime,
-                          DevScalars *sc) {
+                          const double *__restrict__ kap, double *__restrict__ dtv, int dtv_len, DevScalars *sc) {
   const double last = sc->dt_meso_last, next = sc->dt_meso_next;
   double dt = last + (next - last) * frac;
   if ((next_write_time - time) > eps_small && (next_write_time - time) < dt) dt = next_write_time - time;
   if (time + dt > simtime) dt = simtime - time;
-  sc->dt = dt;
+  if (threadIdx.x == 0) sc->dt = dt;
+  if (dtv)
+    for (int t = threadIdx.x; t < dtv_len; t += blockDim.x) dtv[t] = dt / kap[t];
+}
+
+// dt/kappa's buffer for a kernel that forms dt and, where kappa's table is
+// small (a projected grid's; one block forms it within a microsecond or two),
+// dt/kappa with it; null where k_dtv is left to do it.  The caller's entry
+// point advances dt_stamp after the launch.
+double *claim_dtv(a3g_ctx *ctx) {
+  if (!ctx->have_geometry || ctx->kappa_len > 2048) return nullptr;
+  ctx->dtv_valid = true;
+  ctx->dtv_stamp = ctx->dt_stamp + 1;
+  return ctx->dtv_buf;
 }
 
 int launch_cfl_maxima_meso(a3g_ctx *ctx, int slot) {
@@ -247,88 +333,80 @@ int launch_cfl_maxima_meso_ptr(a3g_ctx *ctx, const float *m) {
 
 int launch_fast_dt(a3g_ctx *ctx, double frac, double time, double next_write_time, double simtime) {
   tbegin(ctx, A3G_K_OTHER);
-  k_fast_dt<<<1, 1, 0, ctx->stream>>>(frac, ctx->prm.eps_small, time, next_write_time, simtime, ctx->sc);
+  k_fast_dt<<<1, 256, 0, ctx->stream>>>(frac, ctx->prm.eps_small, time, next_write_time, simtime, ctx->kappa.p,
+                                        claim_dtv(ctx), (int)ctx->kappa_len, ctx->sc);
   tend(ctx);
   A3G_LAUNCH_CHECK(ctx);
   return A3G_OK;
 }
 
-int launch_cfl_maxima(a3g_ctx *ctx) {
+static DtArgs dt_args(const a3g_ctx *ctx, int n_gs_aloft, double time, double next_write_time, double simtime,
+                      int fresh, int meso) {
+  return DtArgs{ctx->grid.latlon,  ctx->prm.use_diffusion, ctx->prm.use_cn,  n_gs_aloft,       ctx->grid.dx,
+                ctx->grid.dy,      ctx->prm.cfl,           ctx->prm.dt_min,  ctx->prm.dt_max,  ctx->prm.imp_dt_fac,
+                ctx->prm.eps_small, time,                  next_write_time,  simtime,          fresh,
+                meso};
+}
+
+// blocks of k_cfl: two rows a warp at least, and a few blocks per SM
+static int cfl_blocks(const Layout &L) {
+  const int n = (L.ny * L.nz + 15) / 16;
+  return n < CFL_BLOCKS ? n : CFL_BLOCKS;
+}
+
+static int run_cfl(a3g_ctx *ctx, int finish, const DtArgs &args, double *dtv) {
   const Layout &L = ctx->L;
-  A3G_CUDA(cudaMemsetAsync(ctx->sc->vmax, 0, sizeof(ctx->sc->vmax), ctx->stream));
+  tbegin(ctx, A3G_K_CFL);
+  k_cfl<<<cfl_blocks(L), 256, 0, ctx->stream>>>(L, ctx->grid.latlon, ctx->vx, ctx->vy, ctx->vz, ctx->vf, ctx->snx,
+                                               ctx->sny, ctx->kappa, ctx->dz_vec, ctx->cfl_part,
+                                               ctx->block_count + 1, finish, args, dtv, (int)ctx->kappa_len, ctx->sc);
+  tend(ctx);
+  A3G_LAUNCH_CHECK(ctx);
+  return A3G_OK;
+}
+
+int launch_cfl_maxima(a3g_ctx *ctx) { return run_cfl(ctx, 0, dt_args(ctx, 0, 0.0, 0.0, 0.0, 0, 0), nullptr); }
+
+// The diffusion time limit, formed the first time a dt needs it; *fresh is 1
+// when it was formed now.
+static int diffusion_limit(a3g_ctx *ctx, int *fresh) {
+  const Layout &L = ctx->L;
+  *fresh = 0;
+  if (!ctx->prm.use_diffusion || ctx->h_sc->have_diffuse) return A3G_OK;
   const long ncell = (long)L.nx * L.ny * L.nz;
   int blocks = (int)((ncell + 255) / 256);
   if (blocks > 148 * 8) blocks = 148 * 8;
+  const double init = ctx->prm.dt_max;
+  A3G_CUDA(cudaMemcpyAsync(&ctx->sc->time_diffuse, &init, sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
   tbegin(ctx, A3G_K_CFL);
-  k_cfl<<<blocks, 256, 0, ctx->stream>>>(L, ctx->grid.latlon, ctx->vx, ctx->vy, ctx->vz, ctx->vf,
-                                         ctx->snx, ctx->sny, ctx->kappa, ctx->dz_vec, ctx->sc);
+  k_diff_limit<<<blocks, 256, 0, ctx->stream>>>(L, ctx->snx, ctx->sny, ctx->snz, ctx->kappa, ctx->kx, ctx->ky,
+                                                ctx->kz, ctx->sc);
   tend(ctx);
   A3G_LAUNCH_CHECK(ctx);
+  *fresh = 1;
+  ctx->h_sc->have_diffuse = 1;  // host mirror; the device flag is set by dt_finalize
   return A3G_OK;
 }
 
 // dt from maxima already in sc->vmax (local, or set from an all-reduce).
 int launch_dt_from_maxima(a3g_ctx *ctx, int n_gs_aloft, double time, double next_write_time,
                           double simtime, int meso) {
-  const Layout &L = ctx->L;
-  const long ncell = (long)L.nx * L.ny * L.nz;
-  int blocks = (int)((ncell + 255) / 256);
-  if (blocks > 148 * 8) blocks = 148 * 8;
-  int fresh = 0;
-  if (ctx->prm.use_diffusion && !ctx->h_sc->have_diffuse) {
-    const double init = ctx->prm.dt_max;
-    A3G_CUDA(cudaMemcpyAsync(&ctx->sc->time_diffuse, &init, sizeof(double), cudaMemcpyHostToDevice,
-                             ctx->stream));
-    tbegin(ctx, A3G_K_CFL);
-    k_diff_limit<<<blocks, 256, 0, ctx->stream>>>(L, ctx->snx, ctx->sny, ctx->snz, ctx->kappa,
-                                                  ctx->kx, ctx->ky, ctx->kz, ctx->sc);
-    tend(ctx);
-    A3G_LAUNCH_CHECK(ctx);
-    fresh = 1;
-    ctx->h_sc->have_diffuse = 1;
-  }
+  int fresh;
+  int rc = diffusion_limit(ctx, &fresh);
+  if (rc) return rc;
   tbegin(ctx, A3G_K_OTHER);
-  k_dt_finalize<<<1, 1, 0, ctx->stream>>>(
-      ctx->grid.latlon, ctx->prm.use_diffusion, ctx->prm.use_cn, n_gs_aloft, ctx->grid.dx,
-      ctx->grid.dy, ctx->prm.cfl, ctx->prm.dt_min, ctx->prm.dt_max, ctx->prm.imp_dt_fac,
-      ctx->prm.eps_small, time, next_write_time, simtime, fresh, meso, ctx->sc);
+  k_dt_finalize<<<1, 1, 0, ctx->stream>>>(dt_args(ctx, n_gs_aloft, time, next_write_time, simtime, fresh, meso),
+                                          ctx->sc);
   tend(ctx);
   A3G_LAUNCH_CHECK(ctx);
   return A3G_OK;
 }
 
 int launch_cfl(a3g_ctx *ctx, double time, double next_write_time, double simtime) {
-  const Layout &L = ctx->L;
-  A3G_CUDA(cudaMemsetAsync(ctx->sc->vmax, 0, sizeof(ctx->sc->vmax), ctx->stream));
-  const long ncell = (long)L.nx * L.ny * L.nz;
-  int blocks = (int)((ncell + 255) / 256);
-  if (blocks > 148 * 8) blocks = 148 * 8;
-  tbegin(ctx, A3G_K_CFL);
-  k_cfl<<<blocks, 256, 0, ctx->stream>>>(L, ctx->grid.latlon, ctx->vx, ctx->vy, ctx->vz, ctx->vf,
-                                         ctx->snx, ctx->sny, ctx->kappa, ctx->dz_vec, ctx->sc);
-  tend(ctx);
-  A3G_LAUNCH_CHECK(ctx);
-  int fresh = 0;
-  if (ctx->prm.use_diffusion && !ctx->h_sc->have_diffuse) {
-    const double init = ctx->prm.dt_max;
-    A3G_CUDA(cudaMemcpyAsync(&ctx->sc->time_diffuse, &init, sizeof(double), cudaMemcpyHostToDevice,
-                             ctx->stream));
-    tbegin(ctx, A3G_K_CFL);
-    k_diff_limit<<<blocks, 256, 0, ctx->stream>>>(L, ctx->snx, ctx->sny, ctx->snz, ctx->kappa,
-                                                  ctx->kx, ctx->ky, ctx->kz, ctx->sc);
-    tend(ctx);
-    A3G_LAUNCH_CHECK(ctx);
-    fresh = 1;
-    ctx->h_sc->have_diffuse = 1;  // host mirror; the device flag is set by finalize
-  }
-  tbegin(ctx, A3G_K_OTHER);
-  k_dt_finalize<<<1, 1, 0, ctx->stream>>>(
-      ctx->grid.latlon, ctx->prm.use_diffusion, ctx->prm.use_cn, ctx->n_gs_aloft, ctx->grid.dx,
-      ctx->grid.dy, ctx->prm.cfl, ctx->prm.dt_min, ctx->prm.dt_max, ctx->prm.imp_dt_fac,
-      ctx->prm.eps_small, time, next_write_time, simtime, fresh, 0, ctx->sc);
-  tend(ctx);
-  A3G_LAUNCH_CHECK(ctx);
-  return A3G_OK;
+  int fresh;
+  int rc = diffusion_limit(ctx, &fresh);
+  if (rc) return rc;
+  return run_cfl(ctx, 1, dt_args(ctx, ctx->n_gs_aloft, time, next_write_time, simtime, fresh, 0), claim_dtv(ctx));
 }
 
 // ---------------------------------------------------------------------------
@@ -362,126 +440,119 @@ __device__ __forceinline__ DD dd_shfl(DD v, int o) {
 // 2 yz1*kappa(0,:,:), 3 yz2*kappa(nx+1,:,:), 4 xz1*kappa(:,0,:),
 // 5 xz2*kappa(:,ny+1,:), 6 xy2*kappa(:,:,nz+1).
 constexpr int NJOBS = 7;
-constexpr int TOT_BLOCKS = 296;
 
+// nb blocks a grain for the airborne mass, fb for each face; the last block of
+// the grid to finish combines the partial sums in a fixed order and writes the
+// ns*NJOBS results to `out` (pinned host memory).
+// Airborne mass: a warp takes a row, a lane eight cells of it at a time (four
+// 16-byte loads in flight), added pairwise in double, times kappa -- once when
+// it does not vary along i -- and carried in double-double: a relative error of
+// three roundings per term, far inside the 1e-13 the totals keep.
+// Bound by the read of the level where that is large: 720x360x60, 10 grains,
+// 349 -> 205 us; and by latency where it is small, in which every face took 296
+// blocks and the combination a kernel and a copy of their own: 93x131x37, 2
+// grains, 32 -> 9 us.
 __global__ void __launch_bounds__(256) k_totals(Layout L, const double *__restrict__ c,
                                                 Geo3 kap, const double *__restrict__ yz1,
                                                 const double *__restrict__ yz2,
                                                 const double *__restrict__ xz1,
                                                 const double *__restrict__ xz2,
                                                 const double *__restrict__ xy1,
-                                                const double *__restrict__ xy2,
-                                                double *__restrict__ part) {
-  // job is the slowest grid index: the airborne-mass blocks of every grain
-  // are resident together (more loads in flight) before the small face sums
-  const int job = blockIdx.z, g = blockIdx.y;
+                                                const double *__restrict__ xy2, int nb, int fb,
+                                                double *__restrict__ part, unsigned *__restrict__ counter,
+                                                double *__restrict__ out) {
+  const int g = blockIdx.y, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   __shared__ double sh[2][8];
   DD acc = {0.0, 0.0};
-  long n;
-  switch (job) {
-    case 0: n = (long)L.nx * L.ny * L.nz; break;
-    case 1: case 6: n = (long)L.nx * L.ny; break;
-    case 2: case 3: n = (long)L.ny * L.nz; break;
-    default: n = (long)L.nx * L.nz; break;
-  }
-  if (job == 0) {
-    // airborne mass: block b sums a contiguous run of the (j,k) rows, threads
-    // along i.  A thread adds its few cells of a row in double (their loads
-    // all in flight at once), times kappa once per row when kappa does not
-    // vary along i, and carries the row terms in double-double: a relative
-    // error of a few ulps per row term, far inside the 1e-13 the totals keep
-    const double *cg = c + (long)g * L.PG;
+  if ((int)blockIdx.x < nb) {
     const int nrow = L.ny * L.nz;
-    const int per = (nrow + (int)gridDim.x - 1) / (int)gridDim.x;
-    const int r0 = (int)blockIdx.x * per, r1 = min(nrow, r0 + per);
-    int j = r0 % L.ny + 1, k = r0 / L.ny + 1;
     const bool row_const = kap.si == 0;
-    const int bd = (int)blockDim.x;
-    for (int r = r0; r < r1; r++) {
-      const double *row = cg + (long)r * L.P;
-      double part = 0.0;
-      for (int i0 = 0; i0 < L.nx; i0 += 4 * bd) {
-        double v[4];
+    for (int r = blockIdx.x * 8 + w; r < nrow; r += nb * 8) {
+      const int j = r % L.ny + 1, k = r / L.ny + 1;
+      const double *row = c + (long)g * L.PG + (long)r * L.P;
+      const double kr = row_const ? kap.at(1, j, k) : 0.0;
+      for (int i0 = 2 * lane; i0 < L.nx; i0 += 256) {
+        double v[8];
 #pragma unroll
         for (int q = 0; q < 4; q++) {
-          const int i = i0 + (int)threadIdx.x + q * bd;
-          v[q] = i < L.nx ? (row_const ? row[i] : row[i] * kap.at(i + 1, j, k)) : 0.0;
+          const int i = i0 + 64 * q;
+          const double2 x = i < L.nx ? *reinterpret_cast<const double2 *>(row + i) : make_double2(0.0, 0.0);
+          v[2 * q] = x.x;
+          v[2 * q + 1] = i + 1 < L.nx ? x.y : 0.0;
         }
+        if (!row_const) {
 #pragma unroll
-        for (int q = 0; q < 4; q++) part = part + v[q];
-      }
-      if (row_const) part = part * kap.at(1, j, k);
-      acc = dd_add(acc, part);
-      if (++j > L.ny) {
-        j = 1;
-        k++;
+          for (int q = 0; q < 8; q++) {
+            const int i = i0 + 64 * (q >> 1) + (q & 1);
+            if (i < L.nx) v[q] = v[q] * kap.at(i + 1, j, k);
+          }
+        }
+        const double s = ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
+        acc = dd_add(acc, row_const ? s * kr : s);
       }
     }
-    n = 0;
-  }
-  for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < n; t += (long)gridDim.x * blockDim.x) {
-    double v;
-    if (job == 1 || job == 6) {
-      const int i = (int)(t % L.nx) + 1, j = (int)(t / L.nx) + 1;
-      const double *a = (job == 1) ? xy1 : xy2;
-      v = a[(long)g * L.nx * L.ny + t] * kap.at(i, j, job == 1 ? 0 : L.nz + 1);
-    } else if (job == 2 || job == 3) {
-      const int j = (int)(t % L.ny) + 1, k = (int)(t / L.ny) + 1;
-      const double *a = (job == 2) ? yz1 : yz2;
-      v = a[(long)g * L.ny * L.nz + t] * kap.at(job == 2 ? 0 : L.nx + 1, j, k);
-    } else {
-      const int i = (int)(t % L.nx) + 1, k = (int)(t / L.nx) + 1;
-      const double *a = (job == 4) ? xz1 : xz2;
-      v = a[(long)g * L.nx * L.nz + t] * kap.at(i, job == 4 ? 0 : L.ny + 1, k);
+  } else {
+    const int f = ((int)blockIdx.x - nb) / fb, b = ((int)blockIdx.x - nb) % fb, job = f + 1;
+    const long n = (job == 1 || job == 6) ? (long)L.nx * L.ny : (job <= 3) ? (long)L.ny * L.nz : (long)L.nx * L.nz;
+    for (long t = b * 256L + threadIdx.x; t < n; t += fb * 256L) {
+      double v;
+      if (job == 1 || job == 6) {
+        const int i = (int)(t % L.nx) + 1, j = (int)(t / L.nx) + 1;
+        v = (job == 1 ? xy1 : xy2)[g * n + t] * kap.at(i, j, job == 1 ? 0 : L.nz + 1);
+      } else if (job <= 3) {
+        const int j = (int)(t % L.ny) + 1, k = (int)(t / L.ny) + 1;
+        v = (job == 2 ? yz1 : yz2)[g * n + t] * kap.at(job == 2 ? 0 : L.nx + 1, j, k);
+      } else {
+        const int i = (int)(t % L.nx) + 1, k = (int)(t / L.nx) + 1;
+        v = (job == 4 ? xz1 : xz2)[g * n + t] * kap.at(i, job == 4 ? 0 : L.ny + 1, k);
+      }
+      acc = dd_add(acc, v);
     }
-    acc = dd_add(acc, v);
   }
   for (int o = 16; o > 0; o >>= 1) acc = dd_add(acc, dd_shfl(acc, o));
-  const int w = threadIdx.x >> 5;
-  if ((threadIdx.x & 31) == 0) { sh[0][w] = acc.hi; sh[1][w] = acc.lo; }
+  if (lane == 0) { sh[0][w] = acc.hi; sh[1][w] = acc.lo; }
   __syncthreads();
+  const int nx = gridDim.x;
   if (threadIdx.x == 0) {
     DD s = {0.0, 0.0};
-    for (int q = 0; q < (int)(blockDim.x >> 5); q++) s = dd_add(s, DD{sh[0][q], sh[1][q]});
-    const long o = (((long)g * NJOBS + job) * gridDim.x + blockIdx.x) * 2;
+    for (int q = 0; q < 8; q++) s = dd_add(s, DD{sh[0][q], sh[1][q]});
+    const long o = ((long)g * nx + blockIdx.x) * 2;
     part[o] = s.hi;
     part[o + 1] = s.lo;
   }
-}
-
-// one warp per (g, job): lanes take every 32nd block partial, then a fixed
-// shuffle tree (the same order on every run)
-__global__ void k_totals_final(int ns, int nblk, const double *__restrict__ part,
-                               double *__restrict__ out) {
-  const int t = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;  // (g, job)
-  if (t >= ns * NJOBS) return;  // whole warps
-  DD s = {0.0, 0.0};
-  for (int b = lane; b < nblk; b += 32) {
-    const long o = ((long)t * nblk + b) * 2;
-    s = dd_add(s, DD{part[o], part[o + 1]});
+  if (!last_block(counter, gridDim.x * gridDim.y)) return;
+  // a warp per (g, job): lanes take every 32nd partial, then a fixed shuffle tree (the same order on every run)
+  for (int t = w; t < L.ns * NJOBS; t += 8) {
+    const int gg = t / NJOBS, job = t % NJOBS;
+    const int b0 = job == 0 ? 0 : nb + (job - 1) * fb, b1 = job == 0 ? nb : b0 + fb;
+    DD s = {0.0, 0.0};
+    for (int b = b0 + lane; b < b1; b += 32) {
+      const double *p = part + ((long)gg * nx + b) * 2;
+      s = dd_add(s, DD{__ldcg(p), __ldcg(p + 1)});
+    }
+    for (int o = 16; o > 0; o >>= 1) s = dd_add(s, dd_shfl(s, o));
+    if (lane == 0) out[t] = s.hi + s.lo;
   }
-  for (int o = 16; o > 0; o >>= 1) s = dd_add(s, dd_shfl(s, o));
-  if (lane == 0) out[t] = s.hi + s.lo;  // out[g*NJOBS + job]
 }
 
-// the partial sums of the totals, copied (asynchronously) to h_dst
-// (ns*NJOBS doubles of pinned memory)
+// The totals' sums, written to h_dst (ns*NJOBS doubles of pinned memory) by the
+// time the stream gets past this launch.
 int launch_totals_partials(a3g_ctx *ctx, double *h_dst) {
   const Layout &L = ctx->L;
-  const int ns = L.ns;
-  dim3 grid(TOT_BLOCKS, ns, NJOBS);
+  const int rows = L.ny * L.nz;
+  // four rows a warp at least, eight blocks per SM at most; 4096 face cells a block, 16 blocks at most
+  int nb = (rows + 31) / 32;
+  const int most = 148 * 8 / L.ns > 1 ? 148 * 8 / L.ns : 1;
+  if (nb > most) nb = most;
+  const long face = (long)L.nx * (L.ny > L.nz ? L.ny : L.nz) > (long)L.ny * L.nz
+                        ? (long)L.nx * (L.ny > L.nz ? L.ny : L.nz) : (long)L.ny * L.nz;
+  const int fb = face > 15 * 4096 ? 16 : (int)(face / 4096) + 1;
   tbegin(ctx, A3G_K_TOTALS);
-  k_totals<<<grid, 256, 0, ctx->stream>>>(L, ctx->c0, ctx->kappa, ctx->out_yz1, ctx->out_yz2,
-                                          ctx->out_xz1, ctx->out_xz2, ctx->out_xy1, ctx->out_xy2,
-                                          ctx->red_buf);
+  k_totals<<<dim3(nb + 6 * fb, L.ns), 256, 0, ctx->stream>>>(
+      L, ctx->c0, ctx->kappa, ctx->out_yz1, ctx->out_yz2, ctx->out_xz1, ctx->out_xz2, ctx->out_xy1, ctx->out_xy2, nb,
+      fb, ctx->red_buf, ctx->block_count, h_dst);
   tend(ctx);
   A3G_LAUNCH_CHECK(ctx);
-  double *fin = ctx->red_buf + (size_t)2 * TOT_BLOCKS * NJOBS * ns;
-  tbegin(ctx, A3G_K_TOTALS);
-  k_totals_final<<<(ns * NJOBS * 32 + 127) / 128, 128, 0, ctx->stream>>>(ns, TOT_BLOCKS, ctx->red_buf, fin);
-  tend(ctx);
-  A3G_LAUNCH_CHECK(ctx);
-  A3G_CUDA(cudaMemcpyAsync(h_dst, fin, sizeof(double) * ns * NJOBS, cudaMemcpyDeviceToHost, ctx->stream));
   return A3G_OK;
 }
 
@@ -504,44 +575,6 @@ void totals_volumes(a3g_ctx *ctx, const double *h_src, double *out4, double *mas
   out4[1] = depv;
   out4[2] = outv;
   out4[3] = aloft + depv + outv;
-}
-
-int launch_totals(a3g_ctx *ctx, double *out4, double *mass_aloft) {
-  const Layout &L = ctx->L;
-  const int ns = L.ns;
-  dim3 grid(TOT_BLOCKS, ns, NJOBS);
-  tbegin(ctx, A3G_K_TOTALS);
-  k_totals<<<grid, 256, 0, ctx->stream>>>(L, ctx->c0, ctx->kappa, ctx->out_yz1, ctx->out_yz2,
-                                          ctx->out_xz1, ctx->out_xz2, ctx->out_xy1, ctx->out_xy2,
-                                          ctx->red_buf);
-  tend(ctx);
-  A3G_LAUNCH_CHECK(ctx);
-  double *fin = ctx->red_buf + (size_t)2 * TOT_BLOCKS * NJOBS * ns;
-  tbegin(ctx, A3G_K_TOTALS);
-  k_totals_final<<<(ns * NJOBS * 32 + 127) / 128, 128, 0, ctx->stream>>>(ns, TOT_BLOCKS, ctx->red_buf, fin);
-  tend(ctx);
-  A3G_LAUNCH_CHECK(ctx);
-  A3G_CUDA(cudaMemcpyAsync(ctx->h_tot, fin, sizeof(double) * ns * NJOBS, cudaMemcpyDeviceToHost,
-                           ctx->stream));
-  A3G_CUDA(cudaStreamSynchronize(ctx->stream));
-  // volumes in the reference's order, src/Output_Vars.f90:1285-1290,1395-1401,1440-1456
-  const double rho = ctx->prm.magma_density, km3 = 1.0e9;
-  double aloft = 0.0, depv = 0.0, outv = 0.0;
-  for (int g = 0; g < ns; g++) {
-    const double *r = ctx->h_tot + (size_t)g * NJOBS;
-    if (mass_aloft) mass_aloft[g] = r[0];
-    aloft = aloft + r[0] / rho / km3;
-  }
-  for (int g = 0; g < ns; g++) depv = depv + ctx->h_tot[(size_t)g * NJOBS + 1] / rho / km3;
-  for (int g = 0; g < ns; g++) {
-    const double *r = ctx->h_tot + (size_t)g * NJOBS;
-    outv = outv + (r[2] + r[3] + r[4] + r[5] + r[6]) / rho / km3;
-  }
-  out4[0] = aloft;
-  out4[1] = depv;
-  out4[2] = outv;
-  out4[3] = aloft + depv + outv;
-  return A3G_OK;
 }
 
 // ---------------------------------------------------------------------------
@@ -588,36 +621,50 @@ int launch_plane_flags(a3g_ctx *ctx) {
 // ---------------------------------------------------------------------------
 // winds and source
 // ---------------------------------------------------------------------------
+// A warp takes whole rows (no division per cell), four cells a lane in flight;
+// bound by the 48 B a cell (140x120x40: 13 -> 7 us).
 __global__ void __launch_bounds__(256) k_interp_winds(Layout L, const float *__restrict__ last,
                                                       const float *__restrict__ next, long n, double frac,
                                                       double *__restrict__ vx, double *__restrict__ vy,
                                                       double *__restrict__ vz) {
-  for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < n; t += (long)gridDim.x * blockDim.x) {
-    const int i = (int)(t % L.nx) + 1;
-    const long r = t / L.nx;
-    const int j = (int)(r % L.ny) + 1;
-    const int k = (int)(r / L.ny) + 1;
-    const long c = L.cell(i, j, k);
-    const float dx = next[t] - last[t];
-    const float dy = next[n + t] - last[n + t];
-    const float dz = next[2 * n + t] - last[2 * n + t];
-    vx[c] = ((double)last[t] + (double)dx * frac) * 3.6;
-    vy[c] = ((double)last[n + t] + (double)dy * frac) * 3.6;
-    vz[c] = ((double)last[2 * n + t] + (double)dz * frac) * 3.6;
-  }
+  constexpr int U = 4;
+  const int lane = threadIdx.x & 31, nrow = L.ny * L.nz;
+  for (int r = blockIdx.x * 8 + (threadIdx.x >> 5); r < nrow; r += gridDim.x * 8)
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+      const float *a = last + d * n + (long)r * L.nx, *b = next + d * n + (long)r * L.nx;
+      double *v = (d == 0 ? vx : d == 1 ? vy : vz) + (long)r * L.P;
+      for (int i0 = lane; i0 < L.nx; i0 += 32 * U) {
+        float x[U], y[U];
+#pragma unroll
+        for (int q = 0; q < U; q++) {
+          const bool in = i0 + 32 * q < L.nx;
+          x[q] = in ? a[i0 + 32 * q] : 0.0f;
+          y[q] = in ? b[i0 + 32 * q] : 0.0f;
+        }
+#pragma unroll
+        for (int q = 0; q < U; q++)
+          if (i0 + 32 * q < L.nx) v[i0 + 32 * q] = ((double)x[q] + (double)(y[q] - x[q]) * frac) * 3.6;
+      }
+    }
+}
+
+// the winds between the met steps `last` and `next` (3 FP32 arrays each)
+int launch_interp_pair(a3g_ctx *ctx, const float *last, const float *next, double frac) {
+  const Layout &L = ctx->L;
+  const int rows = (L.ny * L.nz + 7) / 8;
+  tbegin(ctx, A3G_K_WINDS);
+  k_interp_winds<<<rows < 148 * 8 ? rows : 148 * 8, 256, 0, ctx->stream>>>(
+      L, last, next, (long)L.nx * L.ny * L.nz, frac, ctx->vx, ctx->vy, ctx->vz);
+  tend(ctx);
+  A3G_LAUNCH_CHECK(ctx);
+  return A3G_OK;
 }
 
 int launch_interp_winds(a3g_ctx *ctx, double frac) {
   const long n = ctx->met_n;
-  int blocks = (int)((n + 255) / 256);
-  if (blocks > 148 * 16) blocks = 148 * 16;
-  tbegin(ctx, A3G_K_WINDS);
-  k_interp_winds<<<blocks, 256, 0, ctx->stream>>>(ctx->L, ctx->met + (size_t)3 * n * ctx->met_last,
-                                                  ctx->met + (size_t)3 * n * ctx->met_next, n, frac, ctx->vx,
-                                                  ctx->vy, ctx->vz);
-  tend(ctx);
-  A3G_LAUNCH_CHECK(ctx);
-  return A3G_OK;
+  return launch_interp_pair(ctx, ctx->met + (size_t)3 * n * ctx->met_last, ctx->met + (size_t)3 * n * ctx->met_next,
+                            frac);
 }
 
 // Calc_Vmod_Topo (src/Topography.f90:2138-2166) on the interior, fused with
@@ -1040,17 +1087,47 @@ int launch_output_vars(a3g_ctx *ctx, double time, double *load, double *maxh, do
 // ---------------------------------------------------------------------------
 // NetCDF output arrays and restart (src/write_NETCDF.f90): FP32 (op = 4,
 // src/Ash3d_VariableModules.f90:31) arrays with x fastest, the layout the
-// writer passes to nf90_put_var.  One thread per cell of a row; blockIdx.y =
-// j, blockIdx.z strides over the (k, g) planes.
+// writer passes to nf90_put_var.
 // ---------------------------------------------------------------------------
-// ashcon(i,j,k,g) = real(concen_pd(i,j,k,g,ts1), kind=op) (:3296-3298)
-__global__ void k_pack_ashcon(Layout L, const double *__restrict__ c, float *__restrict__ ashcon) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = blockIdx.y;
-  if (i >= L.nx) return;
-  for (int kg = blockIdx.z; kg < L.nz * L.ns; kg += gridDim.z) {
-    const int k = kg % L.nz, g = kg / L.nz;
-    ashcon[((long)kg * L.ny + j) * L.nx + i] = __double2float_rn(c[(long)g * L.PG + L.cell(i + 1, j + 1, k + 1)]);
+// ashcon(i,j,k,g) = real(concen_pd(i,j,k,g,ts1), kind=op) (:3296-3298), and
+// NC_RestartFile_LoadConcen (:3701-3707): concen_pd(i,j,k,g) = real(ashcon, ip).
+// A warp takes whole rows (the level's pitch P, the array's nx), eight cells a
+// lane in flight; bound by the 12 B a cell.  720x360x60, 10 grains: 620 -> 330
+// us each way against a block per 256 cells.
+constexpr int NC_U = 8;
+__global__ void __launch_bounds__(256) k_pack_ashcon(Layout L, const double *__restrict__ c,
+                                                     float *__restrict__ ashcon) {
+  const int lane = threadIdx.x & 31;
+  const long nrow = (long)L.ny * L.nz * L.ns;
+  for (long r = blockIdx.x * 8L + (threadIdx.x >> 5); r < nrow; r += gridDim.x * 8L) {
+    const double *src = c + r * L.P;
+    float *dst = ashcon + r * L.nx;
+    for (int i0 = lane; i0 < L.nx; i0 += 32 * NC_U) {
+      double v[NC_U];
+#pragma unroll
+      for (int q = 0; q < NC_U; q++) v[q] = i0 + 32 * q < L.nx ? src[i0 + 32 * q] : 0.0;
+#pragma unroll
+      for (int q = 0; q < NC_U; q++)
+        if (i0 + 32 * q < L.nx) dst[i0 + 32 * q] = __double2float_rn(v[q]);
+    }
+  }
+}
+
+__global__ void __launch_bounds__(256) k_unpack_ashcon(Layout L, const float *__restrict__ ashcon,
+                                                       double *__restrict__ c) {
+  const int lane = threadIdx.x & 31;
+  const long nrow = (long)L.ny * L.nz * L.ns;
+  for (long r = blockIdx.x * 8L + (threadIdx.x >> 5); r < nrow; r += gridDim.x * 8L) {
+    const float *src = ashcon + r * L.nx;
+    double *dst = c + r * L.P;
+    for (int i0 = lane; i0 < L.nx; i0 += 32 * NC_U) {
+      float v[NC_U];
+#pragma unroll
+      for (int q = 0; q < NC_U; q++) v[q] = i0 + 32 * q < L.nx ? src[i0 + 32 * q] : 0.0f;
+#pragma unroll
+      for (int q = 0; q < NC_U; q++)
+        if (i0 + 32 * q < L.nx) dst[i0 + 32 * q] = (double)v[q];
+    }
   }
 }
 
@@ -1070,17 +1147,6 @@ __global__ void k_pack_depocon(Layout L, const double *__restrict__ xy1, const d
   }
 }
 
-// NC_RestartFile_LoadConcen (:3701-3707): concen_pd(i,j,k,g) = real(ashcon, ip)
-__global__ void k_unpack_ashcon(Layout L, const float *__restrict__ ashcon, double *__restrict__ c) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = blockIdx.y;
-  if (i >= L.nx) return;
-  for (int kg = blockIdx.z; kg < L.nz * L.ns; kg += gridDim.z) {
-    const int k = kg % L.nz, g = kg / L.nz;
-    c[(long)g * L.PG + L.cell(i + 1, j + 1, k + 1)] = (double)ashcon[((long)kg * L.ny + j) * L.nx + i];
-  }
-}
-
 // outflow_xy1_pd(i,j,g) = DepositGranularity(i,j,g) = real(depocon(i,j,g), ip)
 __global__ void k_unpack_depocon(Layout L, const float *__restrict__ depocon, double *__restrict__ xy1) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1096,10 +1162,15 @@ static dim3 netcdf_grid(const Layout &L, int planes) {
   return dim3((L.nx + 255) / 256, L.ny, planes < 65535 ? planes : 65535);
 }
 
+static unsigned row_blocks(const Layout &L) {  // eight rows a block, eight blocks per SM
+  const long n = ((long)L.ny * L.nz * L.ns + 7) / 8;
+  return (unsigned)(n < 148 * 8 ? n : 148 * 8);
+}
+
 int launch_netcdf_pack(a3g_ctx *ctx, float *ashcon, float *depocon) {
   const Layout &L = ctx->L;
   tbegin(ctx, A3G_K_OTHER);
-  if (ashcon) k_pack_ashcon<<<netcdf_grid(L, L.nz * L.ns), 256, 0, ctx->stream>>>(L, ctx->c0, ashcon);
+  if (ashcon) k_pack_ashcon<<<row_blocks(L), 256, 0, ctx->stream>>>(L, ctx->c0, ashcon);
   if (depocon)
     k_pack_depocon<<<netcdf_grid(L, L.ns), 256, 0, ctx->stream>>>(L, ctx->out_xy1, ctx->dz_vec, depocon);
   tend(ctx);
@@ -1110,7 +1181,7 @@ int launch_netcdf_pack(a3g_ctx *ctx, float *ashcon, float *depocon) {
 int launch_netcdf_unpack(a3g_ctx *ctx, const float *ashcon, const float *depocon) {
   const Layout &L = ctx->L;
   tbegin(ctx, A3G_K_OTHER);
-  if (ashcon) k_unpack_ashcon<<<netcdf_grid(L, L.nz * L.ns), 256, 0, ctx->stream>>>(L, ashcon, ctx->c0);
+  if (ashcon) k_unpack_ashcon<<<row_blocks(L), 256, 0, ctx->stream>>>(L, ashcon, ctx->c0);
   if (depocon) k_unpack_depocon<<<netcdf_grid(L, L.ns), 256, 0, ctx->stream>>>(L, depocon, ctx->out_xy1);
   tend(ctx);
   A3G_LAUNCH_CHECK(ctx);
