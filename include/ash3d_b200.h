@@ -398,7 +398,8 @@ int a3g_kernel_times(a3g_ctx *ctx, double *ms, uint64_t *count);
  * the concentration and wind from chunks that TMA tensor copies stage in
  * shared memory (default for y and z; where the geometry varies along i or
  * the fall speed within a grain, variant 6 runs variant 1).  dir 5: the adjoint advection sweeps,
- * variant 0 four-cell blocks (default), 1 one cell per thread.  All variants
+ * variant 0 marches fed by TMA chunks (default; four-cell blocks where the
+ * geometry varies along i), 1 one cell per thread.  All variants
  * produce identical results; only their speed differs. */
 int a3g_set_variant(a3g_ctx *ctx, int32_t dir, int32_t variant);
 int a3g_get_variant(a3g_ctx *ctx, int32_t dir, int32_t *variant);

@@ -55,6 +55,26 @@ template <int LIM>
 __device__ __forceinline__ void lim_coef(double dq, double dqu, double eps, double &a, double &b) {
   if (LIM == A3G_LIM_LAXWEN) { a = 1.0; b = 0.0; return; }
   if (LIM == A3G_LIM_BW) { a = 0.0; b = 1.0; return; }
+  if (LIM == A3G_LIM_SUPERBEE) {
+    // the branch by comparison, without the quotient: (a, b) is (0, 0) for
+    // theta < 0, (0, 1) at 0, (0, 2) on (0, 1/2], (1, 0) between 1/2 and 1,
+    // (0, 1) on [1, 2] and (2, 0) above.  RN(dqu/dq) equals 1/2, 1 or 2 only
+    // when the exact quotient does, and lies on the same side of them; it is 0
+    // for a dqu that is not only where the quotient underflows.
+    const double u = fabs(dqu), d = fabs(dq);
+    const bool same = (__double2hiint(dqu) ^ __double2hiint(dq)) >= 0;
+    if (fabs(dq) < eps) {  // no cycle (NOCYCLE): the clamp
+      a = same ? 2.0 : 0.0;
+      b = 0.0;
+      return;
+    }
+    const bool le_half = u + u <= d, lt1 = u < d, le2 = u <= d + d;
+    a = le_half ? 0.0 : lt1 ? 1.0 : le2 ? 0.0 : 2.0;
+    b = le_half ? 2.0 : lt1 ? 0.0 : le2 ? 1.0 : 0.0;
+    if (!same) a = b = 0.0;
+    if (u < 0x1p-700 && (u == 0.0 || dqu / dq == 0.0)) b = 1.0;
+    return;
+  }
   const bool clamp = fabs(dqu) > 3.0 * fabs(dq) || fabs(dq) < eps;
   const double th = clamp ? copysign(3.0, dqu * dq) : div_rn(dqu, dq);
   double phi, dphi;
@@ -203,7 +223,7 @@ __global__ void __launch_bounds__(256) k_adj_advect(Layout L, int nocycle, doubl
 // and forms each of the V+3 interfaces they read (c0-1 .. c0+V+1) once,
 // instead of the four a cell-per-thread gather forms for every cell; the
 // expressions and their order are lam_at's, so the results are the same
-// bits.  Not x-periodic (the wrapped ghosts stay with the gather kernel).
+// bits.  Runs where the marches below do not.  Not x-periodic (the wrapped ghosts stay with the gather kernel).
 // DIR 0: lanes are consecutive blocks along i; DIR 1, 2: lanes along i.
 template <int DIR, int LIM, int V, bool CK>
 __device__ __forceinline__ void adj_block_body(const Layout &L, int nocycle, double eps, int n, int c0, long st,
@@ -346,6 +366,352 @@ __global__ void __launch_bounds__(128) k_adj_advect_blk(Layout L, int nocycle, d
                                       pvf, vf.sk, gsig, gdtv, lam_lo0);
 }
 
+// ---------------------------------------------------------------------------
+// Marched form of the adjoint sweep (the default; not x-periodic): a lane walks
+// its line and forms each interface once, in lam_at's expressions, so the
+// results are the same bits.  Reading cell x completes interface J = x-1
+// (which needs q(J+1)), then lam_dq(J-1), then lam_q(J-2).
+// ---------------------------------------------------------------------------
+struct AdjMarch {
+  double q, d0, dm;        // q(J), dq(J), dq(J-1)
+  double v, vm;            // vel(J), vel(J-1)
+  double lam, lamm, t;     // lam(J), lam(J-1), t(J-1)
+  double pos, neg;         // max, min of 0 and usig(J-1)
+  double e1, e2;           // b*e of J-1 and of J-2 where their upwind side is the right
+  double base, ldq, L1;    // lam_dq(J-1) without its neighbours' terms, lam_dq(J-2), lam_q(J-2) without lam_dq
+};
+
+// Takes cell J+1 (its q, vel, lam) with sigma(J)/2 and dt/kappa(J); returns lam_q(J-2).
+template <int LIM>
+__device__ __forceinline__ double adj_march_step(AdjMarch &m, double qx, double vx, double lx, double hs, double dtv,
+                                                 double eps, int nocycle) {
+  const double d1 = qx - m.q;
+  const double us = (m.vm + m.v) * hs;
+  const double p = pos_part(us), n = neg_part(us);
+  const bool up = us > 0.0;
+  const double tJ = -(dtv * m.lam);
+  double ea = 0.0, eb = 0.0;
+  if (LIM != A3G_LIM_NONE && (nocycle || !(fabs(m.d0) <= eps))) {
+    const double aus = fabs(us);
+    const double e = 0.5 * aus * (1.0 - dtv * aus) * (m.t - tJ);  // t(J-1) - t(J)
+    double a, b;
+    lim_coef<LIM>(m.d0, up ? m.dm : d1, eps, a, b);
+    ea = a * e;
+    eb = b * e;
+  }
+  const double ldq = m.base + (up ? eb : 0.0) + m.e2;  // lam_dq(J-1)
+  const double out = m.L1 + m.ldq - ldq;
+  m.L1 = m.lamm + (n - m.neg) * m.t + (p - m.pos) * m.t;
+  m.base = p * tJ + n * m.t + ea;
+  m.ldq = ldq;
+  m.e2 = m.e1;
+  m.e1 = up ? 0.0 : eb;
+  m.pos = p;
+  m.neg = n;
+  m.lamm = m.lam;
+  m.lam = lx;
+  m.t = tJ;
+  m.vm = m.v;
+  m.v = vx;
+  m.dm = m.d0;
+  m.d0 = d1;
+  m.q = qx;
+  return out;
+}
+
+// State before cell x = s0 is taken (J = s0-1) from values by index.
+template <class Q, class V, class T, class L>
+__device__ __forceinline__ AdjMarch adj_march_start(int s0, Q q, V v, T t, L lam) {
+  AdjMarch m;
+  const double qa = q(s0 - 2);
+  m.q = q(s0 - 1);
+  m.d0 = m.q - qa;
+  m.dm = qa - q(s0 - 3);
+  m.v = v(s0 - 1);
+  m.vm = v(s0 - 2);
+  m.lam = lam(s0 - 1);
+  m.lamm = 0.0;
+  m.t = t(s0 - 2);
+  m.pos = m.neg = m.e1 = m.e2 = m.base = m.ldq = m.L1 = 0.0;
+  return m;
+}
+
+// Columns (y and z): k_advect_colt's mapping and chunks, with lam as a third
+// array of the chunk.  140x120x40, 4 grains: y 48 -> 29 us, z 61 -> 29 us
+// against blocks of four cells, which form 7 interfaces for 4 cells (and took
+// a certified quotient for each).
+constexpr int ADJ_WARPS = 2;
+constexpr int ADJ_BUF_D = 3 * ACH * 32 + 2 * ACH;  // q, vel, lam; pairs (sigma/2, dt/kappa)
+
+template <int DIR, int LIM>
+__global__ void __launch_bounds__(32 * ADJ_WARPS, 8) k_adj_colt(
+    const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tv,
+    const __grid_constant__ CUtensorMap tl, Layout L, int nocycle, double eps, int nseg, int seg,
+    const double *__restrict__ cq, const double *__restrict__ lin, double *__restrict__ lout,
+    const double *__restrict__ vel, Geo4 vf, Geo3 sig, Geo3 dtvt, const int32_t *__restrict__ aloft, DevScalars *sc,
+    const double *__restrict__ lam_lo) {
+  extern __shared__ __align__(128) unsigned char adj_smem[];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  uint64_t *bar = reinterpret_cast<uint64_t *>(adj_smem) + 2 * wid;
+  double *wsm = reinterpret_cast<double *>(adj_smem + 128) + (long)wid * 2 * ADJ_BUF_D;
+  const int nother = (DIR == 1) ? L.nz : L.ny;
+  const int nti = (L.nx + 31) >> 5;
+  const long t = (long)blockIdx.x * ADJ_WARPS + wid;
+  if (t >= (long)nti * nother * L.ns * nseg) return;  // whole warps only; no block barrier below
+  const int g = (int)(t % L.ns);
+  long rr = t / L.ns;
+  const int it = (int)(rr % nti);
+  rr /= nti;
+  const int o = (int)(rr % nother) + 1;
+  const int s0 = (int)(rr / nother) * seg + 1;
+  const int a = (it << 5) + lane + 1;
+  const bool valid = a <= L.nx;
+  const int n = (DIR == 1) ? L.ny : L.nz;
+  const int s1 = min(n, s0 + seg - 1);
+  const int st = (DIR == 1) ? (int)L.P : (int)L.PY;
+  const int ac = valid ? a : 1;
+  const long base = (DIR == 1) ? L.cell(ac, 1, o) : L.cell(ac, o, 1);
+  double *po = lout + (long)g * L.PG + base;
+  if (!aloft[g]) {
+    if (valid)
+      for (int c = s0; c <= s1; c++) po[(c - 1) * st] = 0.0;
+    return;
+  }
+  const LineGeo gsig = line_of<DIR>(sig, 1, o), gdtv = line_of<DIR>(dtvt, 1, o);  // constant along i
+  // chunk k holds the cells s0+k*ACH .. and the geometry of the interfaces one before them
+  const int nx_ = s1 + 3 - s0 + 1, nchunk = (nx_ + ACH - 1) / ACH;
+  auto issue = [&](int k) {
+    double *qb = wsm + (k & 1) * ADJ_BUF_D;
+    const int X = s0 + k * ACH;
+    if (lane == 0) {
+      uint64_t *b = &bar[k & 1];
+      mbar_arrive_expect_tx(b, 3u * ACH * 32u * 8u);
+      const int y = (DIR == 1) ? X - 1 : o - 1, z = (DIR == 1) ? o - 1 : X - 1;
+      tma_load_4d(qb, &tq, b, it << 5, y, z, g);
+      tma_load_4d(qb + ACH * 32, &tv, b, it << 5, y, z, 0);
+      tma_load_4d(qb + 2 * ACH * 32, &tl, b, it << 5, y, z, g);
+    }
+    const int J = X + lane - 1;
+    if (lane < ACH && J <= n + 2)  // usig is zero outside interfaces 1 .. n+1
+      reinterpret_cast<double2 *>(qb + 3 * ACH * 32)[lane] =
+          make_double2(J >= 1 && J <= n + 1 ? 0.5 * gsig.at(J) : 0.0, gdtv.at(J));
+  };
+  if (lane == 0) {
+    mbar_init(&bar[0], 1);
+    mbar_init(&bar[1], 1);
+    mbar_init_fence();
+  }
+  __syncwarp();
+  issue(0);
+  const double vf0 = (DIR == 2) ? vf.p[(long)g * vf.sg] : 0.0;  // one fall speed per grain
+  const double *pq = cq + (long)g * L.PG + base, *pl = lin + (long)g * L.PG + base, *pv = vel + base;
+  const double lam0 = (DIR == 2 && lam_lo) ? lam_lo[(long)g * L.nx * L.ny + (long)(o - 1) * L.nx + (ac - 1)] : 0.0;
+  auto Q = [&](int c) { return c >= 1 && c <= n ? pq[(c - 1) * st] : 0.0; };
+  auto V = [&](int c) { return pv[((c < 1 ? 1 : c) - 1) * st] + vf0; };
+  auto Lm = [&](int c) { return c >= 1 ? pl[(c - 1) * st] : c == 0 ? lam0 : 0.0; };
+  auto T = [&](int c) { return c < 0 ? 0.0 : -(gdtv.at(c) * Lm(c)); };
+  AdjMarch m = adj_march_start(s0, Q, V, T, Lm);
+  const double vedge = pv[(n - 1) * st];  // the wind beyond the line
+  po += (long)(s0 - 1) * st;              // cell x-3's place, once x-3 >= s0
+  uint32_t ph = 0u;
+  for (int k = 0, x = s0; k < nchunk; k++) {
+    const int bi = k & 1;
+    if (k + 1 < nchunk) issue(k + 1);
+    if (!mbar_wait(&bar[bi], (ph >> bi) & 1u)) {
+      if (lane == 0) raise_error(sc, A3G_ERR_TIMEOUT, 6);
+      return;
+    }
+    ph ^= 1u << bi;
+    double *qv = wsm + bi * ADJ_BUF_D + lane;
+    if (x <= n + 1 && n + 1 < x + ACH) qv[(ACH + n + 1 - x) * 32] = vedge;
+    __syncwarp();
+    const double2 *gb = reinterpret_cast<const double2 *>(wsm + bi * ADJ_BUF_D + 3 * ACH * 32);
+    const int cnt = min(ACH, s1 + 3 - x + 1);
+    auto step = [&](int e) {
+      const double2 sd = gb[e];
+      const double y = adj_march_step<LIM>(m, qv[e * 32], qv[(ACH + e) * 32] + vf0, qv[(2 * ACH + e) * 32], sd.x, sd.y,
+                                           eps, nocycle);
+      if (x + e - 3 >= s0) {
+        if (valid) *po = y;
+        po += st;
+      }
+    };
+    int e = 0;
+    for (; e + 2 <= cnt; e += 2) {
+      step(e);
+      step(e + 1);
+    }
+    if (e < cnt) step(e);
+    x += ACH;
+    __syncwarp();
+  }
+}
+
+// Rows (x): k_advect_xm's mapping and swizzled chunks, a row per lane.  Chunk
+// k holds the cells s0+8k ..; the new lam of cell x-4 takes the place of cell
+// x's old one, so that a chunk's new values start on an even cell; the first
+// and last chunk of a segment, which also hold other segments' cells, are
+// stored by the lanes.  140x120x40, 4 grains: 133 -> 31 us (the blocks' lanes
+// were four cells apart, a sector each).
+constexpr int AJX_WARP_B = 7 * AXM_BUF;  // 2 concentration, 2 wind, 3 lam buffers
+constexpr int AJX_SMEM = 512 + 512 + ADJ_WARPS * AJX_WARP_B;
+
+template <int LIM>
+__global__ void __launch_bounds__(32 * ADJ_WARPS, 8) k_adj_xm(
+    const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tv,
+    const __grid_constant__ CUtensorMap tl, const __grid_constant__ CUtensorMap to, Layout L, int nocycle, double eps,
+    int nseg, int seg, const double *__restrict__ cq, const double *__restrict__ lin, double *__restrict__ lout,
+    const double *__restrict__ vel, Geo3 sig, Geo3 dtvt, const int32_t *__restrict__ aloft, DevScalars *sc) {
+  extern __shared__ unsigned char ajx_smem[];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  unsigned char *const sm = ajx_smem + ((512u - (smem_u32(ajx_smem) & 511u)) & 511u);  // the swizzle's period
+  uint64_t *bar = reinterpret_cast<uint64_t *>(sm) + 2 * wid;
+  unsigned char *const qbuf = sm + 512 + wid * AJX_WARP_B, *const vbuf = qbuf + 2 * AXM_BUF,
+                *const lbuf = vbuf + 2 * AXM_BUF;
+  const int nrows = L.ny * L.nz;
+  const int ntile = (nrows + 31) >> 5;
+  const long t = (long)blockIdx.x * ADJ_WARPS + wid;
+  if (t >= (long)ntile * L.ns * nseg) return;  // whole warps only; no block barrier below
+  const int g = (int)(t % L.ns);
+  const long rr = t / L.ns;
+  const int r0 = (int)(rr % ntile) * 32;
+  const int s0 = (int)(rr / ntile) * seg + 1;
+  const int n = L.nx, s1 = min(n, s0 + seg - 1);
+  const int r = min(r0 + lane, nrows - 1);
+  const int j = r % L.ny + 1, k = r / L.ny + 1;
+  const long grow = (long)g * nrows;
+  double *const po = lout + (grow + r0) * L.P;
+  if (!aloft[g]) {
+    for (int row = 0; row < min(32, nrows - r0); row++)
+      for (int c = s0 + lane; c <= s1; c += 32) po[(long)row * L.P + (c - 1)] = 0.0;
+    return;
+  }
+  const int nchunk = (s1 + 4 - s0 + 8) >> 3;  // cells s0 .. s1+4
+  auto issue = [&](int c) {  // chunk c; its lam buffer was stored from two chunks ago
+    if (lane == 0) {
+      uint64_t *b = &bar[c & 1];
+      bulk_wait_read1();
+      mbar_arrive_expect_tx(b, 3u * AXM_BUF);
+      tma_load_2d(qbuf + (c & 1) * AXM_BUF, &tq, b, s0 - 1 + 8 * c, (int)(grow + r0));
+      tma_load_2d(vbuf + (c & 1) * AXM_BUF, &tv, b, s0 - 1 + 8 * c, r0);
+      tma_load_2d(lbuf + (c % 3) * AXM_BUF, &tl, b, s0 - 1 + 8 * c, (int)(grow + r0));
+    }
+  };
+  if (lane == 0) {
+    mbar_init(&bar[0], 1);
+    mbar_init(&bar[1], 1);
+    mbar_init_fence();
+  }
+  __syncwarp();
+  issue(0);
+  const double *const pq = cq + (grow + r) * L.P, *const pl = lin + (grow + r) * L.P, *const pv = vel + (long)r * L.P;
+  const double hs = 0.5 * sig.p[(long)(j + 1) * sig.sj + (long)(k + 1) * sig.sk];
+  const double dtv = dtvt.p[(long)(j + 1) * dtvt.sj + (long)(k + 1) * dtvt.sk];
+  auto Q = [&](int c) { return c >= 1 && c <= n ? pq[c - 1] : 0.0; };
+  auto V = [&](int c) { return pv[(c < 1 ? 1 : c) - 1]; };
+  auto Lm = [&](int c) { return c >= 1 ? pl[c - 1] : 0.0; };
+  auto T = [&](int c) { return -(dtv * Lm(c)); };
+  AdjMarch m = adj_march_start(s0, Q, V, T, Lm);
+  const int row_b = lane << 6, row_s = ((lane >> 1) & 3) << 4;
+  auto pair = [&](unsigned char *b, int p) { return reinterpret_cast<double2 *>(b + row_b + ((p << 4) ^ row_s)); };
+  auto cell = [&](unsigned char *b, int e) { return reinterpret_cast<double *>(pair(b, e >> 1)) + (e & 1); };
+  double held = 0.0;  // lam_q of the cell behind the last one computed
+  auto step = [&](double q, double v, double l, double h) {
+    const double y = held;
+    held = adj_march_step<LIM>(m, q, v, l, h, dtv, eps, nocycle);
+    return y;
+  };
+  const bool whole = r0 + 32 <= nrows;
+  uint32_t ph = 0u;
+  for (int c = 0; c < nchunk; c++) {
+    if (c + 1 < nchunk) issue(c + 1);
+    if (!mbar_wait(&bar[c & 1], (ph >> (c & 1)) & 1u)) {
+      if (lane == 0) {
+        raise_error(sc, A3G_ERR_TIMEOUT, 7);
+        bulk_wait0();
+      }
+      return;
+    }
+    ph ^= 1u << (c & 1);
+    unsigned char *const qb = qbuf + (c & 1) * AXM_BUF, *const vb = vbuf + (c & 1) * AXM_BUF,
+                  *const lb = lbuf + (c % 3) * AXM_BUF;
+    const int X = s0 + 8 * c;  // slot e: cell X+e in, cell X+e-4 out
+    if (X + 7 > n) {           // the edge wind, and its negative beyond: usig(n+2) = 0
+      for (int x = max(n + 1, X); x <= min(n + 2, X + 7); x++) *cell(vb, x - X) = x == n + 1 ? pv[n - 1] : -pv[n - 1];
+    }
+    if (X > 1) {
+#pragma unroll 2
+      for (int p = 0; p < 4; p++) {
+        double2 *l = pair(lb, p);
+        const double2 q = *pair(qb, p), v = *pair(vb, p), w = *l;
+        double2 y;
+        y.x = step(q.x, v.x, w.x, hs);
+        y.y = step(q.y, v.y, w.y, hs);
+        *l = y;
+      }
+    } else {  // interface 0 carries nothing
+      for (int e = 0; e < 8; e++) *cell(lb, e) = step(*cell(qb, e), *cell(vb, e), *cell(lb, e), e == 0 ? 0.0 : hs);
+    }
+    fence_proxy_async_smem();
+    __syncwarp();
+    const int o0 = X - 4;  // first cell of the chunk's new values
+    if (whole && o0 >= s0 && o0 + 7 <= s1) {
+      if (lane == 0) {
+        tma_store_2d(&to, lb, o0 - 1, (int)(grow + r0));
+        bulk_commit();
+      }
+    } else {
+      const int e = lane & 7, x = o0 + e;
+#pragma unroll
+      for (int h = 0; h < 8; h++) {
+        const int row = 4 * h + (lane >> 3);
+        if (r0 + row < nrows && x >= s0 && x <= s1)
+          po[(long)row * L.P + (x - 1)] = *reinterpret_cast<const double *>(
+              lb + (row << 6) + ((((e >> 1) ^ ((row >> 1) & 3)) << 4) | ((e & 1) << 3)));
+      }
+      __syncwarp();
+    }
+  }
+  if (lane == 0) bulk_wait0();
+}
+
+// Launches the marched adjoint sweep; false where its conditions (those of the
+// forward marches) do not hold.
+template <int DIR, int LIM>
+static bool launch_adj_march(a3g_ctx *ctx, const double *cq, const double *lin, double *lout, const double *lam_lo) {
+  const Layout &L = ctx->L;
+  CUtensorMap tq, tv, tl, to;
+  if constexpr (DIR == 0) {
+    if (along<0>(ctx->snx) != 0 || along<0>(ctx->dtv) != 0) return false;
+    if (!tensor_map(ctx, cq, TM_QROWS, &tq) || !tensor_map(ctx, ctx->vx, TM_VROWS, &tv) ||
+        !tensor_map(ctx, lin, TM_QROWS, &tl) || !tensor_map(ctx, lout, TM_QROWS, &to))
+      return false;
+    const long nlw = (long)(((long)L.ny * L.nz + 31) / 32) * L.ns;
+    const int want = march_segments(L.nx, nlw);
+    const int seg = (L.nx + want - 1) / want + 7 & ~7;
+    const int nseg = (L.nx + seg - 1) / seg;
+    k_adj_xm<LIM><<<(unsigned)((nlw * nseg + ADJ_WARPS - 1) / ADJ_WARPS), 32 * ADJ_WARPS, AJX_SMEM, ctx->stream>>>(
+        tq, tv, tl, to, L, ctx->prm.nocycle, ctx->prm.eps_thresh, nseg, seg, cq, lin, lout, ctx->vx, ctx->snx,
+        ctx->dtv, ctx->aloft, ctx->sc);
+  } else {
+    const Geo3 &sg = (DIR == 1) ? ctx->sny : ctx->snz;
+    const double *vel = (DIR == 1) ? ctx->vy : ctx->vz;
+    if (sg.si != 0 || ctx->dtv.si != 0) return false;
+    if (DIR == 2 && (ctx->vf.si != 0 || ctx->vf.sj != 0 || ctx->vf.sk != 0)) return false;
+    const int qk = DIR == 1 ? TM_ADV_QY : TM_ADV_QZ, vk = DIR == 1 ? TM_ADV_VY : TM_ADV_VZ;
+    if (!tensor_map(ctx, cq, qk, &tq) || !tensor_map(ctx, vel, vk, &tv) || !tensor_map(ctx, lin, qk, &tl)) return false;
+    const int n = (DIR == 1) ? L.ny : L.nz, nother = (DIR == 1) ? L.nz : L.ny;
+    const long nlw = (long)((L.nx + 31) / 32) * nother * L.ns;
+    const int want = march_segments(n, nlw);
+    const int seg = (n + want - 1) / want, nseg = (n + seg - 1) / seg;
+    const size_t smem = 128 + (size_t)ADJ_WARPS * 2 * ADJ_BUF_D * sizeof(double);
+    k_adj_colt<DIR, LIM><<<(unsigned)((nlw * nseg + ADJ_WARPS - 1) / ADJ_WARPS), 32 * ADJ_WARPS, smem, ctx->stream>>>(
+        tq, tv, tl, L, ctx->prm.nocycle, ctx->prm.eps_thresh, nseg, seg, cq, lin, lout, vel, ctx->vf, sg, ctx->dtv,
+        ctx->aloft, ctx->sc, lam_lo);
+  }
+  return true;
+}
+
 template <int DIR, int LIM>
 static void launch_adj_dir_lim(a3g_ctx *ctx, const double *cq, const double *lin, double *lout,
                                const double *lam_lo) {
@@ -362,7 +728,7 @@ static void launch_adj_dir_lim(a3g_ctx *ctx, const double *cq, const double *lin
     k_adj_advect<DIR, LIM, false><<<grid, dim3(32, 8), 0, ctx->stream>>>(
         L, ctx->prm.nocycle, ctx->prm.eps_thresh, cq, lin, lout, vel, ctx->vf, sig, ctx->dtv, ctx->aloft,
         lam_lo);
-  } else {
+  } else if (!launch_adj_march<DIR, LIM>(ctx, cq, lin, lout, lam_lo)) {
     constexpr int V = 4;
     const int n = (DIR == 0) ? L.nx : (DIR == 1) ? L.ny : L.nz;
     const int nblk = (n + V - 1) / V;
