@@ -158,6 +158,7 @@ struct a3g_ctx {
   std::vector<int32_t> h_aloft;
   int n_gs_aloft;
   a3g::DevScalars *sc;      // device scalars
+  char *pinned;             // the pinned host buffers below
   a3g::DevScalars *h_sc;    // pinned host mirror
   double *red_buf;          // reduction partials
   size_t red_len;
@@ -206,7 +207,9 @@ struct a3g_ctx {
   double *ov_buf;
   double *ov_zcc;
   double ov_cloudcon, ov_cloudload, ov_depo, ov_density;
-  std::vector<double> h_area;  // sigma_nz_pd(1:nx,1:ny,1)
+  std::vector<double> h_area;  // sigma_nz_pd(1:nx,1:ny,1), j fastest
+  char *h_ov;                  // pinned ring the products leave through
+  cudaEvent_t ov_ev[4];        // end of each piece's copy
   // lag-one host loop: pinned rings of the device scalars (a3g_adjust_dt_async
   // / a3g_wait_dt) and of the totals partials (a3g_timestep_totals_async /
   // a3g_totals_get), each slot guarded by an event
@@ -320,7 +323,7 @@ int launch_cloud_load(a3g_ctx *ctx, const double *c, double *out);
 int launch_adj_cloud_load(a3g_ctx *ctx, const double *w, double *lam);
 int launch_vent_column(a3g_ctx *ctx, int ivent, int jvent, const double *lam, double *out);
 int launch_output_vars(a3g_ctx *ctx, double time, double *load, double *maxh, double *minh, double *maxc,
-                       int32_t *mcl, double *dthick, int32_t *mdep, double *carr, double *darr);
+                       int32_t *mcl, double *dthick, int32_t *mdep, uint8_t *cls, double *carr, double *darr);
 int refresh_dtv(a3g_ctx *ctx);
 // The tensor map of kind `kind` over the level at p (encoded on first use,
 // then cached), copied to *out; false when the driver cannot encode it (the

@@ -456,11 +456,11 @@ class Ash3dGPU:
         if not getattr(self, "_ov_params", False):
             self.set_output_params()
         c = self.cfg
-        f = lambda: np.zeros((c.nx, c.ny), order="F")
+        f = lambda: np.empty((c.nx, c.ny), order="F")  # every element is written
         out = dict(cloud_load=f(), max_height=f(), min_height=f(), max_conc=f(), dep_thick=f(),
                    cloud_arrival=f(), dep_arrival=f())
-        mc = np.zeros((c.nx, c.ny), dtype=np.int32, order="F")
-        md = np.zeros((c.nx, c.ny), dtype=np.int32, order="F")
+        mc = np.empty((c.nx, c.ny), dtype=np.int32, order="F")
+        md = np.empty((c.nx, c.ny), dtype=np.int32, order="F")
         areas = np.zeros(7)
         check(self.lib.a3g_output_vars(self.ctx, time, dptr(out["cloud_load"]), dptr(out["max_height"]),
                                        dptr(out["min_height"]), dptr(out["max_conc"]), iptr(mc),
