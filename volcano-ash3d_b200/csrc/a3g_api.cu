@@ -323,6 +323,7 @@ int a3g_destroy(a3g_ctx *ctx) {
   for (double *p : aptrs) if (p) cudaFree(p);
   if (ctx->nc_buf) cudaFree(ctx->nc_buf);
   if (ctx->vfm_sp) cudaFree(ctx->vfm_sp);
+  if (ctx->diff_tab) cudaFree(ctx->diff_tab);
   for (double *p : ctx->snaps) if (p) cudaFree(p);
   if (ctx->met_copy_ev) cudaEventDestroy(ctx->met_copy_ev);
   if (ctx->met_free_ev) cudaEventDestroy(ctx->met_free_ev);
@@ -360,6 +361,7 @@ static int set_geo3(a3g_ctx *ctx, const double *src, long n0, long n1, long n2, 
 
 static int ensure_cn_buf(a3g_ctx *ctx) {
   for (int d = 0; d < 3; d++) ctx->cn_valid[d] = false;  // geometry or diffusivity changed
+  ctx->diff_valid = false;
   if (!ctx->have_geometry || !ctx->have_diffusivity) return A3G_OK;
   size_t len[3], need = 0;
   for (int d = 0; d < 3; d++) {
@@ -994,13 +996,7 @@ int a3g_diffuse_horz(a3g_ctx *ctx, int32_t itime) {
       if ((rc = launch_diffcn_x(ctx))) return rc;
     }
   } else {
-    if (itime % 2 == 0) {
-      if ((rc = launch_diff_x(ctx))) return rc;
-      if ((rc = launch_diff_y(ctx))) return rc;
-    } else {
-      if ((rc = launch_diff_y(ctx))) return rc;
-      if ((rc = launch_diff_x(ctx))) return rc;
-    }
+    if ((rc = launch_diff_horz(ctx, itime % 2 == 0))) return rc;
     ctx->ts1_zeroed = false;
   }
   return A3G_OK;
@@ -1490,6 +1486,22 @@ static int adj_diffuse_dir(a3g_ctx *ctx, int dir) {
   return A3G_OK;
 }
 
+// DiffuseHorz^T; forward even x then y, odd y then x (src/Diffusion.F90:186-214)
+static int adj_diffuse_horz(a3g_ctx *ctx, int itime) {
+  const int first = (itime % 2 == 0) ? 0 : 1;
+  if (!ctx->prm.use_cn) {
+    bool done = false;
+    int rc = launch_adj_diff_horz(ctx, first == 1, ctx->lam0, ctx->lam1, &done);
+    if (rc) return rc;
+    if (done) {
+      swap_lam(ctx);
+      return A3G_OK;
+    }
+  }
+  int rc = adj_diffuse_dir(ctx, 1 - first);
+  return rc ? rc : adj_diffuse_dir(ctx, first);
+}
+
 int a3g_adj_advect_x(a3g_ctx *ctx) {
   CTX_CHECK(ctx);
   int rc = adj_ready(ctx);
@@ -1513,10 +1525,7 @@ int a3g_adj_diffuse_horz(a3g_ctx *ctx, int32_t itime) {
   int rc = adj_ready(ctx);
   if (rc) return rc;
   if (!ctx->have_diffusivity) return fail(A3G_ERR_STATE, "diffusivity not set");
-  // DiffuseHorz: even x then y, odd y then x (src/Diffusion.F90:186-214)
-  const int first = (itime % 2 == 0) ? 0 : 1;
-  if ((rc = adj_diffuse_dir(ctx, 1 - first))) return rc;
-  return adj_diffuse_dir(ctx, first);
+  return adj_diffuse_horz(ctx, itime);
 }
 
 int a3g_adj_diffuse_vert(a3g_ctx *ctx) {
@@ -1554,9 +1563,7 @@ int a3g_adj_step(a3g_ctx *ctx, int32_t itime) {
   if (rc) return rc;
   if (ctx->prm.use_diffusion) {
     if ((rc = adj_diffuse_dir(ctx, 2))) return rc;  // DiffuseVert^T
-    const int dfirst = (itime % 2 == 0) ? 0 : 1;     // DiffuseHorz: even x then y
-    if ((rc = adj_diffuse_dir(ctx, 1 - dfirst))) return rc;
-    if ((rc = adj_diffuse_dir(ctx, dfirst))) return rc;
+    if ((rc = adj_diffuse_horz(ctx, itime))) return rc;
   }
   if ((rc = adj_advect_dir(ctx, 2, ctx->c1))) return rc;             // AdvectVert^T at state c
   if ((rc = adj_advect_dir(ctx, 1 - first, ctx->stage1))) return rc; // second horizontal sweep at b

@@ -184,6 +184,10 @@ struct a3g_ctx {
   int cn_slot[3];
   uint64_t cn_stamp[3];
 
+  // factors of the explicit diffusion sweeps per (j, k), independent of dt
+  void *diff_tab;
+  bool diff_valid;
+
   a3g::Box box;
   int last_bc;
   bool have_geometry, have_diffusivity, have_vf, have_winds;
@@ -283,8 +287,7 @@ int cuda_fail(cudaError_t e, const char *what);
 int launch_advect_x(a3g_ctx *ctx);
 int launch_advect_y(a3g_ctx *ctx);
 int launch_advect_z(a3g_ctx *ctx);
-int launch_diff_x(a3g_ctx *ctx);
-int launch_diff_y(a3g_ctx *ctx);
+int launch_diff_horz(a3g_ctx *ctx, bool xfirst);
 int launch_diff_z(a3g_ctx *ctx);
 int launch_diffcn_x(a3g_ctx *ctx);
 int launch_diffcn_y(a3g_ctx *ctx);
@@ -318,6 +321,7 @@ int check_device_error(a3g_ctx *ctx);
 int launch_adj_advect(a3g_ctx *ctx, int dir, const double *cq, const double *lin, double *lout,
                       const double *lam_lo);
 int launch_adj_diffuse(a3g_ctx *ctx, int dir, const double *lin, double *lout);
+int launch_adj_diff_horz(a3g_ctx *ctx, bool xfirst, const double *lin, double *lout, bool *done);
 int launch_tl_advect(a3g_ctx *ctx, int dir, const double *cq, const double *din, double *dout, double *dep);
 int launch_cloud_load(a3g_ctx *ctx, const double *c, double *out);
 int launch_adj_cloud_load(a3g_ctx *ctx, const double *w, double *lam);

@@ -456,14 +456,13 @@ __global__ void __launch_bounds__(32 * ADJ_WARPS, 8) k_adj_colt(
   double *wsm = reinterpret_cast<double *>(adj_smem + 128) + (long)wid * 2 * ADJ_BUF_D;
   const int nother = (DIR == 1) ? L.nz : L.ny;
   const int nti = (L.nx + 31) >> 5;
-  const long t = (long)blockIdx.x * ADJ_WARPS + wid;
-  if (t >= (long)nti * nother * L.ns * nseg) return;  // whole warps only; no block barrier below
-  const int g = (int)(t % L.ns);
-  long rr = t / L.ns;
-  const int it = (int)(rr % nti);
-  rr /= nti;
-  const int o = (int)(rr % nother) + 1;
-  const int s0 = (int)(rr / nother) * seg + 1;
+  const unsigned t = blockIdx.x * ADJ_WARPS + wid, ns = L.ns, rr = t / ns, ro = rr / (unsigned)nti;
+  if (ro >= (unsigned)(nother * nseg)) return;  // whole warps only; no block barrier below
+  const int g = (int)(t - rr * ns);
+  const int it = (int)(rr - ro * (unsigned)nti);
+  const int sg_ = (int)(ro / (unsigned)nother);
+  const int o = (int)ro - sg_ * nother + 1;
+  const int s0 = sg_ * seg + 1;
   const int a = (it << 5) + lane + 1;
   const bool valid = a <= L.nx;
   const int n = (DIR == 1) ? L.ny : L.nz;
@@ -570,12 +569,11 @@ __global__ void __launch_bounds__(32 * ADJ_WARPS, 8) k_adj_xm(
                 *const lbuf = vbuf + 2 * AXM_BUF;
   const int nrows = L.ny * L.nz;
   const int ntile = (nrows + 31) >> 5;
-  const long t = (long)blockIdx.x * ADJ_WARPS + wid;
-  if (t >= (long)ntile * L.ns * nseg) return;  // whole warps only; no block barrier below
-  const int g = (int)(t % L.ns);
-  const long rr = t / L.ns;
-  const int r0 = (int)(rr % ntile) * 32;
-  const int s0 = (int)(rr / ntile) * seg + 1;
+  const unsigned t = blockIdx.x * ADJ_WARPS + wid, ns = L.ns, rr = t / ns, rs = rr / (unsigned)ntile;
+  if (rs >= (unsigned)nseg) return;  // whole warps only; no block barrier below
+  const int g = (int)(t - rr * ns);
+  const int r0 = (int)(rr - rs * (unsigned)ntile) * 32;
+  const int s0 = (int)rs * seg + 1;
   const int n = L.nx, s1 = min(n, s0 + seg - 1);
   const int r = min(r0 + lane, nrows - 1);
   const int j = r % L.ny + 1, k = r / L.ny + 1;

@@ -1371,14 +1371,14 @@ __global__ void __launch_bounds__(32 * ACT_WARPS, ACT_MINB) k_advect_colt(
   // buffer b at wsm + 4*ACH*32 + b*2*ACH: pairs (sigma(c+2)/2, dt/kappa(c+1))
   const int nother = (DIR == 1) ? L.nz : L.ny;
   const int nti = (L.nx + 31) >> 5;
-  const long t = (long)blockIdx.x * ACT_WARPS + wid;
-  if (t >= (long)nti * nother * L.ns * nseg) return;  // whole warps only; no block barrier below
-  const int g = (int)(t % L.ns);
-  long rr = t / L.ns;
-  const int it = (int)(rr % nti);
-  rr /= nti;
-  const int o = (int)(rr % nother) + 1;  // k (y sweep) or j (z sweep)
-  const int s0 = (int)(rr / nother) * seg + 1;
+  const unsigned t = blockIdx.x * ACT_WARPS + wid;  // 32-bit: a 64-bit division costs a small grid a microsecond
+  const unsigned ns = L.ns, rr = t / ns, ro = rr / (unsigned)nti;
+  if (ro >= (unsigned)(nother * nseg)) return;  // whole warps only; no block barrier below
+  const int g = (int)(t - rr * ns);
+  const int it = (int)(rr - ro * (unsigned)nti);
+  const int sg_ = (int)(ro / (unsigned)nother);
+  const int o = (int)ro - sg_ * nother + 1;  // k (y sweep) or j (z sweep)
+  const int s0 = sg_ * seg + 1;
   const int a = (it << 5) + lane + 1;  // i
   const bool valid = a <= L.nx;
   const int n = (DIR == 1) ? L.ny : L.nz;
@@ -1546,17 +1546,24 @@ __global__ void __launch_bounds__(32 * ACT_WARPS, ACT_MINB) k_advect_colt(
 }
 
 // Segments a marched line of n cells is cut into, given the warps that whole
-// lines would make: enough to give every SM about 20 warps (its registers hold
-// 16 at once), in segments of at least MARCH_SEG_MIN cells, below which the
-// repeated interface costs more than the added warps give (93x131x37, 2
-// grains: y 56 -> 16 us, z 27 -> 14 us a sweep; whole lines would take 45, 22).
-constexpr int MARCH_SEG_MIN = 10;
+// lines would make: the count with the least waves x cells per wave, where a
+// wave is the 16 warps an SM's registers hold and a segment's start costs
+// about eight cells (its loads, and the interface it repeats).  93x131x37, 2
+// grains: y 56 -> 14 us, z 27 -> 14 us a sweep (whole lines 45, 22);
+// 140x120x40, 4 grains: x 27.4 -> 24.6, y 20.3 -> 18.7 us against 20 warps an
+// SM whatever the waves.
 static inline int march_segments(int n, long warps) {
-  const long want = 148L * 20;
-  if (warps >= want) return 1;
-  const long most = n / MARCH_SEG_MIN > 1 ? n / MARCH_SEG_MIN : 1;
-  const long s = (want + warps - 1) / warps;
-  return (int)(s < most ? s : most);
+  const long wave = 148L * 16;
+  int best = 1;
+  long least = 0;
+  for (int s = 1; s == 1 || (s <= 32 && n / s >= 6); s++) {
+    const long cost = ((warps * s + wave - 1) / wave) * ((n + s - 1) / s + 8);
+    if (s == 1 || cost < least) {
+      best = s;
+      least = cost;
+    }
+  }
+  return best;
 }
 
 // Launches the TMA-fed column march; false when its conditions do not hold
@@ -1625,12 +1632,11 @@ __global__ void __launch_bounds__(32 * AXM_WARPS, ACT_MINB) k_advect_xm(
   unsigned char *const qbuf = sm + 512 + wid * AXM_WARP_B, *const vbuf = qbuf + 3 * AXM_BUF;
   const int nrows = L.ny * L.nz;
   const int ntile = (nrows + 31) >> 5;
-  const long t = (long)blockIdx.x * AXM_WARPS + wid;
-  if (t >= (long)ntile * L.ns * nseg) return;  // whole warps only; no block barrier below
-  const int g = (int)(t % L.ns);
-  const long rr = t / L.ns;
-  const int r0 = (int)(rr % ntile) * 32;
-  const int s0 = (int)(rr / ntile) * seg + 1;
+  const unsigned t = blockIdx.x * AXM_WARPS + wid, ns = L.ns, rr = t / ns, rs = rr / (unsigned)ntile;
+  if (rs >= (unsigned)nseg) return;  // whole warps only; no block barrier below
+  const int g = (int)(t - rr * ns);
+  const int r0 = (int)(rr - rs * (unsigned)ntile) * 32;
+  const int s0 = (int)rs * seg + 1;
   const int n = L.nx, s1 = min(n, s0 + seg - 1);
   const int r = min(r0 + lane, nrows - 1);
   const int j = r % L.ny + 1, k = r / L.ny + 1;

@@ -84,6 +84,176 @@ __global__ void __launch_bounds__(256) k_diff(Layout L, Box box, int periodic,
 }
 
 // ---------------------------------------------------------------------------
+// Explicit diffusion where nothing it uses varies along i (every projected or
+// lon/lat grid with uniform diffusivities): the dt-independent factors come
+// from a table per (j, k), and DiffuseHorz's two sweeps run as one.
+// ---------------------------------------------------------------------------
+// Row (j, k) of the table: the x factors k_ds and sigma/kappa (the same for
+// both faces), then for y and for z k_ds of the face before the cell,
+// sigma/kappa of the face after it and of the face before it.
+struct DiffRow {
+  double kx, sx, ky, syR, syL, kz, szR, szL;
+};
+
+// rows j = 1..ny+1, k = 1..nz+1 (the last ones for their ky and kz only)
+__global__ void k_diff_table(Layout L, Geo3 snx, Geo3 sny, Geo3 snz, Geo3 kap, Geo3 kx, Geo3 ky, Geo3 kz,
+                             DiffRow *__restrict__ tab) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= (L.ny + 1) * (L.nz + 1)) return;
+  const int j = t % (L.ny + 1) + 1, k = t / (L.ny + 1) + 1, i = 1;
+  const double k0 = kap.at(i, j, k);
+  DiffRow r;
+  // :351-360 in the operations of k_diff
+  r.kx = 0.5 * (kx.at(i, j, k) + kx.at(i + 1, j, k)) * (2.0 * snx.at(i + 1, j, k) / (k0 + kap.at(i + 1, j, k)));
+  r.sx = snx.at(i + 1, j, k) / k0;
+  r.ky = 0.5 * (ky.at(i, j - 1, k) + ky.at(i, j, k)) * (2.0 * sny.at(i, j, k) / (kap.at(i, j - 1, k) + k0));
+  r.syR = sny.at(i, j + 1, k) / k0;
+  r.syL = sny.at(i, j, k) / k0;
+  r.kz = 0.5 * (kz.at(i, j, k - 1) + kz.at(i, j, k)) * (2.0 * snz.at(i, j, k) / (kap.at(i, j, k - 1) + k0));
+  r.szR = snz.at(i, j, k + 1) / k0;
+  r.szL = snz.at(i, j, k) / k0;
+  tab[t] = r;
+}
+
+// One cell of a sweep from its neighbours; aL, aR: dt*k_ds of its faces, sL,
+// sR: sigma/kappa of its faces.  A neighbour beyond the grid is the cell
+// itself (Neumann) or the wrapped one.
+__device__ __forceinline__ double diff_cell(double l, double q, double r, double aL, double aR, double sL, double sR) {
+  const double LF = aR * (r - q) * sR;
+  const double RF = -(aL * (q - l) * sL);
+  return q + (LF + RF);
+}
+// Its transpose: own coefficients cL, cR, the left neighbour's cR and the right
+// neighbour's cL; the ghosts' terms fold back last (k_adj_diff's order).
+__device__ __forceinline__ double adj_diff_cell(double l, double q, double r, double cL, double cR, double cRm,
+                                                double cLp, bool first, bool last) {
+  double v = q - cR * q - cL * q;
+  if (!first) v = v + cRm * l;
+  if (!last) v = v + cLp * r;
+  if (first) v = v + (cRm)*l;
+  if (last) v = v + (cLp)*r;
+  return v;
+}
+
+// DiffuseHorz (ADJ: its transpose) in one pass: XFIRST the x sweep, then the y
+// sweep, else the other order.  A warp marches along j with a column per
+// lane; the first and last lane hold the columns beside the warp's 30, so that
+// every x neighbour is a shuffle away, and the rows beside a segment are taken
+// again.  The sweep in between never reaches memory: 16 B a cell instead of 32,
+// and the six divisions a cell that k_diff repeats every step are the table's.
+// 360x161x40, 5 grains: x and y 200 -> 64 us together; 100x100x40, 4 grains: 40
+// -> 15 us.
+template <bool XFIRST, bool ADJ, bool PER>
+__global__ void __launch_bounds__(128) k_diff_xy(Layout L, Box box, int nseg, int seg,
+                                                 const double *__restrict__ cin, double *__restrict__ cout,
+                                                 const DiffRow *__restrict__ tab,
+                                                 const int32_t *__restrict__ aloft,
+                                                 const DevScalars *__restrict__ sc) {
+  const int lane = threadIdx.x & 31;
+  const int nti = (L.nx + 29) / 30;
+  const unsigned w = blockIdx.x * 4 + (threadIdx.x >> 5), wt = w / (unsigned)nti, ws = wt / (unsigned)nseg;
+  const int g = (int)(ws / (unsigned)L.nz), k = (int)ws - g * L.nz + 1;
+  if (g >= L.ns) return;  // whole warps
+  const int it = (int)(w - wt * (unsigned)nti);
+  const int s0 = (int)(wt - ws * (unsigned)nseg) * seg + 1, s1 = min(L.ny, s0 + seg - 1);
+  const int i0 = it * 30 + lane;  // 1-based column of this lane: 0 and nx+1 are the ghosts
+  const int i = i0 < 1 ? (PER ? L.nx : 1) : i0 > L.nx ? (PER ? (i0 - L.nx - 1) % L.nx + 1 : L.nx) : i0;
+  const bool own = lane >= 1 && lane <= 30 && i0 <= L.nx;
+  const double *q0 = cin + (long)g * L.PG + (long)(k - 1) * L.PY + (i - 1);
+  double *p0 = cout + (long)g * L.PG + (long)(k - 1) * L.PY + (i - 1);
+  const bool col_in = i >= box.imin && i <= box.imax && k >= box.kmin && k <= box.kmax;
+  if (!aloft[g] || !__any_sync(0xffffffffu, col_in)) {
+    if (own)
+      for (int j = s0; j <= s1; j++) p0[(long)(j - 1) * L.P] = 0.0;
+    return;
+  }
+  const double dt = sc->dt;
+  const DiffRow *T = tab + (long)(k - 1) * (L.ny + 1) - 1;  // row j at T[j]
+  auto in = [&](int j) { return col_in && j >= box.jmin && j <= box.jmax; };
+  auto xs = [&](double q, int j) {  // the x sweep of row j; lanes 0 and 31 give nothing of use
+    const double l = __shfl_up_sync(0xffffffffu, q, 1), r = __shfl_down_sync(0xffffffffu, q, 1);
+    const double a = dt * T[j].kx, s = T[j].sx;
+    if (ADJ) {
+      const double c = a * s;
+      return adj_diff_cell(l, q, r, c, c, c, c, i == 1, i == L.nx);
+    }
+    return in(j) ? diff_cell(l, q, r, a, a, s, s) : 0.0;
+  };
+  auto ys = [&](double l, double q, double r, int j) {  // the y sweep at row j
+    const double aL = dt * T[j].ky, aR = dt * T[j + 1].ky;
+    if (ADJ) {
+      const double cL = aL * T[j].syL, cR = aR * T[j].syR;
+      const double cRm = j > 1 ? aL * T[j - 1].syR : cL, cLp = j < L.ny ? aR * T[j + 1].syL : cR;
+      return adj_diff_cell(l, q, r, cL, cR, cRm, cLp, j == 1, j == L.ny);
+    }
+    return in(j) ? diff_cell(l, q, r, aL, aR, T[j].syL, T[j].syR) : 0.0;
+  };
+  auto at = [&](int j) { return q0[(long)((j < 1 ? 1 : j > L.ny ? L.ny : j) - 1) * L.P]; };
+  // row j as the y sweep sees it, from row j as loaded
+  auto row = [&](double q, int j) {
+    const int jc = j < 1 ? 1 : j > L.ny ? L.ny : j;  // a ghost row is its neighbour's copy
+    return XFIRST ? xs(q, jc) : q;
+  };
+  double a = row(at(s0 - 1), s0 - 1), b = row(at(s0), s0);
+  double nq = at(s0 + 1);
+#pragma unroll 4
+  for (int j = s0; j <= s1; j++) {
+    const double c = row(nq, j + 1);
+    nq = at(j + 2);
+    double y = ys(a, b, c, j);
+    if (!XFIRST) y = xs(y, j);
+    if (own) p0[(long)(j - 1) * L.P] = y;
+    a = b;
+    b = c;
+  }
+}
+
+// DiffuseVert (ADJ: its transpose) marched along k, lanes along i, every cell
+// read once.  360x161x40, 5 grains: 82 -> 60 us.
+template <bool ADJ>
+__global__ void __launch_bounds__(128) k_diff_z(Layout L, Box box, int nseg, int seg, const double *__restrict__ cin,
+                                                double *__restrict__ cout, const DiffRow *__restrict__ tab,
+                                                const int32_t *__restrict__ aloft,
+                                                const DevScalars *__restrict__ sc) {
+  const int lane = threadIdx.x & 31;
+  const int nti = (L.nx + 31) >> 5;
+  const unsigned w = blockIdx.x * 4 + (threadIdx.x >> 5), wt = w / (unsigned)nti, ws = wt / (unsigned)nseg;
+  const int g = (int)(ws / (unsigned)L.ny), j = (int)ws - g * L.ny + 1;
+  const int i = (int)(w - wt * (unsigned)nti) * 32 + lane + 1;
+  if (g >= L.ns || i > L.nx) return;
+  const int s0 = (int)(wt - ws * (unsigned)nseg) * seg + 1, s1 = min(L.nz, s0 + seg - 1);
+  const double *q0 = cin + (long)g * L.PG + L.cell(i, j, 1);
+  double *p0 = cout + (long)g * L.PG + L.cell(i, j, 1);
+  if (!aloft[g] || i < box.imin || i > box.imax || j < box.jmin || j > box.jmax) {
+    for (int k = s0; k <= s1; k++) p0[(long)(k - 1) * L.PY] = 0.0;
+    return;
+  }
+  const double dt = sc->dt;
+  const long TS = L.ny + 1;
+  const DiffRow *T = tab + (j - 1) - TS;  // row k at T[k*TS]
+  auto at = [&](int k) { return q0[(long)((k < 1 ? 1 : k > L.nz ? L.nz : k) - 1) * L.PY]; };
+  double a = at(s0 - 1), b = at(s0), c = at(s0 + 1);
+#pragma unroll 4
+  for (int k = s0; k <= s1; k++) {
+    const double next = at(k + 2);
+    const DiffRow *t = T + k * TS;
+    const double aL = dt * t->kz, aR = dt * t[TS].kz;
+    double y;
+    if (ADJ) {
+      const double cL = aL * t->szL, cR = aR * t->szR;
+      const double cRm = k > 1 ? aL * t[-TS].szR : cL, cLp = k < L.nz ? aR * t[TS].szL : cR;
+      y = adj_diff_cell(a, b, c, cL, cR, cRm, cLp, k == 1, k == L.nz);
+    } else {
+      y = k >= box.kmin && k <= box.kmax ? diff_cell(a, b, c, aL, aR, t->szL, t->szR) : 0.0;
+    }
+    p0[(long)(k - 1) * L.PY] = y;
+    a = b;
+    b = c;
+    c = next;
+  }
+}
+
+// ---------------------------------------------------------------------------
 // Crank-Nicolson line tables
 // ---------------------------------------------------------------------------
 // Per row of a distinct line: dgtsv's multiplier, the right-hand side's
@@ -807,11 +977,10 @@ __global__ void __launch_bounds__(32 * CXT_WARPS, 8) k_cn_solve_xt2(const __grid
   if (r0 >= nrows) return;  // uniform over the warp
   const long r = r0 + lane;
   const bool valid = r < nrows;
-  const long rc = valid ? r : nrows - 1;
-  const int j = (int)(rc % L.ny) + 1;
-  const long t1 = rc / L.ny;
-  const int k = (int)(t1 % L.nz) + 1;
-  const int g = (int)(t1 / L.nz);
+  const unsigned rc = (unsigned)(valid ? r : nrows - 1), t1 = rc / (unsigned)L.ny, t2 = t1 / (unsigned)L.nz;
+  const int j = (int)(rc - t1 * (unsigned)L.ny) + 1;
+  const int k = (int)(t1 - t2 * (unsigned)L.nz) + 1;
+  const int g = (int)t2;
   const bool active =
       valid && j >= box.jmin && j <= box.jmax && k >= box.kmin && k <= box.kmax && aloft[g] != 0;
   const int rmin = box.imin, rmax = box.imax;
@@ -1064,7 +1233,7 @@ __global__ void __launch_bounds__(64, 8) k_cn_solve_zt(const __grid_constant__ C
   const int nti = (L.nx + 31) >> 5;
   const long ntiles = (long)nti * L.ny * L.ns;
   const long nwarps = (long)gridDim.x * wpb;
-  const long per = (ntiles + nwarps - 1) / nwarps;
+  const long per = ((unsigned)ntiles + (unsigned)nwarps - 1u) / (unsigned)nwarps;
   const long t0 = ((long)blockIdx.x * wpb + wid) * per;
   const long t1 = t0 + per < ntiles ? t0 + per : ntiles;
   const int rmin = box.kmin, rmax = box.kmax;
@@ -1075,10 +1244,10 @@ __global__ void __launch_bounds__(64, 8) k_cn_solve_zt(const __grid_constant__ C
   double *xx = tile + lane + (long)(rmin - 1) * 32;  // row l of this lane's line at xx[l*32]
   const double2 *const row2 = reinterpret_cast<const double2 *>(stab);  // FACT,CL  CC,CR  DU,ZH  ZL,ZLL
   for (long t = t0; t < t1; t++) {
-    const int it = (int)(t % nti);
-    const long r = t / nti;
-    const int j = (int)(r % L.ny) + 1;
-    const int g = (int)(r / L.ny);
+    const unsigned r = (unsigned)t / (unsigned)nti, rg = r / (unsigned)L.ny;
+    const int it = (int)((unsigned)t - r * (unsigned)nti);
+    const int j = (int)(r - rg * (unsigned)L.ny) + 1;
+    const int g = (int)rg;
     const int i = (it << 5) + lane + 1;
     const bool act = i <= L.nx && i >= box.imin && i <= box.imax && j >= box.jmin && j <= box.jmax &&
                      aloft[g] != 0;
@@ -1223,7 +1392,7 @@ __global__ void __launch_bounds__(64, 8) k_cn_solve_yt(const __grid_constant__ C
   const int nti = (L.nx + 31) >> 5;
   const long ngroups = (long)nti * L.nz * L.ns;
   const long nwarps = (long)gridDim.x * wpb;
-  const long per = (ngroups + nwarps - 1) / nwarps;
+  const long per = ((unsigned)ngroups + (unsigned)nwarps - 1u) / (unsigned)nwarps;
   const long t0 = ((long)blockIdx.x * wpb + wid) * per;
   const long t1 = t0 + per < ngroups ? t0 + per : ngroups;
   const int rmin = box.jmin, rmax = box.jmax;
@@ -1232,10 +1401,10 @@ __global__ void __launch_bounds__(64, 8) k_cn_solve_yt(const __grid_constant__ C
   const int cnt_last = ncells - (nch - 1) * YT_CH;
   uint32_t s0 = 0;  // loads of the groups before: load p of this one is the warp's load s0 + p
   for (long t = t0; t < t1; t++) {
-    const int it = (int)(t % nti);
-    const long r = t / nti;
-    const int k = (int)(r % L.nz) + 1;
-    const int g = (int)(r / L.nz);
+    const unsigned r = (unsigned)t / (unsigned)nti, rg = r / (unsigned)L.nz;
+    const int it = (int)((unsigned)t - r * (unsigned)nti);
+    const int k = (int)(r - rg * (unsigned)L.nz) + 1;
+    const int g = (int)rg;
     const int i = (it << 5) + lane + 1;
     const bool act = i <= L.nx && i >= box.imin && i <= box.imax && k >= box.kmin && k <= box.kmax &&
                      aloft[g] != 0;
@@ -1574,24 +1743,103 @@ static bool launch_cn_solve_xt2(a3g_ctx *ctx, const LineMap &map, const CnTab &t
 // ---------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------
+// Brings the explicit sweeps' table up to date; false where something varies
+// along i and k_diff / k_adj_diff have to run.
+static bool diff_table(a3g_ctx *ctx) {
+  if (ctx->snx.si || ctx->sny.si || ctx->snz.si || ctx->kappa.si || ctx->kx.si || ctx->ky.si || ctx->kz.si) return false;
+  const Layout &L = ctx->L;
+  const int n = (L.ny + 1) * (L.nz + 1);
+  if (!ctx->diff_tab) {
+    if (cudaMalloc((void **)&ctx->diff_tab, sizeof(DiffRow) * (size_t)n) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    ctx->bytes += sizeof(DiffRow) * (size_t)n;
+  }
+  if (!ctx->diff_valid) {
+    k_diff_table<<<(n + 127) / 128, 128, 0, ctx->stream>>>(L, ctx->snx, ctx->sny, ctx->snz, ctx->kappa, ctx->kx,
+                                                         ctx->ky, ctx->kz, static_cast<DiffRow *>(ctx->diff_tab));
+    ctx->launches++;
+    ctx->diff_valid = true;
+  }
+  return true;
+}
+
+// segments of a marched line of n cells that leave at least 8 cells each and
+// give the chip about 24 warps an SM
+static int diff_segments(int n, long warps) {
+  const long want = (148L * 24 + warps - 1) / warps, most = n / 8 > 1 ? n / 8 : 1;
+  return (int)(want < 1 ? 1 : want < most ? want : most);
+}
+
+// The horizontal sweeps in one pass, x first or y first; false as diff_table.
+template <bool ADJ>
+static bool run_diff_xy(a3g_ctx *ctx, bool xfirst, const Box &box, const double *cin, double *cout) {
+  if (!diff_table(ctx)) return false;
+  const Layout &L = ctx->L;
+  const long lines = (long)((L.nx + 29) / 30) * L.nz * L.ns;
+  const int seg = (L.ny + diff_segments(L.ny, lines) - 1) / diff_segments(L.ny, lines);
+  const int nseg = (L.ny + seg - 1) / seg;
+  const unsigned blocks = (unsigned)((lines * nseg + 3) / 4);
+  const DiffRow *tab = static_cast<const DiffRow *>(ctx->diff_tab);
+#define A3G_DXY(X_, P_) \
+  k_diff_xy<X_, ADJ, P_><<<blocks, 128, 0, ctx->stream>>>(L, box, nseg, seg, cin, cout, tab, ctx->aloft, ctx->sc)
+  if (ctx->grid.periodic) {
+    if (xfirst) A3G_DXY(true, true); else A3G_DXY(false, true);
+  } else {
+    if (xfirst) A3G_DXY(true, false); else A3G_DXY(false, false);
+  }
+#undef A3G_DXY
+  return true;
+}
+
+template <bool ADJ>
+static bool run_diff_z(a3g_ctx *ctx, const Box &box, const double *cin, double *cout) {
+  if (!diff_table(ctx)) return false;
+  const Layout &L = ctx->L;
+  const long lines = (long)((L.nx + 31) / 32) * L.ny * L.ns;
+  const int seg = (L.nz + diff_segments(L.nz, lines) - 1) / diff_segments(L.nz, lines);
+  const int nseg = (L.nz + seg - 1) / seg;
+  k_diff_z<ADJ><<<(unsigned)((lines * nseg + 3) / 4), 128, 0, ctx->stream>>>(
+      L, box, nseg, seg, cin, cout, static_cast<const DiffRow *>(ctx->diff_tab), ctx->aloft, ctx->sc);
+  return true;
+}
+
 template <int DIR>
 static int launch_diff_dir(a3g_ctx *ctx) {
   const Layout &L = ctx->L;
-  const Geo3 &sig = (DIR == 0) ? ctx->snx : (DIR == 1) ? ctx->sny : ctx->snz;
-  const Geo3 &kk = (DIR == 0) ? ctx->kx : (DIR == 1) ? ctx->ky : ctx->kz;
-  dim3 grid((L.nx + 31) / 32, (L.ny + 7) / 8, L.nz);
   tbegin(ctx, A3G_K_DIFF_X + DIR);
-  k_diff<DIR><<<grid, dim3(32, 8), 0, ctx->stream>>>(L, ctx->box, ctx->grid.periodic, ctx->c0,
-                                                     ctx->c1, sig, ctx->kappa, kk, ctx->aloft,
-                                                     ctx->sc);
+  if (DIR == 2 && run_diff_z<false>(ctx, ctx->box, ctx->c0, ctx->c1)) {
+    // marched
+  } else {
+    const Geo3 &sig = (DIR == 0) ? ctx->snx : (DIR == 1) ? ctx->sny : ctx->snz;
+    const Geo3 &kk = (DIR == 0) ? ctx->kx : (DIR == 1) ? ctx->ky : ctx->kz;
+    dim3 grid((L.nx + 31) / 32, (L.ny + 7) / 8, L.nz);
+    k_diff<DIR><<<grid, dim3(32, 8), 0, ctx->stream>>>(L, ctx->box, ctx->grid.periodic, ctx->c0,
+                                                       ctx->c1, sig, ctx->kappa, kk, ctx->aloft,
+                                                       ctx->sc);
+  }
   tend(ctx);
   A3G_LAUNCH_CHECK(ctx);
   swap_levels(ctx);
   return A3G_OK;
 }
 
-int launch_diff_x(a3g_ctx *ctx) { return launch_diff_dir<0>(ctx); }
-int launch_diff_y(a3g_ctx *ctx) { return launch_diff_dir<1>(ctx); }
+// DiffuseHorz, explicit: both sweeps, x first or y first.
+int launch_diff_horz(a3g_ctx *ctx, bool xfirst) {
+  tbegin(ctx, A3G_K_DIFF_X);
+  const bool fused = run_diff_xy<false>(ctx, xfirst, ctx->box, ctx->c0, ctx->c1);
+  tend(ctx);
+  if (!fused) {
+    int rc = xfirst ? launch_diff_dir<0>(ctx) : launch_diff_dir<1>(ctx);
+    if (!rc) rc = xfirst ? launch_diff_dir<1>(ctx) : launch_diff_dir<0>(ctx);
+    return rc;
+  }
+  A3G_LAUNCH_CHECK(ctx);
+  swap_levels(ctx);
+  return A3G_OK;
+}
+
 int launch_diff_z(a3g_ctx *ctx) { return launch_diff_dir<2>(ctx); }
 
 static inline bool varies(const Geo3 &g, int idx) {  // idx 0:i 1:j 2:k
@@ -1828,11 +2076,25 @@ static int launch_adj_diff_dir(a3g_ctx *ctx, const double *lin, double *lout) {
   const Geo3 &sig = (DIR == 0) ? ctx->snx : (DIR == 1) ? ctx->sny : ctx->snz;
   const Geo3 &kk = (DIR == 0) ? ctx->kx : (DIR == 1) ? ctx->ky : ctx->kz;
   dim3 grid((L.nx + 31) / 32, (L.ny + 7) / 8, L.nz);
+  const Box full{1, L.nx, 1, L.ny, 1, L.nz};
   tbegin(ctx, A3G_K_ADJOINT);
-  k_adj_diff<DIR><<<grid, dim3(32, 8), 0, ctx->stream>>>(L, ctx->grid.periodic, lin, lout, sig, ctx->kappa,
+  if (!(DIR == 2 && run_diff_z<true>(ctx, full, lin, lout)))
+    k_adj_diff<DIR><<<grid, dim3(32, 8), 0, ctx->stream>>>(L, ctx->grid.periodic, lin, lout, sig, ctx->kappa,
                                                          kk, ctx->aloft, ctx->sc);
   tend(ctx);
   A3G_LAUNCH_CHECK(ctx);
+  return A3G_OK;
+}
+
+// lam_out <- (D_h)^T lam_in of the explicit horizontal sweeps in one pass, the
+// x transpose first or the y transpose first; *done false where they have to
+// be launched one by one (launch_adj_diffuse).
+int launch_adj_diff_horz(a3g_ctx *ctx, bool xfirst, const double *lin, double *lout, bool *done) {
+  const Box full{1, ctx->L.nx, 1, ctx->L.ny, 1, ctx->L.nz};
+  tbegin(ctx, A3G_K_ADJOINT);
+  *done = run_diff_xy<true>(ctx, xfirst, full, lin, lout);
+  tend(ctx);
+  if (*done) A3G_LAUNCH_CHECK(ctx);
   return A3G_OK;
 }
 
