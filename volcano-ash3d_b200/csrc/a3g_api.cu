@@ -190,6 +190,7 @@ int a3g_create(const a3g_grid_desc *grid, const a3g_params *params, int device, 
   L.PY = L.P * grid->ny;
   L.PG = L.PY * grid->nz;
   full_box(ctx);
+  ctx->nz0 = ctx->nz1 = Box{1, 0, 1, 0, 1, 0};  // the levels start as zeros
   ctx->h_aloft.assign(grid->ns, 1);
   ctx->n_gs_aloft = grid->ns;
   ctx->last_bc = 0;
@@ -617,6 +618,7 @@ int a3g_upload_concen(a3g_ctx *ctx, const double *concen_level) {
   if (rc) return rc;
   A3G_CUDA(cudaStreamSynchronize(ctx->stream));
   ctx->ts1_zeroed = false;
+  ctx->nz0 = full_box_of(L);
   return A3G_OK;
 }
 
@@ -752,15 +754,20 @@ int a3g_restart_load(a3g_ctx *ctx, const float *ashcon, const float *depocon) {
   rc = launch_netcdf_unpack(ctx, da, dd);
   if (rc) return rc;
   A3G_CUDA(cudaStreamSynchronize(ctx->stream));
-  if (ashcon) ctx->ts1_zeroed = false;
+  if (ashcon) {
+    ctx->ts1_zeroed = false;
+    ctx->nz0 = full_box_of(L);
+  }
   return check_device_error(ctx);
 }
 
 int a3g_step_prologue(a3g_ctx *ctx) {
   CTX_CHECK(ctx);
   // ts0 <- ts1: the state is unchanged unless the last sweep left ts1 zero.
-  if (ctx->ts1_zeroed)
+  if (ctx->ts1_zeroed) {
     A3G_CUDA(cudaMemsetAsync(ctx->c0, 0, sizeof(double) * ctx->L.PG * ctx->L.ns, ctx->stream));
+    ctx->nz0 = Box{1, 0, 1, 0, 1, 0};
+  }
   ctx->ts1_zeroed = true;  // ts1 <- 0; the next sweep that copies back clears this
   return A3G_OK;
 }
@@ -1666,6 +1673,7 @@ int a3g_snapshot_load(a3g_ctx *ctx, int32_t slot) {
   CTX_CHECK(ctx);
   if (slot < 0 || slot >= (int)ctx->snaps.size()) return fail(A3G_ERR_ARG, "snapshot slot out of range");
   A3G_CUDA(cudaMemcpyAsync(ctx->c0, ctx->snaps[slot], level_bytes(ctx), cudaMemcpyDeviceToDevice, ctx->stream));
+  ctx->nz0 = full_box_of(ctx->L);
   ctx->ts1_zeroed = false;  // a restored state survives the next prologue
   return A3G_OK;
 }

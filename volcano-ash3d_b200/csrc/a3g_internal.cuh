@@ -189,6 +189,7 @@ struct a3g_ctx {
   bool diff_valid;
 
   a3g::Box box;
+  a3g::Box nz0, nz1;        // outside these c0, c1 hold zeros (kept up under FAST_SUBGRID; see cover_box)
   int last_bc;
   bool have_geometry, have_diffusivity, have_vf, have_winds;
   bool ts1_zeroed;          // the last sweep left ts1 zero without copy-back
@@ -341,6 +342,72 @@ inline void swap_levels(a3g_ctx *ctx) {
   double *t = ctx->c0;
   ctx->c0 = ctx->c1;
   ctx->c1 = t;
+  const Box b = ctx->nz0;
+  ctx->nz0 = ctx->nz1;
+  ctx->nz1 = b;
+}
+
+// FAST_SUBGRID: a sweep leaves zeros outside its box, so both levels are zero
+// outside a box that follows the cloud (nz0, nz1).  A sweep then has to write
+// only the cells of its own box and of the ones its target may hold nonzero
+// (480x401x50, 6 grains, a cloud in a seventh of the grid: 5.99 -> 3.87 ms a
+// four-step pass, most of it zeros written over zeros before).  Every other
+// writer of a level widens its box (touch) or gives it the whole grid.
+inline Box full_box_of(const Layout &L) { return Box{1, L.nx, 1, L.ny, 1, L.nz}; }
+inline bool empty(const Box &b) { return b.imin > b.imax || b.jmin > b.jmax || b.kmin > b.kmax; }
+inline Box hull(const Box &a, const Box &b) {
+  if (empty(a)) return b;
+  if (empty(b)) return a;
+  auto lo = [](int x, int y) { return x < y ? x : y; };
+  auto hi = [](int x, int y) { return x > y ? x : y; };
+  return Box{lo(a.imin, b.imin), hi(a.imax, b.imax), lo(a.jmin, b.jmin), hi(a.jmax, b.jmax),
+             lo(a.kmin, b.kmin), hi(a.kmax, b.kmax)};
+}
+// the cells a sweep from c0 to c1 over ctx->box has to write
+inline Box cover_box(const a3g_ctx *ctx) {
+  return ctx->prm.fast_subgrid ? hull(ctx->box, ctx->nz1) : full_box_of(ctx->L);
+}
+// the cells c0 may hold nonzero
+inline Box state_box(const a3g_ctx *ctx) { return ctx->prm.fast_subgrid ? ctx->nz0 : full_box_of(ctx->L); }
+// the columns i0..i1 x j0..j1 of c0 are about to be written
+inline void touch(a3g_ctx *ctx, int i0, int i1, int j0, int j1) {
+  const Layout &L = ctx->L;
+  ctx->nz0 = hull(ctx->nz0, Box{i0 > 1 ? i0 : 1, i1 < L.nx ? i1 : L.nx, j0 > 1 ? j0 : 1, j1 < L.ny ? j1 : L.ny, 1, L.nz});
+}
+// the levels change places after a sweep over ctx->box
+inline void sweep_done(a3g_ctx *ctx) {
+  ctx->nz1 = ctx->box;
+  swap_levels(ctx);
+}
+
+// Rows of a plane in tiles of 32: one run of rows where a cover's rows are
+// contiguous (all j), else a run per k; and the cells x0..x1 of a row, x0 = 1
+// (mod 8), x1 the row's end or a multiple of 8.
+struct RowCover {
+  int ny, jmin, nj, kmin, nk, per_k, ntile, x0, x1;
+  __device__ __forceinline__ void tile(int t, int *r0, int *end) const {
+    if (nj == ny) {
+      *r0 = (kmin - 1) * ny + 32 * t;
+      *end = (kmin - 1 + nk) * ny;
+    } else {
+      const int kk = t / per_k;
+      *r0 = (kmin - 1 + kk) * ny + jmin - 1 + 32 * (t - kk * per_k);
+      *end = (kmin - 1 + kk) * ny + jmin - 1 + nj;
+    }
+  }
+};
+static inline RowCover row_cover(const Layout &L, const Box &b) {
+  RowCover c;
+  c.ny = L.ny;
+  c.jmin = b.jmin;
+  c.nj = b.jmax - b.jmin + 1;
+  c.kmin = b.kmin;
+  c.nk = b.kmax - b.kmin + 1;
+  c.per_k = (c.nj + 31) / 32;
+  c.ntile = c.nj == L.ny ? (int)(((long)c.nj * c.nk + 31) / 32) : c.per_k * c.nk;
+  c.x0 = ((b.imin - 1) & ~7) + 1;
+  c.x1 = ((b.imax + 7) & ~7) < L.nx ? (b.imax + 7) & ~7 : L.nx;
+  return c;
 }
 
 // Fortran MAX/MIN for reals (no NaNs reach these in the transport path).

@@ -1358,7 +1358,7 @@ struct FalseT { static constexpr bool value = false; };
 
 template <int DIR, int LIM>
 __global__ void __launch_bounds__(32 * ACT_WARPS, ACT_MINB) k_advect_colt(
-    const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tv, Layout L, Box box,
+    const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tv, Layout L, Box box, Box cov,
     int nocycle, double eps, int nseg, int seg, const double *__restrict__ cin, double *__restrict__ cout,
     const double *__restrict__ vel, const double *__restrict__ vghost, Geo4 vf, Geo3 sig, Geo3 dtvt,
     const int32_t *__restrict__ aloft, DevScalars *sc, double *__restrict__ out1, double *__restrict__ out2) {
@@ -1370,19 +1370,22 @@ __global__ void __launch_bounds__(32 * ACT_WARPS, ACT_MINB) k_advect_colt(
   // buffer b: q chunk at wsm + b*2*ACH*32, v chunk after it; geometry of
   // buffer b at wsm + 4*ACH*32 + b*2*ACH: pairs (sigma(c+2)/2, dt/kappa(c+1))
   const int nother = (DIR == 1) ? L.nz : L.ny;
-  const int nti = (L.nx + 31) >> 5;
+  // lines of the cover: 32-column tiles it0.., other index o0.., sweep index l0..l1
+  const int it0 = (cov.imin - 1) >> 5, nti = ((cov.imax - 1) >> 5) - it0 + 1;
+  const int o0 = (DIR == 1) ? cov.kmin : cov.jmin, no = ((DIR == 1) ? cov.kmax : cov.jmax) - o0 + 1;
+  const int l0 = (DIR == 1) ? cov.jmin : cov.kmin, l1 = (DIR == 1) ? cov.jmax : cov.kmax;
   const unsigned t = blockIdx.x * ACT_WARPS + wid;  // 32-bit: a 64-bit division costs a small grid a microsecond
   const unsigned ns = L.ns, rr = t / ns, ro = rr / (unsigned)nti;
-  if (ro >= (unsigned)(nother * nseg)) return;  // whole warps only; no block barrier below
+  if (ro >= (unsigned)(no * nseg)) return;  // whole warps only; no block barrier below
   const int g = (int)(t - rr * ns);
-  const int it = (int)(rr - ro * (unsigned)nti);
-  const int sg_ = (int)(ro / (unsigned)nother);
-  const int o = (int)ro - sg_ * nother + 1;  // k (y sweep) or j (z sweep)
-  const int s0 = sg_ * seg + 1;
+  const int it = it0 + (int)(rr - ro * (unsigned)nti);
+  const int sg_ = (int)(ro / (unsigned)no);
+  const int o = o0 + (int)ro - sg_ * no;  // k (y sweep) or j (z sweep)
+  const int s0 = l0 + sg_ * seg;
   const int a = (it << 5) + lane + 1;  // i
   const bool valid = a <= L.nx;
   const int n = (DIR == 1) ? L.ny : L.nz;
-  const int s1 = min(n, s0 + seg - 1);
+  const int s1 = min(l1, s0 + seg - 1);
   const int rmin = (DIR == 1) ? box.jmin : box.kmin;
   const int rmax = (DIR == 1) ? box.jmax : box.kmax;
   const int st = (DIR == 1) ? (int)L.P : (int)L.PY;
@@ -1581,14 +1584,15 @@ static bool launch_colt(a3g_ctx *ctx) {
     return false;
   const size_t smem = 128 + (size_t)ACT_WARPS * ACT_WARP_D * sizeof(double);
   static_assert(128 + ACT_WARPS * ACT_WARP_D * 8 <= 48 * 1024, "fits the default dynamic limit");
-  const int n = (DIR == 1) ? L.ny : L.nz;
-  const int nother = (DIR == 1) ? L.nz : L.ny;
-  const long nlw = (long)((L.nx + 31) / 32) * nother * L.ns;  // warps of whole lines
+  const Box cov = cover_box(ctx);
+  const int n = (DIR == 1) ? cov.jmax - cov.jmin + 1 : cov.kmax - cov.kmin + 1;
+  const int nother = (DIR == 1) ? cov.kmax - cov.kmin + 1 : cov.jmax - cov.jmin + 1;
+  const long nlw = (long)((cov.imax - 1) / 32 - (cov.imin - 1) / 32 + 1) * nother * L.ns;  // warps of whole lines
   const int nseg = march_segments(n, nlw);
   const int seg = (n + nseg - 1) / nseg;
   const long nw = nlw * ((n + seg - 1) / seg);
   k_advect_colt<DIR, LIM><<<(unsigned)((nw + ACT_WARPS - 1) / ACT_WARPS), 32 * ACT_WARPS, smem, ctx->stream>>>(
-      tq, tv, L, ctx->box, ctx->prm.nocycle, ctx->prm.eps_thresh, (n + seg - 1) / seg, seg, ctx->c0, ctx->c1, vel,
+      tq, tv, L, ctx->box, cov, ctx->prm.nocycle, ctx->prm.eps_thresh, (n + seg - 1) / seg, seg, ctx->c0, ctx->c1, vel,
       dir_vghost(ctx, DIR), ctx->vf, sg, ctx->dtv, ctx->aloft, ctx->sc, (DIR == 1) ? ctx->out_xz1 : ctx->out_xy1,
       (DIR == 1) ? ctx->out_xz2 : ctx->out_xy2);
   return true;
@@ -1622,7 +1626,7 @@ constexpr int AXM_SMEM = 512 + 512 + AXM_WARPS * AXM_WARP_B;  // barriers, room 
 template <int LIM, bool PER>
 __global__ void __launch_bounds__(32 * AXM_WARPS, ACT_MINB) k_advect_xm(
     const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tv,
-    const __grid_constant__ CUtensorMap to, Layout L, Box box, int nocycle, double eps, int nseg, int seg,
+    const __grid_constant__ CUtensorMap to, Layout L, Box box, RowCover cov, int nocycle, double eps, int nseg, int seg,
     const double *__restrict__ cin, double *__restrict__ cout, const double *__restrict__ vel, Geo3 sig, Geo3 dtvt,
     const int32_t *__restrict__ aloft, DevScalars *sc, double *__restrict__ out1, double *__restrict__ out2) {
   extern __shared__ unsigned char axm_smem[];
@@ -1630,20 +1634,19 @@ __global__ void __launch_bounds__(32 * AXM_WARPS, ACT_MINB) k_advect_xm(
   unsigned char *const sm = axm_smem + ((512u - (smem_u32(axm_smem) & 511u)) & 511u);  // the swizzle's period
   uint64_t *bar = reinterpret_cast<uint64_t *>(sm) + 2 * wid;
   unsigned char *const qbuf = sm + 512 + wid * AXM_WARP_B, *const vbuf = qbuf + 3 * AXM_BUF;
-  const int nrows = L.ny * L.nz;
-  const int ntile = (nrows + 31) >> 5;
-  const unsigned t = blockIdx.x * AXM_WARPS + wid, ns = L.ns, rr = t / ns, rs = rr / (unsigned)ntile;
+  const unsigned t = blockIdx.x * AXM_WARPS + wid, ns = L.ns, rr = t / ns, rs = rr / (unsigned)cov.ntile;
   if (rs >= (unsigned)nseg) return;  // whole warps only; no block barrier below
   const int g = (int)(t - rr * ns);
-  const int r0 = (int)(rr - rs * (unsigned)ntile) * 32;
-  const int s0 = (int)rs * seg + 1;
-  const int n = L.nx, s1 = min(n, s0 + seg - 1);
+  int r0, nrows;  // the tile's first row, the end of its run of rows
+  cov.tile((int)(rr - rs * (unsigned)cov.ntile), &r0, &nrows);
+  const int s0 = cov.x0 + (int)rs * seg;
+  const int n = L.nx, s1 = min(cov.x1, s0 + seg - 1);
   const int r = min(r0 + lane, nrows - 1);
   const int j = r % L.ny + 1, k = r / L.ny + 1;
   const int rmin = box.imin, rmax = box.imax;
   const bool al = r0 + lane < nrows && j >= box.jmin && j <= box.jmax && k >= box.kmin && k <= box.kmax &&
                   aloft[g] != 0;
-  const long grow = (long)g * nrows;  // this grain's first row in the level
+  const long grow = (long)g * L.ny * L.nz;  // this grain's first row in the level
   double *const po = cout + (grow + r0) * L.P;
   auto zero = [&](int ca, int cb) {   // cells ca..cb of the tile's rows: the reference leaves zeros
     for (int row = 0; row < min(32, nrows - r0); row++)
@@ -1829,14 +1832,16 @@ static bool launch_advect_xm(a3g_ctx *ctx) {
   if (!tensor_map(ctx, ctx->c0, TM_QROWS, &tq) || !tensor_map(ctx, ctx->vx, TM_VROWS, &tv) ||
       !tensor_map(ctx, ctx->c1, TM_QROWS, &to))
     return false;
-  const long nlw = (long)(((long)L.ny * L.nz + 31) / 32) * L.ns;
-  const int want = march_segments(L.nx, nlw);
-  const int seg = (L.nx + want - 1) / want + 7 & ~7;  // whole chunks
-  const int nseg = (L.nx + seg - 1) / seg;
+  const RowCover cov = row_cover(L, cover_box(ctx));
+  const int nxc = cov.x1 - cov.x0 + 1;
+  const long nlw = (long)cov.ntile * L.ns;
+  const int want = march_segments(nxc, nlw);
+  const int seg = (nxc + want - 1) / want + 7 & ~7;  // whole chunks
+  const int nseg = (nxc + seg - 1) / seg;
   const unsigned blocks = (unsigned)((nlw * nseg + AXM_WARPS - 1) / AXM_WARPS);
 #define A3G_XM(PER_)                                                                                           \
   k_advect_xm<LIM, PER_><<<blocks, 32 * AXM_WARPS, AXM_SMEM, ctx->stream>>>(                                    \
-      tq, tv, to, L, ctx->box, ctx->prm.nocycle, ctx->prm.eps_thresh, nseg, seg, ctx->c0, ctx->c1, ctx->vx,     \
+      tq, tv, to, L, ctx->box, cov, ctx->prm.nocycle, ctx->prm.eps_thresh, nseg, seg, ctx->c0, ctx->c1, ctx->vx,     \
       ctx->snx, ctx->dtv, ctx->aloft, ctx->sc, ctx->out_yz1, ctx->out_yz2)
   if (ctx->grid.periodic) A3G_XM(true); else A3G_XM(false);
 #undef A3G_XM

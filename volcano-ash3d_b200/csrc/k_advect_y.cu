@@ -14,7 +14,7 @@ int launch_advect_y(a3g_ctx *ctx) {
   A3G_LIM_SWITCH(launch_dir_lim, 1, )
   tend(ctx);
   A3G_LAUNCH_CHECK(ctx);
-  swap_levels(ctx);
+  sweep_done(ctx);
   return A3G_OK;
 }
 

@@ -144,21 +144,21 @@ __device__ __forceinline__ double adj_diff_cell(double l, double q, double r, do
 // 360x161x40, 5 grains: x and y 200 -> 64 us together; 100x100x40, 4 grains: 40
 // -> 15 us.
 template <bool XFIRST, bool ADJ, bool PER>
-__global__ void __launch_bounds__(128) k_diff_xy(Layout L, Box box, int nseg, int seg,
+__global__ void __launch_bounds__(128) k_diff_xy(Layout L, Box box, Box cov, int nseg, int seg,
                                                  const double *__restrict__ cin, double *__restrict__ cout,
                                                  const DiffRow *__restrict__ tab,
                                                  const int32_t *__restrict__ aloft,
                                                  const DevScalars *__restrict__ sc) {
   const int lane = threadIdx.x & 31;
-  const int nti = (L.nx + 29) / 30;
+  const int nti = (cov.imax - cov.imin + 30) / 30, nk = cov.kmax - cov.kmin + 1;
   const unsigned w = blockIdx.x * 4 + (threadIdx.x >> 5), wt = w / (unsigned)nti, ws = wt / (unsigned)nseg;
-  const int g = (int)(ws / (unsigned)L.nz), k = (int)ws - g * L.nz + 1;
+  const int g = (int)(ws / (unsigned)nk), k = (int)ws - g * nk + cov.kmin;
   if (g >= L.ns) return;  // whole warps
   const int it = (int)(w - wt * (unsigned)nti);
-  const int s0 = (int)(wt - ws * (unsigned)nseg) * seg + 1, s1 = min(L.ny, s0 + seg - 1);
-  const int i0 = it * 30 + lane;  // 1-based column of this lane: 0 and nx+1 are the ghosts
+  const int s0 = (int)(wt - ws * (unsigned)nseg) * seg + cov.jmin, s1 = min(cov.jmax, s0 + seg - 1);
+  const int i0 = cov.imin - 1 + it * 30 + lane;  // 1-based column of this lane: 0 and nx+1 are the ghosts
   const int i = i0 < 1 ? (PER ? L.nx : 1) : i0 > L.nx ? (PER ? (i0 - L.nx - 1) % L.nx + 1 : L.nx) : i0;
-  const bool own = lane >= 1 && lane <= 30 && i0 <= L.nx;
+  const bool own = lane >= 1 && lane <= 30 && i0 <= cov.imax;
   const double *q0 = cin + (long)g * L.PG + (long)(k - 1) * L.PY + (i - 1);
   double *p0 = cout + (long)g * L.PG + (long)(k - 1) * L.PY + (i - 1);
   const bool col_in = i >= box.imin && i <= box.imax && k >= box.kmin && k <= box.kmax;
@@ -211,17 +211,17 @@ __global__ void __launch_bounds__(128) k_diff_xy(Layout L, Box box, int nseg, in
 // DiffuseVert (ADJ: its transpose) marched along k, lanes along i, every cell
 // read once.  360x161x40, 5 grains: 82 -> 60 us.
 template <bool ADJ>
-__global__ void __launch_bounds__(128) k_diff_z(Layout L, Box box, int nseg, int seg, const double *__restrict__ cin,
+__global__ void __launch_bounds__(128) k_diff_z(Layout L, Box box, Box cov, int nseg, int seg, const double *__restrict__ cin,
                                                 double *__restrict__ cout, const DiffRow *__restrict__ tab,
                                                 const int32_t *__restrict__ aloft,
                                                 const DevScalars *__restrict__ sc) {
   const int lane = threadIdx.x & 31;
-  const int nti = (L.nx + 31) >> 5;
+  const int nti = (cov.imax - cov.imin + 32) >> 5, nj = cov.jmax - cov.jmin + 1;
   const unsigned w = blockIdx.x * 4 + (threadIdx.x >> 5), wt = w / (unsigned)nti, ws = wt / (unsigned)nseg;
-  const int g = (int)(ws / (unsigned)L.ny), j = (int)ws - g * L.ny + 1;
-  const int i = (int)(w - wt * (unsigned)nti) * 32 + lane + 1;
-  if (g >= L.ns || i > L.nx) return;
-  const int s0 = (int)(wt - ws * (unsigned)nseg) * seg + 1, s1 = min(L.nz, s0 + seg - 1);
+  const int g = (int)(ws / (unsigned)nj), j = (int)ws - g * nj + cov.jmin;
+  const int i = cov.imin + (int)(w - wt * (unsigned)nti) * 32 + lane;
+  if (g >= L.ns || i > cov.imax) return;
+  const int s0 = (int)(wt - ws * (unsigned)nseg) * seg + cov.kmin, s1 = min(cov.kmax, s0 + seg - 1);
   const double *q0 = cin + (long)g * L.PG + L.cell(i, j, 1);
   double *p0 = cout + (long)g * L.PG + L.cell(i, j, 1);
   if (!aloft[g] || i < box.imin || i > box.imax || j < box.jmin || j > box.jmax) {
@@ -963,7 +963,7 @@ constexpr int CXT_SMEM = 1024 + 1024 + CXT_WARPS * 3 * CXT_BUF;  // room to alig
 
 __global__ void __launch_bounds__(32 * CXT_WARPS, 8) k_cn_solve_xt2(const __grid_constant__ CUtensorMap tin,
                                                                    const __grid_constant__ CUtensorMap tout,
-                                                                   Layout L, Box box, LineMap map,
+                                                                   Layout L, Box box, RowCover cov, LineMap map,
                                                                    double *__restrict__ cout, CnTab tab,
                                                                    const int32_t *__restrict__ aloft,
                                                                    DevScalars *sc) {
@@ -972,15 +972,15 @@ __global__ void __launch_bounds__(32 * CXT_WARPS, 8) k_cn_solve_xt2(const __grid
   unsigned char *const sm = x2_smem + ((1024u - (smem_u32(x2_smem) & 1023u)) & 1023u);  // the swizzle's period
   uint64_t *bar = reinterpret_cast<uint64_t *>(sm) + 3 * w;
   unsigned char *const bufs = sm + 1024 + w * 3 * CXT_BUF;
-  const long nrows = (long)L.ny * L.nz * L.ns;
-  const long r0 = ((long)blockIdx.x * CXT_WARPS + w) * 32;
-  if (r0 >= nrows) return;  // uniform over the warp
-  const long r = r0 + lane;
-  const bool valid = r < nrows;
-  const unsigned rc = (unsigned)(valid ? r : nrows - 1), t1 = rc / (unsigned)L.ny, t2 = t1 / (unsigned)L.nz;
-  const int j = (int)(rc - t1 * (unsigned)L.ny) + 1;
-  const int k = (int)(t1 - t2 * (unsigned)L.nz) + 1;
-  const int g = (int)t2;
+  const unsigned tw = blockIdx.x * CXT_WARPS + w;
+  const int g = (int)(tw / (unsigned)cov.ntile);
+  if (g >= L.ns) return;  // uniform over the warp
+  int p0, pend;  // the tile's first row of the plane, the end of its run of rows
+  cov.tile((int)(tw - (unsigned)g * (unsigned)cov.ntile), &p0, &pend);
+  const int r0 = g * L.ny * L.nz + p0, nval = min(32, pend - p0);  // its first row of the level, its own rows
+  const bool valid = lane < nval;
+  const int pr = valid ? p0 + lane : pend - 1;
+  const int k = pr / L.ny + 1, j = pr - (k - 1) * L.ny + 1;
   const bool active =
       valid && j >= box.jmin && j <= box.jmax && k >= box.kmin && k <= box.kmax && aloft[g] != 0;
   const int rmin = box.imin, rmax = box.imax;
@@ -989,14 +989,13 @@ __global__ void __launch_bounds__(32 * CXT_WARPS, 8) k_cn_solve_xt2(const __grid
   const int xa = (rmin - 1) & ~1, off = (rmin - 1) - xa;  // 0-based cell of position 0; positions before the box
   const int np = off + ncells, nch = (np + CX_CH - 1) / CX_CH;
   const bool any = __any_sync(0xffffffffu, active);
-  {  // cells that no chunk store covers (outside the FAST_SUBGRID box): zeros
-    const int nr = (int)(nrows - r0 < 32 ? nrows - r0 : 32);
-    const int za = any ? xa : L.nx, zb = any ? xa + nch * CX_CH : L.nx;
-    if (za > 0 || zb < L.nx)
-      for (int row = 0; row < nr; row++) {
-        double *xr = cout + (r0 + row) * P;
-        for (int c = lane; c < za; c += 32) xr[c] = 0.0;
-        for (int c = zb + lane; c < L.nx; c += 32) xr[c] = 0.0;
+  {  // cells of the cover that no chunk store reaches: zeros
+    const int za = any ? xa : cov.x1, zb = any ? xa + nch * CX_CH : cov.x1;
+    if (za > cov.x0 - 1 || zb < cov.x1)
+      for (int row = 0; row < nval; row++) {
+        double *xr = cout + (long)(r0 + row) * P;
+        for (int c = cov.x0 - 1 + lane; c < za; c += 32) xr[c] = 0.0;
+        for (int c = zb + lane; c < cov.x1; c += 32) xr[c] = 0.0;
       }
   }
   if (!any) return;
@@ -1013,13 +1012,13 @@ __global__ void __launch_bounds__(32 * CXT_WARPS, 8) k_cn_solve_xt2(const __grid
       const int ch = p < nch ? p : 2 * nch - 2 - p;
       bulk_wait_read0();
       mbar_arrive_expect_tx(&bar[p % 3], CXT_BUF);
-      tma_load_2d(bufs + (p % 3) * CXT_BUF, &tin, &bar[p % 3], xa + ch * CX_CH, (int)r0);
+      tma_load_2d(bufs + (p % 3) * CXT_BUF, &tin, &bar[p % 3], xa + ch * CX_CH, r0);
     }
   };
   issue(0);
   issue(1);
   // this lane's parking place of chunk ch: park[ch*CX_CH]
-  double *const park = cout + (r0 + (lane >> 4)) * P + xa + (lane & 15);
+  double *const park = cout + (long)(r0 + (lane >> 4)) * P + xa + (lane & 15);
   const long u = map.u(j, k);
   CnRun R;
   cn_load_run(tab, u, R);
@@ -1179,9 +1178,20 @@ __global__ void __launch_bounds__(32 * CXT_WARPS, 8) k_cn_solve_xt2(const __grid
     }
     fence_proxy_async_smem();
     __syncwarp();
-    if (lane == 0) {  // rows past the last one lie outside the tensor
-      tma_store_2d(&tout, b, xa + ch * CX_CH, (int)r0);
-      bulk_commit();
+    if (nval == 32) {
+      if (lane == 0) {
+        tma_store_2d(&tout, b, xa + ch * CX_CH, r0);
+        bulk_commit();
+      }
+    } else {  // the rows past the run's end belong to others
+      const int e = lane & 15, x = xa + ch * CX_CH + e;
+#pragma unroll 1
+      for (int row = lane >> 4; row < nval; row += 2) {
+        if (x < L.nx)
+          cout[(long)(r0 + row) * P + x] =
+              *reinterpret_cast<const double *>(b + (row << 7) + ((((e >> 1) ^ (row & 7)) << 4) | ((e & 1) << 3)));
+      }
+      __syncwarp();
     }
   }
   if (lane == 0) {
@@ -1214,7 +1224,7 @@ __host__ __device__ __forceinline__ long zt_warp_doubles(int nz) {
 
 __global__ void __launch_bounds__(64, 8) k_cn_solve_zt(const __grid_constant__ CUtensorMap tin,
                                                     const __grid_constant__ CUtensorMap tout, Layout L,
-                                                    Box box, LineMap map, CnTab tab,
+                                                    Box box, Box cov, LineMap map, CnTab tab,
                                                     const int32_t *__restrict__ aloft, DevScalars *sc,
                                                     int wpb) {
   extern __shared__ __align__(128) unsigned char zt_smem[];
@@ -1230,8 +1240,8 @@ __global__ void __launch_bounds__(64, 8) k_cn_solve_zt(const __grid_constant__ C
     prefetch_tensormap(&tout);
   }
   __syncwarp();
-  const int nti = (L.nx + 31) >> 5;
-  const long ntiles = (long)nti * L.ny * L.ns;
+  const int it0 = (cov.imin - 1) >> 5, nti = ((cov.imax - 1) >> 5) - it0 + 1, nj = cov.jmax - cov.jmin + 1;
+  const long ntiles = (long)nti * nj * L.ns;
   const long nwarps = (long)gridDim.x * wpb;
   const long per = ((unsigned)ntiles + (unsigned)nwarps - 1u) / (unsigned)nwarps;
   const long t0 = ((long)blockIdx.x * wpb + wid) * per;
@@ -1244,9 +1254,9 @@ __global__ void __launch_bounds__(64, 8) k_cn_solve_zt(const __grid_constant__ C
   double *xx = tile + lane + (long)(rmin - 1) * 32;  // row l of this lane's line at xx[l*32]
   const double2 *const row2 = reinterpret_cast<const double2 *>(stab);  // FACT,CL  CC,CR  DU,ZH  ZL,ZLL
   for (long t = t0; t < t1; t++) {
-    const unsigned r = (unsigned)t / (unsigned)nti, rg = r / (unsigned)L.ny;
-    const int it = (int)((unsigned)t - r * (unsigned)nti);
-    const int j = (int)(r - rg * (unsigned)L.ny) + 1;
+    const unsigned r = (unsigned)t / (unsigned)nti, rg = r / (unsigned)nj;
+    const int it = it0 + (int)((unsigned)t - r * (unsigned)nti);
+    const int j = cov.jmin + (int)(r - rg * (unsigned)nj);
     const int g = (int)rg;
     const int i = (it << 5) + lane + 1;
     const bool act = i <= L.nx && i >= box.imin && i <= box.imax && j >= box.jmin && j <= box.jmax &&
@@ -1373,7 +1383,7 @@ constexpr int YT_BUF_D = YT_CH * 32 + YT_CH * CN_ROW;  // doubles of a buffer: t
 
 __global__ void __launch_bounds__(64, 8) k_cn_solve_yt(const __grid_constant__ CUtensorMap tin,
                                                     const __grid_constant__ CUtensorMap tout, Layout L,
-                                                    Box box, LineMap map, double *__restrict__ cout, CnTab tab,
+                                                    Box box, Box cov, LineMap map, double *__restrict__ cout, CnTab tab,
                                                     const int32_t *__restrict__ aloft, DevScalars *sc,
                                                     int wpb) {
   extern __shared__ __align__(128) unsigned char yt_smem[];
@@ -1389,8 +1399,8 @@ __global__ void __launch_bounds__(64, 8) k_cn_solve_yt(const __grid_constant__ C
     prefetch_tensormap(&tout);
   }
   __syncwarp();
-  const int nti = (L.nx + 31) >> 5;
-  const long ngroups = (long)nti * L.nz * L.ns;
+  const int it0 = (cov.imin - 1) >> 5, nti = ((cov.imax - 1) >> 5) - it0 + 1, nk = cov.kmax - cov.kmin + 1;
+  const long ngroups = (long)nti * nk * L.ns;
   const long nwarps = (long)gridDim.x * wpb;
   const long per = ((unsigned)ngroups + (unsigned)nwarps - 1u) / (unsigned)nwarps;
   const long t0 = ((long)blockIdx.x * wpb + wid) * per;
@@ -1401,9 +1411,9 @@ __global__ void __launch_bounds__(64, 8) k_cn_solve_yt(const __grid_constant__ C
   const int cnt_last = ncells - (nch - 1) * YT_CH;
   uint32_t s0 = 0;  // loads of the groups before: load p of this one is the warp's load s0 + p
   for (long t = t0; t < t1; t++) {
-    const unsigned r = (unsigned)t / (unsigned)nti, rg = r / (unsigned)L.nz;
-    const int it = (int)((unsigned)t - r * (unsigned)nti);
-    const int k = (int)(r - rg * (unsigned)L.nz) + 1;
+    const unsigned r = (unsigned)t / (unsigned)nti, rg = r / (unsigned)nk;
+    const int it = it0 + (int)((unsigned)t - r * (unsigned)nti);
+    const int k = cov.kmin + (int)(r - rg * (unsigned)nk);
     const int g = (int)rg;
     const int i = (it << 5) + lane + 1;
     const bool act = i <= L.nx && i >= box.imin && i <= box.imax && k >= box.kmin && k <= box.kmax &&
@@ -1412,12 +1422,12 @@ __global__ void __launch_bounds__(64, 8) k_cn_solve_yt(const __grid_constant__ C
     double *xg = cout + (long)g * L.PG + (long)(k - 1) * L.PY + (i - 1);  // cell (i, 1, k) of this lane
     if (!any) {  // the reference leaves zeros
       if (i <= L.nx)
-        for (int j = 1; j <= L.ny; j++) xg[(long)(j - 1) * L.P] = 0.0;
+        for (int j = cov.jmin; j <= cov.jmax; j++) xg[(long)(j - 1) * L.P] = 0.0;
       continue;
     }
     if (i <= L.nx) {  // cells that no chunk store covers: outside [rmin, rmin + nch*YT_CH)
-      for (int j = 1; j < rmin; j++) xg[(long)(j - 1) * L.P] = 0.0;
-      for (int j = rmin + nch * YT_CH; j <= L.ny; j++) xg[(long)(j - 1) * L.P] = 0.0;
+      for (int j = cov.jmin; j < rmin; j++) xg[(long)(j - 1) * L.P] = 0.0;
+      for (int j = rmin + nch * YT_CH; j <= cov.jmax; j++) xg[(long)(j - 1) * L.P] = 0.0;
     }
     xg += (long)(rmin - 1) * L.P;  // row 0
     const long u = map.u(1, k);    // the coefficients do not vary along i (map.da == 0)
@@ -1694,10 +1704,11 @@ static bool launch_cn_solve_zt(a3g_ctx *ctx, const LineMap &map, const CnTab &ta
     if (!tile_kernel_setup(ctx, k_cn_solve_zt, 32 * wpb, smem, &per_sm, &nsm)) return false;
     ctx->tma_grid[0] = per_sm * nsm;
   }
-  const long ntiles = (long)((L.nx + 31) / 32) * L.ny * L.ns;
+  const Box cov = cover_box(ctx);
+  const long ntiles = (long)((cov.imax - 1) / 32 - (cov.imin - 1) / 32 + 1) * (cov.jmax - cov.jmin + 1) * L.ns;
   const long need = (ntiles + wpb - 1) / wpb;
   const int grid = (int)(need < ctx->tma_grid[0] ? need : ctx->tma_grid[0]);
-  k_cn_solve_zt<<<grid, 32 * wpb, smem, ctx->stream>>>(tin, tout, L, ctx->box, map, tab, ctx->aloft, ctx->sc,
+  k_cn_solve_zt<<<grid, 32 * wpb, smem, ctx->stream>>>(tin, tout, L, ctx->box, cov, map, tab, ctx->aloft, ctx->sc,
                                                        wpb);
   return true;
 }
@@ -1716,10 +1727,11 @@ static bool launch_cn_solve_yt(a3g_ctx *ctx, const LineMap &map, const CnTab &ta
     if (!tile_kernel_setup(ctx, k_cn_solve_yt, 32 * wpb, smem, &per_sm, &nsm)) return false;
     ctx->tma_grid[1] = per_sm * nsm;
   }
-  const long ngroups = (long)((L.nx + 31) / 32) * L.nz * L.ns;
+  const Box cov = cover_box(ctx);
+  const long ngroups = (long)((cov.imax - 1) / 32 - (cov.imin - 1) / 32 + 1) * (cov.kmax - cov.kmin + 1) * L.ns;
   const long need = (ngroups + wpb - 1) / wpb;
   const int grid = (int)(need < ctx->tma_grid[1] ? need : ctx->tma_grid[1]);
-  k_cn_solve_yt<<<grid, 32 * wpb, smem, ctx->stream>>>(tin, tout, L, ctx->box, map, ctx->c1, tab, ctx->aloft,
+  k_cn_solve_yt<<<grid, 32 * wpb, smem, ctx->stream>>>(tin, tout, L, ctx->box, cov, map, ctx->c1, tab, ctx->aloft,
                                                        ctx->sc, wpb);
   return true;
 }
@@ -1734,9 +1746,10 @@ static bool launch_cn_solve_xt2(a3g_ctx *ctx, const LineMap &map, const CnTab &t
     if (!tile_kernel_setup(ctx, k_cn_solve_xt2, 32 * CXT_WARPS, CXT_SMEM, &per_sm, &nsm)) return false;
     ctx->tma_grid[2] = per_sm * nsm;
   }
-  const long nwarps = ((long)L.ny * L.nz * L.ns + 31) / 32;
+  const RowCover cov = row_cover(L, cover_box(ctx));
+  const long nwarps = (long)cov.ntile * L.ns;
   k_cn_solve_xt2<<<(unsigned)((nwarps + CXT_WARPS - 1) / CXT_WARPS), 32 * CXT_WARPS, CXT_SMEM, ctx->stream>>>(
-      tin, tout, L, ctx->box, map, ctx->c1, tab, ctx->aloft, ctx->sc);
+      tin, tout, L, ctx->box, cov, map, ctx->c1, tab, ctx->aloft, ctx->sc);
   return true;
 }
 
@@ -1774,16 +1787,17 @@ static int diff_segments(int n, long warps) {
 
 // The horizontal sweeps in one pass, x first or y first; false as diff_table.
 template <bool ADJ>
-static bool run_diff_xy(a3g_ctx *ctx, bool xfirst, const Box &box, const double *cin, double *cout) {
+static bool run_diff_xy(a3g_ctx *ctx, bool xfirst, const Box &box, const Box &cov, const double *cin, double *cout) {
   if (!diff_table(ctx)) return false;
   const Layout &L = ctx->L;
-  const long lines = (long)((L.nx + 29) / 30) * L.nz * L.ns;
-  const int seg = (L.ny + diff_segments(L.ny, lines) - 1) / diff_segments(L.ny, lines);
-  const int nseg = (L.ny + seg - 1) / seg;
+  const int n = cov.jmax - cov.jmin + 1;
+  const long lines = (long)((cov.imax - cov.imin + 30) / 30) * (cov.kmax - cov.kmin + 1) * L.ns;
+  const int seg = (n + diff_segments(n, lines) - 1) / diff_segments(n, lines);
+  const int nseg = (n + seg - 1) / seg;
   const unsigned blocks = (unsigned)((lines * nseg + 3) / 4);
   const DiffRow *tab = static_cast<const DiffRow *>(ctx->diff_tab);
 #define A3G_DXY(X_, P_) \
-  k_diff_xy<X_, ADJ, P_><<<blocks, 128, 0, ctx->stream>>>(L, box, nseg, seg, cin, cout, tab, ctx->aloft, ctx->sc)
+  k_diff_xy<X_, ADJ, P_><<<blocks, 128, 0, ctx->stream>>>(L, box, cov, nseg, seg, cin, cout, tab, ctx->aloft, ctx->sc)
   if (ctx->grid.periodic) {
     if (xfirst) A3G_DXY(true, true); else A3G_DXY(false, true);
   } else {
@@ -1794,14 +1808,15 @@ static bool run_diff_xy(a3g_ctx *ctx, bool xfirst, const Box &box, const double 
 }
 
 template <bool ADJ>
-static bool run_diff_z(a3g_ctx *ctx, const Box &box, const double *cin, double *cout) {
+static bool run_diff_z(a3g_ctx *ctx, const Box &box, const Box &cov, const double *cin, double *cout) {
   if (!diff_table(ctx)) return false;
   const Layout &L = ctx->L;
-  const long lines = (long)((L.nx + 31) / 32) * L.ny * L.ns;
-  const int seg = (L.nz + diff_segments(L.nz, lines) - 1) / diff_segments(L.nz, lines);
-  const int nseg = (L.nz + seg - 1) / seg;
+  const int n = cov.kmax - cov.kmin + 1;
+  const long lines = (long)((cov.imax - cov.imin + 32) / 32) * (cov.jmax - cov.jmin + 1) * L.ns;
+  const int seg = (n + diff_segments(n, lines) - 1) / diff_segments(n, lines);
+  const int nseg = (n + seg - 1) / seg;
   k_diff_z<ADJ><<<(unsigned)((lines * nseg + 3) / 4), 128, 0, ctx->stream>>>(
-      L, box, nseg, seg, cin, cout, static_cast<const DiffRow *>(ctx->diff_tab), ctx->aloft, ctx->sc);
+      L, box, cov, nseg, seg, cin, cout, static_cast<const DiffRow *>(ctx->diff_tab), ctx->aloft, ctx->sc);
   return true;
 }
 
@@ -1809,7 +1824,7 @@ template <int DIR>
 static int launch_diff_dir(a3g_ctx *ctx) {
   const Layout &L = ctx->L;
   tbegin(ctx, A3G_K_DIFF_X + DIR);
-  if (DIR == 2 && run_diff_z<false>(ctx, ctx->box, ctx->c0, ctx->c1)) {
+  if (DIR == 2 && run_diff_z<false>(ctx, ctx->box, cover_box(ctx), ctx->c0, ctx->c1)) {
     // marched
   } else {
     const Geo3 &sig = (DIR == 0) ? ctx->snx : (DIR == 1) ? ctx->sny : ctx->snz;
@@ -1821,14 +1836,14 @@ static int launch_diff_dir(a3g_ctx *ctx) {
   }
   tend(ctx);
   A3G_LAUNCH_CHECK(ctx);
-  swap_levels(ctx);
+  sweep_done(ctx);
   return A3G_OK;
 }
 
 // DiffuseHorz, explicit: both sweeps, x first or y first.
 int launch_diff_horz(a3g_ctx *ctx, bool xfirst) {
   tbegin(ctx, A3G_K_DIFF_X);
-  const bool fused = run_diff_xy<false>(ctx, xfirst, ctx->box, ctx->c0, ctx->c1);
+  const bool fused = run_diff_xy<false>(ctx, xfirst, ctx->box, cover_box(ctx), ctx->c0, ctx->c1);
   tend(ctx);
   if (!fused) {
     int rc = xfirst ? launch_diff_dir<0>(ctx) : launch_diff_dir<1>(ctx);
@@ -1836,7 +1851,7 @@ int launch_diff_horz(a3g_ctx *ctx, bool xfirst) {
     return rc;
   }
   A3G_LAUNCH_CHECK(ctx);
-  swap_levels(ctx);
+  sweep_done(ctx);
   return A3G_OK;
 }
 
@@ -1945,7 +1960,7 @@ static int launch_cn_dir(a3g_ctx *ctx) {
   }
   tend(ctx);
   A3G_LAUNCH_CHECK(ctx);
-  swap_levels(ctx);
+  sweep_done(ctx);
   ctx->ts1_zeroed = false;
   return A3G_OK;
 }
@@ -2078,7 +2093,7 @@ static int launch_adj_diff_dir(a3g_ctx *ctx, const double *lin, double *lout) {
   dim3 grid((L.nx + 31) / 32, (L.ny + 7) / 8, L.nz);
   const Box full{1, L.nx, 1, L.ny, 1, L.nz};
   tbegin(ctx, A3G_K_ADJOINT);
-  if (!(DIR == 2 && run_diff_z<true>(ctx, full, lin, lout)))
+  if (!(DIR == 2 && run_diff_z<true>(ctx, full, full, lin, lout)))
     k_adj_diff<DIR><<<grid, dim3(32, 8), 0, ctx->stream>>>(L, ctx->grid.periodic, lin, lout, sig, ctx->kappa,
                                                          kk, ctx->aloft, ctx->sc);
   tend(ctx);
@@ -2092,7 +2107,7 @@ static int launch_adj_diff_dir(a3g_ctx *ctx, const double *lin, double *lout) {
 int launch_adj_diff_horz(a3g_ctx *ctx, bool xfirst, const double *lin, double *lout, bool *done) {
   const Box full{1, ctx->L.nx, 1, ctx->L.ny, 1, ctx->L.nz};
   tbegin(ctx, A3G_K_ADJOINT);
-  *done = run_diff_xy<true>(ctx, xfirst, full, lin, lout);
+  *done = run_diff_xy<true>(ctx, xfirst, full, full, lin, lout);
   tend(ctx);
   if (*done) A3G_LAUNCH_CHECK(ctx);
   return A3G_OK;
