@@ -725,6 +725,263 @@ static void launch_cn_solve_gc(a3g_ctx *ctx, const LineMap &map, const CnTab &ta
     k_cn_solve_gc<DIR, GC><<<grid, 128, 0, ctx->stream>>>(L, ctx->box, map, ctx->c0, ctx->c1, tab, ctx->aloft);
 }
 
+// y and z lines whose coefficients vary along i (terrain), where no two lanes
+// share a table row.  A warp holds 32 neighbouring lines of one grain and its
+// block the same lines of the other grains, which so find the table rows in
+// L1; rows are taken CB_U at a time, all their loads before the first of the
+// dependent operations.  Bound by the latency of those loads and the memory
+// behind them: a thread per line with a row at a time, two grains together,
+// waited for one row after another (201x151x41, 5 grains over terrain: y 324
+// -> 64 us, z 84 -> 69 us).
+constexpr int CB_U = 8, CB_WARPS = 8;
+
+// Lines of 32 neighbouring i: where a thread's line of direction DIR starts.
+template <int DIR>
+__device__ __forceinline__ bool cb_line(const Layout &L, int *a, int *b, int *g, long *base, long *st) {
+  const int nti = (L.nx + 31) >> 5;
+  *b = (int)(blockIdx.x / (unsigned)nti) + 1;
+  *a = (int)(blockIdx.x % (unsigned)nti) * 32 + (int)(threadIdx.x & 31) + 1;
+  *g = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (*a > L.nx || *g >= L.ns) return false;
+  *base = (DIR == 1 ? L.cell(*a, 1, *b) : L.cell(*a, *b, 1)) + (long)*g * L.PG;
+  *st = DIR == 1 ? L.P : L.PY;
+  return true;
+}
+template <int DIR>
+static dim3 cb_grid(const Layout &L, int *threads) {
+  const int w = L.ns < CB_WARPS ? L.ns : CB_WARPS;
+  *threads = 32 * w;
+  return dim3(((L.nx + 31) / 32) * (DIR == 1 ? L.nz : L.ny), (L.ns + w - 1) / w);
+}
+
+template <int DIR>
+__global__ void __launch_bounds__(32 * CB_WARPS, 2) k_cn_solve_b(Layout L, Box box, LineMap map,
+                                                                 const double *__restrict__ cin,
+                                                                 double *__restrict__ cout, CnTab tab,
+                                                                 const int32_t *__restrict__ aloft) {
+  int a, b, g;
+  long base, st;
+  if (!cb_line<DIR>(L, &a, &b, &g, &base, &st)) return;
+  const int n = (DIR == 1) ? L.ny : L.nz;
+  const int rmin = (DIR == 1) ? box.jmin : box.kmin, rmax = (DIR == 1) ? box.jmax : box.kmax;
+  const int ncells = rmax - rmin + 1;
+  const bool in = a >= box.imin && a <= box.imax && b >= ((DIR == 1) ? box.kmin : box.jmin) &&
+                  b <= ((DIR == 1) ? box.kmax : box.jmax) && aloft[g] != 0;
+  double *x = cout + base;
+  if (!in) {
+    for (int c = 1; c <= n; c++) x[(long)(c - 1) * st] = 0.0;
+    return;
+  }
+  for (int c = 1; c < rmin; c++) x[(long)(c - 1) * st] = 0.0;
+  for (int c = rmax + 1; c <= n; c++) x[(long)(c - 1) * st] = 0.0;
+  const long u = map.u(a, b);
+  const double *qq = cin + base + (long)(rmin - 1) * st;
+  x += (long)(rmin - 1) * st;
+  const double *tp = tab.p + u;
+  auto co = [&](int f, int l) { return __ldg(tp + f * tab.F + (long)l * tab.U); };
+  // forward elimination with the right-hand side built on the fly, :813-851
+  double qm = __ldg(qq), qc = qm, bp = 0.0;  // BC_left_t0 = q(rmin)
+  int l = 0;
+  for (; l + CB_U < ncells; l += CB_U) {
+    double q[CB_U], cl[CB_U], cc[CB_U], cr[CB_U], fa[CB_U];
+#pragma unroll
+    for (int e = 0; e < CB_U; e++) {
+      q[e] = __ldg(qq + (long)(l + 1 + e) * st);
+      cl[e] = co(CN_CL, l + e);
+      cc[e] = co(CN_CC, l + e);
+      cr[e] = co(CN_CR, l + e);
+      fa[e] = co(CN_FACT, l + e);
+    }
+#pragma unroll
+    for (int e = 0; e < CB_U; e++) {
+      const double B = cl[e] * qm + cc[e] * qc + cr[e] * q[e];
+      bp = (e == 0 && l == 0) ? B : B - fa[e] * bp;
+      x[(long)(l + e) * st] = bp;
+      qm = qc;
+      qc = q[e];
+    }
+  }
+  for (; l < ncells; l++) {
+    const double qp = l + 1 < ncells ? __ldg(qq + (long)(l + 1) * st) : qc;  // BC_right_t0 = q(rmax)
+    const double B = co(CN_CL, l) * qm + co(CN_CC, l) * qc + co(CN_CR, l) * qp;
+    bp = (l == 0) ? B : B - co(CN_FACT, l) * bp;
+    x[(long)l * st] = bp;
+    qm = qc;
+    qc = qp;
+  }
+  // back substitution
+  double xn = div_rn_rcp(bp, co(CN_DP, ncells - 1), co(CN_ZH, ncells - 1));
+  x[(long)(ncells - 1) * st] = xn;
+  l = ncells - 2;  // the next row to do
+  for (; l >= CB_U - 1; l -= CB_U) {
+    double y[CB_U], du[CB_U], dp[CB_U], zh[CB_U];
+#pragma unroll
+    for (int e = 0; e < CB_U; e++) {
+      y[e] = x[(long)(l - e) * st];
+      du[e] = co(CN_DU, l - e);
+      dp[e] = co(CN_DP, l - e);
+      zh[e] = co(CN_ZH, l - e);
+    }
+#pragma unroll
+    for (int e = 0; e < CB_U; e++) {
+      xn = div_rn_rcp(y[e] - du[e] * xn, dp[e], zh[e]);
+      x[(long)(l - e) * st] = xn;
+    }
+  }
+  for (; l >= 0; l--) {
+    xn = div_rn_rcp(x[(long)l * st] - co(CN_DU, l) * xn, co(CN_DP, l), co(CN_ZH, l));
+    x[(long)l * st] = xn;
+  }
+}
+
+// 32 x rows of a grain to a warp, their cells in chunks of 32 through a shared
+// tile: row segments come and go coalesced, the lanes work along their own
+// rows in between, and the chunk after is on its way (in registers) while one
+// is worked on.  A block's warps hold the same rows of several grains.
+constexpr int RT_WARPS = 5, RT_S = 33;
+
+struct RowTile {
+  double *tile, *own;
+  int lane, r0, nr, n, j, k, g;  // first row of the level, rows, cells; this lane's row
+  long P;
+  __device__ __forceinline__ bool init(const Layout &L, double *t, int cells) {
+    lane = threadIdx.x & 31;
+    g = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (g >= L.ns) return false;
+    const int plane = L.ny * L.nz, p0 = blockIdx.x * 32;
+    nr = plane - p0 < 32 ? plane - p0 : 32;
+    r0 = g * plane + p0;
+    const int pr = lane < nr ? p0 + lane : plane - 1;
+    k = pr / L.ny + 1;
+    j = pr - (k - 1) * L.ny + 1;
+    n = cells;
+    P = L.P;
+    tile = t;
+    own = t + lane * RT_S;
+    return true;
+  }
+  // cell c0 + lane of every row, from src (cell 0 of the level's first row)
+  __device__ __forceinline__ void fetch(double (&next)[32], const double *src, int c0) const {
+    const double *p = src + (long)r0 * P + c0 + lane;
+#pragma unroll
+    for (int e = 0; e < 32; e++) next[e] = (e < nr && c0 + lane < n) ? p[(long)e * P] : 0.0;
+  }
+  __device__ __forceinline__ void fill(const double (&next)[32]) const {
+#pragma unroll
+    for (int e = 0; e < 32; e++) tile[e * RT_S + lane] = next[e];
+    __syncwarp();
+  }
+  // columns col.. of the tile to the cells c0.. of every row
+  __device__ __forceinline__ void drain(double *dst, int c0, int col, int cnt) const {
+    __syncwarp();
+    double *p = dst + (long)r0 * P + c0 + lane;
+    if (lane < cnt) {
+#pragma unroll 8
+      for (int e = 0; e < nr; e++) p[(long)e * P] = tile[e * RT_S + col + lane];
+    }
+    __syncwarp();
+  }
+};
+static dim3 rt_grid(const Layout &L, int *threads) {
+  const int w = L.ns < RT_WARPS ? L.ns : RT_WARPS;
+  *threads = 32 * w;
+  return dim3((L.ny * L.nz + 31) / 32, (L.ns + w - 1) / w);
+}
+
+// x lines whose coefficients vary along them (terrain): B' goes out and comes
+// back, the table rows are taken CB_U at a time.  Bound by the latency of
+// those loads; k_cn_solve_xt2, whose fast path needs lines that settle to one
+// row, waits for each of them (201x151x41, 5 grains: 298 -> 138 us).  Four
+// warps a block (two groups for 5 grains, a second wave) measured 194 us.
+__global__ void __launch_bounds__(32 * RT_WARPS, 2) k_cn_solve_xv(Layout L, Box box, LineMap map,
+                                                                  const double *__restrict__ cin,
+                                                                  double *__restrict__ cout, CnTab tab,
+                                                                  const int32_t *__restrict__ aloft) {
+  __shared__ double sh[RT_WARPS][32 * RT_S];
+  const int n = box.imax - box.imin + 1, nch = (n + 31) >> 5;
+  RowTile T;
+  if (!T.init(L, sh[threadIdx.x >> 5], n)) return;  // uniform over the warp
+  const bool act = T.j >= box.jmin && T.j <= box.jmax && T.k >= box.kmin && T.k <= box.kmax && aloft[T.g] != 0;
+  if (n < L.nx)  // cells outside the box
+    for (int row = 0; row < T.nr; row++) {
+      double *xr = cout + (long)(T.r0 + row) * L.P;
+      for (int c = T.lane; c < box.imin - 1; c += 32) xr[c] = 0.0;
+      for (int c = box.imax + T.lane; c < L.nx; c += 32) xr[c] = 0.0;
+    }
+  cin += box.imin - 1;
+  cout += box.imin - 1;
+  const double *q_own = cin + (long)(T.r0 + (T.lane < T.nr ? T.lane : 0)) * L.P;
+  const long u = map.u(T.j, T.k);
+  CnRun R;
+  cn_load_run(tab, u, R);
+  auto co = [&](int f, int l) { return cn_coef(tab, u, R, f, l); };
+  double next[32];
+  double *const own = T.own;
+  // forward elimination with the right-hand side built on the fly, :813-851
+  T.fetch(next, cin, 0);
+  double qm = 0.0, qc = 0.0, bp = 0.0;
+  for (int ch = 0; ch < nch; ch++) {
+    const int c0 = 32 * ch, cnt = n - c0 < 32 ? n - c0 : 32;
+    T.fill(next);
+    if (ch + 1 < nch) {
+      own[32] = q_own[c0 + 32];
+      T.fetch(next, cin, c0 + 32);
+    } else {
+      own[cnt] = own[cnt - 1];  // BC_right_t0 = q(rmax)
+    }
+    if (ch == 0) qm = own[0];  // BC_left_t0 = q(rmin)
+    qc = own[0];
+    for (int e0 = 0; e0 < cnt; e0 += CB_U) {
+      double cl[CB_U], cc[CB_U], cr[CB_U], fa[CB_U];
+#pragma unroll
+      for (int e = 0; e < CB_U; e++) {
+        const int l = c0 + e0 + e < n ? c0 + e0 + e : n - 1;
+        cl[e] = co(CN_CL, l);
+        cc[e] = co(CN_CC, l);
+        cr[e] = co(CN_CR, l);
+        fa[e] = co(CN_FACT, l);
+      }
+#pragma unroll
+      for (int e = 0; e < CB_U; e++) {
+        if (e0 + e >= cnt) break;
+        const double qp = own[e0 + e + 1];
+        const double B = cl[e] * qm + cc[e] * qc + cr[e] * qp;
+        bp = (e == 0 && c0 + e0 == 0) ? B : B - fa[e] * bp;
+        own[e0 + e] = bp;
+        qm = qc;
+        qc = qp;
+      }
+    }
+    if (ch + 1 < nch) T.drain(cout, c0, 0, cnt);
+  }
+  // back substitution; the last chunk is still in the tile
+  double xn = 0.0;
+  __syncwarp();
+  for (int ch = nch - 1; ch >= 0; ch--) {
+    const int c0 = 32 * ch, cnt = n - c0 < 32 ? n - c0 : 32;
+    if (ch != nch - 1) T.fill(next);
+    if (ch > 0) T.fetch(next, cout, c0 - 32);
+    for (int e0 = cnt - 1; e0 >= 0; e0 -= CB_U) {
+      double du[CB_U], dp[CB_U], zh[CB_U];
+#pragma unroll
+      for (int e = 0; e < CB_U; e++) {
+        const int l = c0 + e0 - e > 0 ? c0 + e0 - e : 0;
+        du[e] = co(CN_DU, l);
+        dp[e] = co(CN_DP, l);
+        zh[e] = co(CN_ZH, l);
+      }
+#pragma unroll
+      for (int e = 0; e < CB_U; e++) {
+        if (e0 - e < 0) break;
+        const double b = own[e0 - e];
+        xn = div_rn_rcp((e == 0 && c0 + e0 == n - 1) ? b : b - du[e] * xn, dp[e], zh[e]);
+        own[e0 - e] = act ? xn : 0.0;
+      }
+    }
+    T.drain(cout, c0, 0, cnt);
+  }
+}
+
 // Solve kernel: one thread per line (a, b, grain), lines enumerated with a
 // fastest so that a warp holds neighbouring lines (neighbouring i for y and
 // z lines: coalesced loads and stores).
@@ -1940,7 +2197,11 @@ static int launch_cn_dir(a3g_ctx *ctx) {
   if (rc) return rc;
   const long nlines = (long)map.na * map.nb * L.ns;
   tbegin(ctx, A3G_K_CN_SOLVE_X + DIR);
-  if (DIR == 0 && ctx->tune_cn_x == 2 && launch_cn_solve_xt2(ctx, map, tab)) {
+  if (DIR == 0 && ctx->tune_cn_x == 2 && map.ds) {
+    int threads;
+    const dim3 grid = rt_grid(L, &threads);
+    k_cn_solve_xv<<<grid, threads, 0, ctx->stream>>>(L, box, map, ctx->c0, ctx->c1, tab, ctx->aloft);
+  } else if (DIR == 0 && ctx->tune_cn_x == 2 && launch_cn_solve_xt2(ctx, map, tab)) {
     // tiles through TMA
   } else if (DIR == 0 && ctx->tune_cn_x == 0) {
     const long nwarps = (nlines + 31) / 32;
@@ -1950,6 +2211,10 @@ static int launch_cn_dir(a3g_ctx *ctx) {
     // column tiles through TMA
   } else if (DIR == 1 && ctx->tune_cn_yz == 3 && launch_cn_solve_yt(ctx, map, tab)) {
     // chunk tiles through TMA
+  } else if (DIR != 0 && ctx->tune_cn_yz == 3 && !tab.byrow) {
+    int threads;
+    const dim3 grid = cb_grid<DIR == 0 ? 1 : DIR>(L, &threads);
+    k_cn_solve_b<DIR == 0 ? 1 : DIR><<<grid, threads, 0, ctx->stream>>>(L, box, map, ctx->c0, ctx->c1, tab, ctx->aloft);
   } else if (DIR != 0 && (ctx->tune_cn_yz == 1 || ctx->tune_cn_yz == 3) && L.ns >= 2) {
     launch_cn_solve_gc<DIR == 0 ? 1 : DIR, 2>(ctx, map, tab);
   } else if (DIR != 0 && ctx->tune_cn_yz == 2 && L.ns >= 2) {
@@ -2031,25 +2296,21 @@ __global__ void __launch_bounds__(256) k_adj_diff(Layout L, int periodic, const 
 //   lam_q(r) = CC(r)y(r) + CR(r-1)y(r-1) + CL(r+1)y(r+1)
 // plus CL(0)y(0) in row 0 and CR(n-1)y(n-1) in the last row (the Neumann
 // columns of N).  One thread per line; z is parked in the output line.
-template <int DIR>
-__global__ void __launch_bounds__(128) k_adj_cn(Layout L, LineMap map, const double *__restrict__ lin,
-                                                double *__restrict__ lout, CnTab tab,
-                                                const int32_t *__restrict__ aloft) {
-  const int na = (DIR == 0) ? L.ny : L.nx;
-  const int nb = (DIR == 2) ? L.ny : L.nz;
-  const long nlines = (long)na * nb * L.ns;
-  const long w = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (w >= nlines) return;
-  const int a = (int)(w % na) + 1;
-  const long r0 = w / na;
-  const int b = (int)(r0 % nb) + 1;
-  const int g = (int)(r0 / nb);
-  const int n = (DIR == 0) ? L.nx : (DIR == 1) ? L.ny : L.nz;
+// y and z lines: 32 neighbouring lines of a grain to a warp, rows CB_U at a
+// time with all loads before the first dependent operation (k_cn_solve_b's
+// layout).  ROWS: the table is by row, and divisions by the pivots take three
+// operations; a table by field (geometry that varies along i) has not the
+// values for that, and its rows are divided one by one.  Latency of the loads
+// and of the chain of quotients bound it (121x104x45, 5 grains: y 47 us with
+// div_rn_rcp, 33 now; z 43 -> 21).
+template <int DIR, bool ROWS>
+__global__ void __launch_bounds__(32 * CB_WARPS, 2) k_adj_cn(Layout L, LineMap map, const double *__restrict__ lin,
+                                                             double *__restrict__ lout, CnTab tab,
+                                                             const int32_t *__restrict__ aloft) {
+  int a, b, g;
   long base, st;
-  if (DIR == 0) { base = L.cell(1, a, b); st = 1; }
-  else if (DIR == 1) { base = L.cell(a, 1, b); st = L.P; }
-  else { base = L.cell(a, b, 1); st = L.PY; }
-  base += (long)g * L.PG;
+  if (!cb_line<DIR>(L, &a, &b, &g, &base, &st)) return;
+  const int n = (DIR == 1) ? L.ny : L.nz;
   const double *li = lin + base;
   double *lo = lout + base;
   if (!aloft[g]) {
@@ -2057,31 +2318,181 @@ __global__ void __launch_bounds__(128) k_adj_cn(Layout L, LineMap map, const dou
     return;
   }
   const long u = map.u(a, b);
-  CnRun R;
-  if (DIR == 0) cn_load_run(tab, u, R);
-  auto co = [&](int f, int l) { return (DIR == 0) ? cn_coef(tab, u, R, f, l) : tab.at(f, l, u); };
+  const double2 *const row2 = reinterpret_cast<const double2 *>(tab.p + CN_ROW * u * n);  // FACT,CL CC,CR DU,ZH ZL,ZLL
+  auto two = [&](int r, int c) {  // fields 2c, 2c+1 of row r
+    return ROWS ? __ldg(row2 + 4 * r + c) : make_double2(tab.at(2 * c, r, u), tab.at(2 * c + 1, r, u));
+  };
+  const bool hard = !ROWS || __ldg(tab.runs() + 2 * tab.U + u) != 0.0;
   // U^T z = lam
-  double zp = 0.0;
-  for (int r = 0; r < n; r++) {
-    const double rhs = (r == 0) ? li[0] : li[(long)r * st] - co(CN_DU, r - 1) * zp;
-    zp = rhs / co(CN_DP, r);
-    lo[(long)r * st] = zp;
+  double zp = 0.0, du = 0.0;  // z and DU of the row before
+  for (int r0 = 0; r0 < n; r0 += CB_U) {
+    double x[CB_U], z[CB_U];
+    double2 c[CB_U], d[CB_U];
+#pragma unroll
+    for (int e = 0; e < CB_U; e++) {
+      const int r = r0 + e < n ? r0 + e : n - 1;
+      x[e] = __ldg(li + (long)r * st);
+      c[e] = two(r, 2);
+      d[e] = ROWS ? two(r, 3) : make_double2(0.0, 0.0);
+    }
+    const double zs = zp, dus = du;
+    bool bad = hard;
+#pragma unroll
+    for (int e = 0; e < CB_U; e++) {
+      const double num = (e == 0 && r0 == 0) ? x[e] : x[e] - du * zp;
+      bad = bad || !div_rn_3_takes(num);
+      zp = div_rn_3(num, c[e].y, d[e].x, d[e].y);
+      du = c[e].x;
+      z[e] = zp;
+    }
+    if (bad) {
+      zp = zs;
+      du = dus;
+      for (int e = 0; e < CB_U && r0 + e < n; e++) {
+        const double v = __ldg(li + (long)(r0 + e) * st);
+        zp = ieee_div(r0 + e == 0 ? v : v - du * zp, tab.at(CN_DP, r0 + e, u));
+        du = two(r0 + e, 2).x;
+        lo[(long)(r0 + e) * st] = zp;
+      }
+    } else {
+#pragma unroll
+      for (int e = 0; e < CB_U; e++)
+        if (r0 + e < n) lo[(long)(r0 + e) * st] = z[e];
+    }
   }
-  // L^T y = z, with lam_q(r+1) emitted as soon as y(r) is known
-  double y2 = 0.0;                 // y(r+2)
-  double y1 = lo[(long)(n - 1) * st];  // y(n-1) = z(n-1)
-  for (int r = n - 2; r >= -1; r--) {
-    double y0 = 0.0;
-    if (r >= 0) y0 = lo[(long)r * st] - co(CN_FACT, r + 1) * y1;
-    const int q = r + 1;  // finished row
-    double v = co(CN_CC, q) * y1;
-    if (q > 0) v = v + co(CN_CR, q - 1) * y0;
-    if (q < n - 1) v = v + co(CN_CL, q + 1) * y2;
-    if (q == 0) v = v + co(CN_CL, 0) * y1;
-    if (q == n - 1) v = v + co(CN_CR, n - 1) * y1;
-    lo[(long)q * st] = v;
+  // L^T y = z, with lam_q(q) emitted as soon as y(q-1) is known
+  double y1 = lo[(long)(n - 1) * st], y2 = 0.0;  // y(q), y(q+1)
+  double2 f1 = two(n - 1, 0), g1 = two(n - 1, 1);  // rows q
+  double cl2 = 0.0;                                                            // CL(q+1)
+  {
+    const double2 f0 = two(n - 2, 0), g0 = two(n - 2, 1);
+    const double y0 = lo[(long)(n - 2) * st] - f1.x * y1;
+    double v = g1.x * y1;
+    v = v + g0.y * y0;
+    v = v + g1.y * y1;
+    lo[(long)(n - 1) * st] = v;
+    cl2 = f1.y;
     y2 = y1;
     y1 = y0;
+    f1 = f0;
+    g1 = g0;
+  }
+  auto row = [&](int q, double z, double2 f0, double2 g0) {  // row q from row q-1
+    const double y0 = z - f1.x * y1;
+    double v = g1.x * y1;
+    v = v + g0.y * y0;
+    v = v + cl2 * y2;
+    lo[(long)q * st] = v;
+    cl2 = f1.y;
+    y2 = y1;
+    y1 = y0;
+    f1 = f0;
+    g1 = g0;
+  };
+  int q = n - 2;
+  for (; q >= CB_U; q -= CB_U) {
+    double z[CB_U];
+    double2 f[CB_U], c[CB_U];
+#pragma unroll
+    for (int e = 0; e < CB_U; e++) {
+      z[e] = lo[(long)(q - e - 1) * st];
+      f[e] = two(q - e - 1, 0);
+      c[e] = two(q - e - 1, 1);
+    }
+#pragma unroll
+    for (int e = 0; e < CB_U; e++) row(q - e, z[e], f[e], c[e]);
+  }
+  for (; q >= 1; q--) row(q, lo[(long)(q - 1) * st], two(q - 1, 0), two(q - 1, 1));
+  double v = g1.x * y1;
+  v = v + cl2 * y2;
+  v = v + f1.y * y1;
+  lo[0] = v;
+}
+
+// x lines, through RowTile: upwards for U^T z = lam, then downwards for the
+// rest.  lam_q(q) needs y(q-1), so a chunk's results are its cells shifted by
+// one, and the line's first cell comes last.  121x104x45, 5 grains, x and y
+// together: 190 -> 89 us, a lane per line at the row pitch before.
+__global__ void __launch_bounds__(32 * RT_WARPS, 2) k_adj_cn_x(Layout L, LineMap map, const double *__restrict__ lin,
+                                                               double *__restrict__ lout, CnTab tab,
+                                                               const int32_t *__restrict__ aloft) {
+  __shared__ double sh[RT_WARPS][32 * RT_S];
+  RowTile T;
+  if (!T.init(L, sh[threadIdx.x >> 5], L.nx)) return;  // uniform over the warp
+  const bool act = aloft[T.g] != 0;
+  const int n = L.nx, nch = (n + 31) >> 5;
+  const long u = map.u(T.j, T.k);
+  CnRun R;
+  cn_load_run(tab, u, R);
+  auto co = [&](int f, int l) { return cn_coef(tab, u, R, f, l); };
+  double next[32];
+  double *const own = T.own;
+  T.fetch(next, lin, 0);
+  double zp = 0.0;
+  for (int ch = 0; ch < nch; ch++) {
+    const int c0 = 32 * ch, cnt = n - c0 < 32 ? n - c0 : 32;
+    T.fill(next);
+    if (ch + 1 < nch) T.fetch(next, lin, c0 + 32);
+    for (int e0 = 0; e0 < cnt; e0 += CB_U) {
+      double du[CB_U], dp[CB_U], zh[CB_U];
+#pragma unroll
+      for (int e = 0; e < CB_U; e++) {
+        const int r = c0 + e0 + e < n ? c0 + e0 + e : n - 1;
+        du[e] = co(CN_DU, r > 0 ? r - 1 : 0);
+        dp[e] = co(CN_DP, r);
+        zh[e] = co(CN_ZH, r);
+      }
+#pragma unroll
+      for (int e = 0; e < CB_U; e++) {
+        if (e0 + e >= cnt) break;
+        const double x = own[e0 + e];
+        zp = div_rn_rcp((e == 0 && c0 + e0 == 0) ? x : x - du[e] * zp, dp[e], zh[e]);
+        own[e0 + e] = act ? zp : 0.0;
+      }
+    }
+    if (ch + 1 < nch) T.drain(lout, c0, 0, cnt);
+  }
+  // downwards; the last chunk is still in the tile
+  double y2 = 0.0, y1 = 0.0;
+  __syncwarp();
+  for (int ch = nch - 1; ch >= 0; ch--) {
+    const int c0 = 32 * ch, cnt = n - c0 < 32 ? n - c0 : 32;
+    if (ch != nch - 1) T.fill(next);
+    if (ch > 0) T.fetch(next, lout, c0 - 32);
+    for (int e0 = cnt - 1; e0 >= 0; e0 -= CB_U) {
+      double fa[CB_U], cc[CB_U], cr[CB_U], cl[CB_U];
+#pragma unroll
+      for (int e = 0; e < CB_U; e++) {
+        const int r = c0 + e0 - e > 0 ? c0 + e0 - e : 0;  // y(r) is next, q = r + 1
+        const int q = r + 1 < n ? r + 1 : n - 1;
+        fa[e] = co(CN_FACT, q);
+        cc[e] = co(CN_CC, q);
+        cr[e] = co(CN_CR, r);
+        cl[e] = co(CN_CL, q + 1 < n ? q + 1 : n - 1);
+      }
+#pragma unroll
+      for (int e = 0; e < CB_U; e++) {
+        if (e0 - e < 0) break;
+        const int q = c0 + e0 - e + 1;
+        double y0 = own[e0 - e];
+        if (q < n) {
+          y0 = y0 - fa[e] * y1;
+          double v = cc[e] * y1;
+          v = v + cr[e] * y0;
+          v = v + (q < n - 1 ? cl[e] * y2 : co(CN_CR, n - 1) * y1);
+          own[e0 - e + 1] = act ? v : 0.0;
+        }
+        y2 = y1;
+        y1 = y0;
+      }
+    }
+    T.drain(lout, c0 + 1, 1, c0 + cnt < n ? cnt : cnt - 1);
+  }
+  if (T.lane < T.nr) {
+    double v = co(CN_CC, 0) * y1;
+    v = v + co(CN_CL, 1) * y2;
+    v = v + co(CN_CL, 0) * y1;
+    lout[(long)(T.r0 + T.lane) * L.P] = act ? v : 0.0;
   }
 }
 
@@ -2129,9 +2540,18 @@ static int launch_adj_cn_dir(a3g_ctx *ctx, const double *lin, double *lout) {
   tbegin(ctx, A3G_K_ADJOINT);
   int rc = cn_table<DIR>(ctx, map, sig, kk, &tab);
   if (rc) return rc;
-  const long nlines = (long)map.na * map.nb * L.ns;
-  k_adj_cn<DIR><<<(unsigned)((nlines + 127) / 128), 128, 0, ctx->stream>>>(L, map, lin, lout, tab,
-                                                                           ctx->aloft);
+  if (DIR == 0) {
+    int threads;
+    const dim3 grid = rt_grid(L, &threads);
+    k_adj_cn_x<<<grid, threads, 0, ctx->stream>>>(L, map, lin, lout, tab, ctx->aloft);
+  } else {
+    int threads;
+    const dim3 grid = cb_grid<DIR == 0 ? 1 : DIR>(L, &threads);
+    if (tab.byrow)
+      k_adj_cn<DIR == 0 ? 1 : DIR, true><<<grid, threads, 0, ctx->stream>>>(L, map, lin, lout, tab, ctx->aloft);
+    else
+      k_adj_cn<DIR == 0 ? 1 : DIR, false><<<grid, threads, 0, ctx->stream>>>(L, map, lin, lout, tab, ctx->aloft);
+  }
   tend(ctx);
   A3G_LAUNCH_CHECK(ctx);
   return A3G_OK;
