@@ -339,20 +339,31 @@ __device__ __forceinline__ bool same_bits(double a, double b) {
 // for, and while that is the step's dt (and the host allows it, `may`: same
 // box, geometry and diffusivity) the blocks return at once.  st_new is the
 // slot the next launch reads, so that no block can see this launch's write.
+struct CnTableJob {  // the table of one direction
+  LineMap map;
+  Geo3 sig, kk;
+  const double *st_old;
+  double *st_new, *tab;
+  int may, byrow, lpb, blocks;  // blocks == 0: up to date, or no line to solve
+};
+
 template <int DIR, int LPB>
-__global__ void __launch_bounds__(256) k_cn_table(Layout L, Box box, double imp, LineMap map, Geo3 sig, Geo3 kap,
-                                                  Geo3 kk, DevScalars *sc, const double *__restrict__ st_old,
-                                                  double *__restrict__ st_new, int may, int byrow,
-                                                  double *__restrict__ tab) {
+__device__ __forceinline__ void cn_table_block(const Layout &L, const Box &box, double imp, const Geo3 &kap,
+                                               const CnTableJob &J, DevScalars *sc, int block, double *smem) {
   constexpr bool COMPRESS = (DIR == 0);
   constexpr int TR = LPB == 1 ? 256 : 32;  // rows per tile
-  __shared__ double sD[TR * LPB], sDL[TR * LPB], sDU[TR * LPB], sF[TR * LPB], sP[TR * LPB];
+  double *const sD = smem, *const sDL = sD + TR * LPB, *const sDU = sDL + TR * LPB, *const sF = sDU + TR * LPB,
+                *const sP = sF + TR * LPB;
   __shared__ double cF[LPB], cP[LPB];      // fact and D' of the row before the tile
   __shared__ int sRun[LPB], sBad[LPB], sBrk;
+  const LineMap &map = J.map;
+  const Geo3 &sig = J.sig, &kk = J.kk;
+  const int byrow = J.byrow;
+  double *const __restrict__ tab = J.tab;
   const double dt = sc->dt;
-  if (blockIdx.x == 0 && threadIdx.x == 0) *st_new = dt;
-  if (may && *st_old == dt) return;
-  const int u0 = blockIdx.x * LPB;
+  if (block == 0 && threadIdx.x == 0) *J.st_new = dt;
+  if (J.may && *J.st_old == dt) return;
+  const int u0 = block * LPB;
   const int tid = threadIdx.x;
   // representative fixed indices of a distinct line
   const int amin = (DIR == 0) ? box.jmin : box.imin;
@@ -496,6 +507,24 @@ __global__ void __launch_bounds__(256) k_cn_table(Layout L, Box box, double imp,
     runs[u] = (double)min(sRun[tid], n - 2);
     runs[U + u] = (double)(n - 2);
     runs[2 * U + u] = (double)sBad[tid];
+  }
+}
+
+// The blocks of x, then y, then z.
+__global__ void __launch_bounds__(256) k_cn_tables(Layout L, Box box, double imp, Geo3 kap, CnTableJob jx,
+                                                   CnTableJob jy, CnTableJob jz, DevScalars *sc) {
+  extern __shared__ __align__(16) double ct_smem[];
+  int b = blockIdx.x;
+  if (b < jx.blocks) {
+    if (jx.lpb == 1) cn_table_block<0, 1>(L, box, imp, kap, jx, sc, b, ct_smem);
+    else cn_table_block<0, 32>(L, box, imp, kap, jx, sc, b, ct_smem);
+  } else if ((b -= jx.blocks) < jy.blocks) {
+    if (jy.lpb == 1) cn_table_block<1, 1>(L, box, imp, kap, jy, sc, b, ct_smem);
+    else cn_table_block<1, 32>(L, box, imp, kap, jy, sc, b, ct_smem);
+  } else {
+    b -= jy.blocks;
+    if (jz.lpb == 1) cn_table_block<2, 1>(L, box, imp, kap, jz, sc, b, ct_smem);
+    else cn_table_block<2, 32>(L, box, imp, kap, jz, sc, b, ct_smem);
   }
 }
 // Solve of one line (a, b) of grain g from the table.  The eliminated
@@ -2149,30 +2178,58 @@ static inline bool same_box(const Box &a, const Box &b) {
          a.kmax == b.kmax;
 }
 
-// The factor table of direction DIR for the step's dt: built by k_cn_table,
-// or kept from the previous build when nothing it depends on has changed.
-// No launch at all while the host knows that dt has not been set since.
+static inline int box_cells(const Box &b, int dir) {
+  return dir == 0 ? b.imax - b.imin + 1 : dir == 1 ? b.jmax - b.jmin + 1 : b.kmax - b.kmin + 1;
+}
+
+// What direction DIR needs of the next k_cn_tables; no blocks where the host
+// knows that nothing has changed since the last build.
 template <int DIR>
-static int cn_table(a3g_ctx *ctx, const LineMap &map, const Geo3 &sig, const Geo3 &kk, CnTab *out) {
-  const Box &box = ctx->box;
-  const int n = (DIR == 0) ? box.imax - box.imin + 1 : (DIR == 1) ? box.jmax - box.jmin + 1 : box.kmax - box.kmin + 1;
-  const bool may = ctx->cn_valid[DIR] && same_box(ctx->cn_box[DIR], box);
-  *out = CnTab{ctx->cn_tab[DIR], (long)n * map.U, map.U, n, cn_byrow(DIR, map)};
-  if (may && ctx->cn_stamp[DIR] == ctx->dt_stamp) return A3G_OK;
+static CnTableJob cn_table_job(a3g_ctx *ctx) {
+  CnTableJob j{};
+  const bool may = ctx->cn_valid[DIR] && same_box(ctx->cn_box[DIR], ctx->box);
+  if (!ctx->cn_tab[DIR] || box_cells(ctx->box, DIR) <= 1 || (may && ctx->cn_stamp[DIR] == ctx->dt_stamp)) return j;
   double *const st = ctx->cn_state + 2 * DIR;
-  const int slot = ctx->cn_slot[DIR];
-#define A3G_TABLE(LPB_)                                                                                       \
-  k_cn_table<DIR, LPB_><<<(map.U + LPB_ - 1) / LPB_, 256, 0, ctx->stream>>>(                                   \
-      ctx->L, box, ctx->prm.imp_fac, map, sig, ctx->kappa, kk, ctx->sc, st + slot, st + (slot ^ 1), may ? 1 : 0, \
-      out->byrow ? 1 : 0, ctx->cn_tab[DIR])
+  j.map = line_map<DIR>(ctx);
+  j.sig = (DIR == 0) ? ctx->snx : (DIR == 1) ? ctx->sny : ctx->snz;
+  j.kk = (DIR == 0) ? ctx->kx : (DIR == 1) ? ctx->ky : ctx->kz;
+  j.st_old = st + ctx->cn_slot[DIR];
+  j.st_new = st + (ctx->cn_slot[DIR] ^ 1);
+  j.tab = ctx->cn_tab[DIR];
+  j.may = may ? 1 : 0;
+  j.byrow = cn_byrow(DIR, j.map) ? 1 : 0;
   // many lines: 32 share a block's serial warp; few: a block each, more of its rows at once
-  if (map.U >= 1024) A3G_TABLE(32); else A3G_TABLE(1);
-#undef A3G_TABLE
+  j.lpb = j.map.U >= 1024 ? 32 : 1;
+  j.blocks = (j.map.U + j.lpb - 1) / j.lpb;
+  return j;
+}
+
+// The factor table of direction DIR for the step's dt: built by k_cn_tables,
+// or kept from the previous build when nothing it depends on has changed.
+// No launch at all while the host knows that dt has not been set since.  A
+// build takes the other directions' stale tables along: each is one serial
+// chain per line, and the three run side by side (a step's tables on
+// 93x131x37: 38 us in three launches, 26 in one; 317x211x53: 35, 26;
+// 201x151x41 over terrain: 176, 96).
+template <int DIR>
+static int cn_table(a3g_ctx *ctx, const LineMap &map, CnTab *out) {
+  const Box &box = ctx->box;
+  const int n = box_cells(box, DIR);
+  *out = CnTab{ctx->cn_tab[DIR], (long)n * map.U, map.U, n, cn_byrow(DIR, map)};
+  if (ctx->cn_valid[DIR] && same_box(ctx->cn_box[DIR], box) && ctx->cn_stamp[DIR] == ctx->dt_stamp) return A3G_OK;
+  const CnTableJob jx = cn_table_job<0>(ctx), jy = cn_table_job<1>(ctx), jz = cn_table_job<2>(ctx);
+  const bool wide = jx.lpb > 1 || jy.lpb > 1 || jz.lpb > 1;
+  k_cn_tables<<<jx.blocks + jy.blocks + jz.blocks, 256, 5 * (wide ? 1024 : 256) * sizeof(double), ctx->stream>>>(
+      ctx->L, box, ctx->prm.imp_fac, ctx->kappa, jx, jy, jz, ctx->sc);
   A3G_LAUNCH_CHECK(ctx);
-  ctx->cn_slot[DIR] ^= 1;
-  ctx->cn_stamp[DIR] = ctx->dt_stamp;
-  ctx->cn_valid[DIR] = true;
-  ctx->cn_box[DIR] = box;
+  const int built[3] = {jx.blocks, jy.blocks, jz.blocks};
+  for (int d = 0; d < 3; d++)
+    if (built[d]) {
+      ctx->cn_slot[d] ^= 1;
+      ctx->cn_stamp[d] = ctx->dt_stamp;
+      ctx->cn_valid[d] = true;
+      ctx->cn_box[d] = box;
+    }
   return A3G_OK;
 }
 
@@ -2187,12 +2244,10 @@ static int launch_cn_dir(a3g_ctx *ctx) {
     ctx->ts1_zeroed = true;
     return A3G_OK;
   }
-  const Geo3 &sig = (DIR == 0) ? ctx->snx : (DIR == 1) ? ctx->sny : ctx->snz;
-  const Geo3 &kk = (DIR == 0) ? ctx->kx : (DIR == 1) ? ctx->ky : ctx->kz;
   const LineMap map = line_map<DIR>(ctx);
   CnTab tab;
   tbegin(ctx, A3G_K_CN_TABLE);
-  int rc = cn_table<DIR>(ctx, map, sig, kk, &tab);
+  int rc = cn_table<DIR>(ctx, map, &tab);
   tend(ctx);
   if (rc) return rc;
   const long nlines = (long)map.na * map.nb * L.ns;
@@ -2533,12 +2588,10 @@ static int launch_adj_cn_dir(a3g_ctx *ctx, const double *lin, double *lout) {
                              ctx->stream));
     return A3G_OK;
   }
-  const Geo3 &sig = (DIR == 0) ? ctx->snx : (DIR == 1) ? ctx->sny : ctx->snz;
-  const Geo3 &kk = (DIR == 0) ? ctx->kx : (DIR == 1) ? ctx->ky : ctx->kz;
   const LineMap map = line_map<DIR>(ctx);
   CnTab tab;
   tbegin(ctx, A3G_K_ADJOINT);
-  int rc = cn_table<DIR>(ctx, map, sig, kk, &tab);
+  int rc = cn_table<DIR>(ctx, map, &tab);
   if (rc) return rc;
   if (DIR == 0) {
     int threads;
