@@ -132,6 +132,7 @@ struct LineGeo {        // a ghosted geometry line: value at sweep index c is p[
   const double *p;
   long s;
   __device__ __forceinline__ double at(int c) const { return p[(long)(c + 1) * s]; }
+  __device__ __forceinline__ double ldg(int c) const { return __ldg(p + (long)(c + 1) * s); }
 };
 
 template <int DIR>
@@ -1356,8 +1357,11 @@ static_assert((ACT_WARP_D * 8) % 128 == 0, "warp regions stay 128-byte aligned")
 struct TrueT { static constexpr bool value = true; };
 struct FalseT { static constexpr bool value = false; };
 
-template <int DIR, int LIM>
-__global__ void __launch_bounds__(32 * ACT_WARPS, ACT_MINB) k_advect_colt(
+// VAR: geometry that varies along i (terrain); each lane loads its own
+// sigma and dt/kappa, ACT_U cells at a time, in place of the staged pairs
+// (z on 201x151x41, 5 grains: 90 us in the block kernel, 54 here).
+template <int DIR, int LIM, bool VAR>
+__global__ void __launch_bounds__(32 * ACT_WARPS, VAR ? ACT_MINB - 2 : ACT_MINB) k_advect_colt(
     const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tv, Layout L, Box box, Box cov,
     int nocycle, double eps, int nseg, int seg, const double *__restrict__ cin, double *__restrict__ cout,
     const double *__restrict__ vel, const double *__restrict__ vghost, Geo4 vf, Geo3 sig, Geo3 dtvt,
@@ -1423,6 +1427,7 @@ __global__ void __launch_bounds__(32 * ACT_WARPS, ACT_MINB) k_advect_colt(
         tma_load_4d(qb + ACH * 32, &tv, b, it << 5, o - 1, C0 - 1, 0);
       }
     }
+    if (VAR) return;
     const LineGeo gsig = line_of<DIR>(sig, 1, o), gdtv = line_of<DIR>(dtvt, 1, o);  // constant along i
     double2 *gb = reinterpret_cast<double2 *>(wsm + 4 * ACH * 32 + (k & 1) * 2 * ACH);
     const int I = C0 + lane;
@@ -1444,7 +1449,7 @@ __global__ void __launch_bounds__(32 * ACT_WARPS, ACT_MINB) k_advect_colt(
     const long base = (DIR == 1) ? L.cell(ac, 1, o) : L.cell(ac, o, 1);
     const double *pq = cin + (long)g * L.PG + base;
     const double *pv = vel + base, *pvg = vghost + base;
-    const LineGeo gsig = line_of<DIR>(sig, 1, o), gdtv = line_of<DIR>(dtvt, 1, o);
+    const LineGeo gsig = line_of<DIR>(sig, VAR ? ac : 1, o), gdtv = line_of<DIR>(dtvt, VAR ? ac : 1, o);
     auto qload = [&](int c) -> double {
       return (c >= rmin - 2 && c <= rmax + 2 && c >= 1 && c <= n) ? pq[(c - 1) * st] : 0.0;
     };
@@ -1486,9 +1491,13 @@ __global__ void __launch_bounds__(32 * ACT_WARPS, ACT_MINB) k_advect_colt(
   const bool nocyc = nocycle != 0;
   const int eps_hi = nocyc ? 0 : __double2hiint(eps);  // |d| < eps for certain, by its high word alone
   po += (long)(c0 - 1) * st;                           // cell c's place from here on
+  const LineGeo lsig = line_of<DIR>(sig, ac, o), ldtv = line_of<DIR>(dtvt, ac, o);
+  // sigma(I)/2 and dt/kappa(I-1), I = c+2 the cell at slot e of the chunk
+  auto geo = [&](const double2 *gb, int e, int I) {
+    return VAR ? make_double2(I <= rmax + 1 ? 0.5 * lsig.ldg(I) : 0.0, ldtv.ldg(I - 1)) : gb[e];
+  };
   // the step c from the values of cell c+2 at slot e of the chunk
-  auto step = [&](auto quiet, const double *qv, const double2 *gb, int e) {
-    const double2 sd = gb[e];
+  auto step = [&](auto quiet, const double *qv, double2 sd, int e) {
     const double q0 = m.q0, q2 = qv[e * 32];
     const double vn = (DIR == 2) ? qv[(ACH + e) * 32] + vf0 : qv[(ACH + e) * 32];
     const double sum = march_step<LIM, decltype(quiet)::value>(m, q2, q2 - m.q1, vn, sd.x, sd.y, eps, nocyc);
@@ -1527,18 +1536,24 @@ __global__ void __launch_bounds__(32 * ACT_WARPS, ACT_MINB) k_advect_colt(
       }
       if (LIM == A3G_LIM_NONE || __all_sync(0xffffffffu, top < eps_hi || !al)) {
         for (; e + 2 <= cnt; e += 2) {
-          step(TrueT{}, qv, gb, e);
-          step(TrueT{}, qv, gb, e + 1);
+          const double2 sd0 = geo(gb, e, c + e + 2), sd1 = geo(gb, e + 1, c + e + 3);
+          step(TrueT{}, qv, sd0, e);
+          step(TrueT{}, qv, sd1, e + 1);
         }
       } else {
         for (; e + ACT_U <= cnt; e += ACT_U) {
+          double2 sd[ACT_U];
+          if (VAR) {
 #pragma unroll
-          for (int u = 0; u < ACT_U; u++) step(FalseT{}, qv, gb, e + u);
+            for (int u = 0; u < ACT_U; u++) sd[u] = geo(gb, e + u, c + e + u + 2);
+          }
+#pragma unroll
+          for (int u = 0; u < ACT_U; u++) step(FalseT{}, qv, VAR ? sd[u] : gb[e + u], e + u);
         }
       }
     }
     for (; e < cnt; e++) {
-      const double upd = step(FalseT{}, qv, gb, e);
+      const double upd = step(FalseT{}, qv, geo(gb, e, c + e + 2), e);
       if (DIR == 2 && al && out_hi && c + e == ctop) out2[oo] -= upd;
     }
     c += cnt;
@@ -1575,7 +1590,7 @@ template <int DIR, int LIM>
 static bool launch_colt(a3g_ctx *ctx) {
   const Layout &L = ctx->L;
   const Geo3 &sg = (DIR == 1) ? ctx->sny : ctx->snz;
-  if (sg.si != 0 || ctx->dtv.si != 0) return false;  // geometry must not vary along i
+  const bool var = sg.si != 0 || ctx->dtv.si != 0;
   if (DIR == 2 && (ctx->vf.si != 0 || ctx->vf.sj != 0 || ctx->vf.sk != 0)) return false;
   CUtensorMap tq, tv;
   const double *vel = dir_vel(ctx, DIR);
@@ -1591,10 +1606,14 @@ static bool launch_colt(a3g_ctx *ctx) {
   const int nseg = march_segments(n, nlw);
   const int seg = (n + nseg - 1) / nseg;
   const long nw = nlw * ((n + seg - 1) / seg);
-  k_advect_colt<DIR, LIM><<<(unsigned)((nw + ACT_WARPS - 1) / ACT_WARPS), 32 * ACT_WARPS, smem, ctx->stream>>>(
-      tq, tv, L, ctx->box, cov, ctx->prm.nocycle, ctx->prm.eps_thresh, (n + seg - 1) / seg, seg, ctx->c0, ctx->c1, vel,
-      dir_vghost(ctx, DIR), ctx->vf, sg, ctx->dtv, ctx->aloft, ctx->sc, (DIR == 1) ? ctx->out_xz1 : ctx->out_xy1,
-      (DIR == 1) ? ctx->out_xz2 : ctx->out_xy2);
+  auto run = [&](auto kernel) {
+    kernel<<<(unsigned)((nw + ACT_WARPS - 1) / ACT_WARPS), 32 * ACT_WARPS, smem, ctx->stream>>>(
+        tq, tv, L, ctx->box, cov, ctx->prm.nocycle, ctx->prm.eps_thresh, (n + seg - 1) / seg, seg, ctx->c0, ctx->c1, vel,
+        dir_vghost(ctx, DIR), ctx->vf, sg, ctx->dtv, ctx->aloft, ctx->sc, (DIR == 1) ? ctx->out_xz1 : ctx->out_xy1,
+        (DIR == 1) ? ctx->out_xz2 : ctx->out_xy2);
+  };
+  if (var) run(k_advect_colt<DIR, LIM, true>);
+  else run(k_advect_colt<DIR, LIM, false>);
   return true;
 }
 
@@ -1851,14 +1870,23 @@ static bool launch_advect_xm(a3g_ctx *ctx) {
 // ---------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------
+// warps of k_advect_march in segments of 96 cells
+template <int DIR>
+static inline long march_warps(const Layout &L, int gc) {
+  const long lines = (long)((((DIR == 0) ? L.ny : L.nx) + 31) / 32) * ((DIR == 2) ? L.ny : L.nz);
+  return lines * ((L.ns + gc - 1) / gc) * ((((DIR == 0) ? L.nx : (DIR == 1) ? L.ny : L.nz) + 95) / 96);
+}
+
 template <int DIR, int LIM, int GC, bool PER, bool TOPO = false>
 static void launch_march_gc(a3g_ctx *ctx) {
   const Layout &L = ctx->L;
   const int n = (DIR == 0) ? L.nx : (DIR == 1) ? L.ny : L.nz;
   const int na = (DIR == 0) ? L.ny : L.nx;
   const int nother = (DIR == 2) ? L.ny : L.nz;
-  // segments of about 96 cells (whole lines when they are short)
-  const int nseg = (n + 95) / 96;
+  // segments of about 96 cells (whole lines when they are short), over terrain
+  // of 48 where that gives an SM less than 32 warps
+  const int len = TOPO && march_warps<DIR>(L, GC) < 148 * 32 ? 48 : 96;
+  const int nseg = (n + len - 1) / len;
   const int seg = (n + nseg - 1) / nseg;
   const int ngroups = (L.ns + GC - 1) / GC;
   dim3 grid(((na + 31) / 32) * ngroups, (nother + 3) / 4, (n + seg - 1) / seg);
@@ -1897,18 +1925,21 @@ static void launch_dir_lim(a3g_ctx *ctx) {
   const bool per = (DIR == 0) && ctx->grid.periodic;
   const int variant = ctx->tune_advect[DIR];
   if constexpr (DIR != 2) {
-    // ZScaling_ID 2: the DelD*onD_cc terms live in the marching kernel only
+    // ZScaling_ID 2: the DelD*onD_cc terms live in the marching kernel only.
+    // A grain a thread, or two that share the row's winds: two in x where they
+    // fill the chip (402x301x50, 10 grains: 913 us a sweep, one 934; y 825,
+    // 746).  With the segments of 48 cells, 201x151x41 and 5 grains: x 144 ->
+    // 130 us, y 142 -> 102; 150x120x30 and 2 grains: x 70 -> 33, y 60 -> 32.
     if (ctx->topo_on && ctx->prm.zscaling_id == 2) {
-      const bool g2 = ctx->L.ns >= 2;
       if constexpr (DIR == 0) {
-        if (per) {
-          if (g2) launch_march_gc<DIR, LIM, 2, true, true>(ctx);
-          else launch_march_gc<DIR, LIM, 1, true, true>(ctx);
-          return;
-        }
+        const bool g2 = ctx->L.ns >= 2 && march_warps<DIR>(ctx->L, 2) >= 148 * 32;
+        if (per && g2) launch_march_gc<DIR, LIM, 2, true, true>(ctx);
+        else if (per) launch_march_gc<DIR, LIM, 1, true, true>(ctx);
+        else if (g2) launch_march_gc<DIR, LIM, 2, false, true>(ctx);
+        else launch_march_gc<DIR, LIM, 1, false, true>(ctx);
+      } else {
+        launch_march_gc<DIR, LIM, 1, false, true>(ctx);
       }
-      if (g2) launch_march_gc<DIR, LIM, 2, false, true>(ctx);
-      else launch_march_gc<DIR, LIM, 1, false, true>(ctx);
       return;
     }
   }
