@@ -107,7 +107,7 @@ __device__ bool last_block(unsigned *counter, unsigned nblocks) {
 // products and quotients are formed once, from the row's largest winds --
 // rounding is monotone, so the maximum is the same.  Bound by the winds' 24 B a
 // cell; with per-warp atomics on three words, a memset before and the dt in a
-// kernel of its own this took 26 us on 93x131x37 where the loads take under 2.
+// kernel of its own it took 26 us on 93x131x37 (2 of them the dt kernel), now 14.
 __global__ void __launch_bounds__(256) k_cfl(Layout L, int latlon, const double *__restrict__ vx,
                                              const double *__restrict__ vy,
                                              const double *__restrict__ vz, Geo4 vf, Geo3 snx,
@@ -449,9 +449,9 @@ constexpr int NJOBS = 7;
 // it does not vary along i -- and carried in double-double: a relative error of
 // three roundings per term, far inside the 1e-13 the totals keep.
 // Bound by the read of the level where that is large: 720x360x60, 10 grains,
-// 349 -> 205 us; and by latency where it is small, in which every face took 296
+// 339 -> 215 us; and by latency where it is small, in which every face took 296
 // blocks and the combination a kernel and a copy of their own: 93x131x37, 2
-// grains, 32 -> 9 us.
+// grains, 28 us and the copy -> 17 us.
 __global__ void __launch_bounds__(256) k_totals(Layout L, const double *__restrict__ c,
                                                 Geo3 kap, const double *__restrict__ yz1,
                                                 const double *__restrict__ yz2,
@@ -588,7 +588,9 @@ void totals_volumes(a3g_ctx *ctx, const double *h_src, double *out4, double *mas
 // set when some grain has c >= thresh in that plane.
 // ---------------------------------------------------------------------------
 // A warp takes a row of the box outside which the level is zero, the grains'
-// loads of four cells a lane in flight.  480x401x50, 6 grains: 95 -> 20 us.
+// loads of four cells a lane in flight.  480x401x50, 6 grains: over the box of a
+// cloud in a seventh of the grid 36 us, over the whole grid 106; a thread a cell
+// over the whole grid took 125.
 __global__ void __launch_bounds__(256) k_plane_flags(Layout L, Box nz, const double *__restrict__ c,
                                                      double thresh, int32_t *__restrict__ flags) {
   constexpr int U = 4;
@@ -600,14 +602,17 @@ __global__ void __launch_bounds__(256) k_plane_flags(Layout L, Box nz, const dou
     bool any = false;
     for (int i0 = nz.imin + lane; i0 <= nz.imax; i0 += 32 * U) {
       bool hit[U] = {false, false, false, false};
-#pragma unroll 2
-      for (int g = 0; g < L.ns; g++)
+#pragma unroll 4
+      for (int g = 0; g < L.ns; g++) {
+        double v[U];
 #pragma unroll
-        for (int q = 0; q < U; q++)
-          if (i0 + 32 * q <= nz.imax) hit[q] = hit[q] || row[(long)g * L.PG + i0 + 32 * q - 1] >= thresh;
+        for (int q = 0; q < U; q++) v[q] = __ldg(row + (long)g * L.PG + min(i0 + 32 * q, nz.imax) - 1);
+#pragma unroll
+        for (int q = 0; q < U; q++) hit[q] |= v[q] >= thresh;
+      }
 #pragma unroll
       for (int q = 0; q < U; q++)
-        if (hit[q]) {
+        if (hit[q] && i0 + 32 * q <= nz.imax) {
           any = true;
           if (!flags[i0 + 32 * q]) flags[i0 + 32 * q] = 1;
         }
@@ -642,7 +647,7 @@ int launch_plane_flags(a3g_ctx *ctx) {
 // winds and source
 // ---------------------------------------------------------------------------
 // A warp takes whole rows (no division per cell), four cells a lane in flight;
-// bound by the 48 B a cell (140x120x40: 13 -> 7 us).
+// bound by the 48 B a cell (720x360x60: 130 -> 124 us; 93x131x37: 6.7 -> 6.3).
 __global__ void __launch_bounds__(256) k_interp_winds(Layout L, const float *__restrict__ last,
                                                       const float *__restrict__ next, long n, double frac,
                                                       double *__restrict__ vx, double *__restrict__ vy,
@@ -1019,7 +1024,7 @@ int launch_vent_column(a3g_ctx *ctx, int ivent, int jvent, const double *lam, do
 // One pass up the column (the lowest level at or below CLOUDCON_THRESH is the
 // last one the reference's downward loop meets), the grains' loads of a level
 // in flight together; bound by the 8 B a cell and grain (480x361x50, 8 grains:
-// 265 -> 110 us against two passes).  cls: the cell's area classes, j fastest:
+// 208 -> 121 us against two passes).  cls: the cell's area classes, j fastest:
 // bit 0 deposit, 1 cloud, 2.. CloudLoadArea's five thresholds.
 __global__ void __launch_bounds__(128) k_output_vars(
     Layout L, Box box, const double *__restrict__ c, const double *__restrict__ dz_vec,
@@ -1131,8 +1136,8 @@ int launch_output_vars(a3g_ctx *ctx, double time, double *load, double *maxh, do
 // ashcon(i,j,k,g) = real(concen_pd(i,j,k,g,ts1), kind=op) (:3296-3298), and
 // NC_RestartFile_LoadConcen (:3701-3707): concen_pd(i,j,k,g) = real(ashcon, ip).
 // A warp takes whole rows (the level's pitch P, the array's nx), eight cells a
-// lane in flight; bound by the 12 B a cell.  720x360x60, 10 grains: 620 -> 330
-// us each way against a block per 256 cells.
+// lane in flight; bound by the 12 B a cell.  720x360x60, 10 grains: 601 -> 292
+// us out and 590 -> 331 us in against a block per 256 cells.
 constexpr int NC_U = 8;
 __global__ void __launch_bounds__(256) k_pack_ashcon(Layout L, const double *__restrict__ c,
                                                      float *__restrict__ ashcon) {
