@@ -1339,8 +1339,8 @@ __device__ __forceinline__ double march_step(March &m, double q2, double d2, dou
 // rows through L2.  Taken when the geometry is constant along i and the fall
 // speed is one value per grain.
 //
-// Bound by instruction issue (67 % of cycles on the C2 slab) and the FP64 pipe
-// (45 %).  march_step() forms an interface in about 100 instructions where
+// Bound by instruction issue (68 % of cycles on the C2 slab) and the FP64 pipe
+// (48 %).  march_step() forms an interface in about 100 instructions where
 // block_body's expressions and the checked steps at the line ends took 190,
 // and a chunk whose differences are all within EPS_THRESH on every lane -- the
 // air around a cloud -- takes steps without the limiter: 720x360x60, 10
@@ -1632,8 +1632,8 @@ static bool launch_colt(a3g_ctx *ctx) {
 // rows are not all this plane's (the last of a grain) is stored by the lanes.
 // Taken when sigma and dt/kappa do not vary along the row.
 //
-// Bound, like the column march, by issue (58 % of cycles on the C2 slab, 16
-// warps per SM by registers) and the FP64 pipe (40 %).  720x360x60, 10 grains:
+// Bound, like the column march, by issue (63 % of cycles on the C2 slab, 16
+// warps per SM by registers) and the FP64 pipe (45 %).  720x360x60, 10 grains:
 // 1.08 -> 0.67 ms a sweep against the warp-row kernel, whose lanes pass each
 // value on through shared-memory rings (188 instructions a cell against 95).
 // ---------------------------------------------------------------------------
