@@ -451,7 +451,7 @@ constexpr int NJOBS = 7;
 // Bound by the read of the level where that is large: 720x360x60, 10 grains,
 // 339 -> 215 us; and by latency where it is small, in which every face took 296
 // blocks and the combination a kernel and a copy of their own: 93x131x37, 2
-// grains, 28 us and the copy -> 17 us.
+// grains, 28 us and the copy -> 10.5 us.
 __global__ void __launch_bounds__(256) k_totals(Layout L, const double *__restrict__ c,
                                                 Geo3 kap, const double *__restrict__ yz1,
                                                 const double *__restrict__ yz2,
@@ -497,19 +497,15 @@ __global__ void __launch_bounds__(256) k_totals(Layout L, const double *__restri
     }
   } else {
     const int f = ((int)blockIdx.x - nb) / fb, b = ((int)blockIdx.x - nb) % fb, job = f + 1;
-    const long n = (job == 1 || job == 6) ? (long)L.nx * L.ny : (job <= 3) ? (long)L.ny * L.nz : (long)L.nx * L.nz;
-    for (long t = b * 256L + threadIdx.x; t < n; t += fb * 256L) {
-      double v;
-      if (job == 1 || job == 6) {
-        const int i = (int)(t % L.nx) + 1, j = (int)(t / L.nx) + 1;
-        v = (job == 1 ? xy1 : xy2)[g * n + t] * kap.at(i, j, job == 1 ? 0 : L.nz + 1);
-      } else if (job <= 3) {
-        const int j = (int)(t % L.ny) + 1, k = (int)(t / L.ny) + 1;
-        v = (job == 2 ? yz1 : yz2)[g * n + t] * kap.at(job == 2 ? 0 : L.nx + 1, j, k);
-      } else {
-        const int i = (int)(t % L.nx) + 1, k = (int)(t / L.nx) + 1;
-        v = (job == 4 ? xz1 : xz2)[g * n + t] * kap.at(i, job == 4 ? 0 : L.ny + 1, k);
-      }
+    const bool xy = job == 1 || job == 6, yz = job == 2 || job == 3;
+    const unsigned len = yz ? L.ny : L.nx, n = len * (xy ? L.ny : L.nz);
+    const double *face = (job == 1 ? xy1 : job == 2 ? yz1 : job == 3 ? yz2 : job == 4 ? xz1 : job == 5 ? xz2 : xy2) +
+                         (long)g * n;
+    for (unsigned t = b * 256u + threadIdx.x; t < n; t += fb * 256u) {
+      const int row = (int)(t / len) + 1, at = (int)(t - (row - 1) * len) + 1;
+      const double v = face[t] * (xy ? kap.at(at, row, job == 1 ? 0 : L.nz + 1)
+                                  : yz ? kap.at(job == 2 ? 0 : L.nx + 1, at, row)
+                                       : kap.at(at, job == 4 ? 0 : L.ny + 1, row));
       acc = dd_add(acc, v);
     }
   }
@@ -546,13 +542,14 @@ int launch_totals_partials(a3g_ctx *ctx, double *h_dst) {
   Box nz = state_box(ctx);
   if (empty(nz)) nz = Box{1, 1, 1, 1, 1, 1};
   const int rows = (nz.jmax - nz.jmin + 1) * (nz.kmax - nz.kmin + 1);
-  // four rows a warp at least, eight blocks per SM at most; 4096 face cells a block, 16 blocks at most
+  // four rows a warp at least, eight blocks per SM at most; 1024 face cells a block (4096 made the faces
+  // the last to finish on 93x131x37: 17 us a launch, 10.5 now), 16 blocks at most
   int nb = (rows + 31) / 32;
   const int most = 148 * 8 / L.ns > 1 ? 148 * 8 / L.ns : 1;
   if (nb > most) nb = most;
   const long face = (long)L.nx * (L.ny > L.nz ? L.ny : L.nz) > (long)L.ny * L.nz
                         ? (long)L.nx * (L.ny > L.nz ? L.ny : L.nz) : (long)L.ny * L.nz;
-  const int fb = face > 15 * 4096 ? 16 : (int)(face / 4096) + 1;
+  const int fb = face > 15 * 1024 ? 16 : (int)(face / 1024) + 1;
   tbegin(ctx, A3G_K_TOTALS);
   k_totals<<<dim3(nb + 6 * fb, L.ns), 256, 0, ctx->stream>>>(
       L, ctx->c0, ctx->kappa, ctx->out_yz1, ctx->out_yz2, ctx->out_xz1, ctx->out_xz2, ctx->out_xy1, ctx->out_xy2, nz, nb,
