@@ -1226,25 +1226,21 @@ static void launch_col(a3g_ctx *ctx) {
 // ---------------------------------------------------------------------------
 // The marching step that the TMA-fed sweeps share.
 // ---------------------------------------------------------------------------
-// max(0, x) and min(0, x) by the sign bit: two logic operations per half
-// instead of a compare and two selects.  A NaN stays a NaN in one of them.
-__device__ __forceinline__ double pos_part(double x) {
-  const int h = __double2hiint(x), m = ~(h >> 31);
-  return __hiloint2double(h & m, __double2loint(x) & m);
-}
-__device__ __forceinline__ double neg_part(double x) {
-  const int h = __double2hiint(x), m = h >> 31;
-  return __hiloint2double(h & m, __double2loint(x) & m);
-}
+// max(0, x) and min(0, x); both 0 for a NaN, as dmx and dmn give them, so that
+// a missing wind carries no first-order flux whichever kernel sweeps its cell.
+__device__ __forceinline__ double pos_part(double x) { return x > 0.0 ? x : 0.0; }
+__device__ __forceinline__ double neg_part(double x) { return x < 0.0 ? x : 0.0; }
 
 // Second-order flux of one interface, cf*ldq (0 where the reference cycles),
 // the same value as fss_select's.  Superbee's factor is 0 for ratios dqu/dq
 // <= 0, 2 from 2 up, 1 on [1/2, 1], and 2*theta or theta in between, and
 // rounding to nearest cannot move a quotient across those bounds, so the
-// class comes from comparisons of dqu with dq and 2*dq, the quotient is
-// needed in two classes only, and it is divided by the operator only where
-// one of those lanes holds operands out of quot_rn's range.  `up` may be
-// either for usig = 0, where cf = 0.
+// class comes from comparisons of dqu, with dq's sign taken off, with |dq| and
+// 2|dq|, the quotient is needed in two classes only, and it is divided by the
+// operator only where one of those lanes holds operands out of quot_rn's
+// range.  A ratio that is NaN is in the class of 2 (fmin and fmax pass it
+// over), and cf, which a missing wind makes NaN, reaches every interface that
+// does not cycle.  `up` may be either for usig = 0, where cf = 0.
 static __device__ __noinline__ double ieee_theta(double dqu, double dq, bool twice) {
   const double th = dqu / dq;
   return twice ? th + th : th;
@@ -1255,27 +1251,27 @@ __device__ __forceinline__ double fss_step(double dqm, double dq, double dqp, bo
                                            bool nocycle) {
   if (LIM == A3G_LIM_NONE) return 0.0;
   if (LIM != A3G_LIM_SUPERBEE) return fss_select<LIM>(dqm, dq, dqp, up, cf, true, eps, nocycle);
-  const double dqu = up ? dqm : dqp;
-  const double a = fabs(dqu), b = fabs(dq);
-  const bool lt = a + a < b, gt = a > b;
-  bool ge2 = a >= b + b, none = b <= eps;
-  if (nocycle) {  // the clamp of :201 without the cycle of :183
+  const double dqu = up ? dqm : dqp, b = fabs(dq);
+  const double s = __hiloint2double(__double2hiint(dqu) ^ (__double2hiint(dq) & (int)0x80000000), __double2loint(dqu));
+  const bool lt = s + s < b, gt = s > b;
+  bool ge2 = !(s < b + b), none = s <= 0.0, skip = b <= eps;
+  if (nocycle) {  // the clamp of :201 (by the sign of a zero too) without the cycle of :183
     ge2 = ge2 || b < eps;
-    none = false;
+    none = none && !(s == 0.0 && __double2hiint(s) >= 0);
+    skip = false;
   }
-  none = none || (__double2hiint(dqu) ^ __double2hiint(dq)) < 0;
   const bool need = !none && !ge2 && (lt || gt);
   double th;
-  const bool ok = quot_rn(dqu, dq, &th);
+  const bool ok = quot_rn(s, b, &th);
   int hi = __double2hiint(th) + (lt ? 1 << 20 : 0), lo = __double2loint(th);  // 2*theta of a normal theta
   if (need && !ok) {
-    th = ieee_theta(dqu, dq, lt);
+    th = ieee_theta(s, b, lt);
     hi = __double2hiint(th);
     lo = __double2loint(th);
   }
   const int flat = none ? 0 : (ge2 ? 0x40000000 : 0x3ff00000);  // 0, 2 or 1
   const double phi = __hiloint2double(need ? hi : flat, need ? lo : 0);
-  return cf * (dq * phi);
+  return skip ? 0.0 : cf * (dq * phi);
 }
 
 // The values a march carries from cell c to cell c+1.
