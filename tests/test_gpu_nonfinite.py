@@ -116,3 +116,25 @@ def test_other_limiters(limiter):
 def test_broken_cells_in_the_solves(kind, op, broken):
     cfg = _cfg(**KINDS[kind])
     _compare(cfg, _state(cfg, 11, broken), _winds(cfg, 12, False), [op], {3: 1, 4: 0})
+
+
+@pytest.mark.parametrize("kind", ["projected", "lonlat"])
+@pytest.mark.parametrize("broken", ["nan", "inf", "huge", ""])
+def test_adjoint_sweeps(kind, broken):
+    """The marched transposed sweeps against the one-cell-per-thread gather, over broken states (or missing winds)."""
+    cfg = _cfg(**KINDS[kind])
+    q, winds = _state(cfg, 13, broken), _winds(cfg, 14, not broken)
+    lam = np.asfortranarray(np.random.default_rng(15).standard_normal(q.shape))
+    geo = syn.geometry(cfg)
+    out = []
+    for variant in (0, 1):
+        m = Ash3dGPU(cfg, geo=geo)
+        m.set_variant(5, variant)
+        m.set_interior(q)
+        m.set_winds(*winds)
+        m.set_dt(0.005)
+        out.append([m.adj_advect_x(lam), m.adj_advect_y(lam), m.adj_advect_z(lam, None)])
+        m.close()
+    for name, a, b in zip("xyz", *out):
+        assert np.isnan(b).any() == (broken != "huge"), name
+        assert np.array_equal(a, b, equal_nan=True), name

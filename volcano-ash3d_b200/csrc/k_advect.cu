@@ -1,6 +1,7 @@
 // k_advect.cu -- dt/kappa of the step and the discrete adjoint of the advection
 // sweeps.  The forward sweeps are in k_advect.cuh.
 #include "k_advect.cuh"
+#include "lim_coef.cuh"
 
 namespace a3g {
 
@@ -49,54 +50,6 @@ int refresh_dtv(a3g_ctx *ctx) {
 // periodic wraps, whose adjoint is added back to the wrapped cells.  Full box
 // only (the subgrid box depends on the state).
 // ===========================================================================
-
-// d(ldq) = a*d(dq) + b*d(dqu) on the branch the forward limiter takes.
-template <int LIM>
-__device__ __forceinline__ void lim_coef(double dq, double dqu, double eps, double &a, double &b) {
-  if (LIM == A3G_LIM_LAXWEN) { a = 1.0; b = 0.0; return; }
-  if (LIM == A3G_LIM_BW) { a = 0.0; b = 1.0; return; }
-  if (LIM == A3G_LIM_SUPERBEE) {
-    // the branch by comparison, without the quotient: (a, b) is (0, 0) for
-    // theta < 0, (0, 1) at 0, (0, 2) on (0, 1/2], (1, 0) between 1/2 and 1,
-    // (0, 1) on [1, 2] and (2, 0) above.  RN(dqu/dq) equals 1/2, 1 or 2 only
-    // when the exact quotient does, and lies on the same side of them; it is 0
-    // for a dqu that is not only where the quotient underflows.
-    const double u = fabs(dqu), d = fabs(dq);
-    const bool same = (__double2hiint(dqu) ^ __double2hiint(dq)) >= 0;
-    if (fabs(dq) < eps) {  // no cycle (NOCYCLE): the clamp
-      a = same ? 2.0 : 0.0;
-      b = 0.0;
-      return;
-    }
-    const bool le_half = u + u <= d, lt1 = u < d, le2 = u <= d + d;
-    a = le_half ? 0.0 : lt1 ? 1.0 : le2 ? 0.0 : 2.0;
-    b = le_half ? 2.0 : lt1 ? 0.0 : le2 ? 1.0 : 0.0;
-    if (!same) a = b = 0.0;
-    if (u < 0x1p-700 && (u == 0.0 || dqu / dq == 0.0)) b = 1.0;
-    return;
-  }
-  const bool clamp = fabs(dqu) > 3.0 * fabs(dq) || fabs(dq) < eps;
-  const double th = clamp ? copysign(3.0, dqu * dq) : div_rn(dqu, dq);
-  double phi, dphi;
-  if (LIM == A3G_LIM_FROMM) {
-    phi = 0.5 * (1.0 + th); dphi = 0.5;
-  } else if (LIM == A3G_LIM_MINMOD) {
-    const double m = fmn(1.0, th), dm = (1.0 < th) ? 0.0 : 1.0;
-    phi = fmx(0.0, m); dphi = (0.0 > m) ? 0.0 : dm;
-  } else if (LIM == A3G_LIM_MC) {
-    const double m1 = fmn((1.0 + th) / 2.0, 2.0), dm1 = ((1.0 + th) / 2.0 < 2.0) ? 0.5 : 0.0;
-    const double m2 = fmn(m1, 2.0 * th), dm2 = (m1 < 2.0 * th) ? dm1 : 2.0;
-    phi = fmx(0.0, m2); dphi = (0.0 > m2) ? 0.0 : dm2;
-  } else {  // superbee
-    const double m1 = fmn(1.0, 2.0 * th), dm1 = (1.0 < 2.0 * th) ? 0.0 : 2.0;
-    const double a1 = fmx(0.0, m1), da1 = (0.0 > m1) ? 0.0 : dm1;
-    const double m2 = fmn(2.0, th), dm2 = (2.0 < th) ? 0.0 : 1.0;
-    phi = fmx(a1, m2); dphi = (a1 > m2) ? da1 : dm2;
-  }
-  if (clamp) dphi = 0.0;
-  a = phi - th * dphi;
-  b = dphi;
-}
 
 template <int DIR, int LIM, bool PER>
 __global__ void __launch_bounds__(256) k_adj_advect(Layout L, int nocycle, double eps,
