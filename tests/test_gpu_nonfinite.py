@@ -5,7 +5,7 @@ kernel that swept it.  The sign of a zero aside, bit for bit."""
 import numpy as np
 import pytest
 
-from gpu_common import random_state, random_winds
+from gpu_common import pair, random_state, random_winds
 from topo_common import level_winds
 from volcano_ash3d_b200 import _lib, synthetic as syn
 from volcano_ash3d_b200.model import Ash3dGPU
@@ -138,3 +138,19 @@ def test_adjoint_sweeps(kind, broken):
     for name, a, b in zip("xyz", *out):
         assert np.isnan(b).any() == (broken != "huge"), name
         assert np.array_equal(a, b, equal_nan=True), name
+
+
+@pytest.mark.parametrize("latlon", [False, True])
+def test_a_missing_level_sets_no_time_step(latlon):
+    """Adjust_DT passes over cells whose wind is missing: a thin level without any wind does not bring the settling
+    speed's limit in."""
+    dz = tuple(0.02 if k == 5 else 0.5 for k in range(SIZE[2]))
+    cfg, gpu, ref = pair(_cfg(dz_profile=dz, latlon=latlon, de=0.5, dn=0.5, latLL=20.0))
+    winds = [0.01 * v for v in random_winds(cfg, 16)]
+    winds[2][:, :, 2 + 5] = np.nan
+    winds[2][7, 9, 2 + 8] = np.nan
+    for m in (gpu, ref):
+        m.set_winds(*winds)
+    dt = ref.Adjust_DT(0.0, 1.0e9, 1.0e9)
+    assert gpu.Adjust_DT(0.0, 1.0e9, 1.0e9) == dt
+    gpu.close()

@@ -140,7 +140,7 @@ __global__ void __launch_bounds__(256) k_cfl(Layout L, int latlon, const double 
   for (int r = blockIdx.x * 8 + w; r < nrow; r += gridDim.x * 8) {
     const int j = r % L.ny + 1, k = r / L.ny + 1;
     const long rb = (long)r * L.P;
-    double ax = 0.0, ay = 0.0, az = 0.0;
+    double ax = -INFINITY, ay = -INFINITY, az = -INFINITY;  // of no wind: a row that is all NaN sets no limit
 #pragma unroll 4
     for (int i = lane; i < L.nx; i += 32) {
       const double x = fabs(vx[rb + i]), y = fabs(vy[rb + i]), z = fabs(vz[rb + i]);
