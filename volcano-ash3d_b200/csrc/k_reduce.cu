@@ -584,41 +584,73 @@ void totals_volumes(a3g_ctx *ctx, const double *h_src, double *out4, double *mas
 // subgrid plane occupancy: flags[i] (i=1..nx), flags[nx+1+j], flags[nx+ny+2+k]
 // set when some grain has c >= thresh in that plane.
 // ---------------------------------------------------------------------------
-// A warp takes a row of the box outside which the level is zero, the grains'
-// loads of four cells a lane in flight.  480x401x50, 6 grains: over the box of a
-// cloud in a seventh of the grid 36 us, over the whole grid 106; a thread a cell
-// over the whole grid took 125.
-__global__ void __launch_bounds__(256) k_plane_flags(Layout L, Box nz, const double *__restrict__ c,
+// 2^lw lanes take a row of the box outside which the level is zero (a warp one
+// row of 65 columns and more, several shorter ones), four cells a lane of four
+// grains in flight, and a warp whose lanes have all met the threshold goes on
+// to its next rows; blockIdx.y shares the grains out where the rows alone
+// leave the chip idle.  A block marks planes in shared memory and hands on at
+// its end what is not set yet.
+constexpr int PF_SMEM = 32 * 1024;  // larger extents mark the global words themselves
+__global__ void __launch_bounds__(256) k_plane_flags(Layout L, Box nz, int lw, int per_y, const double *__restrict__ c,
                                                      double thresh, int32_t *__restrict__ flags) {
+  extern __shared__ uint8_t pf_seen[];
   constexpr int U = 4;
-  const int lane = threadIdx.x & 31;
-  const int nj = nz.jmax - nz.jmin + 1, nrow = nj * (nz.kmax - nz.kmin + 1);
-  for (int r = blockIdx.x * 8 + (threadIdx.x >> 5); r < nrow; r += gridDim.x * 8) {
+  const int lane = threadIdx.x & 31, sub = lane & ((1 << lw) - 1), nf = L.nx + L.ny + L.nz + 3;
+  const bool local = nf <= PF_SMEM;
+  if (local)
+    for (int t = threadIdx.x; t < nf; t += 256) pf_seen[t] = 0;
+  __syncthreads();
+  auto mark = [&](int at) {
+    if (local) pf_seen[at] = 1;
+    else if (!__ldcg(flags + at)) flags[at] = 1;
+  };
+  const int ga = blockIdx.y * per_y, gb = min(L.ns, ga + per_y);
+  const int nj = nz.jmax - nz.jmin + 1, nrow = nj * (nz.kmax - nz.kmin + 1), rows = 32 >> lw;  // rows of a warp
+  for (int r0 = (blockIdx.x * 8 + (threadIdx.x >> 5)) * rows; r0 < nrow; r0 += gridDim.x * 8 * rows) {
+    const int r = min(r0 + (lane >> lw), nrow - 1);  // past the last row: that row again
     const int j = r % nj + nz.jmin, k = r / nj + nz.kmin;
     const double *row = c + L.cell(1, j, k);
     bool any = false;
-    for (int i0 = nz.imin + lane; i0 <= nz.imax; i0 += 32 * U) {
-      bool hit[U] = {false, false, false, false};
-#pragma unroll 4
-      for (int g = 0; g < L.ns; g++) {
-        double v[U];
+    for (int i0 = nz.imin; i0 <= nz.imax; i0 += U << lw) {
+      int at[U];  // past the row's end: its last cell again
+      bool hit[U];
 #pragma unroll
-        for (int q = 0; q < U; q++) v[q] = __ldg(row + (long)g * L.PG + min(i0 + 32 * q, nz.imax) - 1);
+      for (int q = 0; q < U; q++) {
+        at[q] = min(i0 + sub + (q << lw), nz.imax);
+        hit[q] = false;
+      }
+      for (int g0 = ga; g0 < gb; g0 += 4) {
+        double v[4][U];
 #pragma unroll
-        for (int q = 0; q < U; q++) hit[q] |= v[q] >= thresh;
+        for (int g = 0; g < 4; g++)
+#pragma unroll
+          for (int q = 0; q < U; q++) v[g][q] = g0 + g < gb ? __ldg(row + (long)(g0 + g) * L.PG + at[q] - 1) : nan("");
+        bool all = true;
+#pragma unroll
+        for (int q = 0; q < U; q++) {
+#pragma unroll
+          for (int g = 0; g < 4; g++) hit[q] |= v[g][q] >= thresh;
+          all = all && hit[q];
+        }
+        if (__all_sync(0xffffffffu, all)) break;
       }
 #pragma unroll
       for (int q = 0; q < U; q++)
-        if (hit[q] && i0 + 32 * q <= nz.imax) {
+        if (hit[q]) {
           any = true;
-          if (!flags[i0 + 32 * q]) flags[i0 + 32 * q] = 1;
+          mark(at[q]);
         }
     }
-    if (__any_sync(0xffffffffu, any) && lane == 0) {
-      if (!flags[L.nx + 1 + j]) flags[L.nx + 1 + j] = 1;
-      if (!flags[L.nx + L.ny + 2 + k]) flags[L.nx + L.ny + 2 + k] = 1;
+    const unsigned mine = __ballot_sync(0xffffffffu, any) >> (lane - sub) & (0xffffffffu >> (32 - (1 << lw)));
+    if (mine && sub == 0) {
+      mark(L.nx + 1 + j);
+      mark(L.nx + L.ny + 2 + k);
     }
   }
+  if (!local) return;
+  __syncthreads();
+  for (int t = threadIdx.x; t < nf; t += 256)
+    if (pf_seen[t] && !__ldcg(flags + t)) flags[t] = 1;
 }
 
 int launch_plane_flags(a3g_ctx *ctx) {
@@ -628,10 +660,18 @@ int launch_plane_flags(a3g_ctx *ctx) {
   // a threshold of zero or less is met by the zeros outside the state's box too
   Box nz = ctx->prm.cloudcon_grid_thresh > 0.0 ? state_box(ctx) : full_box_of(L);
   if (empty(nz)) nz = Box{1, 1, 1, 1, 1, 1};
-  const int rows = ((nz.jmax - nz.jmin + 1) * (nz.kmax - nz.kmin + 1) + 7) / 8;
+  int lw = 0;
+  while (lw < 5 && (4 << lw) < nz.imax - nz.imin + 1) lw++;
+  const int per = 8 * (32 >> lw);  // rows of a block
+  const int rows = ((nz.jmax - nz.jmin + 1) * (nz.kmax - nz.kmin + 1) + per - 1) / per;
+  // grains in one block, or in fours where that leaves less than four blocks an SM
+  int ny = 148 * 4 / rows, most = (L.ns + 3) / 4;
+  ny = ny < 1 ? 1 : ny < most ? ny : most;
+  const int per_y = ((L.ns + ny - 1) / ny + 3) / 4 * 4;
+  const dim3 grid(rows < 148 * 8 ? rows : 148 * 8, (L.ns + per_y - 1) / per_y);
   tbegin(ctx, A3G_K_OTHER);
-  k_plane_flags<<<rows < 148 * 8 ? rows : 148 * 8, 256, 0, ctx->stream>>>(
-      L, nz, ctx->c0, ctx->prm.cloudcon_grid_thresh, ctx->plane_flags);
+  k_plane_flags<<<grid, 256, nf <= (size_t)PF_SMEM ? nf : 0, ctx->stream>>>(
+      L, nz, lw, per_y, ctx->c0, ctx->prm.cloudcon_grid_thresh, ctx->plane_flags);
   tend(ctx);
   A3G_LAUNCH_CHECK(ctx);
   A3G_CUDA(cudaMemcpyAsync(ctx->h_plane_flags, ctx->plane_flags, nf * sizeof(int32_t),
