@@ -1035,7 +1035,7 @@ static void launch_advect_xw(a3g_ctx *ctx, bool tma) {
   k_advect_xw<LIM, GC_, PER_, LC_, TMA_><<<blocks, 32 * XW_WARPS, 0, ctx->stream>>>(                        \
       tq, tv, L, ctx->box, ctx->prm.nocycle, ctx->prm.eps_thresh, ngroups, ctx->c0, ctx->c1, ctx->vx,        \
       ctx->snx, ctx->dtv, ctx->aloft, ctx->sc, ctx->out_yz1, ctx->out_yz2)
-  // rows of constant geometry come here only without tensor maps (k_advect_xm)
+  // rows of constant geometry come here where they are few (launch_dir_lim) or without tensor maps
 #define A3G_XW_LC(GC_, PER_)                      \
   if (lc) { A3G_XW(GC_, PER_, true, false); }     \
   else if (tma) { A3G_XW(GC_, PER_, false, true); } \
@@ -1944,7 +1944,12 @@ static void launch_dir_lim(a3g_ctx *ctx) {
       launch_advect_xt<LIM>(ctx);
       return;
     }
-    if (variant == 5 && launch_advect_xm<LIM>(ctx)) return;
+    // A row per lane needs rows: with few and short ones a warp per row is
+    // sooner done (50x50x23, 1 grain: 6.2 us a sweep, the march 8.2; 60x80x30, 2
+    // grains: 9.3, 10.4; 200x100x20, 1 grain: 10.3, 12.3; but 400x3x40, 2 grains:
+    // 17.9, 10.3; 30x200x20, 2 grains: 12.3, 10.3; 100x100x40, 2 grains: 18, 14).
+    const bool few_rows = ctx->L.nx <= 224 && (long)ctx->L.ny * ctx->L.nz * ctx->L.ns < 5000;
+    if (variant == 5 && !few_rows && launch_advect_xm<LIM>(ctx)) return;
     if (variant == 4 || variant == 5) {
       launch_advect_xw<LIM>(ctx, variant == 5);
       return;
