@@ -209,7 +209,7 @@ __global__ void __launch_bounds__(128) k_diff_xy(Layout L, Box box, Box cov, int
 }
 
 // DiffuseVert (ADJ: its transpose) marched along k, lanes along i, every cell
-// read once.  360x161x40, 5 grains: 82 -> 60 us.
+// read once.  360x161x40, 5 grains: 76 -> 56 us.
 template <bool ADJ>
 __global__ void __launch_bounds__(128) k_diff_z(Layout L, Box box, Box cov, int nseg, int seg, const double *__restrict__ cin,
                                                 double *__restrict__ cout, const DiffRow *__restrict__ tab,
@@ -2065,9 +2065,13 @@ static bool diff_table(a3g_ctx *ctx) {
 }
 
 // segments of a marched line of n cells that leave at least 8 cells each and
-// give the chip about 24 warps an SM
-static int diff_segments(int n, long warps) {
-  const long want = (148L * 24 + warps - 1) / warps, most = n / 8 > 1 ? n / 8 : 1;
+// give the chip about `per_sm` warps an SM: 24 for the fused horizontal sweeps
+// (48 warps: 360x161x40, 5 grains, 50 -> 60 us), 128 for the vertical one, whose
+// whole columns wait on each load in turn (24 warps: 317x211x53, 3 grains, 72 us
+// and 82 for the transpose, where a thread a cell took 72 and 75; 51 and 57 with
+// 128; 317x211x53, 7 grains, 120 and 136 against 135 and 134; 101 and 113).
+static int diff_segments(int n, long warps, long per_sm) {
+  const long want = (148L * per_sm + warps - 1) / warps, most = n / 8 > 1 ? n / 8 : 1;
   return (int)(want < 1 ? 1 : want < most ? want : most);
 }
 
@@ -2078,7 +2082,7 @@ static bool run_diff_xy(a3g_ctx *ctx, bool xfirst, const Box &box, const Box &co
   const Layout &L = ctx->L;
   const int n = cov.jmax - cov.jmin + 1;
   const long lines = (long)((cov.imax - cov.imin + 30) / 30) * (cov.kmax - cov.kmin + 1) * L.ns;
-  const int seg = (n + diff_segments(n, lines) - 1) / diff_segments(n, lines);
+  const int want = diff_segments(n, lines, 24), seg = (n + want - 1) / want;
   const int nseg = (n + seg - 1) / seg;
   const unsigned blocks = (unsigned)((lines * nseg + 3) / 4);
   const DiffRow *tab = static_cast<const DiffRow *>(ctx->diff_tab);
@@ -2093,13 +2097,17 @@ static bool run_diff_xy(a3g_ctx *ctx, bool xfirst, const Box &box, const Box &co
   return true;
 }
 
+// A march needs columns enough: on small grids a thread a cell (k_diff,
+// k_adj_diff) is sooner done (50x50x23, 1 grain: 5.1 us, the march 8.2, its
+// transpose 4.7, 8.2; 60x80x30, 2 grains: 6.2, 6.5 and 6.2, 7.9; but 100x100x40,
+// 1 grain: 10.3, 6.2 and 10.3, 7.8).
 template <bool ADJ>
 static bool run_diff_z(a3g_ctx *ctx, const Box &box, const Box &cov, const double *cin, double *cout) {
-  if (!diff_table(ctx)) return false;
   const Layout &L = ctx->L;
+  if ((long)L.nx * L.ny * L.nz < 250000 || !diff_table(ctx)) return false;
   const int n = cov.kmax - cov.kmin + 1;
   const long lines = (long)((cov.imax - cov.imin + 32) / 32) * (cov.jmax - cov.jmin + 1) * L.ns;
-  const int seg = (n + diff_segments(n, lines) - 1) / diff_segments(n, lines);
+  const int want = diff_segments(n, lines, 128), seg = (n + want - 1) / want;
   const int nseg = (n + seg - 1) / seg;
   k_diff_z<ADJ><<<(unsigned)((lines * nseg + 3) / 4), 128, 0, ctx->stream>>>(
       L, box, cov, nseg, seg, cin, cout, static_cast<const DiffRow *>(ctx->diff_tab), ctx->aloft, ctx->sc);
