@@ -392,7 +392,8 @@ int a3g_kernel_times(a3g_ctx *ctx, double *ms, uint64_t *count);
  * copy (default).  dir 4: the Crank-Nicolson y and z solves, variant 0 one
  * grain per thread, 1 two grains of a line per thread, 2 four, 3 tiles of
  * 32 lines staged in shared memory by TMA tensor copies (default; where the
- * coefficients vary along i, or nz > 256, variant 3 runs variant 1).
+ * coefficients vary along i, and for z where nz > 256, variant 3 runs one
+ * thread per line and grain, eight rows' loads at a time).
  * dir 1, 2 variant 5: the column march (one thread per line and grain, lanes
  * along i, each interface formed once); variant 6, the same march reading
  * the concentration and wind from chunks that TMA tensor copies stage in

@@ -754,8 +754,10 @@ static void launch_cn_solve_gc(a3g_ctx *ctx, const LineMap &map, const CnTab &ta
     k_cn_solve_gc<DIR, GC><<<grid, 128, 0, ctx->stream>>>(L, ctx->box, map, ctx->c0, ctx->c1, tab, ctx->aloft);
 }
 
-// y and z lines whose coefficients vary along i (terrain), where no two lanes
-// share a table row.  A warp holds 32 neighbouring lines of one grain and its
+// y and z lines that no tile takes: coefficients that vary along i (terrain),
+// where no two lanes share a table row, and columns of more than 256 levels,
+// whose 32 share a table by row (ROWS; 160x160x300, 1 grain: 192 us with the factors by field and a thread per
+// line, 222 with that over the table by row, 77 here).  A warp holds 32 neighbouring lines of one grain and its
 // block the same lines of the other grains, which so find the table rows in
 // L1; rows are taken CB_U at a time, all their loads before the first of the
 // dependent operations.  Bound by the latency of those loads and the memory
@@ -783,7 +785,7 @@ static dim3 cb_grid(const Layout &L, int *threads) {
   return dim3(((L.nx + 31) / 32) * (DIR == 1 ? L.nz : L.ny), (L.ns + w - 1) / w);
 }
 
-template <int DIR>
+template <int DIR, bool ROWS>
 __global__ void __launch_bounds__(32 * CB_WARPS, 2) k_cn_solve_b(Layout L, Box box, LineMap map,
                                                                  const double *__restrict__ cin,
                                                                  double *__restrict__ cout, CnTab tab,
@@ -806,8 +808,12 @@ __global__ void __launch_bounds__(32 * CB_WARPS, 2) k_cn_solve_b(Layout L, Box b
   const long u = map.u(a, b);
   const double *qq = cin + base + (long)(rmin - 1) * st;
   x += (long)(rmin - 1) * st;
-  const double *tp = tab.p + u;
-  auto co = [&](int f, int l) { return __ldg(tp + f * tab.F + (long)l * tab.U); };
+  const double *tp = ROWS ? tab.p + CN_ROW * u * ncells : tab.p + u;
+  const double *dpp = tab.p + CN_ROW * tab.F + u * ncells;  // D' of a table by row
+  auto co = [&](int f, int l) {
+    if (ROWS) return __ldg(f == CN_DP ? dpp + l : tp + (long)CN_ROW * l + f);
+    return __ldg(tp + f * tab.F + (long)l * tab.U);
+  };
   // forward elimination with the right-hand side built on the fly, :813-851
   double qm = __ldg(qq), qc = qm, bp = 0.0;  // BC_left_t0 = q(rmin)
   int l = 0;
@@ -2274,11 +2280,13 @@ static int launch_cn_dir(a3g_ctx *ctx) {
     // column tiles through TMA
   } else if (DIR == 1 && ctx->tune_cn_yz == 3 && launch_cn_solve_yt(ctx, map, tab)) {
     // chunk tiles through TMA
-  } else if (DIR != 0 && ctx->tune_cn_yz == 3 && !tab.byrow) {
+  } else if (DIR != 0 && ctx->tune_cn_yz == 3) {
+    constexpr int D = DIR == 0 ? 1 : DIR;
     int threads;
-    const dim3 grid = cb_grid<DIR == 0 ? 1 : DIR>(L, &threads);
-    k_cn_solve_b<DIR == 0 ? 1 : DIR><<<grid, threads, 0, ctx->stream>>>(L, box, map, ctx->c0, ctx->c1, tab, ctx->aloft);
-  } else if (DIR != 0 && (ctx->tune_cn_yz == 1 || ctx->tune_cn_yz == 3) && L.ns >= 2) {
+    const dim3 grid = cb_grid<D>(L, &threads);
+    if (tab.byrow) k_cn_solve_b<D, true><<<grid, threads, 0, ctx->stream>>>(L, box, map, ctx->c0, ctx->c1, tab, ctx->aloft);
+    else k_cn_solve_b<D, false><<<grid, threads, 0, ctx->stream>>>(L, box, map, ctx->c0, ctx->c1, tab, ctx->aloft);
+  } else if (DIR != 0 && ctx->tune_cn_yz == 1 && L.ns >= 2) {
     launch_cn_solve_gc<DIR == 0 ? 1 : DIR, 2>(ctx, map, tab);
   } else if (DIR != 0 && ctx->tune_cn_yz == 2 && L.ns >= 2) {
     launch_cn_solve_gc<DIR == 0 ? 1 : DIR, 4>(ctx, map, tab);
