@@ -1879,9 +1879,9 @@ static void launch_march_gc(a3g_ctx *ctx) {
   const int n = (DIR == 0) ? L.nx : (DIR == 1) ? L.ny : L.nz;
   const int na = (DIR == 0) ? L.ny : L.nx;
   const int nother = (DIR == 2) ? L.ny : L.nz;
-  // segments of about 96 cells (whole lines when they are short), over terrain
-  // of 48 where that gives an SM less than 32 warps
-  const int len = TOPO && march_warps<DIR>(L, GC) < 148 * 32 ? 48 : 96;
+  // segments of about 96 cells (whole lines when they are short); over terrain
+  // of 48 along rows, and along columns where 96 give an SM less than 32 warps
+  const int len = TOPO && (DIR == 0 || march_warps<DIR>(L, GC) < 148 * 32) ? 48 : 96;
   const int nseg = (n + len - 1) / len;
   const int seg = (n + nseg - 1) / nseg;
   const int ngroups = (L.ns + GC - 1) / GC;
@@ -1922,13 +1922,17 @@ static void launch_dir_lim(a3g_ctx *ctx) {
   const int variant = ctx->tune_advect[DIR];
   if constexpr (DIR != 2) {
     // ZScaling_ID 2: the DelD*onD_cc terms live in the marching kernel only.
-    // A grain a thread, or two that share the row's winds: two in x where they
-    // fill the chip (402x301x50, 10 grains: 913 us a sweep, one 934; y 825,
-    // 746).  With the segments of 48 cells, 201x151x41 and 5 grains: x 144 ->
-    // 130 us, y 142 -> 102; 150x120x30 and 2 grains: x 70 -> 33, y 60 -> 32.
+    // Along x two grains a thread share the row's winds, unless a missing second
+    // one makes a sixth of the work or more; along y a grain a thread.  x with
+    // segments of 48 and two grains, with 48 and one, and with 96 and two, us a
+    // sweep of 201x151x41: 3 grains 89, 86, 122; 5 grains 135, 131, 148; 6: 146,
+    // 161, 156; 8: 186, 200, 217; 10: 226, 246, 232; 402x301x50, 4 grains: 381,
+    // 407, 403; 150x120x30, 2 grains: 35, 33, 61; 97x83x25, 8: 42, 54, 56.  y with
+    // one and with two (segments of 96): 402x301x50, 10 grains, 746, 825;
+    // 201x151x41, 5 grains, 102, 142.
     if (ctx->topo_on && ctx->prm.zscaling_id == 2) {
       if constexpr (DIR == 0) {
-        const bool g2 = ctx->L.ns >= 2 && march_warps<DIR>(ctx->L, 2) >= 148 * 32;
+        const bool g2 = ctx->L.ns % 2 == 0 || ctx->L.ns > 6;
         if (per && g2) launch_march_gc<DIR, LIM, 2, true, true>(ctx);
         else if (per) launch_march_gc<DIR, LIM, 1, true, true>(ctx);
         else if (g2) launch_march_gc<DIR, LIM, 2, false, true>(ctx);

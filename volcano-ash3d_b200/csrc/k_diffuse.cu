@@ -756,14 +756,13 @@ static void launch_cn_solve_gc(a3g_ctx *ctx, const LineMap &map, const CnTab &ta
 
 // y and z lines that no tile takes: coefficients that vary along i (terrain),
 // where no two lanes share a table row, and columns of more than 256 levels,
-// whose 32 share a table by row (ROWS; 160x160x300, 1 grain: 192 us with the factors by field and a thread per
-// line, 222 with that over the table by row, 77 here).  A warp holds 32 neighbouring lines of one grain and its
-// block the same lines of the other grains, which so find the table rows in
-// L1; rows are taken CB_U at a time, all their loads before the first of the
-// dependent operations.  Bound by the latency of those loads and the memory
-// behind them: a thread per line with a row at a time, two grains together,
-// waited for one row after another (201x151x41, 5 grains over terrain: y 324
-// -> 64 us, z 84 -> 69 us).
+// whose 32 share a table by row (ROWS).  A warp holds 32 neighbouring lines of
+// one grain and its block the same lines of the other grains, which so find the
+// table rows in L1; rows are taken CB_U at a time, all their loads before the
+// first of the dependent operations.  Bound by the latency of those loads and
+// the memory behind them: a thread per line with a row at a time waited for one
+// row after another (201x151x41, 5 grains over terrain: y 324 -> 64 us, z 84 ->
+// 69 us; z of 160x160x300, 1 grain: 192 us, 222 over a table by row, 77 here).
 constexpr int CB_U = 8, CB_WARPS = 8;
 
 // Lines of 32 neighbouring i: where a thread's line of direction DIR starts.
