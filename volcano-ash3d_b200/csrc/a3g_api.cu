@@ -1029,7 +1029,6 @@ int a3g_adjust_dt(a3g_ctx *ctx, double time, double next_write_time, double simt
   if (ctx->prm.use_diffusion && !ctx->have_diffusivity) return fail(A3G_ERR_STATE, "diffusivity not set");
   int rc = launch_cfl(ctx, time, next_write_time, simtime);
   if (rc) return rc;
-  ctx->dt_stamp++;
   if ((rc = sync_scalars(ctx))) return rc;
   ctx->host_dt = ctx->h_sc->dt;
   if (dt_out) *dt_out = ctx->h_sc->dt;
@@ -1044,7 +1043,6 @@ int a3g_adjust_dt_async(a3g_ctx *ctx, double time, double next_write_time, doubl
   if (ctx->prm.use_diffusion && !ctx->have_diffusivity) return fail(A3G_ERR_STATE, "diffusivity not set");
   int rc = launch_cfl(ctx, time, next_write_time, simtime);
   if (rc) return rc;
-  ctx->dt_stamp++;
   const int slot = (int)(ctx->dt_seq % 4);
   A3G_CUDA(cudaMemcpyAsync(ctx->h_sc_ring + slot, ctx->sc, sizeof(DevScalars), cudaMemcpyDeviceToHost,
                            ctx->stream));
@@ -1285,7 +1283,6 @@ int a3g_fast_dt_async(a3g_ctx *ctx, double interval_frac, double time, double ne
   CTX_CHECK(ctx);
   int rc = launch_fast_dt(ctx, interval_frac, time, next_write_time, simtime);
   if (rc) return rc;
-  ctx->dt_stamp++;
   const int slot = (int)(ctx->dt_seq % 4);
   A3G_CUDA(cudaMemcpyAsync(ctx->h_sc_ring + slot, ctx->sc, sizeof(DevScalars), cudaMemcpyDeviceToHost,
                            ctx->stream));

@@ -301,7 +301,8 @@ int launch_cfl_maxima_meso(a3g_ctx *ctx, int slot);
 int launch_cfl_maxima_meso_ptr(a3g_ctx *ctx, const float *met_step);
 void inv_free(a3g_ctx *ctx);
 int launch_fast_dt(a3g_ctx *ctx, double frac, double time, double next_write_time, double simtime);
-double *claim_dtv(a3g_ctx *ctx);
+double *dtv_target(const a3g_ctx *ctx);
+void dt_formed(a3g_ctx *ctx, const double *dtv);
 int launch_plane_flags(a3g_ctx *ctx);
 int launch_interp_winds(a3g_ctx *ctx, double frac);
 int launch_interp_pair(a3g_ctx *ctx, const float *last, const float *next, double frac);

@@ -317,10 +317,11 @@ int winds(a3g_ctx *ctx, a3g_inv *v, int hour, double frac) {
 }
 
 int set_step_dt(a3g_ctx *ctx, a3g_inv *v, int n) {
-  k_set_dt<<<1, 256, 0, ctx->stream>>>(ctx->sc, v->dts, n, ctx->kappa.p, claim_dtv(ctx), (int)ctx->kappa_len);
+  double *const dtv = dtv_target(ctx);
+  k_set_dt<<<1, 256, 0, ctx->stream>>>(ctx->sc, v->dts, n, ctx->kappa.p, dtv, (int)ctx->kappa_len);
   A3G_LAUNCH_CHECK(ctx);
+  dt_formed(ctx, dtv);
   ctx->host_dt = v->steps[n].dt;
-  ctx->dt_stamp++;
   return A3G_OK;
 }
 

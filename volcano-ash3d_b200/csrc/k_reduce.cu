@@ -300,13 +300,18 @@ __global__ void k_fast_dt(double frac, double eps_small, double time, double nex
 
 // dt/kappa's buffer for a kernel that forms dt and, where kappa's table is
 // small (a projected grid's; one block forms it within a microsecond or two),
-// dt/kappa with it; null where k_dtv is left to do it.  The caller's entry
-// point advances dt_stamp after the launch.
-double *claim_dtv(a3g_ctx *ctx) {
-  if (!ctx->have_geometry || ctx->kappa_len > 2048) return nullptr;
+// dt/kappa with it; null where k_dtv is left to do it.
+double *dtv_target(const a3g_ctx *ctx) {
+  return ctx->have_geometry && ctx->kappa_len <= 2048 ? ctx->dtv_buf : nullptr;
+}
+
+// After such a kernel's launch, and only if it was not refused: dt is another,
+// and dt/kappa (dtv, from dtv_target) is of that dt.
+void dt_formed(a3g_ctx *ctx, const double *dtv) {
+  ctx->dt_stamp++;
+  if (!dtv) return;
   ctx->dtv_valid = true;
-  ctx->dtv_stamp = ctx->dt_stamp + 1;
-  return ctx->dtv_buf;
+  ctx->dtv_stamp = ctx->dt_stamp;
 }
 
 int launch_cfl_maxima_meso(a3g_ctx *ctx, int slot) {
@@ -333,10 +338,12 @@ int launch_cfl_maxima_meso_ptr(a3g_ctx *ctx, const float *m) {
 
 int launch_fast_dt(a3g_ctx *ctx, double frac, double time, double next_write_time, double simtime) {
   tbegin(ctx, A3G_K_OTHER);
-  k_fast_dt<<<1, 256, 0, ctx->stream>>>(frac, ctx->prm.eps_small, time, next_write_time, simtime, ctx->kappa.p,
-                                        claim_dtv(ctx), (int)ctx->kappa_len, ctx->sc);
+  double *const dtv = dtv_target(ctx);
+  k_fast_dt<<<1, 256, 0, ctx->stream>>>(frac, ctx->prm.eps_small, time, next_write_time, simtime, ctx->kappa.p, dtv,
+                                        (int)ctx->kappa_len, ctx->sc);
   tend(ctx);
   A3G_LAUNCH_CHECK(ctx);
+  dt_formed(ctx, dtv);
   return A3G_OK;
 }
 
@@ -406,7 +413,10 @@ int launch_cfl(a3g_ctx *ctx, double time, double next_write_time, double simtime
   int fresh;
   int rc = diffusion_limit(ctx, &fresh);
   if (rc) return rc;
-  return run_cfl(ctx, 1, dt_args(ctx, ctx->n_gs_aloft, time, next_write_time, simtime, fresh, 0), claim_dtv(ctx));
+  double *const dtv = dtv_target(ctx);
+  rc = run_cfl(ctx, 1, dt_args(ctx, ctx->n_gs_aloft, time, next_write_time, simtime, fresh, 0), dtv);
+  if (!rc) dt_formed(ctx, dtv);
+  return rc;
 }
 
 // ---------------------------------------------------------------------------
