@@ -71,3 +71,19 @@ def test_dt_over_kappa(form_dt):
         assert form_dt(m) != 0
     assert np.array_equal(_swept(m, 0.013), want)
     m.close()
+
+
+def test_explicit_diffusion_factors():
+    """A refused table launch has not filled the explicit sweeps' table."""
+    def diffused(m):
+        m.set_dt(0.013)
+        m.DiffuseHorz(1)
+        return m.interior()
+
+    want = diffused(_model())
+    m = _model()
+    m.set_dt(0.013)
+    with Refusing(m):
+        assert m.lib.a3g_diffuse_horz(m.ctx, 1) != 0
+    assert np.array_equal(diffused(m), want)
+    m.close()

@@ -2064,9 +2064,9 @@ static bool diff_table(a3g_ctx *ctx) {
     k_diff_table<<<(n + 127) / 128, 128, 0, ctx->stream>>>(L, ctx->snx, ctx->sny, ctx->snz, ctx->kappa, ctx->kx,
                                                          ctx->ky, ctx->kz, static_cast<DiffRow *>(ctx->diff_tab));
     ctx->launches++;
-    ctx->diff_valid = true;
+    ctx->diff_valid = cudaPeekAtLastError() == cudaSuccess;  // the caller's check reports a refused launch
   }
-  return true;
+  return ctx->diff_valid;
 }
 
 // segments of a marched line of n cells that leave at least 8 cells each and
