@@ -354,7 +354,13 @@ int a3g_kernel_launches(a3g_ctx *ctx, uint64_t *count);
  *      cpu_time/system_clock totals, src/Ash3d.F90:727-759) ---- */
 /* The cudaStream_t all of this context's work is queued on. */
 int a3g_get_stream(a3g_ctx *ctx, void **stream);
-/* Kernel classes reported by a3g_kernel_times. */
+/* Kernel classes reported by a3g_kernel_times.  A launch that does several
+ * things counts once: DIFF_X holds both horizontal sweeps of the explicit
+ * diffusion where one launch does them (geometry and diffusivities that do not
+ * vary along i; DIFF_Y is then 0), CN_TABLE the factor tables of all
+ * directions, counted where dt or the box may have changed, CFL the maxima and the dt formed
+ * from them, TOTALS all mass totals, ADJOINT every transposed sweep, with the
+ * tables that it rebuilds. */
 #define A3G_K_ADVECT_X   0
 #define A3G_K_ADVECT_Y   1
 #define A3G_K_ADVECT_Z   2

@@ -2080,10 +2080,9 @@ static int diff_segments(int n, long warps, long per_sm) {
   return (int)(want < 1 ? 1 : want < most ? want : most);
 }
 
-// The horizontal sweeps in one pass, x first or y first; false as diff_table.
+// The horizontal sweeps in one pass, x first or y first; diff_table holds.
 template <bool ADJ>
-static bool run_diff_xy(a3g_ctx *ctx, bool xfirst, const Box &box, const Box &cov, const double *cin, double *cout) {
-  if (!diff_table(ctx)) return false;
+static void run_diff_xy(a3g_ctx *ctx, bool xfirst, const Box &box, const Box &cov, const double *cin, double *cout) {
   const Layout &L = ctx->L;
   const int n = cov.jmax - cov.jmin + 1;
   const long lines = (long)((cov.imax - cov.imin + 30) / 30) * (cov.kmax - cov.kmin + 1) * L.ns;
@@ -2099,7 +2098,6 @@ static bool run_diff_xy(a3g_ctx *ctx, bool xfirst, const Box &box, const Box &co
     if (xfirst) A3G_DXY(true, false); else A3G_DXY(false, false);
   }
 #undef A3G_DXY
-  return true;
 }
 
 // A march needs columns enough: on small grids a thread a cell (k_diff,
@@ -2139,16 +2137,17 @@ static int launch_diff_dir(a3g_ctx *ctx) {
   return A3G_OK;
 }
 
-// DiffuseHorz, explicit: both sweeps, x first or y first.
+// DiffuseHorz, explicit: both sweeps, x first or y first.  One timed launch
+// (A3G_K_DIFF_X) where they are fused, one each where they are not.
 int launch_diff_horz(a3g_ctx *ctx, bool xfirst) {
-  tbegin(ctx, A3G_K_DIFF_X);
-  const bool fused = run_diff_xy<false>(ctx, xfirst, ctx->box, cover_box(ctx), ctx->c0, ctx->c1);
-  tend(ctx);
-  if (!fused) {
+  if (!diff_table(ctx)) {
     int rc = xfirst ? launch_diff_dir<0>(ctx) : launch_diff_dir<1>(ctx);
     if (!rc) rc = xfirst ? launch_diff_dir<1>(ctx) : launch_diff_dir<0>(ctx);
     return rc;
   }
+  tbegin(ctx, A3G_K_DIFF_X);
+  run_diff_xy<false>(ctx, xfirst, ctx->box, cover_box(ctx), ctx->c0, ctx->c1);
+  tend(ctx);
   A3G_LAUNCH_CHECK(ctx);
   sweep_done(ctx);
   return A3G_OK;
@@ -2224,16 +2223,19 @@ static CnTableJob cn_table_job(a3g_ctx *ctx) {
 // chain per line, and the three run side by side (a step's tables on
 // 93x131x37: 38 us in three launches, 26 in one; 317x211x53: 35, 26;
 // 201x151x41 over terrain: 176, 96).
+// `timed`: the launch has a bracket of its own (the caller has none open).
 template <int DIR>
-static int cn_table(a3g_ctx *ctx, const LineMap &map, CnTab *out) {
+static int cn_table(a3g_ctx *ctx, const LineMap &map, bool timed, CnTab *out) {
   const Box &box = ctx->box;
   const int n = box_cells(box, DIR);
   *out = CnTab{ctx->cn_tab[DIR], (long)n * map.U, map.U, n, cn_byrow(DIR, map)};
   if (ctx->cn_valid[DIR] && same_box(ctx->cn_box[DIR], box) && ctx->cn_stamp[DIR] == ctx->dt_stamp) return A3G_OK;
   const CnTableJob jx = cn_table_job<0>(ctx), jy = cn_table_job<1>(ctx), jz = cn_table_job<2>(ctx);
   const bool wide = jx.lpb > 1 || jy.lpb > 1 || jz.lpb > 1;
+  if (timed) tbegin(ctx, A3G_K_CN_TABLE);
   k_cn_tables<<<jx.blocks + jy.blocks + jz.blocks, 256, 5 * (wide ? 1024 : 256) * sizeof(double), ctx->stream>>>(
       ctx->L, box, ctx->prm.imp_fac, ctx->kappa, jx, jy, jz, ctx->sc);
+  if (timed) tend(ctx);
   A3G_LAUNCH_CHECK(ctx);
   const int built[3] = {jx.blocks, jy.blocks, jz.blocks};
   for (int d = 0; d < 3; d++)
@@ -2259,9 +2261,7 @@ static int launch_cn_dir(a3g_ctx *ctx) {
   }
   const LineMap map = line_map<DIR>(ctx);
   CnTab tab;
-  tbegin(ctx, A3G_K_CN_TABLE);
-  int rc = cn_table<DIR>(ctx, map, &tab);
-  tend(ctx);
+  int rc = cn_table<DIR>(ctx, map, true, &tab);
   if (rc) return rc;
   const long nlines = (long)map.na * map.nb * L.ns;
   tbegin(ctx, A3G_K_CN_SOLVE_X + DIR);
@@ -2586,11 +2586,13 @@ static int launch_adj_diff_dir(a3g_ctx *ctx, const double *lin, double *lout) {
 // x transpose first or the y transpose first; *done false where they have to
 // be launched one by one (launch_adj_diffuse).
 int launch_adj_diff_horz(a3g_ctx *ctx, bool xfirst, const double *lin, double *lout, bool *done) {
+  *done = diff_table(ctx);
+  if (!*done) return A3G_OK;
   const Box full{1, ctx->L.nx, 1, ctx->L.ny, 1, ctx->L.nz};
   tbegin(ctx, A3G_K_ADJOINT);
-  *done = run_diff_xy<true>(ctx, xfirst, full, full, lin, lout);
+  run_diff_xy<true>(ctx, xfirst, full, full, lin, lout);
   tend(ctx);
-  if (*done) A3G_LAUNCH_CHECK(ctx);
+  A3G_LAUNCH_CHECK(ctx);
   return A3G_OK;
 }
 
@@ -2606,7 +2608,7 @@ static int launch_adj_cn_dir(a3g_ctx *ctx, const double *lin, double *lout) {
   const LineMap map = line_map<DIR>(ctx);
   CnTab tab;
   tbegin(ctx, A3G_K_ADJOINT);
-  int rc = cn_table<DIR>(ctx, map, &tab);
+  int rc = cn_table<DIR>(ctx, map, false, &tab);
   if (rc) return rc;
   if (DIR == 0) {
     int threads;
