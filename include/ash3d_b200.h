@@ -595,6 +595,14 @@ int a3g_mass_aloft_noalloc(int device, const double *conc, const double *kappa, 
  * the given device; *mismatches receives the number of differing quotients
  * (0 is expected: the sweeps rely on bit-identical quotients). */
 int a3g_selftest_div(int device, uint64_t n, uint64_t seed, uint64_t *mismatches);
+/* The same for the two quotients that carry a proof instead of a check of
+ * their result: n seeded pairs for each of the limiter's ratio and the back
+ * substitution's.  counts[4]: wrong ratios, wrong back substitutions (both have to
+ * be 0), then the pairs of each that are left to the division operator.
+ * *estimate receives the largest relative error of the device's reciprocal
+ * estimate over all leading 20-bit mantissas, which the first proof takes to be
+ * below 2^-19. */
+int a3g_selftest_quotients(int device, uint64_t n, uint64_t seed, uint64_t *counts, double *estimate);
 
 #ifdef __cplusplus
 }

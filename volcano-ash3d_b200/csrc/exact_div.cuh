@@ -133,8 +133,8 @@ __device__ __forceinline__ double div_rn_rcp(double a, double b, double y) {
 // ulp(q) from every midpoint m of two doubles (a - b*m is a nonzero multiple
 // of 2^-53 ulp(q)): q = RN(a/b) whenever b < 2(1 - 2^-22).  Divisors whose
 // leading 20 mantissa bits are all ones are refused; the estimate's error is
-// at most 2^-19.9 over all leading 20-bit mantissas (the bits it depends on),
-// measured on B200.  |a| >= 2^-700 and 2^-200 <= |b| < 2^201 keep every
+// at most 2^-19.93 over all leading 20-bit mantissas (measured on B200:
+// a3g_selftest_quotients, which a test holds below 2^-19).  |a| >= 2^-700 and 2^-200 <= |b| < 2^201 keep every
 // intermediate normal and the residual exact (see above); a zero dividend is
 // refused.
 __device__ __forceinline__ bool quot_rn(double a, double b, double *q) {

@@ -14,6 +14,8 @@
 #include "a3g_internal.cuh"
 #include "exact_div.cuh"
 
+#include <cstring>
+
 namespace a3g {
 
 __device__ __forceinline__ void atomic_max_pos(double *addr, double v) {
@@ -1327,7 +1329,83 @@ __global__ void k_selftest_div(uint64_t n, uint64_t seed, unsigned long long *ba
   if (local) atomicAdd(bad, local);
 }
 
+// A mantissa in [1, 2): any, just below 2, a few ulps from 1 or 2, or short (exact quotients).
+__device__ double test_mantissa(uint64_t h) {
+  uint64_t m = (h >> 8) & 0x000fffffffffffffULL;
+  const int fam = (int)(h & 3);
+  if (fam == 1) m |= 0x000fffff00000000ULL & ~((h >> 62) << 32);
+  if (fam == 2) m = (h & 4) ? (h >> 60) : 0x000fffffffffffffULL - (h >> 60);
+  if (fam == 3) m &= 0x000ffff000000000ULL;
+  return __longlong_as_double((long long)(0x3ff0000000000000ULL | m));
+}
+
+// counts: wrong quotients of quot_rn and of div_rn_3 (a zero's sign aside),
+// then the operands either leaves to the division operator
+__global__ void k_selftest_quotients(uint64_t n, uint64_t seed, unsigned long long *counts) {
+  unsigned long long c[4] = {0, 0, 0, 0};
+  for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < n; t += (uint64_t)gridDim.x * blockDim.x) {
+    const uint64_t h = mix64(seed ^ (3 * t + 2));
+    const double ma = test_mantissa(mix64(seed ^ (3 * t))), mb = test_mantissa(mix64(seed ^ (3 * t + 1)));
+    // the limiter's ratio: |b| in 2^-210 .. 2^210, |a| from 2|b| down 40 (one in four: 700) binades
+    double b = ldexp(mb, (int)(h % 420) - 210), q;
+    double a = ldexp(ma, ilogb(b) - (int)((h >> 12) % ((h >> 10 & 3) ? 40 : 700)));
+    if (h & (1ull << 40)) a = -a;
+    if (h & (1ull << 41)) b = -b;
+    if (fabs(a) < 2.0 * fabs(b)) {
+      if (quot_rn(a, b, &q)) c[0] += __double_as_longlong(q) != __double_as_longlong(a / b);
+      else c[2]++;
+    }
+    // the back substitution's: a pivot in 1 .. 2^8, a dividend down to the subnormals
+    b = ldexp(mb, (int)(h >> 24 & 7));
+    a = ldexp(ma, (h >> 30 & 3) ? (int)((h >> 44) % 200) - 100 : -(int)((h >> 44) % 1090));
+    if (h & (1ull << 42)) a = -a;
+    if (div_rn_3_covers(b) && div_rn_3_takes(a)) {
+      const double zh = 1.0 / b, r = fma(-b, zh, 1.0), zl = r / b, zll = fma(-b, zl, r) / b;
+      const double v = div_rn_3(a, zh, zl, zll), want = a / b;
+      c[1] += __double_as_longlong(v) != __double_as_longlong(want) && !(v == 0.0 && want == 0.0);
+    } else {
+      c[3]++;
+    }
+  }
+  for (int q = 0; q < 4; q++)
+    if (c[q]) atomicAdd(counts + q, c[q]);
+}
+
+// The largest |1 - b*rcp_approx(b)| over every leading 20-bit mantissa, the
+// lower word zero, all ones or any, at the ends and the middle of quot_rn's
+// exponents.
+__global__ void k_selftest_estimate(uint64_t seed, unsigned long long *worst) {
+  double m = 0.0;
+  for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < 9u << 20; t += gridDim.x * blockDim.x) {
+    const uint64_t lead = t & 0xfffffu, kind = t >> 20;
+    const uint64_t low = kind % 3 == 0 ? 0 : kind % 3 == 1 ? 0xffffffffu : mix64(seed ^ t) & 0xffffffffu;
+    const uint64_t e = kind < 3 ? 1023 - 200 : kind < 6 ? 1023 : 1023 + 200;
+    const double b = __longlong_as_double((long long)(e << 52 | lead << 32 | low));
+    m = fmax(m, fabs(fma(-b, rcp_approx(b), 1.0)));
+  }
+  atomicMax(worst, (unsigned long long)__double_as_longlong(m));
+}
+
 }  // namespace a3g
+
+extern "C" int a3g_selftest_quotients(int device, uint64_t n, uint64_t seed, uint64_t *counts, double *estimate) {
+  if (!counts || !estimate) { a3g::set_error("null counts or estimate"); return A3G_ERR_ARG; }
+  A3G_CUDA(cudaSetDevice(device));
+  unsigned long long *d = nullptr, h[5];
+  A3G_CUDA(cudaMalloc((void **)&d, sizeof(h)));
+  cudaError_t e = cudaMemset(d, 0, sizeof(h));
+  if (e == cudaSuccess) {
+    a3g::k_selftest_quotients<<<148 * 8, 256>>>(n, seed, d);
+    a3g::k_selftest_estimate<<<148 * 8, 256>>>(seed, d + 4);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) e = cudaMemcpy(h, d, sizeof(h), cudaMemcpyDeviceToHost);
+  cudaFree(d);
+  if (e != cudaSuccess) return a3g::cuda_fail(e, "a3g_selftest_quotients");
+  for (int q = 0; q < 4; q++) counts[q] = h[q];
+  std::memcpy(estimate, &h[4], sizeof(double));
+  return A3G_OK;
+}
 
 extern "C" int a3g_selftest_div(int device, uint64_t n, uint64_t seed, uint64_t *mismatches) {
   if (!mismatches) { a3g::set_error("null mismatches"); return A3G_ERR_ARG; }
