@@ -984,18 +984,45 @@ int launch_source(a3g_ctx *ctx, int ivent, int jvent, double dt) {
 // ---------------------------------------------------------------------------
 // CloudLoad(i,j) = sum_k sum_g c(i,j,k,g) * dz(k) / 1e3 (tonnes/km^2), in the
 // order of src/Output_Vars.f90:1061-1069, without the cloud mask.
+// Sums over the grains, in order, of the levels 0 .. cnt-1 of a column from p
+// on: OV_K levels side by side and four grains, so that loads are in flight
+// whatever the number of grains.  One level at a time with the grains' loads
+// unrolled by eight left 1 to 7 grains, and the rest of a count that is no
+// multiple of eight, waiting for one load after another.  us a launch by
+// events for that (the compiler's own unrolling before it) and now: column
+// load, 140x120x40, 4 grains, 41 (25), 19; 12: 61 (39), 30; 60: 512 (291), 250;
+// products, 480x361x50, 1 grain, 78 (120 in two passes), 70; 4: 208 (149), 79; 8:
+// 122 (208), 123.  Eight levels, two to eight grains or sixteen levels at a time
+// were slower from four grains up (480x361x50, 4: 95 .. 107).
+constexpr int OV_K = 4;
+__device__ __forceinline__ void level_sums(const Layout &L, const double *__restrict__ p, int cnt, double (&t)[OV_K]) {
+#pragma unroll
+  for (int e = 0; e < OV_K; e++) t[e] = 0.0;
+  if (cnt >= OV_K) {
+#pragma unroll 4
+    for (int g = 0; g < L.ns; g++, p += L.PG)
+#pragma unroll
+      for (int e = 0; e < OV_K; e++) t[e] = t[e] + __ldg(p + e * L.PY);
+  } else {
+    for (int g = 0; g < L.ns; g++, p += L.PG)
+#pragma unroll
+      for (int e = 0; e < OV_K; e++)
+        if (e < cnt) t[e] = t[e] + __ldg(p + e * L.PY);
+  }
+}
+
 __global__ void k_cloud_load(Layout L, const double *__restrict__ c, const double *__restrict__ dz_vec,
                              double *__restrict__ out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
   const int j = blockIdx.y + 1;
   if (i > L.nx) return;
   double load = 0.0;
-#pragma unroll 2
-  for (int k = 1; k <= L.nz; k++) {
-    double s = 0.0;
-#pragma unroll 8
-    for (int g = 0; g < L.ns; g++) s = s + c[(long)g * L.PG + L.cell(i, j, k)];
-    load = load + s * dz_vec[k + 1] / 1.0e3;
+  for (int k0 = 1; k0 <= L.nz; k0 += OV_K) {
+    double s[OV_K];
+    level_sums(L, c + L.cell(i, j, k0), L.nz - k0 + 1, s);
+#pragma unroll
+    for (int e = 0; e < OV_K; e++)
+      if (k0 + e <= L.nz) load = load + s[e] * dz_vec[k0 + e + 1] / 1.0e3;
   }
   out[(long)(j - 1) * L.nx + (i - 1)] = load;
 }
@@ -1076,10 +1103,9 @@ int launch_vent_column(a3g_ctx *ctx, int ivent, int jvent, const double *lam, do
 // AshThicknessCalculator (:855-895), the arrival-time marks (:1226-1236).
 // ---------------------------------------------------------------------------
 // One pass up the column (the lowest level at or below CLOUDCON_THRESH is the
-// last one the reference's downward loop meets), the grains' loads of a level
-// in flight together; bound by the 8 B a cell and grain (480x361x50, 8 grains:
-// 208 -> 121 us against two passes).  cls: the cell's area classes, j fastest:
-// bit 0 deposit, 1 cloud, 2.. CloudLoadArea's five thresholds.
+// last one the reference's downward loop meets); bound by the 8 B a cell and
+// grain.  cls: the cell's area classes, j fastest: bit 0 deposit, 1 cloud, 2..
+// CloudLoadArea's five thresholds.
 __global__ void __launch_bounds__(128) k_output_vars(
     Layout L, Box box, const double *__restrict__ c, const double *__restrict__ dz_vec,
     const double *__restrict__ zcc, const double *__restrict__ dep, double cloudcon, double cloudload_th,
@@ -1104,19 +1130,22 @@ __global__ void __launch_bounds__(128) k_output_vars(
   unsigned bits = md ? 1u : 0u;
   if (L.ns > 0 && i >= box.imin && i <= box.imax && j >= box.jmin && j <= box.jmax) {
     bool low = false;
-    const double *p = c + L.cell(i, j, 1);
-#pragma unroll 2
-    for (int k = 1; k <= L.nz; k++, p += L.PY) {
-      double t = 0.0;
-#pragma unroll 8
-      for (int g = 0; g < L.ns; g++) t = t + p[(long)g * L.PG];
-      ld = ld + t * dz_vec[k + 1] / 1.0e3;
-      if (t >= cloudcon) mh = zcc[k - 1] + 0.5 * dz_vec[k + 1];
-      if (!low && t <= cloudcon) {
-        low = true;
-        nh = zcc[k - 1] - 0.5 * dz_vec[k + 1];
+    for (int k0 = 1; k0 <= L.nz; k0 += OV_K) {
+      double s[OV_K];
+      level_sums(L, c + L.cell(i, j, k0), L.nz - k0 + 1, s);
+#pragma unroll
+      for (int e = 0; e < OV_K; e++) {
+        const int k = k0 + e;
+        if (k > L.nz) break;
+        const double t = s[e];
+        ld = ld + t * dz_vec[k + 1] / 1.0e3;
+        if (t >= cloudcon) mh = zcc[k - 1] + 0.5 * dz_vec[k + 1];
+        if (!low && t <= cloudcon) {
+          low = true;
+          nh = zcc[k - 1] - 0.5 * dz_vec[k + 1];
+        }
+        mx = (k == 1) ? t : fmx(mx, t);
       }
-      mx = (k == 1) ? t : fmx(mx, t);
     }
     mc = ld >= cloudload_th;
     if (mc) {
