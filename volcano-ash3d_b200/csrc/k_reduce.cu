@@ -700,41 +700,46 @@ int launch_plane_flags(a3g_ctx *ctx) {
 // ---------------------------------------------------------------------------
 // winds and source
 // ---------------------------------------------------------------------------
-// A warp takes whole rows (no division per cell), four cells a lane in flight;
-// bound by the 48 B a cell (720x360x60: 130 -> 124 us; 93x131x37: 6.7 -> 6.3).
-__global__ void __launch_bounds__(256) k_interp_winds(Layout L, const float *__restrict__ last,
+// 2^lw lanes take up to 4 * 2^lw cells of a row of one of the three winds, four
+// cells a lane in flight (no division per cell); bound by the 48 B a cell.  us
+// for a thread a cell, for a warp taking whole rows of all three winds, and here:
+// 720x360x60, 136, 141, 134; 480x401x50, 85, 90, 81; 400x3x40, 4.2, 8.2, 4.2;
+// 1000x20x10, 4.7, 13.4, 4.2.
+__global__ void __launch_bounds__(256) k_interp_winds(Layout L, int lw, const float *__restrict__ last,
                                                       const float *__restrict__ next, long n, double frac,
                                                       double *__restrict__ vx, double *__restrict__ vy,
                                                       double *__restrict__ vz) {
   constexpr int U = 4;
-  const int lane = threadIdx.x & 31, nrow = L.ny * L.nz;
-  for (int r = blockIdx.x * 8 + (threadIdx.x >> 5); r < nrow; r += gridDim.x * 8)
+  const int lane = threadIdx.x & 31, sub = lane & ((1 << lw) - 1), rows = 32 >> lw, nrow = L.ny * L.nz;
+  const int d = blockIdx.z, i0 = blockIdx.y * (U << lw) + sub;
+  const float *const a0 = last + d * n, *const b0 = next + d * n;
+  double *const v0 = d == 0 ? vx : d == 1 ? vy : vz;
+  for (int r = (blockIdx.x * 8 + (threadIdx.x >> 5)) * rows + (lane >> lw); r < nrow; r += gridDim.x * 8 * rows) {
+    const float *a = a0 + (long)r * L.nx, *b = b0 + (long)r * L.nx;
+    double *v = v0 + (long)r * L.P;
+    float x[U], y[U];
 #pragma unroll
-    for (int d = 0; d < 3; d++) {
-      const float *a = last + d * n + (long)r * L.nx, *b = next + d * n + (long)r * L.nx;
-      double *v = (d == 0 ? vx : d == 1 ? vy : vz) + (long)r * L.P;
-      for (int i0 = lane; i0 < L.nx; i0 += 32 * U) {
-        float x[U], y[U];
-#pragma unroll
-        for (int q = 0; q < U; q++) {
-          const bool in = i0 + 32 * q < L.nx;
-          x[q] = in ? a[i0 + 32 * q] : 0.0f;
-          y[q] = in ? b[i0 + 32 * q] : 0.0f;
-        }
-#pragma unroll
-        for (int q = 0; q < U; q++)
-          if (i0 + 32 * q < L.nx) v[i0 + 32 * q] = ((double)x[q] + (double)(y[q] - x[q]) * frac) * 3.6;
-      }
+    for (int q = 0; q < U; q++) {
+      const bool in = i0 + (q << lw) < L.nx;
+      x[q] = in ? a[i0 + (q << lw)] : 0.0f;
+      y[q] = in ? b[i0 + (q << lw)] : 0.0f;
     }
+#pragma unroll
+    for (int q = 0; q < U; q++)
+      if (i0 + (q << lw) < L.nx) v[i0 + (q << lw)] = ((double)x[q] + (double)(y[q] - x[q]) * frac) * 3.6;
+  }
 }
 
 // the winds between the met steps `last` and `next` (3 FP32 arrays each)
 int launch_interp_pair(a3g_ctx *ctx, const float *last, const float *next, double frac) {
   const Layout &L = ctx->L;
-  const int rows = (L.ny * L.nz + 7) / 8;
+  int lw = 0;
+  while (lw < 5 && (4 << lw) < L.nx) lw++;
+  const int per = 8 * (32 >> lw), chunks = (L.nx + (4 << lw) - 1) / (4 << lw);  // rows of a block, turns of a row
+  const int rows = (L.ny * L.nz + per - 1) / per, most = 148 * 16 / (3 * chunks) + 1;
   tbegin(ctx, A3G_K_WINDS);
-  k_interp_winds<<<rows < 148 * 8 ? rows : 148 * 8, 256, 0, ctx->stream>>>(
-      L, last, next, (long)L.nx * L.ny * L.nz, frac, ctx->vx, ctx->vy, ctx->vz);
+  k_interp_winds<<<dim3(rows < most ? rows : most, chunks, 3), 256, 0, ctx->stream>>>(
+      L, lw, last, next, (long)L.nx * L.ny * L.nz, frac, ctx->vx, ctx->vy, ctx->vz);
   tend(ctx);
   A3G_LAUNCH_CHECK(ctx);
   return A3G_OK;
