@@ -453,7 +453,7 @@ __device__ __forceinline__ DD dd_shfl(DD v, int o) {
 // 5 xz2*kappa(:,ny+1,:), 6 xy2*kappa(:,:,nz+1).
 constexpr int NJOBS = 7;
 
-// nb blocks a grain for the airborne mass, fb for each face; the last block of
+// nb blocks a grain for the airborne mass, fxy and fs for a face; the last block of
 // the grid to finish combines the partial sums in a fixed order and writes the
 // ns*NJOBS results to `out` (pinned host memory).
 // Airborne mass: a warp takes a row, a lane eight cells of it at a time (four
@@ -470,7 +470,7 @@ __global__ void __launch_bounds__(256) k_totals(Layout L, const double *__restri
                                                 const double *__restrict__ xz1,
                                                 const double *__restrict__ xz2,
                                                 const double *__restrict__ xy1,
-                                                const double *__restrict__ xy2, Box nz, int nb, int fb,
+                                                const double *__restrict__ xy2, Box nz, int nb, int fxy, int fs,
                                                 double *__restrict__ part, unsigned *__restrict__ counter,
                                                 double *__restrict__ out) {
   const int g = blockIdx.y, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -508,8 +508,12 @@ __global__ void __launch_bounds__(256) k_totals(Layout L, const double *__restri
       }
     }
   } else {
-    const int f = ((int)blockIdx.x - nb) / fb, b = ((int)blockIdx.x - nb) % fb, job = f + 1;
-    const bool xy = job == 1 || job == 6, yz = job == 2 || job == 3;
+    // the xy faces' blocks first, fxy each, then the others', fs each
+    const int x = (int)blockIdx.x - nb;
+    const bool xy = x < 2 * fxy;
+    const int job = xy ? (x < fxy ? 1 : 6) : (x - 2 * fxy) / fs + 2;
+    const int fb = xy ? fxy : fs, b = xy ? x % fxy : (x - 2 * fxy) % fs;
+    const bool yz = job == 2 || job == 3;
     const unsigned len = yz ? L.ny : L.nx, n = len * (xy ? L.ny : L.nz);
     const double *face = (job == 1 ? xy1 : job == 2 ? yz1 : job == 3 ? yz2 : job == 4 ? xz1 : job == 5 ? xz2 : xy2) +
                          (long)g * n;
@@ -536,7 +540,8 @@ __global__ void __launch_bounds__(256) k_totals(Layout L, const double *__restri
   // a warp per (g, job): lanes take every 32nd partial, then a fixed shuffle tree (the same order on every run)
   for (int t = w; t < L.ns * NJOBS; t += 8) {
     const int gg = t / NJOBS, job = t % NJOBS;
-    const int b0 = job == 0 ? 0 : nb + (job - 1) * fb, b1 = job == 0 ? nb : b0 + fb;
+    const int b0 = job == 0 ? 0 : job == 1 ? nb : job == 6 ? nb + fxy : nb + 2 * fxy + (job - 2) * fs;
+    const int b1 = b0 + (job == 0 ? nb : job == 1 || job == 6 ? fxy : fs);
     DD s = {0.0, 0.0};
     for (int b = b0 + lane; b < b1; b += 32) {
       const double *p = part + ((long)gg * nx + b) * 2;
@@ -555,17 +560,20 @@ int launch_totals_partials(a3g_ctx *ctx, double *h_dst) {
   if (empty(nz)) nz = Box{1, 1, 1, 1, 1, 1};
   const int rows = (nz.jmax - nz.jmin + 1) * (nz.kmax - nz.kmin + 1);
   // four rows a warp at least, eight blocks per SM at most; 1024 face cells a block (4096 made the faces
-  // the last to finish on 93x131x37: 17 us a launch, 10.5 now), 16 blocks at most
+  // the last to finish on 93x131x37: 17 us a launch, 10.5 now), from 16 blocks a face on 4096, and 64 at most
+  // (16 at most were too few for 1000x1000x4, 1 grain: 77 us, 296 blocks 34, these 28)
   int nb = (rows + 31) / 32;
   const int most = 148 * 8 / L.ns > 1 ? 148 * 8 / L.ns : 1;
   if (nb > most) nb = most;
-  const long face = (long)L.nx * (L.ny > L.nz ? L.ny : L.nz) > (long)L.ny * L.nz
-                        ? (long)L.nx * (L.ny > L.nz ? L.ny : L.nz) : (long)L.ny * L.nz;
-  const int fb = face > 15 * 1024 ? 16 : (int)(face / 1024) + 1;
+  auto face_blocks = [](long cells) {
+    const long some = cells / 1024 + 1, many = cells / 4096 > 16 ? cells / 4096 : 16, n = some < many ? some : many;
+    return (int)(n < 64 ? n : 64);
+  };
+  const int fxy = face_blocks((long)L.nx * L.ny), fs = face_blocks((long)(L.nx > L.ny ? L.nx : L.ny) * L.nz);
   tbegin(ctx, A3G_K_TOTALS);
-  k_totals<<<dim3(nb + 6 * fb, L.ns), 256, 0, ctx->stream>>>(
+  k_totals<<<dim3(nb + 2 * fxy + 4 * fs, L.ns), 256, 0, ctx->stream>>>(
       L, ctx->c0, ctx->kappa, ctx->out_yz1, ctx->out_yz2, ctx->out_xz1, ctx->out_xz2, ctx->out_xy1, ctx->out_xy2, nz, nb,
-      fb, ctx->red_buf, ctx->block_count, h_dst);
+      fxy, fs, ctx->red_buf, ctx->block_count, h_dst);
   tend(ctx);
   A3G_LAUNCH_CHECK(ctx);
   return A3G_OK;
