@@ -1565,12 +1565,15 @@ __global__ void __launch_bounds__(32 * ACT_WARPS, VAR ? ACT_MINB - 2 : ACT_MINB)
 // about eight cells (its loads, and the interface it repeats).  93x131x37, 2
 // grains: y 56 -> 14 us, z 27 -> 14 us a sweep (whole lines 45, 22);
 // 140x120x40, 4 grains: x 27.4 -> 24.6, y 20.3 -> 18.7 us against 20 warps an
-// SM whatever the waves.
+// SM whatever the waves.  At most 32, or 128 where whole lines are less than 16
+// warps (1000x20x10, 1 grain: x 12.3 -> 10.3, its transpose 16.4 -> 12.3 us; at
+// 2000x100x10, 2 grains, 37 instead of 32 took the transpose from 42 to 52).
 static inline int march_segments(int n, long warps) {
   const long wave = 148L * 16;
+  const int most = warps < 16 ? 128 : 32;
   int best = 1;
   long least = 0;
-  for (int s = 1; s == 1 || (s <= 32 && n / s >= 6); s++) {
+  for (int s = 1; s == 1 || (s <= most && n / s >= 6); s++) {
     const long cost = ((warps * s + wave - 1) / wave) * ((n + s - 1) / s + 8);
     if (s == 1 || cost < least) {
       best = s;
