@@ -2210,8 +2210,10 @@ static CnTableJob cn_table_job(a3g_ctx *ctx) {
   j.tab = ctx->cn_tab[DIR];
   j.may = may ? 1 : 0;
   j.byrow = cn_byrow(DIR, j.map) ? 1 : 0;
-  // many lines: 32 share a block's serial warp; few: a block each, more of its rows at once
-  j.lpb = j.map.U >= 1024 ? 32 : 1;
+  // many lines: 32 share a block's serial warp; few: a block each, more of its rows at once (the three
+  // tables of 20, 20 and 400 lines 16 us a block each, 19 with 32; of 624, 672 and 728 lines 50 and 25;
+  // of 1224, 1360 and 1440 lines 102 and 30)
+  j.lpb = j.map.U >= 512 ? 32 : 1;
   j.blocks = (j.map.U + j.lpb - 1) / j.lpb;
   return j;
 }
