@@ -335,12 +335,13 @@ struct AdjMarch {
 };
 
 // Takes cell J+1 (its q, vel, lam) with sigma(J)/2 and dt/kappa(J); returns lam_q(J-2).
-template <int LIM>
+// ANY: the caller does not know that the winds are numbers.
+template <int LIM, bool ANY>
 __device__ __forceinline__ double adj_march_step(AdjMarch &m, double qx, double vx, double lx, double hs, double dtv,
                                                  double eps, int nocycle) {
   const double d1 = qx - m.q;
   const double us = (m.vm + m.v) * hs;
-  const double p = pos_part(us), n = neg_part(us);
+  const double p = ANY ? pos_part(us) : pos_bits(us), n = ANY ? neg_part(us) : neg_bits(us);
   const bool up = us > 0.0;
   const double tJ = -(dtv * m.lam);
   double ea = 0.0, eb = 0.0;
@@ -479,9 +480,13 @@ __global__ void __launch_bounds__(32 * ADJ_WARPS, 8) k_adj_colt(
     __syncwarp();
     const double2 *gb = reinterpret_cast<const double2 *>(wsm + bi * ADJ_BUF_D + 3 * ACH * 32);
     const int cnt = min(ACH, s1 + 3 - x + 1);
-    auto step = [&](int e) {
+    // whether every wind that the chunk's interfaces take is a number: their sum is
+    double sum = m.vm + m.v + vf0;
+#pragma unroll
+    for (int u = 0; u < ACH; u += 2) sum = sum + (qv[(ACH + u) * 32] + qv[(ACH + u + 1) * 32]);
+    auto step = [&](auto any, int e) {
       const double2 sd = gb[e];
-      const double y = adj_march_step<LIM>(m, qv[e * 32], qv[(ACH + e) * 32] + vf0, qv[(2 * ACH + e) * 32], sd.x, sd.y,
+      const double y = adj_march_step<LIM, decltype(any)::value>(m, qv[e * 32], qv[(ACH + e) * 32] + vf0, qv[(2 * ACH + e) * 32], sd.x, sd.y,
                                            eps, nocycle);
       if (x + e - 3 >= s0) {
         if (valid) *po = y;
@@ -489,11 +494,13 @@ __global__ void __launch_bounds__(32 * ADJ_WARPS, 8) k_adj_colt(
       }
     };
     int e = 0;
+    if (__any_sync(0xffffffffu, !finite_bits(sum)))
+      for (; e < cnt; e++) step(TrueT{}, e);
     for (; e + 2 <= cnt; e += 2) {
-      step(e);
-      step(e + 1);
+      step(FalseT{}, e);
+      step(FalseT{}, e + 1);
     }
-    if (e < cnt) step(e);
+    if (e < cnt) step(FalseT{}, e);
     x += ACH;
     __syncwarp();
   }
@@ -567,9 +574,9 @@ __global__ void __launch_bounds__(32 * ADJ_WARPS, 8) k_adj_xm(
   auto pair = [&](unsigned char *b, int p) { return reinterpret_cast<double2 *>(b + row_b + ((p << 4) ^ row_s)); };
   auto cell = [&](unsigned char *b, int e) { return reinterpret_cast<double *>(pair(b, e >> 1)) + (e & 1); };
   double held = 0.0;  // lam_q of the cell behind the last one computed
-  auto step = [&](double q, double v, double l, double h) {
+  auto step = [&](auto any, double q, double v, double l, double h) {
     const double y = held;
-    held = adj_march_step<LIM>(m, q, v, l, h, dtv, eps, nocycle);
+    held = adj_march_step<LIM, decltype(any)::value>(m, q, v, l, h, dtv, eps, nocycle);
     return y;
   };
   const bool whole = r0 + 32 <= nrows;
@@ -590,18 +597,26 @@ __global__ void __launch_bounds__(32 * ADJ_WARPS, 8) k_adj_xm(
     if (X + 7 > n) {           // the edge wind, and its negative beyond: usig(n+2) = 0
       for (int x = max(n + 1, X); x <= min(n + 2, X + 7); x++) *cell(vb, x - X) = x == n + 1 ? pv[n - 1] : -pv[n - 1];
     }
-    if (X > 1) {
+    // whether every wind that the chunk's interfaces take is a number: their sum is
+    double sum = m.vm + m.v;
+#pragma unroll
+    for (int p = 0; p < 4; p++) {
+      const double2 v = *pair(vb, p);
+      sum = sum + (v.x + v.y);
+    }
+    if (X > 1 && !__any_sync(0xffffffffu, !finite_bits(sum))) {
 #pragma unroll 2
       for (int p = 0; p < 4; p++) {
         double2 *l = pair(lb, p);
         const double2 q = *pair(qb, p), v = *pair(vb, p), w = *l;
         double2 y;
-        y.x = step(q.x, v.x, w.x, hs);
-        y.y = step(q.y, v.y, w.y, hs);
+        y.x = step(FalseT{}, q.x, v.x, w.x, hs);
+        y.y = step(FalseT{}, q.y, v.y, w.y, hs);
         *l = y;
       }
     } else {  // interface 0 carries nothing
-      for (int e = 0; e < 8; e++) *cell(lb, e) = step(*cell(qb, e), *cell(vb, e), *cell(lb, e), e == 0 ? 0.0 : hs);
+      for (int e = 0; e < 8; e++)
+        *cell(lb, e) = step(TrueT{}, *cell(qb, e), *cell(vb, e), *cell(lb, e), X == 1 && e == 0 ? 0.0 : hs);
     }
     fence_proxy_async_smem();
     __syncwarp();

@@ -1230,48 +1230,62 @@ static void launch_col(a3g_ctx *ctx) {
 // a missing wind carries no first-order flux whichever kernel sweeps its cell.
 __device__ __forceinline__ double pos_part(double x) { return x > 0.0 ? x : 0.0; }
 __device__ __forceinline__ double neg_part(double x) { return x < 0.0 ? x : 0.0; }
+// The same of a number, by the sign bit (a NaN stays one in either): 9
+// instructions a cell fewer in the y march's steps.
+__device__ __forceinline__ double pos_bits(double x) {
+  const int h = __double2hiint(x), m = ~(h >> 31);
+  return __hiloint2double(h & m, __double2loint(x) & m);
+}
+__device__ __forceinline__ double neg_bits(double x) {
+  const int h = __double2hiint(x), m = h >> 31;
+  return __hiloint2double(h & m, __double2loint(x) & m);
+}
+__device__ __forceinline__ bool finite_bits(double x) { return (__double2hiint(x) & 0x7fffffff) < 0x7ff00000; }
 
 // Second-order flux of one interface, cf*ldq (0 where the reference cycles),
-// the same value as fss_select's.  Superbee's factor is 0 for ratios dqu/dq
-// <= 0, 2 from 2 up, 1 on [1/2, 1], and 2*theta or theta in between, and
-// rounding to nearest cannot move a quotient across those bounds, so the
-// class comes from comparisons of dqu, with dq's sign taken off, with |dq| and
-// 2|dq|, the quotient is needed in two classes only, and it is divided by the
+// the same value as fss_select's, cf = 0.5*aus*(1 - dtv*aus).  Superbee's factor
+// is 0 for ratios dqu/dq <= 0, 2 from 2 up, 1 on [1/2, 1], and 2*theta or theta in
+// between, and rounding to nearest cannot move a quotient across those bounds,
+// so the class comes from comparisons of dqu, with dq's sign taken off, with |dq|
+// and 2|dq|, the quotient is needed in two classes only, and it is divided by the
 // operator only where one of those lanes holds operands out of quot_rn's
 // range.  A ratio that is NaN is in the class of 2 (fmin and fmax pass it
-// over), and cf, which a missing wind makes NaN, reaches every interface that
-// does not cycle.  `up` may be either for usig = 0, where cf = 0.
+// over).  ANY: aus may be NaN (a missing wind), which reaches every interface
+// that does not cycle, and no other.  `up` may be either for usig = 0, where
+// cf = 0.  NOCYCLE, which no reference build sets, goes by the general rule.
 static __device__ __noinline__ double ieee_theta(double dqu, double dq, bool twice) {
   const double th = dqu / dq;
   return twice ? th + th : th;
 }
 
 template <int LIM>
-__device__ __forceinline__ double fss_step(double dqm, double dq, double dqp, bool up, double cf, double eps,
-                                           bool nocycle) {
+static __device__ __noinline__ double fss_nocycle(double dqm, double dq, double dqp, bool up, double cf, double eps) {
+  return fss_select<LIM>(dqm, dq, dqp, up, cf, true, eps, 1);
+}
+
+template <int LIM, bool ANY>
+__device__ __forceinline__ double fss_step(double dqm, double dq, double dqp, bool up, double aus, double dtv,
+                                           double eps, bool nocycle) {
   if (LIM == A3G_LIM_NONE) return 0.0;
-  if (LIM != A3G_LIM_SUPERBEE) return fss_select<LIM>(dqm, dq, dqp, up, cf, true, eps, nocycle);
+  if (LIM != A3G_LIM_SUPERBEE)
+    return fss_select<LIM>(dqm, dq, dqp, up, 0.5 * aus * (1.0 - dtv * aus), true, eps, nocycle);
+  if (nocycle) return fss_nocycle<LIM>(dqm, dq, dqp, up, 0.5 * aus * (1.0 - dtv * aus), eps);
   const double dqu = up ? dqm : dqp, b = fabs(dq);
   const double s = __hiloint2double(__double2hiint(dqu) ^ (__double2hiint(dq) & (int)0x80000000), __double2loint(dqu));
-  const bool lt = s + s < b, gt = s > b;
-  bool ge2 = !(s < b + b), none = s <= 0.0, skip = b <= eps;
-  if (nocycle) {  // the clamp of :201 (by the sign of a zero too) without the cycle of :183
-    ge2 = ge2 || b < eps;
-    none = none && !(s == 0.0 && __double2hiint(s) >= 0);
-    skip = false;
-  }
+  const bool lt = s + s < b, gt = s > b, ge2 = !(s < b + b), skip = b <= eps, none = skip || s <= 0.0;
   const bool need = !none && !ge2 && (lt || gt);
   double th;
-  const bool ok = quot_rn(s, b, &th);
+  const bool ok = quot_rn(dqu, dq, &th);
   int hi = __double2hiint(th) + (lt ? 1 << 20 : 0), lo = __double2loint(th);  // 2*theta of a normal theta
   if (need && !ok) {
-    th = ieee_theta(s, b, lt);
+    th = ieee_theta(dqu, dq, lt);
     hi = __double2hiint(th);
     lo = __double2loint(th);
   }
   const int flat = none ? 0 : (ge2 ? 0x40000000 : 0x3ff00000);  // 0, 2 or 1
   const double phi = __hiloint2double(need ? hi : flat, need ? lo : 0);
-  return skip ? 0.0 : cf * (dq * phi);
+  const double cf = 0.5 * aus * (1.0 - dtv * aus);
+  return ANY && skip ? 0.0 : cf * (dq * phi);
 }
 
 // The values a march carries from cell c to cell c+1.
@@ -1286,17 +1300,16 @@ struct March {
 // q2 - q(c+1), vn = vel(c+2), hs = sigma(c+2)/2 and dtv1 = dt/kappa(c+1).
 // Returns the sum whose product with dt/kappa(c) is taken off q(c) (:264-281).
 // usig = 0.5*(v+v')*sigma is (v+v')*(sigma/2): halving is exact.  QUIET: the
-// caller knows that |dq| <= EPS_THRESH at this interface.
-template <int LIM, bool QUIET>
+// caller knows that |dq| <= EPS_THRESH at this interface; ANY: it does not know
+// that the winds are numbers.
+template <int LIM, bool QUIET, bool ANY>
 __device__ __forceinline__ double march_step(March &m, double q2, double d2, double vn, double hs, double dtv1,
                                              double eps, bool nocycle) {
   const double usC = (m.vB + vn) * hs;
-  const double upC = pos_part(usC), unC = neg_part(usC);
+  const double upC = ANY ? pos_part(usC) : pos_bits(usC), unC = ANY ? neg_part(usC) : neg_bits(usC);
   double fss1 = 0.0;
   if (!QUIET && LIM != A3G_LIM_NONE) {
-    const double aus = fabs(m.us);
-    const double cf = 0.5 * aus * (1.0 - dtv1 * aus);
-    fss1 = fss_step<LIM>(m.d0, m.d1, d2, __double2hiint(m.us) >= 0, cf, eps, nocycle);
+    fss1 = fss_step<LIM, ANY>(m.d0, m.d1, d2, __double2hiint(m.us) >= 0, fabs(m.us), dtv1, eps, nocycle);
   }
   double fsr1 = m.upB * m.d1;
   double fsl1 = m.unB * m.d1;
@@ -1493,10 +1506,11 @@ __global__ void __launch_bounds__(32 * ACT_WARPS, VAR ? ACT_MINB - 2 : ACT_MINB)
     return VAR ? make_double2(I <= rmax + 1 ? 0.5 * lsig.ldg(I) : 0.0, ldtv.ldg(I - 1)) : gb[e];
   };
   // the step c from the values of cell c+2 at slot e of the chunk
-  auto step = [&](auto quiet, const double *qv, double2 sd, int e) {
+  auto step = [&](auto quiet, auto any, const double *qv, double2 sd, int e) {
     const double q0 = m.q0, q2 = qv[e * 32];
     const double vn = (DIR == 2) ? qv[(ACH + e) * 32] + vf0 : qv[(ACH + e) * 32];
-    const double sum = march_step<LIM, decltype(quiet)::value>(m, q2, q2 - m.q1, vn, sd.x, sd.y, eps, nocyc);
+    const double sum = march_step<LIM, decltype(quiet)::value, decltype(any)::value>(m, q2, q2 - m.q1, vn, sd.x, sd.y,
+                                                                                     eps, nocyc);
     const double upd = m.dtv0 * sum;
     if (al) *po = q0 - upd;
     po += st;
@@ -1519,8 +1533,16 @@ __global__ void __launch_bounds__(32 * ACT_WARPS, VAR ? ACT_MINB - 2 : ACT_MINB)
     __syncwarp();
     const double2 *gb = reinterpret_cast<const double2 *>(wsm + 4 * ACH * 32 + bi * 2 * ACH);
     int e = 0;
-    // a chunk that holds the z sweep's ctop (a box off the ground) runs the loop
-    if (!(DIR == 2 && out_hi && ctop <= rmax)) {
+    // whether every wind that the chunk's interfaces take is a number: their sum is
+    double sum = m.vB + m.us + vf0;
+#pragma unroll
+    for (int u = 0; u < ACH; u += 2) sum = sum + (qv[(ACH + u) * 32] + qv[(ACH + u + 1) * 32]);
+    if (__any_sync(0xffffffffu, al && !finite_bits(sum))) {
+      for (; e < cnt; e++) {
+        const double upd = step(FalseT{}, TrueT{}, qv, geo(gb, e, c + e + 2), e);
+        if (DIR == 2 && al && out_hi && c + e == ctop) out2[oo] -= upd;
+      }
+    } else if (!(DIR == 2 && out_hi && ctop <= rmax)) {  // the z sweep's ctop (a box off the ground) is the last loop's
       // the differences the chunk's interfaces limit: d1 and the first cnt-1 new ones
       int top = __double2hiint(m.d1) & 0x7fffffff;
       double prev = m.q1;
@@ -1533,8 +1555,8 @@ __global__ void __launch_bounds__(32 * ACT_WARPS, VAR ? ACT_MINB - 2 : ACT_MINB)
       if (LIM == A3G_LIM_NONE || __all_sync(0xffffffffu, top < eps_hi || !al)) {
         for (; e + 2 <= cnt; e += 2) {
           const double2 sd0 = geo(gb, e, c + e + 2), sd1 = geo(gb, e + 1, c + e + 3);
-          step(TrueT{}, qv, sd0, e);
-          step(TrueT{}, qv, sd1, e + 1);
+          step(TrueT{}, FalseT{}, qv, sd0, e);
+          step(TrueT{}, FalseT{}, qv, sd1, e + 1);
         }
       } else {
         for (; e + ACT_U <= cnt; e += ACT_U) {
@@ -1544,12 +1566,12 @@ __global__ void __launch_bounds__(32 * ACT_WARPS, VAR ? ACT_MINB - 2 : ACT_MINB)
             for (int u = 0; u < ACT_U; u++) sd[u] = geo(gb, e + u, c + e + u + 2);
           }
 #pragma unroll
-          for (int u = 0; u < ACT_U; u++) step(FalseT{}, qv, VAR ? sd[u] : gb[e + u], e + u);
+          for (int u = 0; u < ACT_U; u++) step(FalseT{}, FalseT{}, qv, VAR ? sd[u] : gb[e + u], e + u);
         }
       }
     }
     for (; e < cnt; e++) {
-      const double upd = step(FalseT{}, qv, geo(gb, e, c + e + 2), e);
+      const double upd = step(FalseT{}, FalseT{}, qv, geo(gb, e, c + e + 2), e);
       if (DIR == 2 && al && out_hi && c + e == ctop) out2[oo] -= upd;
     }
     c += cnt;
@@ -1744,9 +1766,10 @@ __global__ void __launch_bounds__(32 * AXM_WARPS, ACT_MINB) k_advect_xm(
   const int row_b = lane << 6, row_s = ((lane >> 1) & 3) << 4;
   auto pair = [&](unsigned char *b, int p) { return reinterpret_cast<double2 *>(b + row_b + ((p << 4) ^ row_s)); };
   auto cell = [&](unsigned char *b, int e) { return reinterpret_cast<double *>(pair(b, e >> 1)) + (e & 1); };
-  auto step = [&](auto quiet, double q2, double vn) {
+  auto step = [&](auto quiet, auto any, double q2, double vn) {
     const double q0 = m.q0;
-    const double sum = march_step<LIM, decltype(quiet)::value>(m, q2, q2 - m.q1, vn, hs, dtv, eps, nocyc);
+    const double sum =
+        march_step<LIM, decltype(quiet)::value, decltype(any)::value>(m, q2, q2 - m.q1, vn, hs, dtv, eps, nocyc);
     const double upd = dtv * sum;
     return q0 - upd;
   };
@@ -1754,8 +1777,8 @@ __global__ void __launch_bounds__(32 * AXM_WARPS, ACT_MINB) k_advect_xm(
     double2 *q = pair(qb, p);
     const double2 x = *q, v = *pair(vb, p);
     double2 y;
-    y.x = step(quiet, x.x, v.x);
-    y.y = step(quiet, x.y, v.y);
+    y.x = step(quiet, FalseT{}, x.x, v.x);
+    y.y = step(quiet, FalseT{}, x.y, v.y);
     *q = y;
   };
   const bool whole = r0 + 32 <= nrows, all_al = __all_sync(0xffffffffu, al);
@@ -1783,20 +1806,24 @@ __global__ void __launch_bounds__(32 * AXM_WARPS, ACT_MINB) k_advect_xm(
         }
       }
     }
-    // the differences the chunk's interfaces limit: d1 and the first 7 new ones
+    // the differences the chunk's interfaces limit: d1 and the first 7 new ones;
+    // and whether every wind they take is a number: their sum is
     int top = __double2hiint(m.d1) & 0x7fffffff;
+    double sum = m.vB + m.us;
     {
       double prev = m.q1;
 #pragma unroll
       for (int p = 0; p < 4; p++) {
-        const double2 x = *pair(qb, p);
+        const double2 x = *pair(qb, p), v = *pair(vb, p);
+        sum = sum + (v.x + v.y);
         top = max(top, __double2hiint(x.x - prev) & 0x7fffffff);
         if (p < 3) top = max(top, __double2hiint(x.y - x.x) & 0x7fffffff);
         prev = x.y;
       }
     }
     const bool quiet = LIM == A3G_LIM_NONE || __all_sync(0xffffffffu, top < eps_hi || !al);
-    if (e0 == 0 && e1 == 7) {
+    const bool any = __any_sync(0xffffffffu, al && !finite_bits(sum));
+    if (e0 == 0 && e1 == 7 && !any) {
       if (quiet) {
         for (int p = 0; p < 4; p++) two(TrueT{}, qb, vb, p);
       } else {
@@ -1809,7 +1836,7 @@ __global__ void __launch_bounds__(32 * AXM_WARPS, ACT_MINB) k_advect_xm(
       for (int e = 0; e < 8; e++) {
         double *q = cell(qb, e);
         double y = 0.0;  // outside the box
-        if (e >= e0 && e <= e1) y = step(FalseT{}, *q, *cell(vb, e));
+        if (e >= e0 && e <= e1) y = step(FalseT{}, TrueT{}, *q, *cell(vb, e));
         *q = y;
       }
     }
