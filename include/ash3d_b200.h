@@ -391,11 +391,13 @@ int a3g_kernel_times(a3g_ctx *ctx, double *ms, uint64_t *count);
  * for x only 3, warps marching 32 rows through shared-memory tiles, 4,
  * one warp per row walking it in 32-cell chunks with the lanes along i, and
  * 5, warps marching 32 rows, a row per lane, through chunks that TMA tensor
- * copies bring and take away (where the geometry varies along i, variant 4
- * with its interior chunks staged by TMA) (defaults: x 5, y 6, z 6).
+ * copies bring and take away (on few short rows variant 4; where the geometry
+ * varies along i, variant 4 with its interior chunks staged by TMA) (defaults:
+ * x 5, y 6, z 6).
  * dir 3: the Crank-Nicolson x solve, variant 0 warp-tiled, 1 one thread per
  * line, 2 warp-tiled with each tile loaded one chunk ahead by a TMA tensor
- * copy (default).  dir 4: the Crank-Nicolson y and z solves, variant 0 one
+ * copy (default; where the coefficients vary along i, tiles loaded through
+ * registers, eight rows' coefficients at a time).  dir 4: the Crank-Nicolson y and z solves, variant 0 one
  * grain per thread, 1 two grains of a line per thread, 2 four, 3 tiles of
  * 32 lines staged in shared memory by TMA tensor copies (default; where the
  * coefficients vary along i, and for z where nz > 256, variant 3 runs one
@@ -403,8 +405,9 @@ int a3g_kernel_times(a3g_ctx *ctx, double *ms, uint64_t *count);
  * dir 1, 2 variant 5: the column march (one thread per line and grain, lanes
  * along i, each interface formed once); variant 6, the same march reading
  * the concentration and wind from chunks that TMA tensor copies stage in
- * shared memory (default for y and z; where the geometry varies along i or
- * the fall speed within a grain, variant 6 runs variant 1).  dir 5: the adjoint advection sweeps,
+ * shared memory (default for y and z; where the geometry varies along i each
+ * lane loads its own; where the fall speed varies within a grain, variant 6 runs
+ * variant 1).  dir 5: the adjoint advection sweeps,
  * variant 0 marches fed by TMA chunks (default; four-cell blocks where the
  * geometry varies along i), 1 one cell per thread.  All variants
  * produce identical results; only their speed differs. */

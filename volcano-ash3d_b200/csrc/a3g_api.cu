@@ -195,22 +195,23 @@ int a3g_create(const a3g_grid_desc *grid, const a3g_params *params, int device, 
   ctx->n_gs_aloft = grid->ns;
   ctx->last_bc = 0;
   // fastest measured advection variants on B200: marches fed by TMA chunks,
-  // along rows (x) and columns (y, z) -- 720x360x60, 10 grains: x 0.67 ms
-  // against 1.08 for the warp rows, y 0.58 and z 0.66 against 1.43 and 1.64
-  // for 4-cell blocks.  Where their conditions do not hold the warp rows and
-  // the blocks run; a3g_set_variant overrides them
+  // along rows (x) and columns (y, z) -- 720x360x60, 10 grains, ash in every
+  // cell: x 0.70 ms against 1.26 for the warp rows, y 0.71 and z 0.77 against
+  // 1.43 and 1.64 for 4-cell blocks.  Where their conditions do not hold, and
+  // for x on few short rows, the warp rows and the blocks run; a3g_set_variant
+  // overrides them
   ctx->tune_advect[0] = 5;
   ctx->tune_advect[1] = 6;
   ctx->tune_advect[2] = 6;
-  // CN x solve: row tiles through TMA (C2 0.82 ms against 1.35 for the
-  // synchronous tile loads of variant 0)
+  // CN x solve: row tiles through TMA (the same state: 0.70 ms against 1.35 for
+  // the synchronous tile loads of variant 0)
   ctx->tune_cn_x = 2;
   ctx->ov_cloudcon = 1.0e-3;   // CLOUDCON_THRESH, src/Output_Vars.f90:119
   ctx->ov_cloudload = 2.0e-1;  // CLOUDLOAD_THRESH, :114
   ctx->ov_depo = 1.0e-2;       // DEPO_THRESH, :113
   ctx->ov_density = 1000.0;    // DepositDensity, src/Tephra.f90:55
-  // CN y and z solves through TMA tiles (C2 on B200: y 0.91, z 0.71 ms against
-  // 1.55 and 1.23 for two grains per thread)
+  // CN y and z solves through TMA tiles (y 0.88, z 0.53 ms against 1.55 and 1.23
+  // for two grains per thread)
   ctx->tune_cn_yz = 3;
   auto dmalloc = [&](void **p, size_t n) -> cudaError_t {
     cudaError_t e = cudaMalloc(p, n);

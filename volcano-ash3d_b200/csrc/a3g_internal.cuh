@@ -9,9 +9,11 @@
 //     loads a row, which is exact because no ghost value survives from one
 //     operator to the next in the reference (each operator re-runs Set_BC or
 //     its own Neumann fill first).
-//   * two levels c0/c1 ping-pong; a sweep reads c0 and writes every interior
-//     cell of c1 (zeros outside the active box and for grains not aloft,
-//     which is the zero-then-copy-back of the reference), then they swap.
+//   * two levels c0/c1 ping-pong; a sweep reads c0 and leaves every interior
+//     cell of c1 as its result (zeros outside the active box and for grains
+//     not aloft, which is the zero-then-copy-back of the reference), then they
+//     swap.  It writes them all, except under FAST_SUBGRID, where it writes its
+//     box and the cells that c1 may still hold (cover_box).
 //   * winds vx/vy/vz: interior only, same pitch.
 //   * geometry and diffusivity: stored with ghosts but compressed by
 //     broadcast strides (a stride of 0 means "does not vary along that
@@ -196,11 +198,11 @@ struct a3g_ctx {
   double host_dt;
   uint64_t launches;
   size_t bytes;
-  // kernel variant per advection direction (0 march, 1 block V=4, 2 block V=8)
+  // kernel variant per advection direction (a3g_set_variant)
   int tune_advect[3];
-  int tune_cn_x;            // CN x solve: 0 warp-tiled, 1 one thread per line
-  int tune_cn_yz;           // CN y/z solves: 0 one grain per thread, 1 two grains per thread
-  bool adj_gather;          // adjoint advection: cell-per-thread gather (true) or 4-cell blocks (false)
+  int tune_cn_x;            // CN x solve
+  int tune_cn_yz;           // CN y/z solves
+  bool adj_gather;          // adjoint advection: cell-per-thread gather (true), or marches and 4-cell blocks
   // discrete adjoint (a3g_adj_*)
   double *lam0, *lam1;      // lam and its scratch level
   double *lam_dep;          // adjoint of DepositGranularity (ns,ny,nx)

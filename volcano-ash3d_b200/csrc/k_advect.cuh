@@ -1348,12 +1348,12 @@ __device__ __forceinline__ double march_step(March &m, double q2, double d2, dou
 // rows through L2.  Taken when the geometry is constant along i and the fall
 // speed is one value per grain.
 //
-// Bound by instruction issue (68 % of cycles on the C2 slab) and the FP64 pipe
-// (48 %).  march_step() forms an interface in about 100 instructions where
-// block_body's expressions and the checked steps at the line ends took 190,
-// and a chunk whose differences are all within EPS_THRESH on every lane -- the
-// air around a cloud -- takes steps without the limiter: 720x360x60, 10
-// grains, y 1.12 -> 0.58 ms and z 1.27 -> 0.66 ms a sweep.
+// Bound by instruction issue (68 % of cycles on 720x120x60, 10 grains) and the
+// FP64 pipe (50 %).  march_step() forms an interface in about 100 instructions
+// where block_body's expressions and the checked steps at the line ends took
+// 190, and a chunk whose differences are all within EPS_THRESH on every lane --
+// the air around a cloud -- takes steps without the limiter: 720x360x60, 10
+// grains, ash in every cell, y 1.12 -> 0.71 ms and z 1.22 -> 0.77 ms a sweep.
 // Lines are cut into segments of `seg` cells where whole lines would leave
 // the chip short of warps (launch_colt); a segment repeats one interface.
 // ---------------------------------------------------------------------------
@@ -1653,10 +1653,11 @@ static bool launch_colt(a3g_ctx *ctx) {
 // rows are not all this plane's (the last of a grain) is stored by the lanes.
 // Taken when sigma and dt/kappa do not vary along the row.
 //
-// Bound, like the column march, by issue (63 % of cycles on the C2 slab, 16
-// warps per SM by registers) and the FP64 pipe (45 %).  720x360x60, 10 grains:
-// 1.08 -> 0.67 ms a sweep against the warp-row kernel, whose lanes pass each
-// value on through shared-memory rings (188 instructions a cell against 95).
+// Bound, like the column march, by issue (65 % of cycles on 720x120x60, 10
+// grains, 16 warps per SM by registers) and the FP64 pipe (48 %).  720x360x60, 10
+// grains, ash in every cell: 1.26 -> 0.70 ms a sweep against the warp-row kernel,
+// whose lanes pass each value on through shared-memory rings (188 instructions a
+// cell against 97).
 // ---------------------------------------------------------------------------
 constexpr int AXM_WARPS = 2;
 constexpr int AXM_BUF = 32 * 8 * 8;                    // bytes of a chunk

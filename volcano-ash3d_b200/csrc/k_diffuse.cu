@@ -3,8 +3,9 @@
 // Explicit: diff_x/diff_y/diff_z, src/Diffusion.F90:266-650 (LeVeque eq. 4.11)
 //   update(l) = dt*k_ds(l+1)*dq(l+1)*(sig(l+1)/kap(l)) - dt*k_ds(l)*dq(l)*(sig(l)/kap(l))
 //   with k_ds = 0.5*(k_{l-1}+k_l) * 2*sig/(kap_{l-1}+kap_l) and Neumann ghosts
-//   (periodic in x).  One thread per cell, all grains in a loop: the
-//   grain-independent products dt*k_ds and sig/kap are formed once.
+//   (periodic in x).  Where nothing varies along i, warps march along j (x and y
+//   in one pass) and k with the factors that dt does not touch in a table; else,
+//   and in z on small grids, one thread per cell takes all grains in a loop.
 //
 // Crank-Nicolson: diffCN_x/y/z, src/Diffusion.F90:671-1428 (eq. 4.13), each
 // line solved by LAPACK dgtsv in the reference.  The matrices are strictly
@@ -14,8 +15,8 @@
 // B'(i+1) = B(i+1) - fact*B'(i); then x(n) = B'(n)/D'(n),
 // x(i) = (B'(i) - DU(i)*x(i+1))/D'(i).  The factorisation (fact, D', DU) and
 // the right-hand-side weights depend only on geometry, diffusivity and dt, so
-// a per-step table holds them once per distinct line geometry (a projected
-// grid has one per k) and the solve kernel runs one thread per (line, grain).
+// a table, rebuilt when dt changes, holds them once per distinct line geometry (a
+// projected grid has one per k) and a lane solves one line of one grain.
 // A line that would need a row interchange (or a zero pivot) raises
 // A3G_ERR_PIVOT instead of silently diverging from dgtsv.
 #include "a3g_internal.cuh"
@@ -1243,11 +1244,13 @@ constexpr int ZT_BAR_BYTES = 128;  // barriers ahead of the tiles (keeps tiles 1
 // take their coefficients from registers.
 //
 // Bound by the latency of the two recurrences at 16 warps per SM (registers),
-// with 24 B per cell of traffic at 4.5 TB/s.  720x360x60, 10 grains: 1.27 ->
-// 0.82 ms, 317x211x53, 7 grains: 275 -> 180 us, against dense tiles that the
-// lanes copied into an odd-stride one and certified quotients (96 warp
-// instructions a cell against 55).  Issuing loads two chunks ahead instead of
-// one changed nothing; parking the values a sector each per row cost 1.33 ms.
+// with 24 B per cell of traffic at 5.3 TB/s.  720x360x60, 10 grains, ash in
+// every cell: 1.15 -> 0.70 ms (a cloud in still air, whose tails go by the
+// division operator, 1.27 -> 0.82), 317x211x53, 7 grains: 275 -> 180 us, against
+// dense tiles that the lanes copied into an odd-stride one and certified
+// quotients (96 warp instructions a cell against 55).  Issuing loads two chunks
+// ahead instead of one changed nothing; parking the values a sector each per row
+// cost 1.33 ms.
 constexpr int CXT_WARPS = 2;
 constexpr int CXT_BUF = 32 * CX_CH * 8;
 constexpr int CXT_SMEM = 1024 + 1024 + CXT_WARPS * 3 * CXT_BUF;  // room to align, barriers, buffers
@@ -1668,8 +1671,8 @@ __global__ void __launch_bounds__(64, 8) k_cn_solve_zt(const __grid_constant__ C
 // by chunk from the last (the last chunk's B' stays in a register, the others
 // are read a chunk ahead).  Warps are persistent and take contiguous runs of
 // line groups (neighbouring i, then k), which share table rows.
-// Bound as the x solve; 720x360x60, 10 grains: 1.04 -> 0.91 ms, 93x131x37, 2
-// grains: 45 -> 29 us a solve.
+// Bound as the x solve; 720x360x60, 10 grains, ash in every cell: 0.99 -> 0.88
+// ms, 93x131x37, 2 grains: 45 -> 29 us a solve.
 constexpr int YT_BUF_D = YT_CH * 32 + YT_CH * CN_ROW;  // doubles of a buffer: the tile, the table rows
 
 __global__ void __launch_bounds__(64, 8) k_cn_solve_yt(const __grid_constant__ CUtensorMap tin,

@@ -5,9 +5,10 @@
 //    to the CPU loop (NaNs are skipped as the reference's `if (tmp.gt.max)`
 //    skips them; a met step's are combined with atomicMax on the IEEE bit
 //    patterns of non-negative doubles).
-//  * mass totals (src/Output_Vars.f90:1255-1459): per-grain sums of c*kappa
-//    accumulated in double-double (TwoSum) and combined in a fixed order, so
-//    the result is deterministic and within a few ulp of the exact sum.
+//  * mass totals (src/Output_Vars.f90:1255-1459): per-grain sums of c*kappa,
+//    eight cells of a row added pairwise in double, their sums accumulated in
+//    double-double (TwoSum) and combined in a fixed order, so the result is
+//    deterministic and within a few ulp of the exact sum.
 //  * subgrid plane occupancy for get_minmax_index (src/Calc_Mesh.f90:432-542).
 //  * met-step interpolation (src/MesoInterpolater.f90:207-223) and the vent
 //    column source insertion (src/Ash3d.F90:428-431).
