@@ -460,7 +460,9 @@ constexpr int NJOBS = 7;
 // Airborne mass: a warp takes a row, a lane eight cells of it at a time (four
 // 16-byte loads in flight), added pairwise in double, times kappa -- once when
 // it does not vary along i -- and carried in double-double: a relative error of
-// three roundings per term, far inside the 1e-13 the totals keep.
+// three roundings per term, far inside the 1e-13 the totals keep (against sums in
+// extended precision on six grids, projected and lon/lat, 0.25 to 0.43 x 2^-53 on
+// average and 0.93 at most, as with every cell in double-double).
 // Bound by the read of the level where that is large: 720x360x60, 10 grains,
 // 339 -> 215 us; and by latency where it is small, in which every face took 296
 // blocks and the combination a kernel and a copy of their own: 93x131x37, 2
